@@ -5,15 +5,15 @@
 //                      examples/CentroidData.h:41-59, accumulating
 //                      MultipoleMoments::operator+=(Particle) in particle order
 //                      (examples/MultipoleMoments.h:274-353, non-HEXADECAPOLE)
-//     upward_level     Subtree::populateTree (src/Subtree.h:352-384): every
+//     upward_climb     Subtree::populateTree (src/Subtree.h:352-384): every
 //                      parent combines its children with CentroidData::
 //                      operator+= (examples/CentroidData.h:61-73,
 //                      examples/MultipoleMoments.h:204-271, :458-469) in the
 //                      order the reference's FIFO delivers them.  That order is
 //                      reproduced without a queue: leaves hold FIFO rank
-//                      (0, leaf DFS rank), empty leaves (0, n_leaves + rank),
-//                      and a parent's rank is (1 + chain, t) of its
-//                      latest-ranked child -- parents enter the FIFO in the
+//                      (0, position) with all leaves before all empty leaves,
+//                      each in DFS order (fifo_of, k_build.cu), and a parent's
+//                      rank is (1 + chain, position) of its latest-ranked child -- parents enter the FIFO in the
 //                      order their last child leaves it.
 //     finalize         per-node traversal records (WalkRec, QuadRec).
 //  K7 traverse_f64     warp-per-bucket walk (pt_walk.cuh) with the FP64
@@ -73,8 +73,11 @@ __device__ __forceinline__ void mom_add_particle(Mom& q, double px, double py, d
   q.yz += pm * d1 * d2;
 }
 
-// CentroidData::operator+= with MultipoleMoments::operator+=(MultipoleMoments).
+// CentroidData::operator+= with MultipoleMoments::operator+=(MultipoleMoments);
+// the radius follows from the box, centre and count of the last combine
+// (mom_radius), so it is left to the caller.
 __device__ __forceinline__ void mom_combine(Mom& q, int& count, const Mom& c, int ccount) {
+#pragma unroll
   for (int d = 0; d < 3; d++) {
     if (c.lo[d] < q.lo[d]) q.lo[d] = c.lo[d];
     if (c.hi[d] > q.hi[d]) q.hi[d] = c.hi[d];
@@ -83,14 +86,16 @@ __device__ __forceinline__ void mom_combine(Mom& q, int& count, const Mom& c, in
   q.mass += c.mass;
   if (q.mass == 0.0) {
     q.soft = 0.5 * (q.soft + c.soft);
+#pragma unroll
     for (int d = 0; d < 3; d++) q.cm[d] = 0.5 * (q.cm[d] + c.cm[d]);
   } else if (m1 == 0.0) {
-    q.mass = c.mass; q.soft = c.soft; q.radius = c.radius;
+    q.mass = c.mass; q.soft = c.soft;
     q.cm[0] = c.cm[0]; q.cm[1] = c.cm[1]; q.cm[2] = c.cm[2];
     q.xx = c.xx; q.xy = c.xy; q.xz = c.xz; q.yy = c.yy; q.yz = c.yz; q.zz = c.zz;
   } else if (c.mass != 0.0) {
     q.soft = (m1 * q.soft + c.mass * c.soft) / q.mass;
     double c0 = q.cm[0], c1 = q.cm[1], c2 = q.cm[2];
+#pragma unroll
     for (int d = 0; d < 3; d++) q.cm[d] = (m1 * q.cm[d] + c.mass * c.cm[d]) / q.mass;
     double d0 = c0 - q.cm[0], d1 = c1 - q.cm[1], d2 = c2 - q.cm[2];
     q.xx += m1 * d0 * d0;
@@ -110,8 +115,12 @@ __device__ __forceinline__ void mom_combine(Mom& q, int& count, const Mom& c, in
     q.yz += c.yz + c.mass * d1 * d2;
   }
   count += ccount;
+}
+
+__device__ __forceinline__ void mom_radius(Mom& q, int count) {
   if (count > 1) {
     double e[3];
+#pragma unroll
     for (int d = 0; d < 3; d++) {
       double a = q.cm[d] - q.lo[d], b = q.hi[d] - q.cm[d];
       e[d] = (a > b) ? a : b;
@@ -162,39 +171,84 @@ __global__ void __launch_bounds__(256) leaf_moments(Nodes nd, int64_t nnodes, Pa
   nd.count[i] = cnt;
 }
 
-__global__ void __launch_bounds__(128) upward_level(Nodes nd, int64_t begin, int64_t count) {
-  int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (t >= count) return;
-  int64_t i = begin + t;
-  if (nd.type[i] != kTypeInternal) return;
-  int c0 = nd.first_child[i];
-  uint64_t f[8];
-  int ord[8];
-  for (int c = 0; c < 8; c++) {
-    f[c] = nd.fifo[c0 + c];
-    ord[c] = c;
-  }
-  // ascending FIFO rank (all distinct): insertion sort of 8
-  for (int a = 1; a < 8; a++) {
-    int k = ord[a];
-    int b = a - 1;
-    while (b >= 0 && f[ord[b]] > f[k]) {
-      ord[b + 1] = ord[b];
-      b--;
+// The upward pass over all levels in one launch: eight lanes per Internal node
+// (lane c holds child c).  The nodes without Internal children start; the group
+// that brings a parent its last finished Internal child goes on with the parent
+// (a counter per node, no waiting).  The combine itself is serial -- the order
+// the reference's FIFO delivers the children in decides the sums' last bits --
+// so all eight lanes run it on fields shuffled from the child's lane, after one
+// round of loads for the eight children.  One launch per level, one thread per
+// node and a load chain per child took 98 us at N = 4096 and 207 us at 2^20
+// (10-20 us per level).
+__global__ void __launch_bounds__(128) upward_climb(Nodes nd, int64_t ninternal) {
+  const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
+  if (g >= ninternal) return;
+  const int lane = threadIdx.x & 31, c = lane & 7;
+  const unsigned gm = 0xffu << (lane & 24);
+  const int4 first = nd.inode[g];
+  int node = first.x, c0 = first.y;
+  if (nd.npend[node] != 0) return;
+  while (true) {
+    const int j = c0 + c;
+    double v[20];  // this lane's child, past L1: another SM may have written it in this launch
+    const double2* m = reinterpret_cast<const double2*>(nd.mom + j);
+#pragma unroll
+    for (int k = 0; k < 10; k++) {
+      const double2 p = __ldcg(m + k);
+      v[2 * k] = p.x;
+      v[2 * k + 1] = p.y;
     }
-    ord[b + 1] = k;
+    const int count = __ldcg(nd.count + j);
+    const unsigned long long f = __ldcg(reinterpret_cast<const unsigned long long*>(nd.fifo) + j);
+    int rank = 0;  // ascending FIFO position (all distinct)
+#pragma unroll
+    for (int o = 1; o < 8; o++) rank += __shfl_xor_sync(gm, f, o) < f;
+    Mom q;
+    mom_clear(q);
+    int cnt = 0, src = 0;
+    for (int a = 0; a < 8; a++) {
+      src = __ffs(__ballot_sync(gm, rank == a) & gm) - 1;
+      Mom t;
+      t.mass = __shfl_sync(gm, v[0], src);
+      t.cm[0] = __shfl_sync(gm, v[1], src);
+      t.cm[1] = __shfl_sync(gm, v[2], src);
+      t.cm[2] = __shfl_sync(gm, v[3], src);
+      t.soft = __shfl_sync(gm, v[4], src);
+      t.xx = __shfl_sync(gm, v[6], src);
+      t.xy = __shfl_sync(gm, v[7], src);
+      t.xz = __shfl_sync(gm, v[8], src);
+      t.yy = __shfl_sync(gm, v[9], src);
+      t.yz = __shfl_sync(gm, v[10], src);
+      t.zz = __shfl_sync(gm, v[11], src);
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        t.lo[d] = __shfl_sync(gm, v[12 + d], src);
+        t.hi[d] = __shfl_sync(gm, v[15 + d], src);
+      }
+      mom_combine(q, cnt, t, __shfl_sync(gm, count, src));
+    }
+    mom_radius(q, cnt);
+    const unsigned long long last = __shfl_sync(gm, f, src);
+    if (c == 0) {
+      nd.fifo[node] = (((last >> 48) + 1ull) << 48) | (last & ((1ull << 48) - 1ull));
+      nd.mom[node] = q;
+      nd.count[node] = cnt;
+    }
+    const int parent = nd.parent[node];
+    if (parent < 0) return;
+    int go = 0;
+    if (c == 0) {
+      __threadfence();
+      if (atomicAdd(nd.arrived + parent, 1) + 1 == nd.npend[parent]) {
+        nd.arrived[parent] = 0;  // ready for the next upward pass over this tree
+        go = 1;
+      }
+      __threadfence();
+    }
+    if (!__shfl_sync(gm, go, lane & 24)) return;
+    node = parent;
+    c0 = nd.first_child[node];
   }
-  Mom q;
-  mom_clear(q);
-  int cnt = 0;
-  for (int a = 0; a < 8; a++) {
-    int c = c0 + ord[a];
-    mom_combine(q, cnt, nd.mom[c], nd.count[c]);
-  }
-  uint64_t last = f[ord[7]];
-  nd.fifo[i] = (((last >> 40) + 1ull) << 40) | (last & ((1ull << 40) - 1ull));
-  nd.mom[i] = q;
-  nd.count[i] = cnt;
 }
 
 __global__ void __launch_bounds__(256) finalize_records(Nodes nd, int64_t nnodes, double gfac, int want_f32) {
@@ -596,8 +650,8 @@ static inline unsigned blocks_for(int64_t n, int t = 256) { return (unsigned)((n
 void launch_leaf_moments(Nodes nd, int64_t nnodes, Particles p, cudaStream_t st) {
   if (nnodes > 0) { note_launch(); leaf_moments<<<blocks_for(nnodes), 256, 0, st>>>(nd, nnodes, p); }
 }
-void launch_upward_level(Nodes nd, int64_t begin, int64_t count, cudaStream_t st) {
-  if (count > 0) { note_launch(); upward_level<<<blocks_for(count, 128), 128, 0, st>>>(nd, begin, count); }
+void launch_upward(Nodes nd, int64_t ninternal, cudaStream_t st) {
+  if (ninternal > 0) { note_launch(); upward_climb<<<blocks_for(8 * ninternal, 128), 128, 0, st>>>(nd, ninternal); }
 }
 void launch_finalize(Nodes nd, int64_t nnodes, double gfac, int want_f32, cudaStream_t st) {
   if (nnodes > 0) { note_launch(); finalize_records<<<blocks_for(nnodes), 256, 0, st>>>(nd, nnodes, gfac, want_f32); }

@@ -1,6 +1,5 @@
 // k_sort.cu -- K3 stable LSD radix sort of the 64-bit SFC keys with a uint32
-// payload (onesweep), K4 particle permutation, and the device-wide exclusive
-// scan used by the octree build.
+// payload (onesweep) and K4 particle permutation.
 //
 // Replaces std::sort(particles) (src/Subtree.h:281, Particle::operator<
 // src/Particle.C:61-79), which moves ~170-byte AoS particles; here only the
@@ -199,100 +198,6 @@ __global__ void __launch_bounds__(kSortThreads, 2) radix_onesweep(const uint64_t
     kout[dst] = key;
     vout[dst] = S.val[i];
   }
-}
-
-// ---------------------------------------------------------------- scan
-constexpr int kScanThreads = 256;
-constexpr int kScanItems = 8;
-constexpr int kScanTile = kScanThreads * kScanItems;
-
-// Exclusive scan of one tile; writes the tile total to sums[blockIdx.x].
-__global__ void __launch_bounds__(kScanThreads) scan_tiles(const uint32_t* in, uint32_t* out,
-                                                           int64_t n, uint32_t* __restrict__ sums) {
-  __shared__ uint32_t wsum[kScanThreads / 32];
-  int64_t base = (int64_t)blockIdx.x * kScanTile + threadIdx.x * kScanItems;
-  uint32_t v[kScanItems];
-  uint32_t t = 0;
-#pragma unroll
-  for (int j = 0; j < kScanItems; j++) {
-    int64_t i = base + j;
-    v[j] = (i < n) ? in[i] : 0u;
-    t += v[j];
-  }
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  uint32_t inc = t;
-  for (int o = 1; o < 32; o <<= 1) {
-    uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += y;
-  }
-  if (lane == 31) wsum[w] = inc;
-  __syncthreads();
-  if (w == 0) {
-    uint32_t s = (lane < kScanThreads / 32) ? wsum[lane] : 0u;
-    for (int o = 1; o < 32; o <<= 1) {
-      uint32_t y = __shfl_up_sync(0xffffffffu, s, o);
-      if (lane >= o) s += y;
-    }
-    if (lane < kScanThreads / 32) wsum[lane] = s;
-  }
-  __syncthreads();
-  uint32_t run = inc - t + (w ? wsum[w - 1] : 0u);
-#pragma unroll
-  for (int j = 0; j < kScanItems; j++) {
-    int64_t i = base + j;
-    if (i < n) out[i] = run;
-    run += v[j];
-  }
-  if (threadIdx.x == kScanThreads - 1) sums[blockIdx.x] = run;
-}
-
-__global__ void __launch_bounds__(kScanThreads) scan_add(uint32_t* __restrict__ out, int64_t n,
-                                                         const uint32_t* __restrict__ sums) {
-  uint32_t a = sums[blockIdx.x];
-  int64_t base = (int64_t)blockIdx.x * kScanTile;
-  for (int j = threadIdx.x; j < kScanTile; j += kScanThreads) {
-    int64_t i = base + j;
-    if (i < n) out[i] += a;
-  }
-}
-
-__global__ void scan_total(const uint32_t* __restrict__ in, const uint32_t* __restrict__ out, int64_t n,
-                           uint32_t* total) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) *total = (n > 0) ? out[n - 1] + in[n - 1] : 0u;
-}
-
-// Bytes of scratch scan_exclusive needs for n elements.
-size_t scan_scratch_bytes(int64_t n) {
-  size_t b = 0;
-  int64_t m = n;
-  do {
-    m = (m + kScanTile - 1) / kScanTile;
-    b += (size_t)(m + 17) * sizeof(uint32_t);
-  } while (m > 1);
-  return b + 64;
-}
-
-// out[i] = sum_{j<i} in[j]; *total (device) = sum of all.  in may equal out.
-void scan_exclusive(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* scratch, uint32_t* total,
-                    cudaStream_t st) {
-  if (n <= 0) {
-    cudaMemsetAsync(total, 0, sizeof(uint32_t), st);
-    return;
-  }
-  // keep the last input element for the total before an in-place scan
-  uint32_t* last = scratch;
-  cudaMemcpyAsync(last, in + (n - 1), sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
-  uint32_t* sums = scratch + 16;
-  int64_t tiles = (n + kScanTile - 1) / kScanTile;
-  note_launch();
-  scan_tiles<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, n, sums);
-  if (tiles > 1) {
-    scan_exclusive(sums, sums, tiles, sums + tiles + 1, sums + tiles, st);
-    note_launch();
-    scan_add<<<(unsigned)tiles, kScanThreads, 0, st>>>(out, n, sums);
-  }
-  note_launch();
-  scan_total<<<1, 32, 0, st>>>(last, out + (n - 1), 1, total);
 }
 
 // ---------------------------------------------------------------- sort driver

@@ -3,11 +3,11 @@
 //
 // One force pass (pt_compute_forces) runs, on the handle's stream:
 //   K1 bbox + universe -> K2 keys -> K3 radix sort -> K4 permute
-//   -> K5 level-synchronous octree build (+ bucket DFS order)
+//   -> K5 octree build, all levels at once (+ bucket DFS order)
 //   -> K6 leaf moments + upward pass + traversal records
 //   -> K7 traversal (FP64 or mixed), optionally with interaction lists.
-// The host reads back one 4-byte count per tree level (to size the next
-// level) and the status word at the end; everything else stays on the device.
+// The host reads back the tree's node counts (to size the node arrays) and the
+// status word; everything else stays on the device.
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -36,9 +36,8 @@ struct pt_handle {
   uint64_t* key_alt = nullptr;
   uint32_t *idx = nullptr, *idx_alt = nullptr;
   unsigned char* sort_scratch = nullptr;  // onesweep histograms, tile counters, look-back words
-  uint32_t* scan_scratch = nullptr;
-  size_t scan_scratch_elems = 0;
-  uint32_t* d_total = nullptr;
+  uint32_t* tree_counts = nullptr;  // per tile of particles: Internal nodes by level, leaves
+  uint32_t* d_total = nullptr;      // their sums
   double* bbox_partial = nullptr;
   int bbox_blocks = 0;
   double* d_uni = nullptr;  // 12 doubles
@@ -51,9 +50,8 @@ struct pt_handle {
   int64_t cap_srcf = 0;
 
   Nodes nd{};
-  int64_t node_cap = 0, nnodes = 0;
-  uint32_t* flags = nullptr;
-  std::vector<int64_t> lev;
+  int64_t node_cap = 0, nnodes = 0, ninternal = 0;
+  int depth = 0;  // deepest level of the tree
   int32_t* buckets = nullptr;
   unsigned long long* bucket_work = nullptr;  // interactions per bucket of the last pass
   int64_t nbuckets = 0, cap_buckets = 0;
@@ -188,65 +186,34 @@ int ensure_particles(pt_handle* h, int64_t n) {
   CKR(dalloc(h, &h->idx, c));
   CKR(dalloc(h, &h->idx_alt, c));
   CKR(dalloc(h, &h->sort_scratch, sort_scratch_bytes(c)));
-  size_t ss = scan_scratch_bytes(8 * c + 64);
-  h->scan_scratch_elems = ss / sizeof(uint32_t) + 1;
-  CKR(dalloc(h, &h->scan_scratch, h->scan_scratch_elems));
+  CKR(dalloc(h, &h->tree_counts, (size_t)tree_columns() * tree_tiles(c)));
   h->cap_n = c;
   return PT_OK;
 }
 
+// Room for `need` nodes; the arrays hold nothing that outlives a build.
 int grow_nodes(pt_handle* h, int64_t need) {
   if (need <= h->node_cap) return PT_OK;
-  int64_t nc = std::max<int64_t>(need + need / 2, 1024);
-  Nodes o = h->nd;
-  Nodes nn{};
-  int64_t keep = h->nnodes;
-  // build arrays are copied, the rest are (re)computed after the build
-  CKR(dalloc(h, &nn.key, nc));
-  CKR(dalloc(h, &nn.type, nc));
-  CKR(dalloc(h, &nn.depth, nc));
-  CKR(dalloc(h, &nn.pstart, nc));
-  CKR(dalloc(h, &nn.pcount, nc));
-  CKR(dalloc(h, &nn.parent, nc));
-  CKR(dalloc(h, &nn.first_child, nc));
-  CKR(dalloc(h, &nn.count, nc));
-  CKR(dalloc(h, &nn.mom, nc));
-  CKR(dalloc(h, &nn.walk, nc));
-  CKR(dalloc(h, &nn.walks, walk_sib_size(nc)));
-  CKR(dalloc(h, &nn.quad, nc));
-  CKR(dalloc(h, &nn.quadf, nc));
-  CKR(dalloc(h, &nn.fifo, nc));
-  CKR(dalloc(h, &nn.nleaf_sub, nc));
-  CKR(dalloc(h, &nn.nempty_sub, nc));
-  CKR(dalloc(h, &nn.leaf_base, nc));
-  CKR(dalloc(h, &nn.empty_base, nc));
-  if (keep > 0 && o.key) {
-    cudaStream_t st = h->stream;
-    CK(cudaMemcpyAsync(nn.key, o.key, keep * sizeof(uint64_t), cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(nn.type, o.type, keep * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(nn.depth, o.depth, keep * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(nn.pstart, o.pstart, keep * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(nn.pcount, o.pcount, keep * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(nn.parent, o.parent, keep * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(nn.first_child, o.first_child, keep * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(nn.leaf_base, o.leaf_base, keep * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(nn.empty_base, o.empty_base, keep * sizeof(int32_t), cudaMemcpyDeviceToDevice, st));
-    CK(cudaStreamSynchronize(st));
-  }
-  dfree(o.key); dfree(o.type); dfree(o.depth); dfree(o.pstart); dfree(o.pcount); dfree(o.parent);
-  dfree(o.first_child); dfree(o.count); dfree(o.mom); dfree(o.walk); dfree(o.walks); dfree(o.quad); dfree(o.quadf);
-  dfree(o.fifo); dfree(o.nleaf_sub); dfree(o.nempty_sub); dfree(o.leaf_base); dfree(o.empty_base);
-  h->nd = nn;
-  // flags holds the current level's child ranks while the build is running:
-  // the new buffer must start with the old contents.
-  uint32_t* nf = nullptr;
-  CK(cudaMalloc((void**)&nf, nc * sizeof(uint32_t)));
-  if (h->flags && h->node_cap > 0) {
-    CK(cudaMemcpyAsync(nf, h->flags, h->node_cap * sizeof(uint32_t), cudaMemcpyDeviceToDevice, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-  }
-  dfree(h->flags);
-  h->flags = nf;
+  const int64_t nc = std::max<int64_t>(need + need / 4, 1024);
+  Nodes& o = h->nd;
+  h->node_cap = 0;
+  CKR(dalloc(h, &o.key, nc));
+  CKR(dalloc(h, &o.type, nc));
+  CKR(dalloc(h, &o.depth, nc));
+  CKR(dalloc(h, &o.pstart, nc));
+  CKR(dalloc(h, &o.pcount, nc));
+  CKR(dalloc(h, &o.parent, nc));
+  CKR(dalloc(h, &o.first_child, nc));
+  CKR(dalloc(h, &o.count, nc));
+  CKR(dalloc(h, &o.mom, nc));
+  CKR(dalloc(h, &o.walk, nc));
+  CKR(dalloc(h, &o.walks, walk_sib_size(nc)));
+  CKR(dalloc(h, &o.quad, nc));
+  CKR(dalloc(h, &o.quadf, nc));
+  CKR(dalloc(h, &o.fifo, nc));
+  CKR(dalloc(h, &o.inode, nc / 8 + 1));
+  CKR(dalloc(h, &o.npend, nc));
+  CKR(dalloc(h, &o.arrived, nc));
   h->node_cap = nc;
   return PT_OK;
 }
@@ -299,44 +266,27 @@ int keys_and_sort(pt_handle* h) {
   return PT_OK;
 }
 
-// K5: octree build, levels, bucket order.
+// K5: octree build and bucket order.
 int build_tree(pt_handle* h) {
   cudaStream_t st = h->stream;
   const int64_t n = h->n;
-  if (h->node_cap < 1024) {
-    h->nnodes = 0;
-    CKR(grow_nodes(h, std::max<int64_t>(1024, n / 2 + 1024)));
-  }
-  h->nnodes = 1;
-  launch_init_root(h->nd, n, h->cfg.bucket, st);
-  h->lev.assign(1, 0);
-  int64_t begin = 0, count = 1;
-  while (true) {
-    launch_flag_internal(h->nd.type, begin, count, h->flags, st);
-    scan_exclusive(h->flags, h->flags, count, h->scan_scratch, h->d_total, st);
-    uint32_t ni = 0;
-    CK(cudaMemcpyAsync(&ni, h->d_total, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    h->lev.push_back(begin + count);
-    if (ni == 0) break;
-    int64_t next = begin + count;
-    int64_t need = next + 8 * (int64_t)ni;
-    if (need > h->node_cap) {
-      h->nnodes = next;
-      CKR(grow_nodes(h, need));
-    }
-    launch_build_children(h->nd, h->p.key, begin, count, h->flags, next, h->cfg.bucket, h->node_cap, h->d_status, st);
-    begin = next;
-    count = 8 * (int64_t)ni;
-    h->nnodes = need;
-  }
-  const int L = (int)h->lev.size() - 1;
-  for (int l = L - 1; l >= 0; l--) launch_count_subtree(h->nd, h->lev[l], h->lev[l + 1] - h->lev[l], st);
-  for (int l = 0; l < L; l++) launch_base_topdown(h->nd, h->lev[l], h->lev[l + 1] - h->lev[l], st);
-  int32_t nl = 0;
-  CK(cudaMemcpyAsync(&nl, h->nd.nleaf_sub, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+  launch_tree_count(h->p.key, n, h->cfg.bucket, h->tree_counts, h->d_total, st);
+  uint32_t tot[kMaxDepth + 1];  // Internal nodes of each level, leaves
+  CK(cudaMemcpyAsync(tot, h->d_total, sizeof(tot), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  h->nbuckets = nl;
+  int64_t ni = 0;
+  int depth = 0;
+  for (int l = 0; l < kMaxDepth; l++) {
+    ni += tot[l];
+    if (tot[l]) depth = l + 1;
+  }
+  const int64_t nl = tot[kMaxDepth];
+  h->nnodes = 0;
+  CKR(grow_nodes(h, 1 + 8 * ni));
+  h->nnodes = 1 + 8 * ni;
+  h->ninternal = ni;
+  h->depth = depth;
+  h->nbuckets = 0;
   if (nl > h->cap_buckets) {
     // an eighth of headroom: the bucket count drifts from pass to pass as the
     // particles move, and a cudaFree on every new maximum would stall the device
@@ -345,7 +295,9 @@ int build_tree(pt_handle* h) {
     CKR(dalloc(h, &h->bucket_work, cap));
     h->cap_buckets = cap;
   }
-  launch_assign_buckets(h->nd, h->nnodes, h->buckets, nl, st);
+  h->nbuckets = nl;
+  launch_tree_emit(h->nd, h->p.key, n, h->cfg.bucket, h->tree_counts, h->d_total, ni, h->node_cap, nl, h->buckets,
+                   h->d_status, st);
   CK(cudaGetLastError());
   CK(cudaEventRecord(h->ev[3], st));
   return PT_OK;
@@ -355,8 +307,7 @@ int build_tree(pt_handle* h) {
 int upward(pt_handle* h) {
   cudaStream_t st = h->stream;
   launch_leaf_moments(h->nd, h->nnodes, h->p, st);
-  const int L = (int)h->lev.size() - 1;
-  for (int l = L - 1; l >= 0; l--) launch_upward_level(h->nd, h->lev[l], h->lev[l + 1] - h->lev[l], st);
+  launch_upward(h->nd, h->ninternal, st);
   const double gfac = (4.0 / 3.0) / (h->cfg.theta * h->cfg.theta);  // GravityVisitor.h:14,18
   const int mixed = h->cfg.precision == PT_MIXED;
   launch_finalize(h->nd, h->nnodes, gfac, mixed, st);
@@ -736,7 +687,7 @@ int forces(pt_handle* h, int64_t b0, int64_t b1) {
   k.n_open = c[2];
   k.n_nodes = h->nnodes;
   k.n_buckets = h->nbuckets;
-  k.depth = (int32_t)h->lev.size() - 2;
+  k.depth = h->depth;
   k.launches = (int32_t)(launches_so_far() - launches0);
   CK(cudaEventElapsedTime(&k.ms_keys, h->ev[0], h->ev[1]));
   CK(cudaEventElapsedTime(&k.ms_sort, h->ev[1], h->ev[2]));
@@ -853,7 +804,7 @@ int pt_create(const pt_config* cfg, pt_handle** out) {
   if (dalloc(h, &h->d_counters, 3) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_work, 1) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_vmax2, 1) != PT_OK) return bail(PT_E_NOMEM);
-  if (dalloc(h, &h->d_total, 4) != PT_OK) return bail(PT_E_NOMEM);
+  if (dalloc(h, &h->d_total, tree_columns()) != PT_OK) return bail(PT_E_NOMEM);
   if (cudaMemset(h->d_status, 0, sizeof(unsigned)) != cudaSuccess) return bail(PT_E_CUDA);
   *out = h;
   return PT_OK;
@@ -867,13 +818,13 @@ int pt_destroy(pt_handle* h) {
                     &h->p.ax, &h->p.ay, &h->p.az, &h->p.pot, &h->p.potf, &h->tmp_d};
   for (auto pp : dbl) dfree(*pp);
   dfree(h->p.order); dfree(h->tmp_i); dfree(h->p.key); dfree(h->key_alt); dfree(h->idx); dfree(h->idx_alt);
-  dfree(h->sort_scratch); dfree(h->scan_scratch); dfree(h->d_total); dfree(h->bbox_partial); dfree(h->d_uni);
+  dfree(h->sort_scratch); dfree(h->tree_counts); dfree(h->d_total); dfree(h->bbox_partial); dfree(h->d_uni);
   dfree(h->d_status); dfree(h->d_counters); dfree(h->d_work); dfree(h->d_vmax2); dfree(h->srcf); dfree(h->softf);
   Nodes& o = h->nd;
   dfree(o.key); dfree(o.type); dfree(o.depth); dfree(o.pstart); dfree(o.pcount); dfree(o.parent);
   dfree(o.first_child); dfree(o.count); dfree(o.mom); dfree(o.walk); dfree(o.walks); dfree(o.quad); dfree(o.quadf);
-  dfree(o.fifo); dfree(o.nleaf_sub); dfree(o.nempty_sub); dfree(o.leaf_base); dfree(o.empty_base);
-  dfree(h->flags); dfree(h->buckets); dfree(h->bucket_work); dfree(h->list_count); dfree(h->list_off); dfree(h->list_node);
+  dfree(o.fifo); dfree(o.inode); dfree(o.npend); dfree(o.arrived);
+  dfree(h->buckets); dfree(h->bucket_work); dfree(h->list_count); dfree(h->list_off); dfree(h->list_node);
   dfree(h->list_kind); dfree(h->dsum); dfree(h->adj); dfree(h->nadj); dfree(h->d_htab); dfree(h->ewd); dfree(h->sph); dfree(h->sph_nbr); dfree(h->sph_nd2);
   dfree(h->sph_list_d); dfree(h->sph_list_i); dfree(h->sph_state);
   dfree(h->pool_pc); dfree(h->pool_pp); dfree(h->l_pc_start); dfree(h->l_pp_start); dfree(h->l_pc_count);
@@ -1493,8 +1444,7 @@ bool lists_cover_all(const pt_handle* h) {
 int recompute_moments(pt_handle* h) {
   cudaStream_t st = h->stream;
   launch_leaf_moments(h->nd, h->nnodes, h->p, st);
-  const int L = (int)h->lev.size() - 1;
-  for (int l = L - 1; l >= 0; l--) launch_upward_level(h->nd, h->lev[l], h->lev[l + 1] - h->lev[l], st);
+  launch_upward(h->nd, h->ninternal, st);
   const double gfac = (4.0 / 3.0) / (h->cfg.theta * h->cfg.theta);
   launch_finalize(h->nd, h->nnodes, gfac, h->cfg.precision == PT_MIXED, st);
   CK(cudaGetLastError());

@@ -107,11 +107,10 @@ struct Nodes {
   double2* walks;       // sibling-block copy of walk's classification fields (walk_sib_index)
   QuadRec* quad;
   QuadRecF* quadf;
-  uint64_t* fifo;       // upward-pass FIFO position key (depth-of-chain << 40 | rank)
-  int32_t* nleaf_sub;   // Leaf nodes in subtree
-  int32_t* nempty_sub;  // EmptyLeaf nodes in subtree
-  int32_t* leaf_base;   // DFS rank base of Leaf nodes in subtree
-  int32_t* empty_base;  // DFS rank base of EmptyLeaf nodes in subtree
+  uint64_t* fifo;       // upward-pass FIFO position key (depth-of-chain << 48 | position)
+  int4* inode;          // Internal nodes, level by level: node, first child, first particle, level
+  int32_t* npend;       // Internal node: how many of its children are Internal
+  int32_t* arrived;     // Internal node: those finished in the running upward pass (0 between passes)
 };
 
 struct TravParams {

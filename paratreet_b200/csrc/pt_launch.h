@@ -18,9 +18,6 @@ void launch_vmax2(const double* vx, const double* vy, const double* vz, int64_t 
                   int grid, cudaStream_t st);
 
 // k_sort.cu
-size_t scan_scratch_bytes(int64_t n);
-void scan_exclusive(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* scratch, uint32_t* total,
-                    cudaStream_t st);
 size_t sort_scratch_bytes(int64_t n);
 // 0 on success, -1 if the kernel attribute could not be set; spin_limit =
 // polls of an unpublished tile before the look-back gives up (kErrSort)
@@ -29,18 +26,20 @@ int radix_sort_pairs(uint64_t* k0, uint32_t* v0, uint64_t* k1, uint32_t* v1, int
 void gather_f64(const double* in, double* out, const uint32_t* idx, int64_t n, int grid, cudaStream_t st);
 void gather_i32(const int32_t* in, int32_t* out, const uint32_t* idx, int64_t n, int grid, cudaStream_t st);
 
-// k_build.cu
-void launch_init_root(Nodes nd, int64_t n, int bucket, cudaStream_t st);
-void launch_flag_internal(const int32_t* type, int64_t begin, int64_t count, uint32_t* flags, cudaStream_t st);
-void launch_build_children(Nodes nd, const uint64_t* keys, int64_t begin, int64_t count, const uint32_t* rank,
-                           int64_t next_begin, int bucket, int64_t cap, unsigned* status, cudaStream_t st);
-void launch_count_subtree(Nodes nd, int64_t begin, int64_t count, cudaStream_t st);
-void launch_base_topdown(Nodes nd, int64_t begin, int64_t count, cudaStream_t st);
-void launch_assign_buckets(Nodes nd, int64_t nnodes, int32_t* buckets, int nleaves, cudaStream_t st);
+// k_build.cu: the columns and tiles of the per-tile counts, the counting pass
+// (totals[L] = Internal nodes of level L, the last one the leaves), and the pass
+// that writes the nodes and the buckets
+int tree_columns();
+int tree_tiles(int64_t n);
+void launch_tree_count(const uint64_t* keys, int64_t n, int bucket, uint32_t* counts, uint32_t* totals,
+                       cudaStream_t st);
+void launch_tree_emit(Nodes nd, const uint64_t* keys, int64_t n, int bucket, const uint32_t* counts,
+                      const uint32_t* totals, int64_t ninternal, int64_t cap, int64_t nbuckets, int32_t* buckets,
+                      unsigned* status, cudaStream_t st);
 
 // k_fp64.cu
 void launch_leaf_moments(Nodes nd, int64_t nnodes, Particles p, cudaStream_t st);
-void launch_upward_level(Nodes nd, int64_t begin, int64_t count, cudaStream_t st);
+void launch_upward(Nodes nd, int64_t ninternal, cudaStream_t st);
 void launch_finalize(Nodes nd, int64_t nnodes, double gfac, int want_f32, cudaStream_t st);
 void launch_traverse_f64(const TravParams& P, const Mom* mom, int grid, cudaStream_t st);
 void launch_replay_f64(const TravParams& P, int grid, cudaStream_t st);
