@@ -17,8 +17,9 @@
 //                      order their last child leaves it.
 //     finalize         per-node traversal records (WalkRec, QuadRec).
 //  K7 traverse_f64     warp-per-bucket walk (pt_walk.cuh) with the FP64
-//                      GravityVisitor leaf / node evaluators -- bit-identical
-//                      to the reference built -DUSE_DOUBLE_FP.
+//                      GravityVisitor leaf / node terms, summed in the
+//                      reference's order -- bit-identical to the reference
+//                      built -DUSE_DOUBLE_FP.
 //  K8 kick_perturb     Particle::kick + Particle::perturb
 //                      (src/Particle.C:7-21) fused, and the leapfrog variant.
 //  K9 direct_sum       FP64 spline direct sum (force-error yardstick).
@@ -290,127 +291,340 @@ __global__ void __launch_bounds__(256) finalize_records(Nodes nd, int64_t nnodes
 }
 
 // ---------------------------------------------------------------- traversal
+// One warp per bucket.  The reference fixes the order in which each target adds
+// its interactions, not the order in which the terms are computed, so a bucket's
+// interactions are collected in walk order (up to 64 entries), their terms are
+// computed for all targets by groups of lanes in parallel, and the sums then
+// run over the entries in walk order:
+//   terms  lane l of group l / nt is target l mod nt; the G = 32 / nt groups take
+//          different entries.  A leaf's term is its own partial sum (the
+//          reference's leaf() adds a leaf's pairs into a local first), in particle
+//          order.  Leaves are taken by descending size, so the groups' loops are
+//          of similar length; then quadrupole, then monopole nodes.
+//   sums   the terms wait in shared memory as [entry][target][ax ay az pot]; lane
+//          4 t + c adds component c of target t over the entries, in order.
+// With more than 16 targets (one group) each lane keeps its target's sums itself.
+// Bound by the FP64 pipe (45-80 operations per term, with the IEEE square roots
+// and divisions) and by latency.  With one lane per target and nothing else (a
+// bucket holds 4-10 particles, so 4-10 of 32 lanes worked) the 2^20 mixture took
+// 84.8 ms and the 4096-particle Plummer 1.01 ms; this takes 28.6 and 0.74 ms.
 constexpr int kTravWarps = 4;
+constexpr int kF64Entries = 64;
+constexpr int kF64Terms = 256;  // (entry, target) terms held in shared memory
+enum : int { kEntLeaf = 0, kEntQuad = 1, kEntMono = 2 };
+
+struct F64Warp {
+  double term[4 * kF64Terms];
+  BucketGeom geom;
+  union {
+    WalkSeg stack[kWalkStack];
+    int32_t queue[kBfsQueue];  // basic-down order
+  };
+  int32_t ent[kF64Entries];      // node | kind << 30, walk order
+  uint8_t order[kF64Entries];    // entries by kind and size
+};
 
 struct F64Eval {
-  const Particles* p;
-  const WalkRec* walk;
-  const QuadRec* quad;
-  double* stage;  // this warp's [5][32] source staging
-  int lane, nt;
+  const TravParams* P;
+  F64Warp* w;
+  int lane, nt, grp, G, cap, n;
   double xi, yi, zi, si;
-  double ax, ay, az, pot, potf;
-  double ox, oy, oz;
-  const BucketGeom* g;
-  unsigned long long n_pp, n_pc;
-  int record;
-  int64_t nlist, lbase;
-  int32_t* lnode;
-  int8_t* lkind;
+  double s[5];  // G > 1: sums of (target, component) pairs lane and lane + 32, then their pot; else ax ay az pot potf
+  unsigned nsrc, npc;
+  int64_t lat;  // where the next list entry goes (recording)
+  bool record;
 
-  // GravityVisitor::leaf, examples/GravityVisitor.h:144-160
-  __device__ void p2p(int node) {
-    const int s0 = walk[node].pstart, sn = walk[node].pcount;
-    double pax = 0.0, pay = 0.0, paz = 0.0, ppf = 0.0;
-    for (int base = 0; base < sn; base += 32) {
-      int cnt = min(32, sn - base);
-      __syncwarp();
-      if (lane < cnt) {
-        int j = s0 + base + lane;
-        stage[0 * 32 + lane] = p->x[j];
-        stage[1 * 32 + lane] = p->y[j];
-        stage[2 * 32 + lane] = p->z[j];
-        stage[3 * 32 + lane] = p->m[j];
-        stage[4 * 32 + lane] = p->soft[j];
-      }
-      __syncwarp();
+  __device__ void begin(const TravParams& Q, F64Warp& W, int t0, int ntargets, int l, int64_t rec) {
+    P = &Q;
+    w = &W;
+    lane = l;
+    nt = ntargets;
+    G = 32 / nt;
+    grp = lane / nt;
+    cap = min(kF64Entries, kF64Terms / nt);
+    if (G == 1) cap = kF64Entries;
+    n = 0;
+    nsrc = npc = 0;
+    record = rec >= 0;
+    lat = rec;
+    xi = yi = zi = si = 0.0;
+    const int t = lane % nt;
+    if (grp < G) {
+      xi = Q.p.x[t0 + t];
+      yi = Q.p.y[t0 + t];
+      zi = Q.p.z[t0 + t];
+      si = Q.p.soft[t0 + t];
+    }
+#pragma unroll
+    for (int k = 0; k < 5; k++) s[k] = 0.0;
+    if (!Q.accumulate) return;  // later replica walks continue each particle's sums
+    if (G == 1) {
       if (lane < nt) {
-        for (int j = 0; j < cnt; j++) {
-          double xs = stage[j], ys = stage[32 + j], zs = stage[64 + j], ms = stage[96 + j], ss = stage[128 + j];
-          double dx = (xs + ox) - xi;
-          double dy = (ys + oy) - yi;
-          double dz = (zs + oz) - zi;
-          double rsq = dx * dx + dy * dy + dz * dz;
-          double twoh = ss + si;
-          if (rsq != 0) {
-            double a, b;
-            spline_f64(rsq, twoh, a, b);
-            double bm = b * ms;
-            pax += dx * bm;
-            pay += dy * bm;
-            paz += dz * bm;
-            ppf += -ms * a;
-          }
+        const int i = t0 + lane;
+        s[0] = Q.p.ax[i]; s[1] = Q.p.ay[i]; s[2] = Q.p.az[i]; s[3] = Q.p.pot[i]; s[4] = Q.p.potf[i];
+      }
+    } else {
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int p = lane + 32 * h;
+        if (p < 4 * nt) {
+          const int i = t0 + (p >> 2), c = p & 3;
+          s[h] = c == 0 ? Q.p.ax[i] : c == 1 ? Q.p.ay[i] : c == 2 ? Q.p.az[i] : Q.p.potf[i];
+          if (c == 3) s[2 + h] = Q.p.pot[i];
         }
       }
-    }
-    ax += pax;
-    ay += pay;
-    az += paz;
-    potf += ppf;
-    n_pp += (unsigned long long)sn * (unsigned long long)nt;
-    if (record) {
-      if (lane == 0) { lnode[lbase + nlist] = node; lkind[lbase + nlist] = 0; }
-      ++nlist;
     }
   }
 
-  // GravityVisitor::node, examples/GravityVisitor.h:184-224 (non-HEXADECAPOLE);
-  // mono = openSoftening held (decided in the walk), i.e. addGravity (:130-139)
-  __device__ void p2c(int node, bool mono) {
-    const WalkRec w = walk[node];
-    const QuadRec q = quad[node];
-    n_pc += (unsigned long long)nt;
-    if (record) {
-      if (lane == 0) { lnode[lbase + nlist] = node; lkind[lbase + nlist] = mono ? 2 : 1; }
-      ++nlist;
-    }
-    if (w.count == 0) return;
-    const double cx = w.cm[0] + ox, cy = w.cm[1] + oy, cz = w.cm[2] + oz;
-    if (mono) {
-      if (lane < nt) {  // addGravity, :130-139
-        double dx = cx - xi, dy = cy - yi, dz = cz - zi;
-        double rsq = dx * dx + dy * dy + dz * dz;
-        if (rsq != 0) {
-          double f = q.mass / (rsq * sqrt(rsq));
-          ax += dx * f;
-          ay += dy * f;
-          az += dz * f;
-          potf += -q.mass / sqrt(rsq);
-        }
+  __device__ void store(int t0) {
+    const Particles& q = P->p;
+    if (G == 1) {
+      if (lane < nt) {
+        const int i = t0 + lane;
+        q.ax[i] = s[0]; q.ay[i] = s[1]; q.az[i] = s[2]; q.pot[i] = s[3]; q.potf[i] = s[4];
       }
       return;
     }
-    if (lane < nt) {
-      double rx = (xi - w.cm[0]) - ox;
-      double ry = (yi - w.cm[1]) - oy;
-      double rz = (zi - w.cm[2]) - oz;
-      double rsq = rx * rx + ry * ry + rz * rz;
-      double dir = 1.0 / sqrt(rsq);
-      double twoh = q.soft + si;
-      double a, b, c, d;
-      splineq_f64(dir, rsq, twoh, a, b, c, d);
-      double qx = q.xx * rx + q.xy * ry + q.xz * rz;
-      double qy = q.xy * rx + q.yy * ry + q.yz * rz;
-      double qz = q.xz * rx + q.yz * ry + q.zz * rz;
-      double qir = 0.5 * (qx * rx + qy * ry + qz * rz);
-      double tr = 0.5 * (q.xx + q.yy + q.zz);
-      double qir3 = b * q.mass + d * qir - c * tr;
-      double pp = -q.mass * a - c * qir + b * tr;
-      pot += pp;
-      potf += pp;
-      ax += -qir3 * rx + c * qx;
-      ay += -qir3 * ry + c * qy;
-      az += -qir3 * rz + c * qz;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int p = lane + 32 * h;
+      if (p < 4 * nt) {
+        const int i = t0 + (p >> 2), c = p & 3;
+        double* const out = c == 0 ? q.ax : c == 1 ? q.ay : c == 2 ? q.az : q.potf;
+        out[i] = s[h];
+        if (c == 3) q.pot[i] = s[2 + h];
+      }
     }
+  }
+
+  // Runs of terminals from the walk: children c0 + k, in child order.
+  __device__ void emit(int c0, uint32_t pp, uint32_t pq, uint32_t pm) {
+    const uint32_t run = pp | pq | pm;
+    const int m = __popc(run);
+    if (n + m > cap) flush();
+    if (lane < 8 && ((run >> lane) & 1u)) {
+      const int kind = ((pp >> lane) & 1u) ? kEntLeaf : ((pq >> lane) & 1u) ? kEntQuad : kEntMono;
+      const int at = __popc(run & ((1u << lane) - 1u));
+      w->ent[n + at] = (c0 + lane) | (kind << 30);
+      if (record) {
+        P->list_node[lat + at] = c0 + lane;
+        P->list_kind[lat + at] = (int8_t)kind;
+      }
+    }
+    lat += m;
+    n += m;
+  }
+
+  // One entry of a recorded list.
+  __device__ void push(int node, int kind) {
+    if (n == cap) flush();
+    if (lane == 0) w->ent[n] = node | (kind << 30);
+    ++n;
+  }
+
+  // GravityVisitor::leaf, examples/GravityVisitor.h:144-160
+  __device__ void leaf_term(int node, double v[4]) const {
+    const int s0 = P->walk[node].pstart, sn = P->walk[node].pcount;
+    const Particles& q = P->p;
+    double pax = 0.0, pay = 0.0, paz = 0.0, ppf = 0.0;
+    double nx = q.x[s0], ny = q.y[s0], nz = q.z[s0], nm = q.m[s0], ns = q.soft[s0];
+    for (int j = 1; j <= sn; j++) {
+      const double xs = nx, ys = ny, zs = nz, ms = nm, ss = ns;
+      if (j < sn) {  // the next source, ahead of this one's chain of divisions
+        nx = q.x[s0 + j];
+        ny = q.y[s0 + j];
+        nz = q.z[s0 + j];
+        nm = q.m[s0 + j];
+        ns = q.soft[s0 + j];
+      }
+      const double dx = (xs + P->ox) - xi;
+      const double dy = (ys + P->oy) - yi;
+      const double dz = (zs + P->oz) - zi;
+      const double rsq = dx * dx + dy * dy + dz * dz;
+      const double twoh = ss + si;
+      if (rsq != 0) {
+        double a, b;
+        spline_f64(rsq, twoh, a, b);
+        const double bm = b * ms;
+        pax += dx * bm;
+        pay += dy * bm;
+        paz += dz * bm;
+        ppf += -ms * a;
+      }
+    }
+    v[0] = pax;
+    v[1] = pay;
+    v[2] = paz;
+    v[3] = ppf;
+  }
+
+  // GravityVisitor::node, examples/GravityVisitor.h:184-224 (non-HEXADECAPOLE)
+  __device__ void quad_term(int node, double v[4]) const {
+    const double2* wr = reinterpret_cast<const double2*>(P->walk + node);
+    const double2 c01 = wr[0];
+    const double cz = wr[1].x;
+    const QuadRec q = P->quad[node];
+    const double rx = (xi - c01.x) - P->ox;
+    const double ry = (yi - c01.y) - P->oy;
+    const double rz = (zi - cz) - P->oz;
+    const double rsq = rx * rx + ry * ry + rz * rz;
+    const double dir = 1.0 / sqrt(rsq);
+    const double twoh = q.soft + si;
+    double a, b, c, d;
+    splineq_f64(dir, rsq, twoh, a, b, c, d);
+    const double qx = q.xx * rx + q.xy * ry + q.xz * rz;
+    const double qy = q.xy * rx + q.yy * ry + q.yz * rz;
+    const double qz = q.xz * rx + q.yz * ry + q.zz * rz;
+    const double qir = 0.5 * (qx * rx + qy * ry + qz * rz);
+    const double tr = 0.5 * (q.xx + q.yy + q.zz);
+    const double qir3 = b * q.mass + d * qir - c * tr;
+    v[3] = -q.mass * a - c * qir + b * tr;
+    v[0] = -qir3 * rx + c * qx;
+    v[1] = -qir3 * ry + c * qy;
+    v[2] = -qir3 * rz + c * qz;
+  }
+
+  // openSoftening held (decided in the walk): addGravity, :130-139
+  __device__ void mono_term(int node, double v[4]) const {
+    const WalkRec* wr = P->walk + node;
+    const double mass = P->quad[node].mass;
+    const double cx = wr->cm[0] + P->ox, cy = wr->cm[1] + P->oy, cz = wr->cm[2] + P->oz;
+    const double dx = cx - xi, dy = cy - yi, dz = cz - zi;
+    const double rsq = dx * dx + dy * dy + dz * dz;
+    v[0] = v[1] = v[2] = v[3] = 0.0;
+    if (rsq != 0) {
+      const double f = mass / (rsq * sqrt(rsq));
+      v[0] = dx * f;
+      v[1] = dy * f;
+      v[2] = dz * f;
+      v[3] = -mass / sqrt(rsq);
+    }
+  }
+
+  // Evaluate the collected entries and add them to the sums.
+  __device__ void flush() {
+    __syncwarp();
+    // kinds and leaf sizes of this lane's two entries
+    int key[2];
+    unsigned src = 0;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int e = lane + 32 * h;
+      key[h] = -1;
+      if (e < n) {
+        const int x = w->ent[e], kind = (unsigned)x >> 30;
+        if (kind == kEntLeaf) {
+          const int sn = P->walk[x].pcount;
+          src += (unsigned)sn;
+          key[h] = 1 + sn;
+        } else {
+          key[h] = kind == kEntQuad ? 1 : 0;
+        }
+      }
+    }
+    const int nquad = __popc(__ballot_sync(kFull, key[0] == 1)) + __popc(__ballot_sync(kFull, key[1] == 1));
+    const int nmono = __popc(__ballot_sync(kFull, key[0] == 0)) + __popc(__ballot_sync(kFull, key[1] == 0));
+    const int nleaf = n - nquad - nmono;
+    nsrc += __reduce_add_sync(kFull, src);
+    npc += (unsigned)(nquad + nmono);
+    if (G == 1) {
+      for (int e = 0; e < n; e++) {
+        const int x = w->ent[e], kind = (unsigned)x >> 30, node = x & 0x3fffffff;
+        if (lane < nt) {
+          double v[4];
+          if (kind == kEntLeaf) leaf_term(node, v);
+          else if (kind == kEntQuad) quad_term(node, v);
+          else mono_term(node, v);
+          s[0] += v[0];
+          s[1] += v[1];
+          s[2] += v[2];
+          if (kind == kEntQuad) s[3] += v[3];
+          s[4] += v[3];
+        }
+      }
+      n = 0;
+      __syncwarp();
+      return;
+    }
+    // entries by descending key: one round per distinct key
+    {
+      const unsigned lt = (1u << lane) - 1u;
+      int done = 0;
+      int k0 = key[0], k1 = key[1];
+      while (done < n) {
+        const int top = __reduce_max_sync(kFull, max(k0, k1));
+        const unsigned m0 = __ballot_sync(kFull, k0 == top), m1 = __ballot_sync(kFull, k1 == top);
+        if (k0 == top) {
+          w->order[done + __popc(m0 & lt)] = (uint8_t)lane;
+          k0 = -1;
+        }
+        if (k1 == top) {
+          w->order[done + __popc(m0) + __popc(m1 & lt)] = (uint8_t)(lane + 32);
+          k1 = -1;
+        }
+        done += __popc(m0) + __popc(m1);
+      }
+    }
+    __syncwarp();
+    if (grp < G) {
+      const int t = lane % nt;
+      int k = grp;
+      for (; k < nleaf; k += G) {
+        const int e = w->order[k];
+        double v[4];
+        leaf_term(w->ent[e] & 0x3fffffff, v);
+        double2* o = reinterpret_cast<double2*>(w->term + 4 * (e * nt + t));
+        o[0] = make_double2(v[0], v[1]);
+        o[1] = make_double2(v[2], v[3]);
+      }
+      for (; k < n; k += G) {
+        const int e = w->order[k], x = w->ent[e];
+        double v[4];
+        if (((unsigned)x >> 30) == kEntQuad) quad_term(x & 0x3fffffff, v);
+        else mono_term(x & 0x3fffffff, v);
+        double2* o = reinterpret_cast<double2*>(w->term + 4 * (e * nt + t));
+        o[0] = make_double2(v[0], v[1]);
+        o[1] = make_double2(v[2], v[3]);
+      }
+    }
+    __syncwarp();
+    const int per = 4 * nt;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int p = lane + 32 * h;
+      if (p < per) {
+        double a = s[h], b = s[2 + h];
+        for (int e = 0; e < n; e++) {
+          const double v = w->term[e * per + p];
+          a += v;
+          if (((unsigned)w->ent[e] >> 30) == kEntQuad) b += v;  // pot: quadrupole node() terms only
+        }
+        s[h] = a;
+        s[2 + h] = b;
+      }
+    }
+    n = 0;
+    __syncwarp();
   }
 };
 
-__global__ void __launch_bounds__(kTravWarps * 32) traverse_f64(TravParams P, const Mom* __restrict__ mom) {
-  __shared__ WalkFrame stacks[kTravWarps][kWalkStack];
-  __shared__ int32_t queues[kTravWarps][kBfsQueue];  // basic-down order only
-  __shared__ double stage[kTravWarps][5 * 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+// The bucket's walk in the handle's order; its geometry stays in shared memory
+// (the terms need the registers).
+template <bool kBfs, class Sink>
+__device__ __forceinline__ bool walk_one(const TravParams& P, F64Warp& W, int lane, Sink& sink,
+                                         unsigned long long& opens) {
+  if constexpr (kBfs)
+    return walk_bucket_bfs(P.walk, P.nnodes, W.geom, P.ox, P.oy, P.oz, W.queue, kBfsQueue, lane, sink, opens, P.status);
+  else
+    return walk_preorder(P.walk, P.walks, P.nnodes, W.geom, P.ox, P.oy, P.oz, W.stack, lane, sink, opens, P.status);
+}
+
+// CTAs per SM: 42 KB of shared memory each
+template <bool kBfs>
+__global__ void __launch_bounds__(kTravWarps * 32, 5) traverse_f64(TravParams P, const Mom* __restrict__ mom) {
+  __shared__ F64Warp warps[kTravWarps];
+  F64Warp& W = warps[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
   unsigned long long c_pp = 0, c_pc = 0, c_open = 0;
   while (true) {
     unsigned bi = 0;
@@ -423,16 +637,13 @@ __global__ void __launch_bounds__(kTravWarps * 32) traverse_f64(TravParams P, co
       if (lane == 0) atomicOr(P.status, kErrCapacity);
       continue;
     }
-    BucketGeom g;
-    load_bucket_geom(mom, tnode, g);
+    __syncwarp();
+    if (lane == 0) load_bucket_geom(mom, tnode, W.geom);
+    __syncwarp();
     const int tbase = P.walk[tnode].pstart, ntot = P.walk[tnode].pcount;
     if (P.mode == 1) {  // count the interaction list only
-      ListRecorder rec{lane, 1, 0, 0, nullptr, nullptr};
-      if (!(P.bfs ? walk_bucket_bfs(P.walk, P.nnodes, g, P.ox, P.oy, P.oz, queues[wid], kBfsQueue, lane, rec,
-                                    c_open, P.status)
-                  : walk_bucket(P.walk, P.nnodes, g, P.ox, P.oy, P.oz, stacks[wid], lane, rec, c_open, P.status)) &&
-          lane == 0)
-        atomicOr(P.status, kErrStack);
+      ListCounter rec{0};
+      if (!walk_one<kBfs>(P, W, lane, rec, c_open) && lane == 0) atomicOr(P.status, kErrStack);
       if (lane == 0) P.list_count[b - P.b_begin] = rec.n;
       continue;
     }
@@ -443,53 +654,17 @@ __global__ void __launch_bounds__(kTravWarps * 32) traverse_f64(TravParams P, co
       const int t0 = tbase + tc, nt = min(32, ntot - tc);
       unsigned long long opens = 0;
       F64Eval ev;
-      ev.p = &P.p;
-      ev.walk = P.walk;
-      ev.quad = P.quad;
-      ev.stage = stage[wid];
-      ev.lane = lane;
-      ev.nt = nt;
-      ev.xi = ev.yi = ev.zi = ev.si = 0.0;
-      if (lane < nt) {
-        ev.xi = P.p.x[t0 + lane];
-        ev.yi = P.p.y[t0 + lane];
-        ev.zi = P.p.z[t0 + lane];
-        ev.si = P.p.soft[t0 + lane];
-      }
-      ev.ax = ev.ay = ev.az = ev.pot = ev.potf = 0.0;
-      if (P.accumulate && lane < nt) {  // later replica walks continue each particle's sum
-        ev.ax = P.p.ax[t0 + lane];
-        ev.ay = P.p.ay[t0 + lane];
-        ev.az = P.p.az[t0 + lane];
-        ev.pot = P.p.pot[t0 + lane];
-        ev.potf = P.p.potf[t0 + lane];
-      }
-      ev.ox = P.ox; ev.oy = P.oy; ev.oz = P.oz;
-      ev.g = &g;
-      ev.n_pp = 0; ev.n_pc = 0;
-      ev.record = (P.mode == 2 && tc == 0);
-      ev.nlist = 0;
-      ev.lbase = ev.record ? P.list_off[b - P.b_begin] : 0;
-      ev.lnode = P.list_node;
-      ev.lkind = P.list_kind;
-      if (!(P.bfs ? walk_bucket_bfs(P.walk, P.nnodes, g, P.ox, P.oy, P.oz, queues[wid], kBfsQueue, lane, ev,
-                                    opens, P.status)
-                  : walk_bucket(P.walk, P.nnodes, g, P.ox, P.oy, P.oz, stacks[wid], lane, ev, opens, P.status)) &&
-          lane == 0)
-        atomicOr(P.status, kErrStack);
+      ev.begin(P, W, t0, nt, lane, P.mode == 2 && tc == 0 ? P.list_off[b - P.b_begin] : -1);
+      if (!walk_one<kBfs>(P, W, lane, ev, opens) && lane == 0) atomicOr(P.status, kErrStack);
+      ev.flush();
+      ev.store(t0);
       if (tc == 0) c_open += opens;
-      if (lane < nt) {
-        int i = t0 + lane;
-        P.p.ax[i] = ev.ax;
-        P.p.ay[i] = ev.ay;
-        P.p.az[i] = ev.az;
-        P.p.pot[i] = ev.pot;
-        P.p.potf[i] = ev.potf;
-      }
-      c_pp += ev.n_pp;
-      c_pc += ev.n_pc;
+      const unsigned long long pp = (unsigned long long)ev.nsrc * (unsigned long long)nt;
+      const unsigned long long pc = (unsigned long long)ev.npc * (unsigned long long)nt;
+      c_pp += pp;
+      c_pc += pc;
       if (P.bucket_work && lane == 0) {  // this chunk's interactions, added to the bucket's
-        unsigned long long wk = ev.n_pp + ev.n_pc;
+        unsigned long long wk = pp + pc;
         if (tc > 0 || P.accumulate) wk += P.bucket_work[b];
         P.bucket_work[b] = wk;
       }
@@ -505,9 +680,9 @@ __global__ void __launch_bounds__(kTravWarps * 32) traverse_f64(TravParams P, co
 // Frozen-list replay: evaluates each bucket's recorded interaction list (in the
 // recorded order, i.e. the walk's) with the FP64 evaluator, without walking.
 // Used to differentiate the force pass for a fixed interaction list.
-__global__ void __launch_bounds__(kTravWarps * 32) replay_f64(TravParams P) {
-  __shared__ double stage[kTravWarps][5 * 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+__global__ void __launch_bounds__(kTravWarps * 32, 5) replay_f64(TravParams P) {
+  __shared__ F64Warp warps[kTravWarps];
+  const int lane = threadIdx.x & 31;
   while (true) {
     unsigned bi = 0;
     if (lane == 0) bi = atomicAdd(P.work, 1u);
@@ -520,28 +695,7 @@ __global__ void __launch_bounds__(kTravWarps * 32) replay_f64(TravParams P) {
     for (int tc = 0; tc < ntot; tc += 32) {
       const int t0 = tbase + tc, nt = min(32, ntot - tc);
       F64Eval ev;
-      ev.p = &P.p;
-      ev.walk = P.walk;
-      ev.quad = P.quad;
-      ev.stage = stage[wid];
-      ev.lane = lane;
-      ev.nt = nt;
-      ev.xi = ev.yi = ev.zi = ev.si = 0.0;
-      if (lane < nt) {
-        ev.xi = P.p.x[t0 + lane];
-        ev.yi = P.p.y[t0 + lane];
-        ev.zi = P.p.z[t0 + lane];
-        ev.si = P.p.soft[t0 + lane];
-      }
-      ev.ax = ev.ay = ev.az = ev.pot = ev.potf = 0.0;
-      ev.ox = P.ox; ev.oy = P.oy; ev.oz = P.oz;
-      ev.g = nullptr;
-      ev.n_pp = 0; ev.n_pc = 0;
-      ev.record = 0;
-      ev.nlist = 0;
-      ev.lbase = 0;
-      ev.lnode = nullptr;
-      ev.lkind = nullptr;
+      ev.begin(P, warps[threadIdx.x >> 5], t0, nt, lane, -1);
       for (int64_t e = e0; e < e1; e++) {
         const int node = P.list_node[e];
         const int kind = P.list_kind[e];
@@ -549,17 +703,10 @@ __global__ void __launch_bounds__(kTravWarps * 32) replay_f64(TravParams P) {
           if (lane == 0) atomicOr(P.status, kErrCapacity);
           continue;
         }
-        if (kind == 0) ev.p2p(node);
-        else ev.p2c(node, kind == 2);
+        ev.push(node, kind == 0 ? kEntLeaf : kind == 2 ? kEntMono : kEntQuad);
       }
-      if (lane < nt) {
-        const int i = t0 + lane;
-        P.p.ax[i] = ev.ax;
-        P.p.ay[i] = ev.ay;
-        P.p.az[i] = ev.az;
-        P.p.pot[i] = ev.pot;
-        P.p.potf[i] = ev.potf;
-      }
+      ev.flush();
+      ev.store(t0);
     }
   }
 }
@@ -658,7 +805,8 @@ void launch_finalize(Nodes nd, int64_t nnodes, double gfac, int want_f32, cudaSt
 }
 void launch_traverse_f64(const TravParams& P, const Mom* mom, int grid, cudaStream_t st) {
   note_launch();
-  traverse_f64<<<grid, kTravWarps * 32, 0, st>>>(P, mom);
+  if (P.bfs) traverse_f64<true><<<grid, kTravWarps * 32, 0, st>>>(P, mom);
+  else traverse_f64<false><<<grid, kTravWarps * 32, 0, st>>>(P, mom);
 }
 void launch_replay_f64(const TravParams& P, int grid, cudaStream_t st) {
   note_launch();

@@ -13,10 +13,11 @@
 // node is opened, lanes 0..7 classify its 8 contiguous children in parallel
 // (64-byte WalkRec each, one coalesced 512-byte read) into P2P / P2C
 // (quadrupole) / P2C (softened monopole, GravityVisitor::openSoftening) /
-// open; four ballots give the per-child masks.  The terminal children before
-// the first opened child are handed to the evaluator in child order, the
-// remaining masks are pushed on a per-warp shared-memory frame stack, and the
-// walk descends.  Every decision is warp-uniform.  The tests use
+// open; four ballots give the per-child masks (a frame's bits: P2P 0-7, P2C
+// quadrupole 8-15, P2C monopole 16-23, open 24-31).  The terminal children
+// before the first opened child are handed to the evaluator in child order, the
+// rest waits on a per-warp shared-memory stack (walk_preorder).  Every decision
+// is warp-uniform.  The tests use
 // __dadd_rn/__dmul_rn so that they evaluate identically (no FMA contraction)
 // in every translation unit: all traversal forms see the same interactions.
 #pragma once
@@ -25,17 +26,12 @@
 
 namespace pt {
 
-constexpr int kWalkStack = 32;
+constexpr int kWalkStack = 128;  // pre-order walk: at most 4 entries more per level than it takes off
 constexpr int kBfsQueue = 512;  // pending sibling frames of a breadth-first walk
 constexpr unsigned kFull = 0xffffffffu;
 
 // Child classes.
 enum : int { kClsNone = 0, kClsP2P = 1, kClsQuad = 2, kClsOpen = 3, kClsMono = 4 };
-
-struct WalkFrame {
-  int32_t c0;     // index of child 0
-  uint32_t bits;  // P2P (0-7) | P2C quadrupole (8-15) | P2C monopole (16-23) | open (24-31)
-};
 
 // Squared gap between a box and a point as Space::intersect of the
 // reference's utility submodule accumulates it (stand-in convention: per axis
@@ -189,53 +185,105 @@ __device__ __forceinline__ uint32_t classify_children(const WalkRec* __restrict_
   return pp | (pq << 8) | (pm << 16) | (op << 24);
 }
 
-// Walk the tree for one bucket; ev.p2p(node), ev.p2c(node, mono) are called in
-// the reference's per-bucket order.  Returns false on stack overflow.
-template <class Eval>
-__device__ __forceinline__ bool walk_bucket(const WalkRec* __restrict__ walk, int64_t nnodes, const BucketGeom& g,
-                                            double ox, double oy, double oz, WalkFrame* stack, int lane, Eval& ev,
-                                            unsigned long long& n_open, unsigned* status) {
+// One stack entry of the pre-order walk: terminals of the frame above that come
+// first (pc0, pbits), then a classified frame (its children from c0 on).
+struct __align__(16) WalkSeg {
+  int32_t pc0;
+  uint32_t pbits;
+  int32_t c0;
+  uint32_t bits;
+};
+
+// The classification fields of node >= 1 from its sibling block.
+__device__ __forceinline__ WalkRec load_sibling(const double2* __restrict__ walks, int64_t node) {
+  const double2* sb = walks + walk_sib_index(node, 0);
+  const double2 v0 = sb[0], v1 = sb[8], v2 = sb[16];
+  WalkRec r;
+  r.cm[0] = v0.x;
+  r.cm[1] = v0.y;
+  r.cm[2] = v1.x;
+  r.orsq = v1.y;
+  r.soft = v2.x;
+  const int tc = __double2hiint(v2.y);
+  r.first_child = __double2loint(v2.y);
+  r.type = tc & 7;
+  r.count = tc >> 3;
+  return r;
+}
+
+// Walk the tree for one bucket in the reference's per-bucket order (pre-order).
+// sink.emit(c0, pp, pq, pm) receives runs of terminals among the children from
+// c0 on, in child order.  A popped frame's first four opened children are
+// classified together (lanes 8e .. 8e + 7 take the children of the e-th): all of
+// them would be classified later anyway, so the tests are the same, the steps
+// fewer.  The classified frames wait on the stack, each behind the terminals
+// that precede it in its parent.  Returns false on stack overflow.
+template <class Sink>
+__device__ __forceinline__ bool walk_preorder(const WalkRec* __restrict__ walk, const double2* __restrict__ walks,
+                                              int64_t nnodes, const BucketGeom& g, double ox, double oy, double oz,
+                                              WalkSeg* stack, int lane, Sink& sink, unsigned long long& n_open,
+                                              unsigned* status) {
   int c0 = 0;  // the root, tested as a one-child frame
   uint32_t bits = classify_children(walk, nnodes, 0, 1, g, ox, oy, oz, lane, n_open, status);
   int sp = 0;
+  const int e = lane >> 3, c = lane & 7;
   while (true) {
-    if (bits == 0) {
-      if (sp == 0) break;
-      --sp;
-      WalkFrame f = stack[sp];
-      c0 = f.c0;
-      bits = f.bits;
-      continue;
-    }
-    uint32_t pp = bits & 0xffu, pq = (bits >> 8) & 0xffu, pm = (bits >> 16) & 0xffu, op = bits >> 24;
-    int fo = op ? (__ffs(op) - 1) : 8;
-    uint32_t low = (1u << fo) - 1u;
-    uint32_t run = (pp | pq | pm) & low;
-    while (run) {
-      int k = __ffs(run) - 1;
-      run &= run - 1u;
-      if ((pp >> k) & 1u) ev.p2p(c0 + k);
-      else ev.p2c(c0 + k, ((pm >> k) & 1u) != 0);
-    }
-    pp &= ~low;
-    pq &= ~low;
-    pm &= ~low;
-    if (fo < 8) {
-      op &= ~(1u << fo);
-      uint32_t rem = pp | (pq << 8) | (pm << 16) | (op << 24);
-      if (rem) {
-        if (sp >= kWalkStack) return false;
-        __syncwarp();
-        if (lane == 0) stack[sp] = WalkFrame{c0, rem};
-        __syncwarp();
+    const uint32_t op = bits >> 24;
+    const uint32_t low = op ? (op & (0u - op)) - 1u : 0xffu;  // the children before the first opened one
+    if (bits & (low * 0x00010101u)) sink.emit(c0, bits & low, (bits >> 8) & low, (bits >> 16) & low);
+    if (op) {
+      // the e-th opened child of this frame, and the last of the four taken
+      uint32_t o = op;
+      for (int q = 0; q < e; q++) o &= o - 1u;
+      const int k = o ? __ffs(o) - 1 : 8;
+      const int klast = __reduce_max_sync(kFull, o ? k : -1);
+      const int m = min(4, __popc(op));
+      int fc = -1, code = kClsNone;
+      bool internal = false;
+      if (o) {
+        const int64_t parent = (int64_t)c0 + k;
+        fc = parent == 0 ? walk[0].first_child : __double2loint(walks[walk_sib_index(parent, 2)].y);
+        const int64_t idx = (int64_t)fc + c;
+        if (fc < 1 || idx >= nnodes) {
+          atomicOr(status, kErrCapacity);
+        } else {
+          const WalkRec w = load_sibling(walks, idx);
+          internal = (w.type == kTypeInternal);
+          code = classify_node(w, g, ox, oy, oz);
+        }
+      }
+      const unsigned pp = __ballot_sync(kFull, code == kClsP2P), pq = __ballot_sync(kFull, code == kClsQuad);
+      const unsigned pm = __ballot_sync(kFull, code == kClsMono), po = __ballot_sync(kFull, code == kClsOpen);
+      n_open += (unsigned long long)__popc(__ballot_sync(kFull, internal));
+      // what is left of this frame behind the children taken, then the later
+      // children's frames, each behind the terminals since the one before it
+      const uint32_t above = 0xffu & ~((2u << klast) - 1u);
+      const uint32_t rest = bits & (above * 0x01010101u);
+      if (sp + m + 1 > kWalkStack) return false;
+      __syncwarp();
+      if (rest) {
+        if (lane == 0) stack[sp] = WalkSeg{0, 0u, c0, rest};
         ++sp;
       }
-      int nc0 = walk[c0 + fo].first_child;
-      c0 = nc0;
-      bits = classify_children(walk, nnodes, nc0, 8, g, ox, oy, oz, lane, n_open, status);
-    } else {
-      bits = 0;
+      if (c == 0 && e >= 1 && e < m) {
+        const int kp = 31 - __clz(op & ((1u << k) - 1u));  // the opened child before this one
+        const uint32_t between = ((1u << k) - 1u) & ~((2u << kp) - 1u);
+        const uint32_t b = ((pp >> (8 * e)) & 0xffu) | (((pq >> (8 * e)) & 0xffu) << 8) |
+                           (((pm >> (8 * e)) & 0xffu) << 16) | (((po >> (8 * e)) & 0xffu) << 24);
+        stack[sp + m - 1 - e] = WalkSeg{c0, bits & (between * 0x00010101u), fc, b};
+      }
+      sp += m - 1;
+      __syncwarp();
+      c0 = __shfl_sync(kFull, fc, 0);
+      bits = (pp & 0xffu) | ((pq & 0xffu) << 8) | ((pm & 0xffu) << 16) | ((po & 0xffu) << 24);
+      continue;
     }
+    if (sp == 0) break;
+    --sp;
+    const WalkSeg f = stack[sp];
+    if (f.pbits) sink.emit(f.pc0, f.pbits & 0xffu, (f.pbits >> 8) & 0xffu, (f.pbits >> 16) & 0xffu);
+    c0 = f.c0;
+    bits = f.bits;
   }
   return true;
 }
@@ -246,10 +294,10 @@ __device__ __forceinline__ bool walk_bucket(const WalkRec* __restrict__ walk, in
 // children of an opened node -- processed in child order, each opened child
 // queuing its own frame at the back.  queue is a per-warp ring of qcap frames
 // (first-child indices).  Returns false if the ring overflows.
-template <class Eval>
+template <class Sink>
 __device__ __forceinline__ bool walk_bucket_bfs(const WalkRec* __restrict__ walk, int64_t nnodes,
                                                 const BucketGeom& g, double ox, double oy, double oz,
-                                                int32_t* queue, int qcap, int lane, Eval& ev,
+                                                int32_t* queue, int qcap, int lane, Sink& sink,
                                                 unsigned long long& n_open, unsigned* status) {
   int c0 = 0;  // the root, as a one-child frame
   uint32_t bits = classify_children(walk, nnodes, 0, 1, g, ox, oy, oz, lane, n_open, status);
@@ -257,20 +305,19 @@ __device__ __forceinline__ bool walk_bucket_bfs(const WalkRec* __restrict__ walk
   while (true) {
     const uint32_t pp = bits & 0xffu, pq = (bits >> 8) & 0xffu, pm = (bits >> 16) & 0xffu, op = bits >> 24;
     uint32_t all = pp | pq | pm | op;
-    while (all) {
-      const int k = __ffs(all) - 1;
-      all &= all - 1u;
-      if ((pp >> k) & 1u) {
-        ev.p2p(c0 + k);
-      } else if (((pq | pm) >> k) & 1u) {
-        ev.p2c(c0 + k, ((pm >> k) & 1u) != 0);
-      } else {
+    while (all) {  // runs of terminals between the opened children
+      const uint32_t nxt = all & op, first = nxt & (0u - nxt);
+      const uint32_t run = first ? all & (first - 1u) : all;
+      if (run) sink.emit(c0, pp & run, pq & run, pm & run);
+      all &= ~run;
+      if (first) {
         if (tail - head >= qcap) return false;
-        const int fc = walk[c0 + k].first_child;
+        const int fc = walk[c0 + __ffs(first) - 1].first_child;
         __syncwarp();
         if (lane == 0) queue[tail % qcap] = fc;
         __syncwarp();
         ++tail;
+        all &= ~first;
       }
     }
     if (head == tail) break;
@@ -281,23 +328,10 @@ __device__ __forceinline__ bool walk_bucket_bfs(const WalkRec* __restrict__ walk
   return true;
 }
 
-// Evaluator that only records / counts the interaction list of a bucket.
-// Stored kinds: 0 leaf() P2P, 1 node() quadrupole, 2 node() softened monopole.
-struct ListRecorder {
-  int lane;
-  int mode;  // 1 count, 2 record
+// Sink that only counts the interaction list of a bucket.
+struct ListCounter {
   int64_t n;
-  int64_t base;
-  int32_t* node_out;
-  int8_t* kind_out;
-  __device__ void p2p(int node) {
-    if (mode == 2 && lane == 0) { node_out[base + n] = node; kind_out[base + n] = 0; }
-    ++n;
-  }
-  __device__ void p2c(int node, bool mono) {
-    if (mode == 2 && lane == 0) { node_out[base + n] = node; kind_out[base + n] = mono ? 2 : 1; }
-    ++n;
-  }
+  __device__ void emit(int, uint32_t pp, uint32_t pq, uint32_t pm) { n += __popc(pp | pq | pm); }
 };
 
 }  // namespace pt
