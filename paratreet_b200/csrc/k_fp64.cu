@@ -132,7 +132,8 @@ __device__ __forceinline__ void mom_radius(Mom& q, int count) {
   }
 }
 
-__global__ void __launch_bounds__(256) leaf_moments(Nodes nd, int64_t nnodes, Particles p) {
+__global__ void __launch_bounds__(256) leaf_moments(Nodes nd, int64_t nnodes, Particles p,
+                                                    double4* __restrict__ src) {
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (i >= nnodes) return;
   Mom q;
@@ -141,8 +142,9 @@ __global__ void __launch_bounds__(256) leaf_moments(Nodes nd, int64_t nnodes, Pa
   if (nd.type[i] == kTypeLeaf) {
     int s0 = nd.pstart[i], sn = nd.pcount[i];
     for (int j = s0; j < s0 + sn; j++) {
-      double px = p.x[j], py = p.y[j], pz = p.z[j];
-      mom_add_particle(q, px, py, pz, p.m[j], p.soft[j]);
+      double px = p.x[j], py = p.y[j], pz = p.z[j], pm = p.m[j];
+      mom_add_particle(q, px, py, pz, pm, p.soft[j]);
+      if (src) src[j] = make_double4(px, py, pz, pm);  // the FP64 evaluation's source records
       if (px < q.lo[0]) q.lo[0] = px;
       if (py < q.lo[1]) q.lo[1] = py;
       if (pz < q.lo[2]) q.lo[2] = pz;
@@ -303,13 +305,13 @@ __global__ void __launch_bounds__(256) finalize_records(Nodes nd, int64_t nnodes
 //          of similar length; then quadrupole, then monopole nodes.
 //   sums   the terms wait in shared memory as [entry][target][ax ay az pot]; lane
 //          4 t + c adds component c of target t over the entries, in order.
-// With more than 16 targets (one group) each lane keeps its target's sums itself.
 // Bound by the FP64 pipe (45-80 operations per term, with the IEEE square roots
 // and divisions) and by latency.  With one lane per target and nothing else (a
 // bucket holds 4-10 particles, so 4-10 of 32 lanes worked) the 2^20 mixture took
-// 84.8 ms and the 4096-particle Plummer 1.01 ms; this takes 28.6 and 0.74 ms.
+// 84.8 ms and the 4096-particle Plummer 1.01 ms; this takes 27.6 and 0.6 ms.
 constexpr int kTravWarps = 4;
 constexpr int kF64Entries = 64;
+constexpr int kF64Ctas = 4;  // per SM: 128 registers; 5, 6 and 7 spill (35.8, 44 and 50 against 28.3 ms)
 constexpr int kF64Terms = 256;  // (entry, target) terms held in shared memory
 enum : int { kEntLeaf = 0, kEntQuad = 1, kEntMono = 2 };
 
@@ -320,16 +322,26 @@ struct F64Warp {
     WalkSeg stack[kWalkStack];
     int32_t queue[kBfsQueue];  // basic-down order
   };
-  int32_t ent[kF64Entries];      // node | kind << 30, walk order
-  uint8_t order[kF64Entries];    // entries by kind and size
+  int32_t ent[kF64Entries];    // node | kind << 30, walk order
+  int2 range[kF64Entries];     // a leaf's first particle and count
+  uint8_t order[kF64Entries];  // entries by kind and size
 };
+
+// A particle's (x, y, z, m) record in one 256-bit load.
+__device__ __forceinline__ double4 ld_src(const double4* p) {
+  double4 v;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
 
 struct F64Eval {
   const TravParams* P;
   F64Warp* w;
   int lane, nt, grp, G, cap, n;
   double xi, yi, zi, si;
-  double s[5];  // G > 1: sums of (target, component) pairs lane and lane + 32, then their pot; else ax ay az pot potf
+  // sums of the (target, component) pairs lane + 32 h (4 t + c), and the
+  // potential of those with c = 3
+  double s[4], sp[4];
   unsigned nsrc, npc;
   int64_t lat;  // where the next list entry goes (recording)
   bool record;
@@ -342,66 +354,49 @@ struct F64Eval {
     G = 32 / nt;
     grp = lane / nt;
     cap = min(kF64Entries, kF64Terms / nt);
-    if (G == 1) cap = kF64Entries;
     n = 0;
     nsrc = npc = 0;
     record = rec >= 0;
     lat = rec;
     xi = yi = zi = si = 0.0;
-    const int t = lane % nt;
     if (grp < G) {
-      xi = Q.p.x[t0 + t];
-      yi = Q.p.y[t0 + t];
-      zi = Q.p.z[t0 + t];
-      si = Q.p.soft[t0 + t];
+      const int i = t0 + lane % nt;
+      xi = Q.p.x[i];
+      yi = Q.p.y[i];
+      zi = Q.p.z[i];
+      si = Q.p.soft[i];
     }
 #pragma unroll
-    for (int k = 0; k < 5; k++) s[k] = 0.0;
-    if (!Q.accumulate) return;  // later replica walks continue each particle's sums
-    if (G == 1) {
-      if (lane < nt) {
-        const int i = t0 + lane;
-        s[0] = Q.p.ax[i]; s[1] = Q.p.ay[i]; s[2] = Q.p.az[i]; s[3] = Q.p.pot[i]; s[4] = Q.p.potf[i];
-      }
-    } else {
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int p = lane + 32 * h;
-        if (p < 4 * nt) {
-          const int i = t0 + (p >> 2), c = p & 3;
-          s[h] = c == 0 ? Q.p.ax[i] : c == 1 ? Q.p.ay[i] : c == 2 ? Q.p.az[i] : Q.p.potf[i];
-          if (c == 3) s[2 + h] = Q.p.pot[i];
-        }
+    for (int h = 0; h < 4; h++) {
+      s[h] = sp[h] = 0.0;
+      const int p = lane + 32 * h;
+      if (Q.accumulate && p < 4 * nt) {  // later replica walks continue each particle's sums
+        const int i = t0 + (p >> 2), c = p & 3;
+        s[h] = c == 0 ? Q.p.ax[i] : c == 1 ? Q.p.ay[i] : c == 2 ? Q.p.az[i] : Q.p.potf[i];
+        if (c == 3) sp[h] = Q.p.pot[i];
       }
     }
   }
 
   __device__ void store(int t0) {
     const Particles& q = P->p;
-    if (G == 1) {
-      if (lane < nt) {
-        const int i = t0 + lane;
-        q.ax[i] = s[0]; q.ay[i] = s[1]; q.az[i] = s[2]; q.pot[i] = s[3]; q.potf[i] = s[4];
-      }
-      return;
-    }
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
+    for (int h = 0; h < 4; h++) {
       const int p = lane + 32 * h;
       if (p < 4 * nt) {
         const int i = t0 + (p >> 2), c = p & 3;
         double* const out = c == 0 ? q.ax : c == 1 ? q.ay : c == 2 ? q.az : q.potf;
         out[i] = s[h];
-        if (c == 3) q.pot[i] = s[2 + h];
+        if (c == 3) q.pot[i] = sp[h];
       }
     }
   }
 
   // Runs of terminals from the walk: children c0 + k, in child order.
-  __device__ void emit(int c0, uint32_t pp, uint32_t pq, uint32_t pm) {
+  __device__ void emit(int c0, uint32_t pp, uint32_t pq, uint32_t pm, bool last) {
     const uint32_t run = pp | pq | pm;
     const int m = __popc(run);
-    if (n + m > cap) flush();
+    if (n + m > cap || last) flush();
     if (lane < 8 && ((run >> lane) & 1u)) {
       const int kind = ((pp >> lane) & 1u) ? kEntLeaf : ((pq >> lane) & 1u) ? kEntQuad : kEntMono;
       const int at = __popc(run & ((1u << lane) - 1u));
@@ -422,34 +417,41 @@ struct F64Eval {
     ++n;
   }
 
-  // GravityVisitor::leaf, examples/GravityVisitor.h:144-160
-  __device__ void leaf_term(int node, double v[4]) const {
-    const int s0 = P->walk[node].pstart, sn = P->walk[node].pcount;
-    const Particles& q = P->p;
+  // GravityVisitor::leaf, examples/GravityVisitor.h:144-160, over sn particles
+  // from s0 on
+  __device__ __forceinline__ void leaf_term(int s0, int sn, double v[4]) const {
     double pax = 0.0, pay = 0.0, paz = 0.0, ppf = 0.0;
-    double nx = q.x[s0], ny = q.y[s0], nz = q.z[s0], nm = q.m[s0], ns = q.soft[s0];
-    for (int j = 1; j <= sn; j++) {
-      const double xs = nx, ys = ny, zs = nz, ms = nm, ss = ns;
-      if (j < sn) {  // the next source, ahead of this one's chain of divisions
-        nx = q.x[s0 + j];
-        ny = q.y[s0 + j];
-        nz = q.z[s0 + j];
-        nm = q.m[s0 + j];
-        ns = q.soft[s0 + j];
+    // two sources at a time: their chains of square root and division overlap,
+    // the sums stay in particle order
+    for (int j = 0; j < sn; j += 2) {
+      const double4* rec = P->src + s0 + j;
+      const double* so = P->p.soft + s0 + j;
+      const bool two = j + 1 < sn;
+      const double4 p = ld_src(rec), q = ld_src(two ? rec + 1 : rec);
+      const double ph = so[0] + si, qh = so[two ? 1 : 0] + si;
+      const double px = (p.x + P->ox) - xi, py = (p.y + P->oy) - yi, pz = (p.z + P->oz) - zi;
+      const double qx = (q.x + P->ox) - xi, qy = (q.y + P->oy) - yi, qz = (q.z + P->oz) - zi;
+      const double p2 = px * px + py * py + pz * pz, q2 = qx * qx + qy * qy + qz * qz;
+      const double pr = sqrt(p2), qr = sqrt(q2);
+      double pa = 1.0 / pr, qa = 1.0 / qr;
+      double pb = pa * pa * pa, qb = qa * qa * qa;
+      if (pr < ph || qr < qh) {
+        if (p2 != 0) spline_f64(p2, ph, pa, pb);
+        if (q2 != 0) spline_f64(q2, qh, qa, qb);
       }
-      const double dx = (xs + P->ox) - xi;
-      const double dy = (ys + P->oy) - yi;
-      const double dz = (zs + P->oz) - zi;
-      const double rsq = dx * dx + dy * dy + dz * dz;
-      const double twoh = ss + si;
-      if (rsq != 0) {
-        double a, b;
-        spline_f64(rsq, twoh, a, b);
-        const double bm = b * ms;
-        pax += dx * bm;
-        pay += dy * bm;
-        paz += dz * bm;
-        ppf += -ms * a;
+      if (p2 != 0) {
+        const double bm = pb * p.w;
+        pax += px * bm;
+        pay += py * bm;
+        paz += pz * bm;
+        ppf += -p.w * pa;
+      }
+      if (q2 != 0 && two) {
+        const double bm = qb * q.w;
+        pax += qx * bm;
+        pay += qy * bm;
+        paz += qz * bm;
+        ppf += -q.w * qa;
       }
     }
     v[0] = pax;
@@ -514,9 +516,10 @@ struct F64Eval {
       if (e < n) {
         const int x = w->ent[e], kind = (unsigned)x >> 30;
         if (kind == kEntLeaf) {
-          const int sn = P->walk[x].pcount;
-          src += (unsigned)sn;
-          key[h] = 1 + sn;
+          const int4 r = *reinterpret_cast<const int4*>(&P->walk[x].count);  // count, pstart, pcount, pad
+          w->range[e] = make_int2(r.y, r.z);
+          src += (unsigned)r.z;
+          key[h] = 1 + r.z;
         } else {
           key[h] = kind == kEntQuad ? 1 : 0;
         }
@@ -527,25 +530,6 @@ struct F64Eval {
     const int nleaf = n - nquad - nmono;
     nsrc += __reduce_add_sync(kFull, src);
     npc += (unsigned)(nquad + nmono);
-    if (G == 1) {
-      for (int e = 0; e < n; e++) {
-        const int x = w->ent[e], kind = (unsigned)x >> 30, node = x & 0x3fffffff;
-        if (lane < nt) {
-          double v[4];
-          if (kind == kEntLeaf) leaf_term(node, v);
-          else if (kind == kEntQuad) quad_term(node, v);
-          else mono_term(node, v);
-          s[0] += v[0];
-          s[1] += v[1];
-          s[2] += v[2];
-          if (kind == kEntQuad) s[3] += v[3];
-          s[4] += v[3];
-        }
-      }
-      n = 0;
-      __syncwarp();
-      return;
-    }
     // entries by descending key: one round per distinct key
     {
       const unsigned lt = (1u << lane) - 1u;
@@ -572,7 +556,7 @@ struct F64Eval {
       for (; k < nleaf; k += G) {
         const int e = w->order[k];
         double v[4];
-        leaf_term(w->ent[e] & 0x3fffffff, v);
+        leaf_term(w->range[e].x, w->range[e].y, v);
         double2* o = reinterpret_cast<double2*>(w->term + 4 * (e * nt + t));
         o[0] = make_double2(v[0], v[1]);
         o[1] = make_double2(v[2], v[3]);
@@ -590,17 +574,18 @@ struct F64Eval {
     __syncwarp();
     const int per = 4 * nt;
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
+    for (int h = 0; h < 4; h++) {
       const int p = lane + 32 * h;
-      if (p < per) {
-        double a = s[h], b = s[2 + h];
-        for (int e = 0; e < n; e++) {
-          const double v = w->term[e * per + p];
-          a += v;
-          if (((unsigned)w->ent[e] >> 30) == kEntQuad) b += v;  // pot: quadrupole node() terms only
+      if (32 * h < per && p < per) {
+        double a = s[h], b = sp[h];
+        const double* v = w->term + p;
+        for (int e = 0; e < n; e++, v += per) {
+          const double t = *v;
+          a += t;
+          if (((unsigned)w->ent[e] >> 30) == kEntQuad) b += t;  // pot: quadrupole node() terms only
         }
         s[h] = a;
-        s[2 + h] = b;
+        sp[h] = b;
       }
     }
     n = 0;
@@ -619,17 +604,14 @@ __device__ __forceinline__ bool walk_one(const TravParams& P, F64Warp& W, int la
     return walk_preorder(P.walk, P.walks, P.nnodes, W.geom, P.ox, P.oy, P.oz, W.stack, lane, sink, opens, P.status);
 }
 
-// CTAs per SM: 42 KB of shared memory each
 template <bool kBfs>
-__global__ void __launch_bounds__(kTravWarps * 32, 5) traverse_f64(TravParams P, const Mom* __restrict__ mom) {
+__global__ void __launch_bounds__(kTravWarps * 32, kF64Ctas) traverse_f64(TravParams P, const Mom* __restrict__ mom) {
   __shared__ F64Warp warps[kTravWarps];
   F64Warp& W = warps[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   unsigned long long c_pp = 0, c_pc = 0, c_open = 0;
   while (true) {
-    unsigned bi = 0;
-    if (lane == 0) bi = atomicAdd(P.work, 1u);
-    bi = __shfl_sync(kFull, bi, 0);
+    const unsigned bi = grab_bucket(P.work, P.smq, P.batch, lane);
     int64_t b = P.b_begin + (int64_t)bi;
     if (b >= P.b_end) break;
     const int tnode = P.buckets[b];
@@ -656,7 +638,6 @@ __global__ void __launch_bounds__(kTravWarps * 32, 5) traverse_f64(TravParams P,
       F64Eval ev;
       ev.begin(P, W, t0, nt, lane, P.mode == 2 && tc == 0 ? P.list_off[b - P.b_begin] : -1);
       if (!walk_one<kBfs>(P, W, lane, ev, opens) && lane == 0) atomicOr(P.status, kErrStack);
-      ev.flush();
       ev.store(t0);
       if (tc == 0) c_open += opens;
       const unsigned long long pp = (unsigned long long)ev.nsrc * (unsigned long long)nt;
@@ -680,13 +661,11 @@ __global__ void __launch_bounds__(kTravWarps * 32, 5) traverse_f64(TravParams P,
 // Frozen-list replay: evaluates each bucket's recorded interaction list (in the
 // recorded order, i.e. the walk's) with the FP64 evaluator, without walking.
 // Used to differentiate the force pass for a fixed interaction list.
-__global__ void __launch_bounds__(kTravWarps * 32, 5) replay_f64(TravParams P) {
+__global__ void __launch_bounds__(kTravWarps * 32, kF64Ctas) replay_f64(TravParams P) {
   __shared__ F64Warp warps[kTravWarps];
   const int lane = threadIdx.x & 31;
   while (true) {
-    unsigned bi = 0;
-    if (lane == 0) bi = atomicAdd(P.work, 1u);
-    bi = __shfl_sync(kFull, bi, 0);
+    const unsigned bi = grab_bucket(P.work, P.smq, P.batch, lane);
     const int64_t b = P.b_begin + (int64_t)bi;
     if (b >= P.b_end) break;
     const int tnode = P.buckets[b];
@@ -794,8 +773,8 @@ __global__ void __launch_bounds__(kDirTile) direct_sum_f64(const double* __restr
 // ---------------------------------------------------------------- launchers
 static inline unsigned blocks_for(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
 
-void launch_leaf_moments(Nodes nd, int64_t nnodes, Particles p, cudaStream_t st) {
-  if (nnodes > 0) { note_launch(); leaf_moments<<<blocks_for(nnodes), 256, 0, st>>>(nd, nnodes, p); }
+void launch_leaf_moments(Nodes nd, int64_t nnodes, Particles p, double4* src, cudaStream_t st) {
+  if (nnodes > 0) { note_launch(); leaf_moments<<<blocks_for(nnodes), 256, 0, st>>>(nd, nnodes, p, src); }
 }
 void launch_upward(Nodes nd, int64_t ninternal, cudaStream_t st) {
   if (ninternal > 0) { note_launch(); upward_climb<<<blocks_for(8 * ninternal, 128), 128, 0, st>>>(nd, ninternal); }

@@ -83,45 +83,6 @@ __device__ __forceinline__ bool ensure_region(Region& r, unsigned long long* cur
   return true;
 }
 
-#ifndef PT_SMQ_BATCH
-#define PT_SMQ_BATCH 32
-#endif
-// The next bucket index of a warp (lane 0 grabs, all lanes receive it).  With
-// smq, the warps of one SM take consecutive buckets from a batch of
-// PT_SMQ_BATCH that the SM's queue holds, so the warps resident on an SM work
-// on neighbouring buckets: their targets, results and most of their node
-// records share cache lines.  (On the periodic 256^3 lattice pass, whose outer
-// replica walks leave little work per bucket besides loading its targets and
-// adding to its results, this measured 239.5 -> 214.4 ms; the Plummer pass at
-// N = 2^24 is unchanged.)  A queue word is (batch start + 1) << 32 | next
-// index; zero = no batch yet.
-// The warp that draws index 0 of an empty queue, or the index one past the
-// batch, takes a new batch from the global counter (keeping its first bucket);
-// warps that draw past the batch meanwhile take single buckets.
-__device__ __forceinline__ unsigned grab_bucket(unsigned* work, unsigned long long* smq, int lane) {
-  unsigned bi = 0;
-  if (lane == 0) {
-    if (smq == nullptr) {
-      bi = atomicAdd(work, 1u);
-    } else {
-      unsigned sm;
-      asm volatile("mov.u32 %0, %%smid;" : "=r"(sm));
-      unsigned long long* q = smq + (sm & 255u);
-      const unsigned long long old = atomicAdd(q, 1ull);
-      const unsigned hi = (unsigned)(old >> 32), idx = (unsigned)old;
-      if (hi != 0u && idx < (unsigned)PT_SMQ_BATCH) {
-        bi = hi - 1u + idx;
-      } else if (hi == 0u ? idx == 0u : idx == (unsigned)PT_SMQ_BATCH) {
-        bi = atomicAdd(work, (unsigned)PT_SMQ_BATCH);
-        atomicExch(q, ((unsigned long long)(bi + 1u) << 32) | 1ull);
-      } else {
-        bi = atomicAdd(work, 1u);
-      }
-    }
-  }
-  return __shfl_sync(kFull, bi, 0);
-}
-
 // Room for n more entries of the bucket's list, which occupies [start,
 // r.cur) of the warp's region: when they do not fit, the list so far moves to
 // a new region of at least twice its new length.  False only if the pool is
@@ -167,7 +128,7 @@ __global__ void __launch_bounds__(kWlWarps * 32, PT_WALK_MINB) walk_lists(TravPa
   const int nn32 = (int)min(P.nnodes, (int64_t)INT_MAX);  // node indices are 32-bit
   PROF_START(w);
   while (true) {
-    const unsigned bi = grab_bucket(P.work, P.smq, lane);
+    const unsigned bi = grab_bucket(P.work, P.smq, P.batch, lane);
     const int64_t b = P.b_begin + (int64_t)bi;
     if (b >= P.b_end) break;
     const int64_t lb = b - P.b_begin;
@@ -503,7 +464,7 @@ __device__ __forceinline__ void ev_finish(W& w, const Kahan4& K, float pmono, co
 }
 
 __device__ __forceinline__ bool next_bucket(const TravParams& P, int lane, int64_t& b, int& tnode) {
-  const unsigned bi = grab_bucket(P.work, P.smq, lane);
+  const unsigned bi = grab_bucket(P.work, P.smq, P.batch, lane);
   b = P.b_begin + (int64_t)bi;
   if (b >= P.b_end) return false;
   tnode = P.buckets[b];
@@ -1331,11 +1292,8 @@ void launch_walk_lists(const TravParams& P, const ListParams& L, const Mom* mom,
   if (P.ox == 0.0 && P.oy == 0.0 && P.oz == 0.0) walk_lists<false><<<grid, kWlWarps * 32, 0, st>>>(P, L, mom);
   else walk_lists<true><<<grid, kWlWarps * 32, 0, st>>>(P, L, mom);
 }
-void launch_eval_lists(const TravParams& P, const ListParams& L, const Mom* mom, int grid, cudaStream_t st,
-                       unsigned* work2) {
-  TravParams Q = P;
-  Q.work = work2;
-  if (P.smq) Q.smq = P.smq + 256;  // P2P's queues follow P2C's
+void launch_eval_lists(const TravParams& P, const TravParams& Q, const ListParams& L, const Mom* mom, int grid,
+                       cudaStream_t st) {
   note_launch();
   // the replica walks after the first (periodic passes) leave short P2C
   // lists, where the one-target kernel's smaller per-bucket work measured

@@ -45,6 +45,8 @@ struct pt_handle {
   unsigned long long* d_counters = nullptr;  // 3
   unsigned* d_work = nullptr;
   unsigned long long* d_vmax2 = nullptr;
+  double4* src = nullptr;  // (x, y, z, m) per particle, sorted order (FP64 walk and replay)
+  int64_t cap_src = 0;
   float4* srcf = nullptr;
   float* softf = nullptr;
   int64_t cap_srcf = 0;
@@ -77,8 +79,7 @@ struct pt_handle {
   int32_t *l_pc_count = nullptr, *l_pp_count = nullptr;
   int64_t l_nb_cap = 0;
   unsigned long long* d_lcur = nullptr;  // [0] P2C cursor, [1] P2P cursor, [2] longest list
-  unsigned* d_work3 = nullptr;           // bucket queues of the list kernels (walk, P2C, P2P)
-  unsigned long long* d_smq = nullptr;   // their per-SM batches, 256 words per kernel
+  unsigned long long* d_queue = nullptr;  // bucket queues (kQueueWords each) of up to three kernels
   unsigned l_region = 32768;  // entries per warp region of the list pools
 
   double* sph = nullptr;  // SPH density pass: density, ball^2 (2n), neighbours (k n int32 + k n double)
@@ -129,6 +130,22 @@ unsigned long long launches_so_far() { return g_launches.load(std::memory_order_
 
 namespace {
 
+// A bucket queue: the global counter's word, then 256 words of per-SM batches.
+constexpr int kQueueWords = 257;
+
+void use_queue(pt_handle* h, TravParams& P, int k) {
+  P.work = reinterpret_cast<unsigned*>(h->d_queue + k * kQueueWords);
+  P.smq = h->d_queue + k * kQueueWords + 1;
+}
+
+// Buckets per batch of an SM: 32, or less where the SMs would not each see a
+// few batches.  A batch belongs to its SM: with 32 for 2112 buckets, 66 SMs took
+// everything, one warp each (the others had found the counter at its end and
+// left), and the walk of the 10,000-particle Plummer took 391 us.
+unsigned bucket_batch(const pt_handle* h, int64_t nb) {
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(32, nb / ((int64_t)h->sms * 64)));
+}
+
 int fail(pt_handle* h, int code, const std::string& msg) {
   if (h) h->err = msg;
   return code;
@@ -156,6 +173,11 @@ int dalloc(pt_handle* h, T** ptr, size_t count) {
   }
   if (count == 0) count = 1;
   CK(cudaMalloc((void**)ptr, count * sizeof(T)));
+  return PT_OK;
+}
+
+int zero_queue(pt_handle* h) {
+  CK(cudaMemsetAsync(h->d_queue, 0, kQueueWords * sizeof(unsigned long long), h->stream));
   return PT_OK;
 }
 
@@ -303,10 +325,22 @@ int build_tree(pt_handle* h) {
   return PT_OK;
 }
 
+int ensure_src(pt_handle* h) {
+  if (h->cap_src >= h->cap_n) return PT_OK;
+  h->cap_src = 0;
+  CKR(dalloc(h, &h->src, h->cap_n));
+  h->cap_src = h->cap_n;
+  return PT_OK;
+}
+
 // K6: moments, upward pass, traversal records.
-int upward(pt_handle* h) {
+int upward(pt_handle* h, bool walk = true) {
   cudaStream_t st = h->stream;
-  launch_leaf_moments(h->nd, h->nnodes, h->p, st);
+  // the FP64 walk reads source records (a mixed pass takes it only to record
+  // lists, or where its list pools do not fit)
+  const bool want_src = walk && (h->cfg.precision != PT_MIXED || h->cfg.record_lists);
+  if (want_src) CKR(ensure_src(h));
+  launch_leaf_moments(h->nd, h->nnodes, h->p, want_src ? h->src : nullptr, st);
   launch_upward(h->nd, h->ninternal, st);
   const double gfac = (4.0 / 3.0) / (h->cfg.theta * h->cfg.theta);  // GravityVisitor.h:14,18
   const int mixed = h->cfg.precision == PT_MIXED;
@@ -416,8 +450,6 @@ int run_two_phase(pt_handle* h, TravParams& P) {
     h->l_nb_cap = cap;
   }
   if (!h->d_lcur) CKR(dalloc(h, &h->d_lcur, 3));
-  if (!h->d_work3) CKR(dalloc(h, &h->d_work3, 3));
-  if (!h->d_smq) CKR(dalloc(h, &h->d_smq, 3 * 256));
   const int wgrid = (int)std::max<int64_t>(1, std::min<int64_t>(walk_lists_grid(h->sms), (nb + 3) / 4));
   unsigned long long c0[3];
   CK(cudaMemcpyAsync(c0, h->d_counters, sizeof(c0), cudaMemcpyDeviceToHost, st));
@@ -454,6 +486,7 @@ int run_two_phase(pt_handle* h, TravParams& P) {
         dfree(h->pool_pp);
         h->two_phase = false;
         CK(cudaMemcpyAsync(h->d_counters, c0, sizeof(c0), cudaMemcpyHostToDevice, st));
+        CKR(zero_queue(h));
         if (h->cfg.precision == PT_FP64_LISTS) launch_traverse_f64(P, h->nd.mom, h->sms * 16, st);
         else launch_traverse_mixed(P, h->nd.mom, h->sms * 16, st);
         CK(cudaGetLastError());
@@ -475,11 +508,9 @@ int run_two_phase(pt_handle* h, TravParams& P) {
     L.pp_count = h->l_pp_count;
     L.max_len = reinterpret_cast<unsigned*>(h->d_lcur + 2);
     CK(cudaMemsetAsync(h->d_lcur, 0, 3 * sizeof(unsigned long long), st));
-    CK(cudaMemsetAsync(h->d_work3, 0, 3 * sizeof(unsigned), st));
-    if (h->d_smq) CK(cudaMemsetAsync(h->d_smq, 0, 3 * 256 * sizeof(unsigned long long), st));
+    CK(cudaMemsetAsync(h->d_queue, 0, 3 * kQueueWords * sizeof(unsigned long long), st));
     TravParams A = P;
-    A.work = h->d_work3;
-    A.smq = h->d_smq;
+    use_queue(h, A, 0);
     launch_walk_lists(A, L, h->nd.mom, wgrid, st);
     CK(cudaGetLastError());
     unsigned status = 0;
@@ -505,10 +536,11 @@ int run_two_phase(pt_handle* h, TravParams& P) {
     h->want_pp = std::max(2 * h->cap_pp, cur[1] + cur[1] / 2);
   }
   TravParams E = P;
-  E.work = h->d_work3 + 1;
-  E.smq = h->d_smq ? h->d_smq + 256 : nullptr;
-  if (h->cfg.precision == PT_FP64_LISTS) launch_eval_lists_f64(E, L, h->nd.mom, h->sms * 16, st, h->d_work3 + 2);
-  else launch_eval_lists(E, L, h->nd.mom, h->sms * 16, st, h->d_work3 + 2);
+  use_queue(h, E, 1);
+  TravParams F = P;  // the P2P evaluation's
+  use_queue(h, F, 2);
+  if (h->cfg.precision == PT_FP64_LISTS) launch_eval_lists_f64(E, L, h->nd.mom, h->sms * 16, st, F.work);
+  else launch_eval_lists(E, F, L, h->nd.mom, h->sms * 16, st);
   CK(cudaGetLastError());
   h->tp_lists_valid = (P.b_begin == 0 && P.b_end == h->nbuckets && !h->cfg.periodic);
   return PT_OK;
@@ -574,6 +606,7 @@ int traverse(pt_handle* h, int64_t b0, int64_t b1) {
   P.quad = h->nd.quad;
   P.quadf = h->nd.quadf;
   P.srcf = h->srcf;
+  P.src = h->src;
   P.softf = h->softf;
   P.buckets = h->buckets;
   P.b_begin = b0;
@@ -584,8 +617,9 @@ int traverse(pt_handle* h, int64_t b0, int64_t b1) {
   if (h->nbuckets > 0) CK(cudaMemsetAsync(h->bucket_work, 0, h->nbuckets * sizeof(unsigned long long), st));
   P.nnodes = h->nnodes;
   P.counters = h->d_counters;
-  P.work = h->d_work;
   P.status = h->d_status;
+  use_queue(h, P, 0);
+  P.batch = bucket_batch(h, b1 - b0);
   const int grid = h->sms * 16;
   CK(cudaMemsetAsync(h->d_counters, 0, 3 * sizeof(unsigned long long), st));
   const int64_t nb = b1 - b0;
@@ -606,7 +640,7 @@ int traverse(pt_handle* h, int64_t b0, int64_t b1) {
     h->list_nb = nb + 1;
     P.mode = 1;
     P.list_count = h->list_count;
-    CK(cudaMemsetAsync(h->d_work, 0, sizeof(unsigned), st));
+    CKR(zero_queue(h));
     CKR(run_traversal(h, P, grid));
     std::vector<int64_t> cnt(nb), off(nb + 1);
     CK(cudaMemcpyAsync(cnt.data(), h->list_count, nb * sizeof(int64_t), cudaMemcpyDeviceToHost, st));
@@ -628,7 +662,7 @@ int traverse(pt_handle* h, int64_t b0, int64_t b1) {
     if (h->cfg.precision == PT_MIXED || h->cfg.precision == PT_FP64_LISTS) {
       // lists come from the FP64 walk (identical for every form); then the two-phase pass
       P.mode = 2;
-      CK(cudaMemsetAsync(h->d_work, 0, sizeof(unsigned), st));
+      CKR(zero_queue(h));
       launch_traverse_f64(P, h->nd.mom, grid, st);  // records lists (and FP64 forces)
       CK(cudaMemsetAsync(h->d_counters, 0, 3 * sizeof(unsigned long long), st));
       P.mode = 0;
@@ -652,7 +686,7 @@ int traverse(pt_handle* h, int64_t b0, int64_t b1) {
         P.oz = Z * L;
         P.accumulate = first ? 0 : 1;
         first = false;
-        CK(cudaMemsetAsync(h->d_work, 0, sizeof(unsigned), st));
+        CKR(zero_queue(h));
         CKR(run_traversal(h, P, grid));
       }
   if (h->cfg.periodic) CKR(ewald_correction_pass(h, b0, b1));
@@ -803,6 +837,7 @@ int pt_create(const pt_config* cfg, pt_handle** out) {
   if (dalloc(h, &h->d_status, 1) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_counters, 3) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_work, 1) != PT_OK) return bail(PT_E_NOMEM);
+  if (dalloc(h, &h->d_queue, 3 * kQueueWords) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_vmax2, 1) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_total, tree_columns()) != PT_OK) return bail(PT_E_NOMEM);
   if (cudaMemset(h->d_status, 0, sizeof(unsigned)) != cudaSuccess) return bail(PT_E_CUDA);
@@ -819,7 +854,7 @@ int pt_destroy(pt_handle* h) {
   for (auto pp : dbl) dfree(*pp);
   dfree(h->p.order); dfree(h->tmp_i); dfree(h->p.key); dfree(h->key_alt); dfree(h->idx); dfree(h->idx_alt);
   dfree(h->sort_scratch); dfree(h->tree_counts); dfree(h->d_total); dfree(h->bbox_partial); dfree(h->d_uni);
-  dfree(h->d_status); dfree(h->d_counters); dfree(h->d_work); dfree(h->d_vmax2); dfree(h->srcf); dfree(h->softf);
+  dfree(h->d_status); dfree(h->d_counters); dfree(h->d_work); dfree(h->d_vmax2); dfree(h->src); dfree(h->srcf); dfree(h->softf);
   Nodes& o = h->nd;
   dfree(o.key); dfree(o.type); dfree(o.depth); dfree(o.pstart); dfree(o.pcount); dfree(o.parent);
   dfree(o.first_child); dfree(o.count); dfree(o.mom); dfree(o.walk); dfree(o.walks); dfree(o.quad); dfree(o.quadf);
@@ -828,7 +863,7 @@ int pt_destroy(pt_handle* h) {
   dfree(h->list_kind); dfree(h->dsum); dfree(h->adj); dfree(h->nadj); dfree(h->d_htab); dfree(h->ewd); dfree(h->sph); dfree(h->sph_nbr); dfree(h->sph_nd2);
   dfree(h->sph_list_d); dfree(h->sph_list_i); dfree(h->sph_state);
   dfree(h->pool_pc); dfree(h->pool_pp); dfree(h->l_pc_start); dfree(h->l_pp_start); dfree(h->l_pc_count);
-  dfree(h->l_pp_count); dfree(h->d_lcur); dfree(h->d_work3); dfree(h->d_smq);
+  dfree(h->l_pp_count); dfree(h->d_lcur); dfree(h->d_queue);
   for (auto& e : h->ev)
     if (e) cudaEventDestroy(e);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
@@ -937,7 +972,7 @@ static int sph_density_device(pt_handle* h, bool want_nbr) {
   const int k = sph_k();
   CKR(keys_and_sort(h));
   CKR(build_tree(h));
-  CKR(upward(h));
+  CKR(upward(h, false));
   // the particle arrays were re-sorted: results of an earlier force pass no longer line up
   h->have_forces = false;
   h->forces_current = false;
@@ -1443,7 +1478,8 @@ bool lists_cover_all(const pt_handle* h) {
 // Leaf moments, upward pass and traversal records on the existing topology.
 int recompute_moments(pt_handle* h) {
   cudaStream_t st = h->stream;
-  launch_leaf_moments(h->nd, h->nnodes, h->p, st);
+  CKR(ensure_src(h));
+  launch_leaf_moments(h->nd, h->nnodes, h->p, h->src, st);
   launch_upward(h->nd, h->ninternal, st);
   const double gfac = (4.0 / 3.0) / (h->cfg.theta * h->cfg.theta);
   launch_finalize(h->nd, h->nnodes, gfac, h->cfg.precision == PT_MIXED, st);
@@ -1532,6 +1568,7 @@ int pt_forces_frozen(pt_handle* h, const double* x, const double* y, const doubl
   P.walk = h->nd.walk;
   P.walks = h->nd.walks;
   P.quad = h->nd.quad;
+  P.src = h->src;
   P.buckets = h->buckets;
   P.b_begin = 0;
   P.b_end = h->nbuckets;
@@ -1540,8 +1577,9 @@ int pt_forces_frozen(pt_handle* h, const double* x, const double* y, const doubl
   P.list_node = h->list_node;
   P.list_kind = h->list_kind;
   P.status = h->d_status;
-  P.work = h->d_work;
-  CK(cudaMemsetAsync(h->d_work, 0, sizeof(unsigned), st));
+  use_queue(h, P, 0);
+  P.batch = bucket_batch(h, h->nbuckets);
+  CKR(zero_queue(h));
   launch_replay_f64(P, h->sms * 16, st);
   CK(cudaGetLastError());
   return read_status(h);

@@ -71,6 +71,7 @@ __host__ __device__ __forceinline__ int64_t walk_sib_index(int64_t node, int row
 }
 __host__ __device__ __forceinline__ int64_t walk_sib_size(int64_t nodes) { return ((nodes + 7) >> 3) * 24 + 24; }
 static_assert(sizeof(WalkRec) == 64, "WalkRec is one 64-byte record");
+static_assert(__builtin_offsetof(WalkRec, count) == 48, "count, pstart, pcount, pad are read as one 16-byte word");
 
 // Per-node P2C record (FP64): mass, soft and the 6 second moments.
 struct __align__(16) QuadRec {
@@ -121,6 +122,7 @@ struct TravParams {
   const QuadRecF* quadf;
   const float4* srcf;     // mixed: per-particle (x,y,z) relative to its leaf's cm, mass
   const float* softf;     // mixed: per-particle softening (FP32)
+  const double4* src;     // FP64 walk: per-particle (x, y, z, m), 32-byte aligned
   const int32_t* buckets; // bucket b -> node index (DFS order)
   int64_t b_begin, b_end;
   double ox, oy, oz;      // GravityVisitor offset (periodic replicas; 0 otherwise)
@@ -136,7 +138,8 @@ struct TravParams {
   unsigned long long* counters;  // n_pp, n_pc, n_open
   unsigned int* work;     // dynamic bucket counter
   unsigned int* status;
-  unsigned long long* smq;  // per-SM bucket batches (list kernels; null: one bucket per grab)
+  unsigned long long* smq;  // per-SM bucket batches (256 words, zeroed with the counter)
+  unsigned batch;           // buckets per batch (1: one bucket per grab, no batches)
 };
 
 // Interaction lists of the two-phase mixed traversal (k_mixed2.cu): two pools

@@ -38,7 +38,7 @@ void launch_tree_emit(Nodes nd, const uint64_t* keys, int64_t n, int bucket, con
                       unsigned* status, cudaStream_t st);
 
 // k_fp64.cu
-void launch_leaf_moments(Nodes nd, int64_t nnodes, Particles p, cudaStream_t st);
+void launch_leaf_moments(Nodes nd, int64_t nnodes, Particles p, double4* src, cudaStream_t st);
 void launch_upward(Nodes nd, int64_t ninternal, cudaStream_t st);
 void launch_finalize(Nodes nd, int64_t nnodes, double gfac, int want_f32, cudaStream_t st);
 void launch_traverse_f64(const TravParams& P, const Mom* mom, int grid, cudaStream_t st);
@@ -69,10 +69,10 @@ void launch_ewald_recip(const double* x, const double* y, const double* z, const
 // k_mixed2.cu
 int walk_lists_grid(int sms);
 void launch_walk_lists(const TravParams& P, const ListParams& L, const Mom* mom, int grid, cudaStream_t st);
-// eval_p2c (store or add per P.accumulate) then eval_p2p (add); each takes its
-// bucket queue from P.work and work2 respectively (zeroed by the caller)
-void launch_eval_lists(const TravParams& P, const ListParams& L, const Mom* mom, int grid, cudaStream_t st,
-                       unsigned* work2);
+// eval_p2c (store or add per P.accumulate) then eval_p2p (add); P and Q differ in
+// their bucket queues (zeroed by the caller)
+void launch_eval_lists(const TravParams& P, const TravParams& Q, const ListParams& L, const Mom* mom, int grid,
+                       cudaStream_t st);
 // k_f64lists.cu
 void launch_eval_lists_f64(const TravParams& P, const ListParams& L, const Mom* mom, int grid, cudaStream_t st,
                            unsigned* work2);
