@@ -1,6 +1,6 @@
 // k_keys.cu -- bounding box, universe and SFC keys (compiled with -fmad=false).
 //
-//  K1 bbox_partial / bbox_final: FP64 min/max reduction of the positions
+//  K1 bbox_universe: FP64 min/max reduction of the positions
 //     (the reference's bbox reduction, src/Reader.C:92,106 and
 //     src/Partition.h:368-378) and Driver::remakeUniverse (src/Driver.h:67-80)
 //     evaluated by one thread on the device.  min/max are exact, so the
@@ -23,10 +23,20 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
-// partial[6 * block + k]: min x,y,z then max x,y,z over the block's slice.
-__global__ void __launch_bounds__(256) bbox_partial(const double* __restrict__ x, const double* __restrict__ y,
-                                                    const double* __restrict__ z, int64_t n,
-                                                    double* __restrict__ partial, unsigned* status) {
+// Bounding box and universe in one launch: every CTA reduces its slice to
+// partial[6 * block + k] (min x, y, z then max x, y, z), and the CTA that
+// finishes last (ticket, reset for the next pass) reduces the partials and
+// writes out[0..2] universe lo, out[3..5] universe hi, out[6..11] particle bbox.
+// (A second launch whose six threads each read all partials in turn took 75 us,
+// more than the rest of the keys at any size below 2^24.)
+constexpr int kBoxThreads = 256;
+__global__ void __launch_bounds__(kBoxThreads) bbox_universe(const double* __restrict__ x, const double* __restrict__ y,
+                                                            const double* __restrict__ z, int64_t n,
+                                                            double* __restrict__ partial, unsigned* __restrict__ ticket,
+                                                            double* __restrict__ out, unsigned* status) {
+  __shared__ double s[6][kBoxThreads / 32];
+  __shared__ bool last;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   double mn[3] = {DBL_MAX, DBL_MAX, DBL_MAX}, mx[3] = {-DBL_MAX, -DBL_MAX, -DBL_MAX};
   bool bad = false;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -39,45 +49,55 @@ __global__ void __launch_bounds__(256) bbox_partial(const double* __restrict__ x
     }
   }
   if (bad) atomicOr(status, kErrNonFinite);
-  __shared__ double s[6][8];
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  for (int round = 0; round < 2; round++) {
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
-    double a = warp_min(mn[d]), b = warp_max(mx[d]);
-    if (lane == 0) { s[d][w] = a; s[3 + d][w] = b; }
-  }
-  __syncthreads();
-  if (threadIdx.x < 6) {
-    int k = threadIdx.x;
-    double v = s[k][0];
-    for (int i = 1; i < (int)(blockDim.x >> 5); i++) v = (k < 3) ? fmin(v, s[k][i]) : fmax(v, s[k][i]);
-    partial[6 * blockIdx.x + k] = v;
-  }
-}
-
-// out[0..2] universe lo, out[3..5] universe hi, out[6..11] particle bbox.
-__global__ void bbox_final(const double* __restrict__ partial, int nblocks, double* __restrict__ out) {
-  __shared__ double s[6];
-  if (threadIdx.x < 6) {
-    int k = threadIdx.x;
-    double v = (k < 3) ? DBL_MAX : -DBL_MAX;
-    for (int b = 0; b < nblocks; b++) v = (k < 3) ? fmin(v, partial[6 * b + k]) : fmax(v, partial[6 * b + k]);
-    s[k] = v;
+    for (int d = 0; d < 3; d++) {
+      double a = warp_min(mn[d]), b = warp_max(mx[d]);
+      if (lane == 0) { s[d][w] = a; s[3 + d][w] = b; }
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+      const int k = threadIdx.x;
+      double v = s[k][0];
+      for (int i = 1; i < kBoxThreads / 32; i++) v = (k < 3) ? fmin(v, s[k][i]) : fmax(v, s[k][i]);
+      if (round == 0) partial[6 * blockIdx.x + k] = v;
+      else s[k][0] = v;
+    }
+    if (round == 1) break;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      mn[d] = DBL_MAX;
+      mx[d] = -DBL_MAX;
+    }
+    for (int b = threadIdx.x; b < (int)gridDim.x; b += kBoxThreads) {
+#pragma unroll
+      for (int d = 0; d < 3; d++) {
+        mn[d] = fmin(mn[d], __ldcg(partial + 6 * b + d));
+        mx[d] = fmax(mx[d], __ldcg(partial + 6 * b + 3 + d));
+      }
+    }
   }
   __syncthreads();
   if (threadIdx.x == 0) {
+    *ticket = 0u;
     // Driver::remakeUniverse, src/Driver.h:67-80
-    double sx = s[3] - s[0], sy = s[4] - s[1], sz = s[5] - s[2];
+    double sx = s[3][0] - s[0][0], sy = s[4][0] - s[1][0], sz = s[5][0] - s[2][0];
     double m = (sx > sy) ? sx : sy;
     m = (m > sz) ? m : sz;
     const double fEps = 1.0 + 1.91e-6;
     double h = fEps * 0.5 * m;
     for (int d = 0; d < 3; d++) {
-      double c = (s[d] + s[3 + d]) / 2.0;
+      double c = (s[d][0] + s[3 + d][0]) / 2.0;
       out[d] = c - h;
       out[3 + d] = c + h;
-      out[6 + d] = s[d];
-      out[9 + d] = s[3 + d];
+      out[6 + d] = s[d][0];
+      out[9 + d] = s[3 + d][0];
     }
   }
 }
@@ -126,11 +146,11 @@ __global__ void __launch_bounds__(256) vmax2_kernel(const double* __restrict__ v
 }
 
 void launch_bbox(const double* x, const double* y, const double* z, int64_t n, double* partial, int nblocks,
-                 double* uni, unsigned* status, cudaStream_t st) {
+                 unsigned* ticket, double* uni, unsigned* status, cudaStream_t st) {
+  const int64_t need = (n + kBoxThreads - 1) / kBoxThreads;
+  if (need < nblocks) nblocks = need > 0 ? (int)need : 1;
   note_launch();
-  bbox_partial<<<nblocks, 256, 0, st>>>(x, y, z, n, partial, status);
-  note_launch();
-  bbox_final<<<1, 32, 0, st>>>(partial, nblocks, uni);
+  bbox_universe<<<nblocks, kBoxThreads, 0, st>>>(x, y, z, n, partial, ticket, uni, status);
 }
 
 void launch_keys(const double* x, const double* y, const double* z, int64_t n, const double* uni, uint64_t* key,

@@ -14,7 +14,9 @@
 //              keys stably with __match_any_sync (lane order = key order in a
 //              round, rounds and warps in order), publishes its per-digit
 //              counts, and resolves the counts of all earlier tiles by
-//              decoupled look-back on 64-bit status words (flag | count).  The
+//              decoupled look-back on 64-bit status words (tag | flag | count;
+//              a word of another tag is one an earlier pass left, so the words
+//              are never cleared between passes).  The
 //              ranked tile is staged in shared memory and written out with
 //              consecutive threads on consecutive destinations.
 // The look-back only waits on tiles that claimed their index earlier and
@@ -32,10 +34,14 @@ namespace pt {
 
 constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
-constexpr int kSortRounds = 16;                        // rounds of 32 keys per warp
-constexpr int kSortTile = kSortThreads * kSortRounds;  // 4096 keys per CTA
+// Rounds of 32 keys per warp: 4096 keys per CTA, or 1024 where that leaves SMs
+// without a CTA (a pass then waits for one CTA's 16 serial rounds).
+constexpr int kSortRounds = 16, kSortRoundsSmall = 4;
+constexpr int64_t kSortSmallMax = 1 << 19;
 constexpr unsigned long long kFlagAggregate = 1ull << 32;
 constexpr unsigned long long kFlagInclusive = 2ull << 32;
+constexpr int kTagShift = 34;
+constexpr unsigned kTags = 1u << 30;  // pass tags 1 .. kTags - 1; 0 = memory as it was cleared
 
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
   unsigned long long v;
@@ -82,16 +88,18 @@ __global__ void __launch_bounds__(256) radix_digit_offsets(uint32_t* __restrict_
   g[threadIdx.x] = base + inc - v;
 }
 
+template <int kRounds>
 struct OnesweepShared {
   uint32_t wh[kSortWarps][256];  // per-warp digit counts, then their warp prefixes
   uint32_t dstart[256];          // tile-local start of each digit
   uint32_t gbase[256];           // global destination of each digit's first key of this tile
   uint32_t wsum[kSortWarps];
   int tile;
-  uint64_t key[kSortTile];
-  uint32_t val[kSortTile];
+  uint64_t key[kSortThreads * kRounds];
+  uint32_t val[kSortThreads * kRounds];
 };
 
+template <int kRounds>
 __global__ void __launch_bounds__(kSortThreads, 2) radix_onesweep(const uint64_t* __restrict__ kin,
                                                                   const uint32_t* __restrict__ vin,
                                                                   uint64_t* __restrict__ kout,
@@ -99,22 +107,26 @@ __global__ void __launch_bounds__(kSortThreads, 2) radix_onesweep(const uint64_t
                                                                   const uint32_t* __restrict__ gofs,
                                                                   uint32_t* __restrict__ counter,
                                                                   unsigned long long* __restrict__ look,
-                                                                  unsigned* __restrict__ status, long long spin_limit) {
+                                                                  unsigned* __restrict__ status, long long spin_limit,
+                                                                  unsigned tag) {
+  constexpr int kTile = kSortThreads * kRounds;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  OnesweepShared& S = *reinterpret_cast<OnesweepShared*>(smem_raw);
+  using Shared = OnesweepShared<kRounds>;
+  Shared& S = *reinterpret_cast<Shared*>(smem_raw);
+  const unsigned long long mine = (unsigned long long)tag << kTagShift;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < kSortWarps * 256; i += kSortThreads) (&S.wh[0][0])[i] = 0;
   if (threadIdx.x == 0) S.tile = (int)atomicAdd(counter, 1u);
   __syncthreads();
   const int tile = S.tile;
-  const int64_t tbase = (int64_t)tile * kSortTile;
-  const int64_t base = tbase + (int64_t)w * (32 * kSortRounds);
-  uint64_t k[kSortRounds];
-  uint32_t v[kSortRounds];
-  uint32_t rank[kSortRounds];
+  const int64_t tbase = (int64_t)tile * kTile;
+  const int64_t base = tbase + (int64_t)w * (32 * kRounds);
+  uint64_t k[kRounds];
+  uint32_t v[kRounds];
+  uint32_t rank[kRounds];
   const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
-  for (int r = 0; r < kSortRounds; r++) {
+  for (int r = 0; r < kRounds; r++) {
     const int64_t i = base + r * 32 + lane;
     const bool ok = i < n;
     k[r] = ok ? kin[i] : 0ull;
@@ -140,15 +152,15 @@ __global__ void __launch_bounds__(kSortThreads, 2) radix_onesweep(const uint64_t
   unsigned long long* my = look + (int64_t)tile * 256 + d;
   uint32_t excl = 0;
   if (tile == 0) {
-    st_relaxed_u64(my, kFlagInclusive | total);
+    st_relaxed_u64(my, mine | kFlagInclusive | total);
   } else {
-    st_relaxed_u64(my, kFlagAggregate | total);
+    st_relaxed_u64(my, mine | kFlagAggregate | total);
     // decoupled look-back over the earlier tiles
     int64_t pt = tile - 1;
     long long spins = 0;
     while (pt >= 0) {
       const unsigned long long s = ld_relaxed_u64(look + pt * 256 + d);
-      const unsigned long long f = s & (3ull << 32);
+      const unsigned long long f = (s >> kTagShift) == tag ? s & (3ull << 32) : 0ull;
       if (f == 0) {
         if (++spins > spin_limit) {
           atomicOr(status, kErrSort);
@@ -161,7 +173,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) radix_onesweep(const uint64_t
       if (f == kFlagInclusive) break;
       pt--;
     }
-    st_relaxed_u64(my, kFlagInclusive | (unsigned long long)(excl + total));
+    st_relaxed_u64(my, mine | kFlagInclusive | (unsigned long long)(excl + total));
   }
   S.gbase[d] = gofs[d] + excl;
   // tile-local digit starts: exclusive scan of total over the 256 digits
@@ -180,7 +192,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) radix_onesweep(const uint64_t
   __syncthreads();
   // stage the ranked tile in shared memory
 #pragma unroll
-  for (int r = 0; r < kSortRounds; r++) {
+  for (int r = 0; r < kRounds; r++) {
     const int64_t i = base + r * 32 + lane;
     if (i < n) {
       const uint32_t dd = (uint32_t)((k[r] >> shift) & 0xff);
@@ -190,7 +202,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) radix_onesweep(const uint64_t
     }
   }
   __syncthreads();
-  const int cnt = (int)min((int64_t)kSortTile, n - tbase);
+  const int cnt = (int)min((int64_t)kTile, n - tbase);
   for (int i = threadIdx.x; i < cnt; i += kSortThreads) {
     const uint64_t key = S.key[i];
     const uint32_t dd = (uint32_t)((key >> shift) & 0xff);
@@ -200,68 +212,150 @@ __global__ void __launch_bounds__(kSortThreads, 2) radix_onesweep(const uint64_t
   }
 }
 
+// ---------------------------------------------------------------- small sort
+// Up to kRankMax keys: every key's place is the number of keys before it, counted
+// against all of them (n^2 / 2 comparisons cost less than eight dependent digit
+// passes of about 11 us: 91 us at N = 4096 and 10,000).  A CTA places 32 keys,
+// lane = key, its warps taking every 8th group of four keys.
+constexpr int kRankThreads = 256;
+constexpr int64_t kRankMax = 12288;
+
+__global__ void __launch_bounds__(kRankThreads) rank_sort(const uint64_t* __restrict__ kin, uint64_t* __restrict__ kout,
+                                                         uint32_t* __restrict__ vout, int64_t n) {
+  __shared__ unsigned part[kRankThreads / 32][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int base = blockIdx.x * 32, i = base + lane, m = (int)n;
+  const uint64_t k = i < m ? kin[i] : ~0ull;
+  unsigned before = 0;
+  // keys at lower indices come first when equal, so those of the CTA's own 32
+  // and all others are told apart by the index
+  for (int g = 4 * w; g < m; g += 4 * (kRankThreads / 32)) {
+    uint64_t q[4];
+    if (g + 4 <= m) {
+      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(kin + g), b = *reinterpret_cast<const ulonglong2*>(kin + g + 2);
+      q[0] = a.x;
+      q[1] = a.y;
+      q[2] = b.x;
+      q[3] = b.y;
+    } else {
+#pragma unroll
+      for (int h = 0; h < 4; h++) q[h] = g + h < m ? kin[g + h] : ~0ull;
+    }
+    if (g + 4 <= base) {
+#pragma unroll
+      for (int h = 0; h < 4; h++) before += q[h] <= k;
+    } else if (g >= base + 32) {
+#pragma unroll
+      for (int h = 0; h < 4; h++) before += q[h] < k;
+    } else {
+#pragma unroll
+      for (int h = 0; h < 4; h++) before += q[h] < k || (q[h] == k && g + h < i);
+    }
+  }
+  part[w][lane] = before;
+  __syncthreads();
+  if (w == 0 && i < m) {
+    unsigned r = 0;
+#pragma unroll
+    for (int q = 0; q < kRankThreads / 32; q++) r += part[q][lane];
+    kout[r] = k;
+    vout[r] = (uint32_t)i;
+  }
+}
+
 // ---------------------------------------------------------------- sort driver
 namespace {
 size_t align256(size_t b) { return (b + 255) / 256 * 256; }
-}  // namespace
 
-// Scratch of radix_sort_pairs for n keys: eight digit histograms, eight tile
-// counters, and one 64-bit look-back word per (tile, digit).
-size_t sort_scratch_bytes(int64_t n) {
-  const int64_t tiles = (n + kSortTile - 1) / kSortTile;
-  return align256(8 * 256 * sizeof(uint32_t)) + align256(8 * sizeof(uint32_t)) +
-         align256((size_t)std::max<int64_t>(tiles, 1) * 256 * sizeof(unsigned long long));
+template <int kRounds>
+bool onesweep_passes(uint64_t* ka, uint32_t* va, uint64_t* kb, uint32_t* vb, int64_t n, const uint32_t* ghist,
+                     uint32_t* counters, unsigned long long* look, unsigned* status, long long spin_limit, unsigned tag,
+                     cudaStream_t st) {
+  constexpr size_t kBytes = sizeof(OnesweepShared<kRounds>);
+  static_assert(kBytes <= 227 * 1024, "onesweep tile exceeds shared memory");
+  const int tiles = (int)((n + kSortThreads * kRounds - 1) / (kSortThreads * kRounds));
+  if (cudaFuncSetAttribute(radix_onesweep<kRounds>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBytes) !=
+      cudaSuccess)
+    return false;
+  for (int pass = 0; pass < 8; pass++) {
+    note_launch();
+    radix_onesweep<kRounds><<<tiles, kSortThreads, kBytes, st>>>(ka, va, kb, vb, n, 8 * pass, ghist + 256 * pass,
+                                                                 counters + pass, look, status, spin_limit,
+                                                                 tag + (unsigned)pass);
+    uint64_t* tk = ka; ka = kb; kb = tk;
+    uint32_t* tv = va; va = vb; vb = tv;
+  }
+  return true;
 }
 
-// Sorts (k0, v0) in place by full 64-bit key using (k1, v1) as alternates.
+bool small_tiles(int64_t n) { return n <= kSortSmallMax; }
+int64_t sort_tiles(int64_t n) {
+  const int64_t tile = kSortThreads * (small_tiles(n) ? kSortRoundsSmall : kSortRounds);
+  return std::max<int64_t>((n + tile - 1) / tile, 1);
+}
+}  // namespace
+
+// Scratch of radix_sort_pairs for up to n keys: eight digit histograms, eight
+// tile counters, and one 64-bit look-back word per (tile, digit); the caller
+// clears it once, and again when it starts the tags over.
+size_t sort_scratch_bytes(int64_t n) {
+  const int64_t tiles = std::max(sort_tiles(n), sort_tiles(std::min(n, kSortSmallMax)));
+  return align256(8 * 256 * sizeof(uint32_t)) + align256(8 * sizeof(uint32_t)) +
+         align256((size_t)tiles * 256 * sizeof(unsigned long long));
+}
+
+unsigned sort_tags() { return kTags; }
+
+// Sorts the keys k0 with their indices; (k0, v0) or (k1, v1) hold the result
+// (returns 0 or 1, -1 on an error).  tag: the first of eight tags no sort on this
+// scratch has used since it was cleared, 1 .. kTags - 8.
 int radix_sort_pairs(uint64_t* k0, uint32_t* v0, uint64_t* k1, uint32_t* v1, int64_t n, void* scratch,
-                     unsigned* status, int sms, long long spin_limit, cudaStream_t st) {
-  if (n <= 1) return 0;
-  const int tiles = (int)((n + kSortTile - 1) / kSortTile);
+                     unsigned* status, int sms, long long spin_limit, unsigned tag, cudaStream_t st) {
+  if (n <= 1) return 0;  // v0 holds the identity
+  if (n <= kRankMax) {
+    note_launch();
+    rank_sort<<<(unsigned)((n + 31) / 32), kRankThreads, 0, st>>>(k0, k1, v1, n);
+    return 1;
+  }
   unsigned char* b = static_cast<unsigned char*>(scratch);
   uint32_t* ghist = reinterpret_cast<uint32_t*>(b);
   uint32_t* counters = reinterpret_cast<uint32_t*>(b + align256(8 * 256 * sizeof(uint32_t)));
   unsigned long long* look = reinterpret_cast<unsigned long long*>(
       b + align256(8 * 256 * sizeof(uint32_t)) + align256(8 * sizeof(uint32_t)));
-  const size_t look_bytes = (size_t)tiles * 256 * sizeof(unsigned long long);
-  static_assert(sizeof(OnesweepShared) <= 227 * 1024, "onesweep tile exceeds shared memory");
-  if (cudaFuncSetAttribute(radix_onesweep, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)sizeof(OnesweepShared)) != cudaSuccess)
-    return -1;
   cudaMemsetAsync(ghist, 0, align256(8 * 256 * sizeof(uint32_t)) + align256(8 * sizeof(uint32_t)), st);
   note_launch();
-  radix_histograms<<<sms * 4, kSortThreads, 0, st>>>(k0, n, ghist);
+  radix_histograms<<<(unsigned)std::min<int64_t>(sms * 4, (n + 2047) / 2048), kSortThreads, 0, st>>>(k0, n, ghist);
   note_launch();
   radix_digit_offsets<<<8, 256, 0, st>>>(ghist);
-  uint64_t *ka = k0, *kb = k1;
-  uint32_t *va = v0, *vb = v1;
-  for (int pass = 0; pass < 8; pass++) {
-    cudaMemsetAsync(look, 0, look_bytes, st);
-    note_launch();
-    radix_onesweep<<<tiles, kSortThreads, sizeof(OnesweepShared), st>>>(
-        ka, va, kb, vb, n, 8 * pass, ghist + 256 * pass, counters + pass, look, status, spin_limit);
-    uint64_t* tk = ka; ka = kb; kb = tk;
-    uint32_t* tv = va; va = vb; vb = tv;
-  }
-  // 8 passes: the result is back in (k0, v0)
-  return 0;
+  const bool ok = small_tiles(n)
+                      ? onesweep_passes<kSortRoundsSmall>(k0, v0, k1, v1, n, ghist, counters, look, status, spin_limit, tag, st)
+                      : onesweep_passes<kSortRounds>(k0, v0, k1, v1, n, ghist, counters, look, status, spin_limit, tag, st);
+  return ok ? 0 : -1;  // 8 passes: the result is back in (k0, v0)
 }
 
 // ---------------------------------------------------------------- permute
-template <typename T>
-__global__ void __launch_bounds__(256) gather_kernel(const T* __restrict__ in, T* __restrict__ out,
-                                                     const uint32_t* __restrict__ idx, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = in[idx[i]];
+// All nine particle arrays through one read of the sorted indices.  With a status
+// bit set (a sort that gave up leaves no permutation; a non-finite position) every
+// particle stays where it is: the arrays keep a consistent state.
+__global__ void __launch_bounds__(256) permute_particles(PermuteArrays a, const uint32_t* __restrict__ idx, int64_t n,
+                                                        const unsigned* __restrict__ status) {
+  const bool keep = *status != 0u;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t j = keep ? i : (int64_t)idx[i];
+    double v[8];
+#pragma unroll
+    for (int f = 0; f < 8; f++) v[f] = a.in[f][j];
+    const int32_t o = a.order_in[j];
+#pragma unroll
+    for (int f = 0; f < 8; f++) a.out[f][i] = v[f];
+    a.order_out[i] = o;
+  }
 }
 
-void gather_f64(const double* in, double* out, const uint32_t* idx, int64_t n, int grid, cudaStream_t st) {
+void launch_permute(const PermuteArrays& a, const uint32_t* idx, int64_t n, const unsigned* status, int grid,
+                    cudaStream_t st) {
   note_launch();
-  gather_kernel<double><<<grid, 256, 0, st>>>(in, out, idx, n);
-}
-void gather_i32(const int32_t* in, int32_t* out, const uint32_t* idx, int64_t n, int grid, cudaStream_t st) {
-  note_launch();
-  gather_kernel<int32_t><<<grid, 256, 0, st>>>(in, out, idx, n);
+  permute_particles<<<grid, 256, 0, st>>>(a, idx, n, status);
 }
 
 }  // namespace pt

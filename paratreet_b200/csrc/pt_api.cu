@@ -15,6 +15,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/pt_gravity.h"
@@ -31,10 +32,13 @@ struct pt_handle {
 
   int64_t n = 0, cap_n = 0;
   Particles p{};
-  double* tmp_d = nullptr;
+  unsigned char* slab = nullptr;  // every per-particle array below, one allocation
+  double* tmp[8]{};               // the other half of the permutation (free between passes)
   int32_t* tmp_i = nullptr;
   uint64_t* key_alt = nullptr;
   uint32_t *idx = nullptr, *idx_alt = nullptr;
+  unsigned sort_tag = 1;  // the next sort's first look-back tag
+  size_t sort_bytes = 0;
   unsigned char* sort_scratch = nullptr;  // onesweep histograms, tile counters, look-back words
   uint32_t* tree_counts = nullptr;  // per tile of particles: Internal nodes by level, leaves
   uint32_t* d_total = nullptr;      // their sums
@@ -42,6 +46,7 @@ struct pt_handle {
   int bbox_blocks = 0;
   double* d_uni = nullptr;  // 12 doubles
   unsigned* d_status = nullptr;
+  unsigned* d_ticket = nullptr;  // CTAs that finished the bounding box (0 between passes)
   unsigned long long* d_counters = nullptr;  // 3
   unsigned* d_work = nullptr;
   unsigned long long* d_vmax2 = nullptr;
@@ -197,18 +202,35 @@ int grid_for(const pt_handle* h, int64_t n) {
 
 int ensure_particles(pt_handle* h, int64_t n) {
   if (n <= h->cap_n && h->p.x) return PT_OK;
-  int64_t c = std::max<int64_t>(n, 1);
-  double** dbl[] = {&h->p.x, &h->p.y, &h->p.z, &h->p.vx, &h->p.vy, &h->p.vz, &h->p.m, &h->p.soft,
-                    &h->p.ax, &h->p.ay, &h->p.az, &h->p.pot, &h->p.potf, &h->tmp_d};
-  for (auto pp : dbl) CKR(dalloc(h, pp, c));
-  CKR(dalloc(h, &h->p.order, c));
-  CKR(dalloc(h, &h->tmp_i, c));
-  CKR(dalloc(h, &h->p.key, c));
-  CKR(dalloc(h, &h->key_alt, c));
-  CKR(dalloc(h, &h->idx, c));
-  CKR(dalloc(h, &h->idx_alt, c));
-  CKR(dalloc(h, &h->sort_scratch, sort_scratch_bytes(c)));
-  CKR(dalloc(h, &h->tree_counts, (size_t)tree_columns() * tree_tiles(c)));
+  const int64_t c = (std::max<int64_t>(n, 1) + 31) / 32 * 32;  // every array starts on a 128-byte boundary
+  h->cap_n = h->n = 0;
+  h->have_forces = h->forces_current = h->lists_valid = false;
+  h->p = Particles{};
+  const size_t sort_bytes = (sort_scratch_bytes(c) + 255) / 256 * 256;
+  const size_t count_bytes = ((size_t)tree_columns() * tree_tiles(c) * sizeof(uint32_t) + 255) / 256 * 256;
+  CKR(dalloc(h, &h->slab, (size_t)c * (21 * 8 + 2 * 8 + 4 * 4) + sort_bytes + count_bytes));
+  unsigned char* at = h->slab;
+  auto take = [&](auto** ptr, size_t bytes) {
+    *ptr = reinterpret_cast<std::remove_reference_t<decltype(*ptr)>>(at);
+    at += bytes;
+  };
+  h->sort_scratch = at;
+  at += sort_bytes;
+  take(&h->tree_counts, count_bytes);
+  double** dbl[] = {&h->p.y, &h->p.z, &h->p.vx, &h->p.vy, &h->p.vz, &h->p.m, &h->p.soft,
+                    &h->p.ax, &h->p.ay, &h->p.az, &h->p.pot, &h->p.potf};
+  for (auto pp : dbl) take(pp, c * sizeof(double));
+  for (auto& t : h->tmp) take(&t, c * sizeof(double));
+  take(&h->p.order, c * sizeof(int32_t));
+  take(&h->tmp_i, c * sizeof(int32_t));
+  take(&h->p.key, c * sizeof(uint64_t));
+  take(&h->key_alt, c * sizeof(uint64_t));
+  take(&h->idx, c * sizeof(uint32_t));
+  take(&h->idx_alt, c * sizeof(uint32_t));
+  take(&h->p.x, c * sizeof(double));
+  CK(cudaMemsetAsync(h->sort_scratch, 0, sort_bytes, h->stream));
+  h->sort_tag = 1;
+  h->sort_bytes = sort_bytes;
   h->cap_n = c;
   return PT_OK;
 }
@@ -266,22 +288,35 @@ int keys_and_sort(pt_handle* h) {
   cudaStream_t st = h->stream;
   const int64_t n = h->n;
   const int g = grid_for(h, n);
-  launch_bbox(h->p.x, h->p.y, h->p.z, n, h->bbox_partial, h->bbox_blocks, h->d_uni, h->d_status, st);
+  launch_bbox(h->p.x, h->p.y, h->p.z, n, h->bbox_partial, h->bbox_blocks, h->d_ticket, h->d_uni, h->d_status, st);
   launch_keys(h->p.x, h->p.y, h->p.z, n, h->d_uni, h->p.key, h->idx, g, st);
   CK(cudaGetLastError());
   CK(cudaEventRecord(h->ev[1], st));
-  if (radix_sort_pairs(h->p.key, h->idx, h->key_alt, h->idx_alt, n, h->sort_scratch, h->d_status, h->sms,
-                       h->sort_spin_limit, st))
-    return fail(h, PT_E_CUDA, "radix sort: could not set the shared-memory attribute");
-  // a look-back that gave up leaves indices that are not a permutation: stop
-  // before the gather, so the particle arrays keep their last consistent state
-  CKR(read_status(h));
-  double** fields[] = {&h->p.x, &h->p.y, &h->p.z, &h->p.vx, &h->p.vy, &h->p.vz, &h->p.m, &h->p.soft};
-  for (auto f : fields) {
-    gather_f64(*f, h->tmp_d, h->idx, n, g, st);
-    std::swap(*f, h->tmp_d);
+  if (h->sort_tag + 8 > sort_tags()) {
+    CK(cudaMemsetAsync(h->sort_scratch, 0, h->sort_bytes, st));
+    h->sort_tag = 1;
   }
-  gather_i32(h->p.order, h->tmp_i, h->idx, n, g, st);
+  const int where = radix_sort_pairs(h->p.key, h->idx, h->key_alt, h->idx_alt, n, h->sort_scratch, h->d_status,
+                                     h->sms, h->sort_spin_limit, h->sort_tag, st);
+  if (where < 0) return fail(h, PT_E_CUDA, "radix sort: could not set the shared-memory attribute");
+  h->sort_tag += 8;
+  if (where == 1) {
+    std::swap(h->p.key, h->key_alt);
+    std::swap(h->idx, h->idx_alt);
+  }
+  // a look-back that gave up leaves indices that are not a permutation: the
+  // permutation then leaves every particle where it is, and build_tree, which
+  // reads the status word, stops the pass
+  PermuteArrays A{};
+  double** fields[] = {&h->p.x, &h->p.y, &h->p.z, &h->p.vx, &h->p.vy, &h->p.vz, &h->p.m, &h->p.soft};
+  for (int f = 0; f < 8; f++) {
+    A.in[f] = *fields[f];
+    A.out[f] = h->tmp[f];
+  }
+  A.order_in = h->p.order;
+  A.order_out = h->tmp_i;
+  launch_permute(A, h->idx, n, h->d_status, g, st);
+  for (int f = 0; f < 8; f++) std::swap(*fields[f], h->tmp[f]);
   std::swap(h->p.order, h->tmp_i);
   CK(cudaGetLastError());
   CK(cudaEventRecord(h->ev[2], st));
@@ -295,7 +330,7 @@ int build_tree(pt_handle* h) {
   launch_tree_count(h->p.key, n, h->cfg.bucket, h->tree_counts, h->d_total, st);
   uint32_t tot[kMaxDepth + 1];  // Internal nodes of each level, leaves
   CK(cudaMemcpyAsync(tot, h->d_total, sizeof(tot), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+  CKR(read_status(h));  // synchronises; a failed sort ends the pass here
   int64_t ni = 0;
   int depth = 0;
   for (int l = 0; l < kMaxDepth; l++) {
@@ -755,9 +790,9 @@ int timestep(pt_handle* h, double* dt) {
 
 int unpermute_f64(pt_handle* h, const double* dsrc, double* host_out) {
   if (!host_out) return PT_OK;
-  launch_scatter_f64(dsrc, h->tmp_d, h->p.order, h->n, grid_for(h, h->n), h->stream);
+  launch_scatter_f64(dsrc, h->tmp[0], h->p.order, h->n, grid_for(h, h->n), h->stream);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(host_out, h->tmp_d, h->n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaMemcpyAsync(host_out, h->tmp[0], h->n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   return PT_OK;
 }
 
@@ -834,13 +869,14 @@ int pt_create(const pt_config* cfg, pt_handle** out) {
   h->bbox_blocks = h->sms * 4;
   if (dalloc(h, &h->bbox_partial, 6 * (size_t)h->bbox_blocks) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_uni, 12) != PT_OK) return bail(PT_E_NOMEM);
-  if (dalloc(h, &h->d_status, 1) != PT_OK) return bail(PT_E_NOMEM);
+  if (dalloc(h, &h->d_status, 2) != PT_OK) return bail(PT_E_NOMEM);
+  h->d_ticket = h->d_status + 1;
   if (dalloc(h, &h->d_counters, 3) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_work, 1) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_queue, 3 * kQueueWords) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_vmax2, 1) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_total, tree_columns()) != PT_OK) return bail(PT_E_NOMEM);
-  if (cudaMemset(h->d_status, 0, sizeof(unsigned)) != cudaSuccess) return bail(PT_E_CUDA);
+  if (cudaMemset(h->d_status, 0, 2 * sizeof(unsigned)) != cudaSuccess) return bail(PT_E_CUDA);
   *out = h;
   return PT_OK;
 }
@@ -849,11 +885,7 @@ int pt_destroy(pt_handle* h) {
   if (!h) return PT_OK;
   cudaSetDevice(h->cfg.device);
   if (h->stream) cudaStreamSynchronize(h->stream);
-  double** dbl[] = {&h->p.x, &h->p.y, &h->p.z, &h->p.vx, &h->p.vy, &h->p.vz, &h->p.m, &h->p.soft,
-                    &h->p.ax, &h->p.ay, &h->p.az, &h->p.pot, &h->p.potf, &h->tmp_d};
-  for (auto pp : dbl) dfree(*pp);
-  dfree(h->p.order); dfree(h->tmp_i); dfree(h->p.key); dfree(h->key_alt); dfree(h->idx); dfree(h->idx_alt);
-  dfree(h->sort_scratch); dfree(h->tree_counts); dfree(h->d_total); dfree(h->bbox_partial); dfree(h->d_uni);
+  dfree(h->slab); dfree(h->d_total); dfree(h->bbox_partial); dfree(h->d_uni);
   dfree(h->d_status); dfree(h->d_counters); dfree(h->d_work); dfree(h->d_vmax2); dfree(h->src); dfree(h->srcf); dfree(h->softf);
   Nodes& o = h->nd;
   dfree(o.key); dfree(o.type); dfree(o.depth); dfree(o.pstart); dfree(o.pcount); dfree(o.parent);
@@ -1053,8 +1085,8 @@ int pt_sph_pressure(pt_handle* h, const double* u, double* density, double* ax, 
   CKR(sph_density_device(h, true));
   double* us = h->sph + 2 * n;
   double* out = h->sph + 3 * n;  // ax, ay, az, PdV
-  CK(cudaMemcpyAsync(h->tmp_d, u, n * sizeof(double), cudaMemcpyHostToDevice, st));
-  launch_gather_by_order(h->tmp_d, us, h->p.order, n, grid_for(h, n), st);
+  CK(cudaMemcpyAsync(h->tmp[0], u, n * sizeof(double), cudaMemcpyHostToDevice, st));
+  launch_gather_by_order(h->tmp[0], us, h->p.order, n, grid_for(h, n), st);
   CK(cudaMemsetAsync(out, 0, 4 * n * sizeof(double), st));
   launch_sph_pressure(h->p, h->sph, h->sph + n, us, h->sph_nbr, h->sph_nd2, n, out, out + n, out + 2 * n,
                       out + 3 * n, h->d_status, h->sms * 16, st);

@@ -40,6 +40,14 @@ struct Particles {
   double *ax, *ay, *az, *pot, *potf;
 };
 
+// The particle permutation's arrays: x y z vx vy vz m soft, and the caller order.
+struct PermuteArrays {
+  const double* in[8];
+  double* out[8];
+  const int32_t* order_in;
+  int32_t* order_out;
+};
+
 // Per-node walk record: what one lane needs to classify one child.
 struct __align__(16) WalkRec {
   double cm[3];         // MultipoleMoments::cm

@@ -11,7 +11,7 @@ namespace pt {
 
 // k_keys.cu
 void launch_bbox(const double* x, const double* y, const double* z, int64_t n, double* partial, int nblocks,
-                 double* uni, unsigned* status, cudaStream_t st);
+                 unsigned* ticket, double* uni, unsigned* status, cudaStream_t st);
 void launch_keys(const double* x, const double* y, const double* z, int64_t n, const double* uni, uint64_t* key,
                  uint32_t* idx, int grid, cudaStream_t st);
 void launch_vmax2(const double* vx, const double* vy, const double* vz, int64_t n, unsigned long long* out,
@@ -19,12 +19,14 @@ void launch_vmax2(const double* vx, const double* vy, const double* vz, int64_t 
 
 // k_sort.cu
 size_t sort_scratch_bytes(int64_t n);
-// 0 on success, -1 if the kernel attribute could not be set; spin_limit =
-// polls of an unpublished tile before the look-back gives up (kErrSort)
+unsigned sort_tags();  // look-back tags of a scratch between two clears (8 per sort, from 1 on)
+// 0 or 1: which of (k0, v0) and (k1, v1) holds the result; -1 if the kernel
+// attribute could not be set; spin_limit = polls of an unpublished tile before
+// the look-back gives up (kErrSort)
 int radix_sort_pairs(uint64_t* k0, uint32_t* v0, uint64_t* k1, uint32_t* v1, int64_t n, void* scratch,
-                     unsigned* status, int sms, long long spin_limit, cudaStream_t st);
-void gather_f64(const double* in, double* out, const uint32_t* idx, int64_t n, int grid, cudaStream_t st);
-void gather_i32(const int32_t* in, int32_t* out, const uint32_t* idx, int64_t n, int grid, cudaStream_t st);
+                     unsigned* status, int sms, long long spin_limit, unsigned tag, cudaStream_t st);
+void launch_permute(const PermuteArrays& a, const uint32_t* idx, int64_t n, const unsigned* status, int grid,
+                    cudaStream_t st);
 
 // k_build.cu: the columns and tiles of the per-tile counts, the counting pass
 // (totals[L] = Internal nodes of level L, the last one the leaves), and the pass
