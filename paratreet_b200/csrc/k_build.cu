@@ -26,6 +26,8 @@
 // search for 8 children per thread, counts up and ranks down, a host read per
 // level -- took 0.40 ms at N = 4096, 0.96 ms at 2^20 and 1.4 ms at 2^24, almost
 // all of it launch gaps, host reads and chains of dependent loads.)
+#include <cfloat>
+
 #include "pt_internal.cuh"
 
 namespace pt {
@@ -323,6 +325,16 @@ __global__ void __launch_bounds__(256) tree_children(Nodes nd, const uint64_t* _
   if (type != kTypeInternal) {  // an Internal child's first_child was written with its inode
     nd.first_child[j] = -1;
     nd.fifo[j] = fifo_of(type, start, q.z, pfinish, q.w, c);
+  }
+  if (type == kTypeEmpty) {  // no particles: the moments an upward pass starts from
+    Mom e{};
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      e.lo[d] = DBL_MAX;
+      e.hi[d] = -DBL_MAX;
+    }
+    nd.mom[j] = e;
+    nd.count[j] = 0;
   }
   if (c == 0) {
     nd.npend[q.x] = __popc((in >> (lane & 24)) & 0xffu);

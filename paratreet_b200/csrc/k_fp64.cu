@@ -31,224 +31,189 @@
 
 namespace pt {
 
-__device__ __forceinline__ void mom_clear(Mom& q) {
-  q.mass = 0.0; q.cm[0] = q.cm[1] = q.cm[2] = 0.0; q.soft = 0.0; q.radius = 0.0;
-  q.xx = q.xy = q.xz = q.yy = q.yz = q.zz = 0.0;
-  q.lo[0] = q.lo[1] = q.lo[2] = DBL_MAX;
-  q.hi[0] = q.hi[1] = q.hi[2] = -DBL_MAX;
-  q.reach = 0.0;
-  q.soft_max = 0.0;
-}
+// Moments of one node held by eight lanes (r = lane & 7): lane r < 3 has centre
+// coordinate r and the box along it, lane 3 the softening, lane r < 6 the second
+// moment (i, j) of kQi / kQj; the mass is on every lane.  A combine then takes one
+// IEEE division per lane instead of four in a row on one lane, and the
+// additions of the reference's moments stay in its order.
+struct LaneMom {
+  double mass, lin, quad, lo, hi;
+};
 
-// MultipoleMoments::operator+=(Particle), examples/MultipoleMoments.h:274-353.
-__device__ __forceinline__ void mom_add_particle(Mom& q, double px, double py, double pz, double pm, double ps) {
-  double m1 = q.mass;
-  q.mass += pm;
+__device__ __forceinline__ LaneMom lane_mom_clear() { return {0.0, 0.0, 0.0, DBL_MAX, -DBL_MAX}; }
+// second moments in the order of Mom: xx xy xz yy yz zz
+__device__ __forceinline__ int quad_i(int r) { return r < 3 ? 0 : r < 5 ? 1 : 2; }
+__device__ __forceinline__ int quad_j(int r) { return r < 3 ? r : r == 3 ? 1 : 2; }
+
+// q += (m2, lin2, quad2), a particle (quad2 = 0, leaf = true) or a child's
+// moments: MultipoleMoments::operator+=(Particle), examples/MultipoleMoments.h:
+// 274-353, and CentroidData::operator+= with MultipoleMoments::
+// operator+=(MultipoleMoments).  The group's lanes call it together.
+template <bool kLeaf>
+__device__ __forceinline__ void lane_mom_add(LaneMom& q, double m2, double lin2, double quad2, int r, unsigned gm) {
+  const double m1 = q.mass;
+  q.mass += m2;
   if (q.mass == 0.0) {
-    q.soft = 0.5 * (q.soft + ps);
-    q.cm[0] = 0.5 * (q.cm[0] + px);
-    q.cm[1] = 0.5 * (q.cm[1] + py);
-    q.cm[2] = 0.5 * (q.cm[2] + pz);
+    q.lin = 0.5 * (q.lin + lin2);
     return;
   }
-  q.soft = (m1 * q.soft + pm * ps) / q.mass;
-  double c0 = q.cm[0], c1 = q.cm[1], c2 = q.cm[2];
-  q.cm[0] = (m1 * q.cm[0] + pm * px) / q.mass;
-  q.cm[1] = (m1 * q.cm[1] + pm * py) / q.mass;
-  q.cm[2] = (m1 * q.cm[2] + pm * pz) / q.mass;
-  double d0 = c0 - q.cm[0], d1 = c1 - q.cm[1], d2 = c2 - q.cm[2];
-  q.xx += m1 * d0 * d0;
-  q.yy += m1 * d1 * d1;
-  q.zz += m1 * d2 * d2;
-  q.xy += m1 * d0 * d1;
-  q.xz += m1 * d0 * d2;
-  q.yz += m1 * d1 * d2;
-  d0 = px - q.cm[0];
-  d1 = py - q.cm[1];
-  d2 = pz - q.cm[2];
-  q.xx += pm * d0 * d0;
-  q.yy += pm * d1 * d1;
-  q.zz += pm * d2 * d2;
-  q.xy += pm * d0 * d1;
-  q.xz += pm * d0 * d2;
-  q.yz += pm * d1 * d2;
+  if (!kLeaf && m1 == 0.0) {
+    q.mass = m2;
+    q.lin = lin2;
+    q.quad = quad2;
+    return;
+  }
+  if (!kLeaf && m2 == 0.0) return;
+  const double old = q.lin;
+  q.lin = (m1 * q.lin + m2 * lin2) / q.mass;
+  const double d = old - q.lin, e = lin2 - q.lin;
+  const int i = quad_i(r), j = quad_j(r);
+  const double di = __shfl_sync(gm, d, i, 8), dj = __shfl_sync(gm, d, j, 8);
+  const double ei = __shfl_sync(gm, e, i, 8), ej = __shfl_sync(gm, e, j, 8);
+  q.quad += m1 * di * dj;
+  if (kLeaf) q.quad += m2 * ei * ej;
+  else q.quad += quad2 + m2 * ei * ej;
 }
 
-// CentroidData::operator+= with MultipoleMoments::operator+=(MultipoleMoments);
-// the radius follows from the box, centre and count of the last combine
-// (mom_radius), so it is left to the caller.
-__device__ __forceinline__ void mom_combine(Mom& q, int& count, const Mom& c, int ccount) {
-#pragma unroll
-  for (int d = 0; d < 3; d++) {
-    if (c.lo[d] < q.lo[d]) q.lo[d] = c.lo[d];
-    if (c.hi[d] > q.hi[d]) q.hi[d] = c.hi[d];
+// The group's moments to the node's record.
+__device__ __forceinline__ void lane_mom_store(Mom* __restrict__ out, const LaneMom& q, double radius, double reach,
+                                               double soft_max, int r) {
+  double* o = reinterpret_cast<double*>(out);  // mass cm soft radius | xx .. zz | lo hi | reach soft_max
+  if (r < 4) o[1 + r] = q.lin;
+  if (r < 6) o[6 + r] = q.quad;
+  if (r < 3) {
+    o[12 + r] = q.lo;
+    o[15 + r] = q.hi;
   }
-  double m1 = q.mass;
-  q.mass += c.mass;
-  if (q.mass == 0.0) {
-    q.soft = 0.5 * (q.soft + c.soft);
-#pragma unroll
-    for (int d = 0; d < 3; d++) q.cm[d] = 0.5 * (q.cm[d] + c.cm[d]);
-  } else if (m1 == 0.0) {
-    q.mass = c.mass; q.soft = c.soft;
-    q.cm[0] = c.cm[0]; q.cm[1] = c.cm[1]; q.cm[2] = c.cm[2];
-    q.xx = c.xx; q.xy = c.xy; q.xz = c.xz; q.yy = c.yy; q.yz = c.yz; q.zz = c.zz;
-  } else if (c.mass != 0.0) {
-    q.soft = (m1 * q.soft + c.mass * c.soft) / q.mass;
-    double c0 = q.cm[0], c1 = q.cm[1], c2 = q.cm[2];
-#pragma unroll
-    for (int d = 0; d < 3; d++) q.cm[d] = (m1 * q.cm[d] + c.mass * c.cm[d]) / q.mass;
-    double d0 = c0 - q.cm[0], d1 = c1 - q.cm[1], d2 = c2 - q.cm[2];
-    q.xx += m1 * d0 * d0;
-    q.yy += m1 * d1 * d1;
-    q.zz += m1 * d2 * d2;
-    q.xy += m1 * d0 * d1;
-    q.xz += m1 * d0 * d2;
-    q.yz += m1 * d1 * d2;
-    d0 = c.cm[0] - q.cm[0];
-    d1 = c.cm[1] - q.cm[1];
-    d2 = c.cm[2] - q.cm[2];
-    q.xx += c.xx + c.mass * d0 * d0;
-    q.yy += c.yy + c.mass * d1 * d1;
-    q.zz += c.zz + c.mass * d2 * d2;
-    q.xy += c.xy + c.mass * d0 * d1;
-    q.xz += c.xz + c.mass * d0 * d2;
-    q.yz += c.yz + c.mass * d1 * d2;
+  if (r == 4) o[0] = q.mass;
+  if (r == 5) o[5] = radius;
+  if (r == 6) o[18] = reach;
+  if (r == 7) o[19] = soft_max;
+}
+static_assert(sizeof(Mom) == 20 * sizeof(double), "lane_mom_store writes Mom's twenty doubles");
+
+// CentroidData(particles, n, depth) of every bucket, eight lanes per leaf.  (One
+// thread per node, four divisions in a row per particle, took 15-29 us at up to
+// 10^5 particles; this 9 us at 4096 and 10,000.)
+__global__ void __launch_bounds__(256) leaf_moments(Nodes nd, const int32_t* __restrict__ buckets, int64_t nbuckets,
+                                                    Particles p, double4* __restrict__ src) {
+  const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
+  if (g >= nbuckets) return;
+  const int lane = threadIdx.x & 31, r = lane & 7;
+  const unsigned gm = 0xffu << (lane & 24);
+  const int node = buckets[g];
+  const int s0 = nd.pstart[node], sn = nd.pcount[node];
+  const double* const field = r == 0 ? p.x : r == 1 ? p.y : r == 2 ? p.z : p.soft;
+  LaneMom q = lane_mom_clear();
+  double smax = 0.0;
+  double v = field[s0], m = p.m[s0];
+  for (int j = s0; j < s0 + sn; j++) {
+    const double lin = v, pm = m;
+    if (j + 1 < s0 + sn) {
+      v = field[j + 1];
+      m = p.m[j + 1];
+    }
+    if (src) {  // the FP64 evaluation's source records (x, y, z, m)
+      if (r < 4) reinterpret_cast<double*>(src + j)[r] = r < 3 ? lin : pm;
+    }
+    lane_mom_add<true>(q, pm, lin, 0.0, r, gm);
+    if (lin < q.lo) q.lo = lin;
+    if (lin > q.hi) q.hi = lin;
+    smax = fmax(smax, lin);  // lane 3: the softening
   }
-  count += ccount;
+  const double w = q.hi - q.lo;
+  const double wx = __shfl_sync(gm, w, 0, 8), wy = __shfl_sync(gm, w, 1, 8), wz = __shfl_sync(gm, w, 2, 8);
+  const double radius = sn > 1 ? 0.5 * sqrt(wx * wx + wy * wy + wz * wz) : 1.0;
+  // not part of the reference's data: reach and max softening of the leaf,
+  // used only to select the mixed form's unsoftened fast path
+  const double cx = __shfl_sync(gm, q.lin, 0, 8), cy = __shfl_sync(gm, q.lin, 1, 8), cz = __shfl_sync(gm, q.lin, 2, 8);
+  double r2max = 0.0;
+  for (int j = s0 + r; j < s0 + sn; j += 8) {
+    const double dx = p.x[j] - cx, dy = p.y[j] - cy, dz = p.z[j] - cz;
+    r2max = fmax(r2max, dx * dx + dy * dy + dz * dz);
+  }
+#pragma unroll
+  for (int o = 4; o; o >>= 1) r2max = fmax(r2max, __shfl_xor_sync(gm, r2max, o));
+  smax = __shfl_sync(gm, smax, 3, 8);
+  lane_mom_store(nd.mom + node, q, radius, sqrt(r2max), smax, r);
+  if (r == 0) nd.count[node] = sn;
 }
 
-__device__ __forceinline__ void mom_radius(Mom& q, int count) {
-  if (count > 1) {
-    double e[3];
-#pragma unroll
-    for (int d = 0; d < 3; d++) {
-      double a = q.cm[d] - q.lo[d], b = q.hi[d] - q.cm[d];
-      e[d] = (a > b) ? a : b;
-    }
-    q.radius = sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
-  } else {
-    q.radius = 1.0;
-  }
-}
-
-__global__ void __launch_bounds__(256) leaf_moments(Nodes nd, int64_t nnodes, Particles p,
-                                                    double4* __restrict__ src) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i >= nnodes) return;
-  Mom q;
-  mom_clear(q);
-  int cnt = 0;
-  if (nd.type[i] == kTypeLeaf) {
-    int s0 = nd.pstart[i], sn = nd.pcount[i];
-    for (int j = s0; j < s0 + sn; j++) {
-      double px = p.x[j], py = p.y[j], pz = p.z[j], pm = p.m[j];
-      mom_add_particle(q, px, py, pz, pm, p.soft[j]);
-      if (src) src[j] = make_double4(px, py, pz, pm);  // the FP64 evaluation's source records
-      if (px < q.lo[0]) q.lo[0] = px;
-      if (py < q.lo[1]) q.lo[1] = py;
-      if (pz < q.lo[2]) q.lo[2] = pz;
-      if (px > q.hi[0]) q.hi[0] = px;
-      if (py > q.hi[1]) q.hi[1] = py;
-      if (pz > q.hi[2]) q.hi[2] = pz;
-    }
-    cnt = sn;
-    if (cnt > 1) {
-      double dx = q.hi[0] - q.lo[0], dy = q.hi[1] - q.lo[1], dz = q.hi[2] - q.lo[2];
-      q.radius = 0.5 * sqrt(dx * dx + dy * dy + dz * dz);
-    } else {
-      q.radius = 1.0;
-    }
-    // not part of the reference's data: reach and max softening of the leaf,
-    // used only to select the mixed form's unsoftened fast path
-    double r2max = 0.0, smax = 0.0;
-    for (int j = s0; j < s0 + sn; j++) {
-      double dx = p.x[j] - q.cm[0], dy = p.y[j] - q.cm[1], dz = p.z[j] - q.cm[2];
-      r2max = fmax(r2max, dx * dx + dy * dy + dz * dz);
-      smax = fmax(smax, p.soft[j]);
-    }
-    q.reach = sqrt(r2max);
-    q.soft_max = smax;
-  }
-  nd.mom[i] = q;
-  nd.count[i] = cnt;
-}
-
-// The upward pass over all levels in one launch: eight lanes per Internal node
-// (lane c holds child c).  The nodes without Internal children start; the group
-// that brings a parent its last finished Internal child goes on with the parent
-// (a counter per node, no waiting).  The combine itself is serial -- the order
-// the reference's FIFO delivers the children in decides the sums' last bits --
-// so all eight lanes run it on fields shuffled from the child's lane, after one
-// round of loads for the eight children.  One launch per level, one thread per
-// node and a load chain per child took 98 us at N = 4096 and 207 us at 2^20
-// (10-20 us per level).
-__global__ void __launch_bounds__(128) upward_climb(Nodes nd, int64_t ninternal) {
+// The upward pass over all levels in one launch: eight lanes per Internal node.
+// The nodes without Internal children start; the group that brings a parent its
+// last finished Internal child goes on with the parent (a counter per node, no
+// waiting).  The children's moments are read in one round (lane c child c) and
+// wait in shared memory while the group adds them in the order the reference's
+// FIFO delivers them.  One launch per level, one thread per node and a load
+// chain per child took 98 us at N = 4096 and 207 us at 2^20 (10-20 us per
+// level); this form with every lane doing all of a combine 48 us at 4096; this 38.
+constexpr int kClimbThreads = 128;
+__global__ void __launch_bounds__(kClimbThreads) upward_climb(Nodes nd, int64_t ninternal) {
+  __shared__ double kids[kClimbThreads / 8][8][19];  // odd stride: mass cm soft . | xx .. zz | lo hi, count
   const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
   if (g >= ninternal) return;
-  const int lane = threadIdx.x & 31, c = lane & 7;
+  const int lane = threadIdx.x & 31, r = lane & 7;
   const unsigned gm = 0xffu << (lane & 24);
+  double(*K)[19] = kids[threadIdx.x >> 3];
   const int4 first = nd.inode[g];
   int node = first.x, c0 = first.y;
   if (nd.npend[node] != 0) return;
   while (true) {
-    const int j = c0 + c;
-    double v[20];  // this lane's child, past L1: another SM may have written it in this launch
+    const int j = c0 + r;
+    // past L1: another SM may have written the child in this launch
     const double2* m = reinterpret_cast<const double2*>(nd.mom + j);
+    __syncwarp(gm);
 #pragma unroll
-    for (int k = 0; k < 10; k++) {
+    for (int k = 0; k < 9; k++) {
       const double2 p = __ldcg(m + k);
-      v[2 * k] = p.x;
-      v[2 * k + 1] = p.y;
+      K[r][2 * k] = p.x;
+      K[r][2 * k + 1] = p.y;
     }
     const int count = __ldcg(nd.count + j);
     const unsigned long long f = __ldcg(reinterpret_cast<const unsigned long long*>(nd.fifo) + j);
     int rank = 0;  // ascending FIFO position (all distinct)
 #pragma unroll
     for (int o = 1; o < 8; o++) rank += __shfl_xor_sync(gm, f, o) < f;
-    Mom q;
-    mom_clear(q);
-    int cnt = 0, src = 0;
-    for (int a = 0; a < 8; a++) {
-      src = __ffs(__ballot_sync(gm, rank == a) & gm) - 1;
-      Mom t;
-      t.mass = __shfl_sync(gm, v[0], src);
-      t.cm[0] = __shfl_sync(gm, v[1], src);
-      t.cm[1] = __shfl_sync(gm, v[2], src);
-      t.cm[2] = __shfl_sync(gm, v[3], src);
-      t.soft = __shfl_sync(gm, v[4], src);
-      t.xx = __shfl_sync(gm, v[6], src);
-      t.xy = __shfl_sync(gm, v[7], src);
-      t.xz = __shfl_sync(gm, v[8], src);
-      t.yy = __shfl_sync(gm, v[9], src);
-      t.yz = __shfl_sync(gm, v[10], src);
-      t.zz = __shfl_sync(gm, v[11], src);
+    int cnt = count;
 #pragma unroll
-      for (int d = 0; d < 3; d++) {
-        t.lo[d] = __shfl_sync(gm, v[12 + d], src);
-        t.hi[d] = __shfl_sync(gm, v[15 + d], src);
-      }
-      mom_combine(q, cnt, t, __shfl_sync(gm, count, src));
+    for (int o = 4; o; o >>= 1) cnt += __shfl_xor_sync(gm, cnt, o);
+    __syncwarp(gm);
+    LaneMom q = lane_mom_clear();
+    const int lin = 1 + min(r, 3), quad = 6 + min(r, 5), d = min(r, 2);
+    int src = 0;
+    for (int a = 0; a < 8; a++) {
+      src = __ffs(__ballot_sync(gm, rank == a) & gm) - 1 - (lane & 24);
+      const double* c = K[src];
+      if (c[12 + d] < q.lo) q.lo = c[12 + d];
+      if (c[15 + d] > q.hi) q.hi = c[15 + d];
+      lane_mom_add<false>(q, c[0], c[lin], c[quad], r, gm);
     }
-    mom_radius(q, cnt);
-    const unsigned long long last = __shfl_sync(gm, f, src);
-    if (c == 0) {
+    double e;
+    {
+      const double a = q.lin - q.lo, b = q.hi - q.lin;
+      e = (a > b) ? a : b;
+    }
+    const double ex = __shfl_sync(gm, e, 0, 8), ey = __shfl_sync(gm, e, 1, 8), ez = __shfl_sync(gm, e, 2, 8);
+    const double radius = cnt > 1 ? sqrt(ex * ex + ey * ey + ez * ez) : 1.0;
+    const unsigned long long last = __shfl_sync(gm, f, src, 8);
+    lane_mom_store(nd.mom + node, q, radius, 0.0, 0.0, r);
+    if (r == 0) {
       nd.fifo[node] = (((last >> 48) + 1ull) << 48) | (last & ((1ull << 48) - 1ull));
-      nd.mom[node] = q;
       nd.count[node] = cnt;
     }
     const int parent = nd.parent[node];
     if (parent < 0) return;
+    __threadfence();
+    __syncwarp(gm);
     int go = 0;
-    if (c == 0) {
-      __threadfence();
+    if (r == 0) {
       if (atomicAdd(nd.arrived + parent, 1) + 1 == nd.npend[parent]) {
         nd.arrived[parent] = 0;  // ready for the next upward pass over this tree
         go = 1;
       }
-      __threadfence();
     }
-    if (!__shfl_sync(gm, go, lane & 24)) return;
+    if (!__shfl_sync(gm, go, 0, 8)) return;
+    __threadfence();
     node = parent;
     c0 = nd.first_child[node];
   }
@@ -309,23 +274,33 @@ __global__ void __launch_bounds__(256) finalize_records(Nodes nd, int64_t nnodes
 // and divisions) and by latency.  With one lane per target and nothing else (a
 // bucket holds 4-10 particles, so 4-10 of 32 lanes worked) the 2^20 mixture took
 // 84.8 ms and the 4096-particle Plummer 1.01 ms; this takes 27.6 and 0.6 ms.
+//
+// With fewer buckets than resident warps a pass takes as long as its longest
+// bucket, so there the four warps of a CTA share one bucket (kTeam = 4): warp 0
+// walks and adds the sums, and every warp computes the terms of a quarter of the
+// collected entries.
 constexpr int kTravWarps = 4;
-constexpr int kF64Entries = 64;
+constexpr int kF64Entries = 64;  // per warp
 constexpr int kF64Ctas = 4;  // per SM: 128 registers; 5, 6 and 7 spill (35.8, 44 and 50 against 28.3 ms)
-constexpr int kF64Terms = 256;  // (entry, target) terms held in shared memory
+constexpr int kF64Terms = 256;  // (entry, target) terms held in shared memory, per warp
 enum : int { kEntLeaf = 0, kEntQuad = 1, kEntMono = 2 };
 
-struct F64Warp {
-  double term[4 * kF64Terms];
+template <int kTeam>
+struct F64Work {
+  double term[4 * kF64Terms * kTeam];
   BucketGeom geom;
   union {
     WalkSeg stack[kWalkStack];
     int32_t queue[kBfsQueue];  // basic-down order
   };
-  int32_t ent[kF64Entries];    // node | kind << 30, walk order
-  int2 range[kF64Entries];     // a leaf's first particle and count
-  uint8_t order[kF64Entries];  // entries by kind and size
+  int32_t ent[kF64Entries * kTeam];    // node | kind << 30, walk order
+  int2 range[kF64Entries * kTeam];     // a leaf's first particle and count
+  uint8_t order[kF64Entries * kTeam];  // a warp's entries by kind and size
+  int cmd, t0, nt;                     // team: entries to evaluate (-1: leave) and their targets
+  unsigned nsrc, npc;                  // source particles and nodes of the targets' entries
 };
+
+__device__ __forceinline__ void team_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(kTravWarps * 32) : "memory"); }
 
 // A particle's (x, y, z, m) record in one 256-bit load.
 __device__ __forceinline__ double4 ld_src(const double4* p) {
@@ -334,30 +309,26 @@ __device__ __forceinline__ double4 ld_src(const double4* p) {
   return v;
 }
 
+template <int kTeam>
 struct F64Eval {
   const TravParams* P;
-  F64Warp* w;
+  F64Work<kTeam>* w;
   int lane, nt, grp, G, cap, n;
   double xi, yi, zi, si;
   // sums of the (target, component) pairs lane + 32 h (4 t + c), and the
   // potential of those with c = 3
   double s[4], sp[4];
-  unsigned nsrc, npc;
   int64_t lat;  // where the next list entry goes (recording)
   bool record;
 
-  __device__ void begin(const TravParams& Q, F64Warp& W, int t0, int ntargets, int l, int64_t rec) {
+  // The lane's target among the ntargets from t0 on.
+  __device__ void targets(const TravParams& Q, F64Work<kTeam>& W, int t0, int ntargets, int l) {
     P = &Q;
     w = &W;
     lane = l;
     nt = ntargets;
     G = 32 / nt;
     grp = lane / nt;
-    cap = min(kF64Entries, kF64Terms / nt);
-    n = 0;
-    nsrc = npc = 0;
-    record = rec >= 0;
-    lat = rec;
     xi = yi = zi = si = 0.0;
     if (grp < G) {
       const int i = t0 + lane % nt;
@@ -366,6 +337,23 @@ struct F64Eval {
       zi = Q.p.z[i];
       si = Q.p.soft[i];
     }
+  }
+
+  __device__ void begin(const TravParams& Q, F64Work<kTeam>& W, int t0, int ntargets, int l, int64_t rec) {
+    targets(Q, W, t0, ntargets, l);
+    cap = kTeam * min(kF64Entries, kF64Terms / nt);
+    n = 0;
+    record = rec >= 0;
+    lat = rec;
+    __syncwarp();
+    if (lane == 0) {
+      w->nsrc = w->npc = 0;
+      if (kTeam > 1) {
+        w->t0 = t0;
+        w->nt = nt;
+      }
+    }
+    __syncwarp();
 #pragma unroll
     for (int h = 0; h < 4; h++) {
       s[h] = sp[h] = 0.0;
@@ -503,17 +491,16 @@ struct F64Eval {
     }
   }
 
-  // Evaluate the collected entries and add them to the sums.
-  __device__ void flush() {
-    __syncwarp();
+  // The terms of the entries [e0, e1) (at most kF64Entries), by one warp.
+  __device__ __forceinline__ void terms(int e0, int e1) {
     // kinds and leaf sizes of this lane's two entries
     int key[2];
     unsigned src = 0;
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int e = lane + 32 * h;
+      const int e = e0 + lane + 32 * h;
       key[h] = -1;
-      if (e < n) {
+      if (e < e1) {
         const int x = w->ent[e], kind = (unsigned)x >> 30;
         if (kind == kEntLeaf) {
           const int4 r = *reinterpret_cast<const int4*>(&P->walk[x].count);  // count, pstart, pcount, pad
@@ -525,25 +512,35 @@ struct F64Eval {
         }
       }
     }
-    const int nquad = __popc(__ballot_sync(kFull, key[0] == 1)) + __popc(__ballot_sync(kFull, key[1] == 1));
-    const int nmono = __popc(__ballot_sync(kFull, key[0] == 0)) + __popc(__ballot_sync(kFull, key[1] == 0));
-    const int nleaf = n - nquad - nmono;
-    nsrc += __reduce_add_sync(kFull, src);
-    npc += (unsigned)(nquad + nmono);
+    const int m = e1 - e0;
+    const int nnode = __popc(__ballot_sync(kFull, key[0] == 1 || key[0] == 0)) +
+                      __popc(__ballot_sync(kFull, key[1] == 1 || key[1] == 0));
+    const int nleaf = m - nnode;
+    src = __reduce_add_sync(kFull, src);
+    if (lane == 0) {
+      if (kTeam > 1) {
+        atomicAdd(&w->nsrc, src);
+        atomicAdd(&w->npc, (unsigned)nnode);
+      } else {
+        w->nsrc += src;
+        w->npc += (unsigned)nnode;
+      }
+    }
     // entries by descending key: one round per distinct key
+    uint8_t* const order = w->order + e0;
     {
       const unsigned lt = (1u << lane) - 1u;
       int done = 0;
       int k0 = key[0], k1 = key[1];
-      while (done < n) {
+      while (done < m) {
         const int top = __reduce_max_sync(kFull, max(k0, k1));
         const unsigned m0 = __ballot_sync(kFull, k0 == top), m1 = __ballot_sync(kFull, k1 == top);
         if (k0 == top) {
-          w->order[done + __popc(m0 & lt)] = (uint8_t)lane;
+          order[done + __popc(m0 & lt)] = (uint8_t)(e0 + lane);
           k0 = -1;
         }
         if (k1 == top) {
-          w->order[done + __popc(m0) + __popc(m1 & lt)] = (uint8_t)(lane + 32);
+          order[done + __popc(m0) + __popc(m1 & lt)] = (uint8_t)(e0 + lane + 32);
           k1 = -1;
         }
         done += __popc(m0) + __popc(m1);
@@ -554,15 +551,15 @@ struct F64Eval {
       const int t = lane % nt;
       int k = grp;
       for (; k < nleaf; k += G) {
-        const int e = w->order[k];
+        const int e = order[k];
         double v[4];
         leaf_term(w->range[e].x, w->range[e].y, v);
         double2* o = reinterpret_cast<double2*>(w->term + 4 * (e * nt + t));
         o[0] = make_double2(v[0], v[1]);
         o[1] = make_double2(v[2], v[3]);
       }
-      for (; k < n; k += G) {
-        const int e = w->order[k], x = w->ent[e];
+      for (; k < m; k += G) {
+        const int e = order[k], x = w->ent[e];
         double v[4];
         if (((unsigned)x >> 30) == kEntQuad) quad_term(x & 0x3fffffff, v);
         else mono_term(x & 0x3fffffff, v);
@@ -572,6 +569,27 @@ struct F64Eval {
       }
     }
     __syncwarp();
+  }
+
+  // A team's share of n entries: those of warp q.
+  __device__ __forceinline__ void share(int n_, int q) {
+    const int per = (n_ + kTeam - 1) / kTeam, e0 = min(n_, q * per);
+    terms(e0, min(n_, e0 + per));
+  }
+
+  // Evaluate the collected entries and add them to the sums (team: by warp 0,
+  // whose threads alone hold the sums).
+  __device__ void flush() {
+    __syncwarp();
+    if (kTeam > 1) {
+      if (lane == 0) w->cmd = n;
+      __syncwarp();
+      team_barrier();
+      share(n, 0);
+      team_barrier();
+    } else {
+      terms(0, n);
+    }
     const int per = 4 * nt;
 #pragma unroll
     for (int h = 0; h < 4; h++) {
@@ -579,6 +597,7 @@ struct F64Eval {
       if (32 * h < per && p < per) {
         double a = s[h], b = sp[h];
         const double* v = w->term + p;
+#pragma unroll 4
         for (int e = 0; e < n; e++, v += per) {
           const double t = *v;
           a += t;
@@ -591,12 +610,29 @@ struct F64Eval {
     n = 0;
     __syncwarp();
   }
+
+  // The other warps of a team: evaluate shares until warp 0 sends them away.
+  __device__ void help(const TravParams& Q, F64Work<kTeam>& W, int q, int l) {
+    int last_t0 = -1;
+    while (true) {
+      team_barrier();
+      const int m = *(volatile int*)&W.cmd;
+      if (m < 0) break;
+      const int t0 = *(volatile int*)&W.t0;
+      if (t0 != last_t0) {
+        targets(Q, W, t0, *(volatile int*)&W.nt, l);
+        last_t0 = t0;
+      }
+      share(m, q);
+      team_barrier();
+    }
+  }
 };
 
 // The bucket's walk in the handle's order; its geometry stays in shared memory
 // (the terms need the registers).
-template <bool kBfs, class Sink>
-__device__ __forceinline__ bool walk_one(const TravParams& P, F64Warp& W, int lane, Sink& sink,
+template <bool kBfs, class Work, class Sink>
+__device__ __forceinline__ bool walk_one(const TravParams& P, Work& W, int lane, Sink& sink,
                                          unsigned long long& opens) {
   if constexpr (kBfs)
     return walk_bucket_bfs(P.walk, P.nnodes, W.geom, P.ox, P.oy, P.oz, W.queue, kBfsQueue, lane, sink, opens, P.status);
@@ -604,11 +640,16 @@ __device__ __forceinline__ bool walk_one(const TravParams& P, F64Warp& W, int la
     return walk_preorder(P.walk, P.walks, P.nnodes, W.geom, P.ox, P.oy, P.oz, W.stack, lane, sink, opens, P.status);
 }
 
-template <bool kBfs>
+template <bool kBfs, int kTeam>
 __global__ void __launch_bounds__(kTravWarps * 32, kF64Ctas) traverse_f64(TravParams P, const Mom* __restrict__ mom) {
-  __shared__ F64Warp warps[kTravWarps];
-  F64Warp& W = warps[threadIdx.x >> 5];
+  __shared__ F64Work<kTeam> works[kTravWarps / kTeam];
+  F64Work<kTeam>& W = works[(threadIdx.x >> 5) / kTeam];
   const int lane = threadIdx.x & 31;
+  if (kTeam > 1 && threadIdx.x >= 32) {
+    F64Eval<kTeam> ev;
+    ev.help(P, W, threadIdx.x >> 5, lane);
+    return;
+  }
   unsigned long long c_pp = 0, c_pc = 0, c_open = 0;
   while (true) {
     const unsigned bi = grab_bucket(P.work, P.smq, P.batch, lane);
@@ -635,13 +676,13 @@ __global__ void __launch_bounds__(kTravWarps * 32, kF64Ctas) traverse_f64(TravPa
     for (int tc = 0; tc < ntot; tc += 32) {
       const int t0 = tbase + tc, nt = min(32, ntot - tc);
       unsigned long long opens = 0;
-      F64Eval ev;
+      F64Eval<kTeam> ev;
       ev.begin(P, W, t0, nt, lane, P.mode == 2 && tc == 0 ? P.list_off[b - P.b_begin] : -1);
       if (!walk_one<kBfs>(P, W, lane, ev, opens) && lane == 0) atomicOr(P.status, kErrStack);
       ev.store(t0);
       if (tc == 0) c_open += opens;
-      const unsigned long long pp = (unsigned long long)ev.nsrc * (unsigned long long)nt;
-      const unsigned long long pc = (unsigned long long)ev.npc * (unsigned long long)nt;
+      const unsigned long long pp = (unsigned long long)W.nsrc * (unsigned long long)nt;
+      const unsigned long long pc = (unsigned long long)W.npc * (unsigned long long)nt;
       c_pp += pp;
       c_pc += pc;
       if (P.bucket_work && lane == 0) {  // this chunk's interactions, added to the bucket's
@@ -656,13 +697,18 @@ __global__ void __launch_bounds__(kTravWarps * 32, kF64Ctas) traverse_f64(TravPa
     atomicAdd(&P.counters[1], c_pc);
     atomicAdd(&P.counters[2], c_open);
   }
+  if (kTeam > 1) {
+    if (lane == 0) W.cmd = -1;
+    __syncwarp();
+    team_barrier();
+  }
 }
 
 // Frozen-list replay: evaluates each bucket's recorded interaction list (in the
 // recorded order, i.e. the walk's) with the FP64 evaluator, without walking.
 // Used to differentiate the force pass for a fixed interaction list.
 __global__ void __launch_bounds__(kTravWarps * 32, kF64Ctas) replay_f64(TravParams P) {
-  __shared__ F64Warp warps[kTravWarps];
+  __shared__ F64Work<1> works[kTravWarps];
   const int lane = threadIdx.x & 31;
   while (true) {
     const unsigned bi = grab_bucket(P.work, P.smq, P.batch, lane);
@@ -673,8 +719,8 @@ __global__ void __launch_bounds__(kTravWarps * 32, kF64Ctas) replay_f64(TravPara
     const int64_t e0 = P.list_off[b - P.b_begin], e1 = P.list_off[b - P.b_begin + 1];
     for (int tc = 0; tc < ntot; tc += 32) {
       const int t0 = tbase + tc, nt = min(32, ntot - tc);
-      F64Eval ev;
-      ev.begin(P, warps[threadIdx.x >> 5], t0, nt, lane, -1);
+      F64Eval<1> ev;
+      ev.begin(P, works[threadIdx.x >> 5], t0, nt, lane, -1);
       for (int64_t e = e0; e < e1; e++) {
         const int node = P.list_node[e];
         const int kind = P.list_kind[e];
@@ -773,19 +819,33 @@ __global__ void __launch_bounds__(kDirTile) direct_sum_f64(const double* __restr
 // ---------------------------------------------------------------- launchers
 static inline unsigned blocks_for(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
 
-void launch_leaf_moments(Nodes nd, int64_t nnodes, Particles p, double4* src, cudaStream_t st) {
-  if (nnodes > 0) { note_launch(); leaf_moments<<<blocks_for(nnodes), 256, 0, st>>>(nd, nnodes, p, src); }
+void launch_leaf_moments(Nodes nd, const int32_t* buckets, int64_t nbuckets, Particles p, double4* src,
+                         cudaStream_t st) {
+  if (nbuckets > 0) { note_launch(); leaf_moments<<<blocks_for(8 * nbuckets), 256, 0, st>>>(nd, buckets, nbuckets, p, src); }
 }
 void launch_upward(Nodes nd, int64_t ninternal, cudaStream_t st) {
-  if (ninternal > 0) { note_launch(); upward_climb<<<blocks_for(8 * ninternal, 128), 128, 0, st>>>(nd, ninternal); }
+  if (ninternal > 0) { note_launch(); upward_climb<<<blocks_for(8 * ninternal, kClimbThreads), kClimbThreads, 0, st>>>(nd, ninternal); }
 }
 void launch_finalize(Nodes nd, int64_t nnodes, double gfac, int want_f32, cudaStream_t st) {
   if (nnodes > 0) { note_launch(); finalize_records<<<blocks_for(nnodes), 256, 0, st>>>(nd, nnodes, gfac, want_f32); }
 }
-void launch_traverse_f64(const TravParams& P, const Mom* mom, int grid, cudaStream_t st) {
+void launch_traverse_f64(const TravParams& P, const Mom* mom, int sms, cudaStream_t st) {
+  const int grid = 16 * sms;
   note_launch();
-  if (P.bfs) traverse_f64<true><<<grid, kTravWarps * 32, 0, st>>>(P, mom);
-  else traverse_f64<false><<<grid, kTravWarps * 32, 0, st>>>(P, mom);
+  // Up to 24 buckets per SM (16 warps are resident), a CTA per bucket.  Plummer,
+  // mixture and Hernquist spheres, buckets of 16, at 4,000 / 10,000 particles:
+  // 0.65-0.72 -> 0.32-0.34 and 0.85-1.19 -> 0.68-0.86 ms (0.22 -> 0.13 and 0.41 ->
+  // 0.32 the mixture); from 27 per SM on within 5% either way, and at 52 a warp
+  // per bucket is the better one by a third.
+  const bool team = P.mode != 1 && P.b_end - P.b_begin <= (int64_t)24 * sms;
+  const int threads = kTravWarps * 32;
+  if (P.bfs) {
+    if (team) traverse_f64<true, kTravWarps><<<grid, threads, 0, st>>>(P, mom);
+    else traverse_f64<true, 1><<<grid, threads, 0, st>>>(P, mom);
+  } else {
+    if (team) traverse_f64<false, kTravWarps><<<grid, threads, 0, st>>>(P, mom);
+    else traverse_f64<false, 1><<<grid, threads, 0, st>>>(P, mom);
+  }
 }
 void launch_replay_f64(const TravParams& P, int grid, cudaStream_t st) {
   note_launch();

@@ -214,42 +214,45 @@ __global__ void __launch_bounds__(kSortThreads, 2) radix_onesweep(const uint64_t
 
 // ---------------------------------------------------------------- small sort
 // Up to kRankMax keys: every key's place is the number of keys before it, counted
-// against all of them (n^2 / 2 comparisons cost less than eight dependent digit
+// against all of them (n^2 comparisons cost less than eight dependent digit
 // passes of about 11 us: 91 us at N = 4096 and 10,000).  A CTA places 32 keys,
-// lane = key, its warps taking every 8th group of four keys.
-constexpr int kRankThreads = 256;
+// lane = key, its warps taking every 16th group of 16 keys.
+constexpr int kRankThreads = 512;
+constexpr int kRankWarps = kRankThreads / 32;
+constexpr int kRankGroup = 16;
 constexpr int64_t kRankMax = 12288;
 
 __global__ void __launch_bounds__(kRankThreads) rank_sort(const uint64_t* __restrict__ kin, uint64_t* __restrict__ kout,
                                                          uint32_t* __restrict__ vout, int64_t n) {
-  __shared__ unsigned part[kRankThreads / 32][32];
+  __shared__ unsigned part[kRankWarps][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int base = blockIdx.x * 32, i = base + lane, m = (int)n;
   const uint64_t k = i < m ? kin[i] : ~0ull;
   unsigned before = 0;
-  // keys at lower indices come first when equal, so those of the CTA's own 32
-  // and all others are told apart by the index
-  for (int g = 4 * w; g < m; g += 4 * (kRankThreads / 32)) {
-    uint64_t q[4];
-    if (g + 4 <= m) {
-      const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(kin + g), b = *reinterpret_cast<const ulonglong2*>(kin + g + 2);
-      q[0] = a.x;
-      q[1] = a.y;
-      q[2] = b.x;
-      q[3] = b.y;
-    } else {
+  // keys at lower indices come first when equal: all keys of a group below the
+  // CTA's 32 count with <=, those above with <
+  for (int g = kRankGroup * w; g < m; g += kRankGroup * kRankWarps) {
+    uint64_t q[kRankGroup];
+    if (g + kRankGroup <= m) {
 #pragma unroll
-      for (int h = 0; h < 4; h++) q[h] = g + h < m ? kin[g + h] : ~0ull;
+      for (int h = 0; h < kRankGroup; h += 2) {
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(kin + g + h);
+        q[h] = a.x;
+        q[h + 1] = a.y;
+      }
+    } else {  // past the end: a key that counts for none
+#pragma unroll
+      for (int h = 0; h < kRankGroup; h++) q[h] = g + h < m ? kin[g + h] : ~0ull;
     }
-    if (g + 4 <= base) {
+    if (g + kRankGroup <= base) {
 #pragma unroll
-      for (int h = 0; h < 4; h++) before += q[h] <= k;
+      for (int h = 0; h < kRankGroup; h++) before += q[h] <= k;
     } else if (g >= base + 32) {
 #pragma unroll
-      for (int h = 0; h < 4; h++) before += q[h] < k;
+      for (int h = 0; h < kRankGroup; h++) before += q[h] < k;
     } else {
 #pragma unroll
-      for (int h = 0; h < 4; h++) before += q[h] < k || (q[h] == k && g + h < i);
+      for (int h = 0; h < kRankGroup; h++) before += q[h] < k || (q[h] == k && g + h < i);
     }
   }
   part[w][lane] = before;
@@ -257,7 +260,7 @@ __global__ void __launch_bounds__(kRankThreads) rank_sort(const uint64_t* __rest
   if (w == 0 && i < m) {
     unsigned r = 0;
 #pragma unroll
-    for (int q = 0; q < kRankThreads / 32; q++) r += part[q][lane];
+    for (int q = 0; q < kRankWarps; q++) r += part[q][lane];
     kout[r] = k;
     vout[r] = (uint32_t)i;
   }

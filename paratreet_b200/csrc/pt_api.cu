@@ -375,7 +375,7 @@ int upward(pt_handle* h, bool walk = true) {
   // lists, or where its list pools do not fit)
   const bool want_src = walk && (h->cfg.precision != PT_MIXED || h->cfg.record_lists);
   if (want_src) CKR(ensure_src(h));
-  launch_leaf_moments(h->nd, h->nnodes, h->p, want_src ? h->src : nullptr, st);
+  launch_leaf_moments(h->nd, h->buckets, h->nbuckets, h->p, want_src ? h->src : nullptr, st);
   launch_upward(h->nd, h->ninternal, st);
   const double gfac = (4.0 / 3.0) / (h->cfg.theta * h->cfg.theta);  // GravityVisitor.h:14,18
   const int mixed = h->cfg.precision == PT_MIXED;
@@ -522,7 +522,7 @@ int run_two_phase(pt_handle* h, TravParams& P) {
         h->two_phase = false;
         CK(cudaMemcpyAsync(h->d_counters, c0, sizeof(c0), cudaMemcpyHostToDevice, st));
         CKR(zero_queue(h));
-        if (h->cfg.precision == PT_FP64_LISTS) launch_traverse_f64(P, h->nd.mom, h->sms * 16, st);
+        if (h->cfg.precision == PT_FP64_LISTS) launch_traverse_f64(P, h->nd.mom, h->sms, st);
         else launch_traverse_mixed(P, h->nd.mom, h->sms * 16, st);
         CK(cudaGetLastError());
         return PT_OK;
@@ -586,7 +586,7 @@ int run_traversal(pt_handle* h, TravParams& P, int grid) {
   if (lists_form && P.mode == 0 && h->two_phase) return run_two_phase(h, P);
   if (h->cfg.precision == PT_MIXED && P.mode != 1)
     launch_traverse_mixed(P, h->nd.mom, grid, h->stream);
-  else launch_traverse_f64(P, h->nd.mom, grid, h->stream);
+  else launch_traverse_f64(P, h->nd.mom, h->sms, h->stream);
   CK(cudaGetLastError());
   return PT_OK;
 }
@@ -698,7 +698,7 @@ int traverse(pt_handle* h, int64_t b0, int64_t b1) {
       // lists come from the FP64 walk (identical for every form); then the two-phase pass
       P.mode = 2;
       CKR(zero_queue(h));
-      launch_traverse_f64(P, h->nd.mom, grid, st);  // records lists (and FP64 forces)
+      launch_traverse_f64(P, h->nd.mom, h->sms, st);  // records lists (and FP64 forces)
       CK(cudaMemsetAsync(h->d_counters, 0, 3 * sizeof(unsigned long long), st));
       P.mode = 0;
     }
@@ -1511,7 +1511,7 @@ bool lists_cover_all(const pt_handle* h) {
 int recompute_moments(pt_handle* h) {
   cudaStream_t st = h->stream;
   CKR(ensure_src(h));
-  launch_leaf_moments(h->nd, h->nnodes, h->p, h->src, st);
+  launch_leaf_moments(h->nd, h->buckets, h->nbuckets, h->p, h->src, st);
   launch_upward(h->nd, h->ninternal, st);
   const double gfac = (4.0 / 3.0) / (h->cfg.theta * h->cfg.theta);
   launch_finalize(h->nd, h->nnodes, gfac, h->cfg.precision == PT_MIXED, st);

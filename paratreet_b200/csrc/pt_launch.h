@@ -40,10 +40,11 @@ void launch_tree_emit(Nodes nd, const uint64_t* keys, int64_t n, int bucket, con
                       unsigned* status, cudaStream_t st);
 
 // k_fp64.cu
-void launch_leaf_moments(Nodes nd, int64_t nnodes, Particles p, double4* src, cudaStream_t st);
+void launch_leaf_moments(Nodes nd, const int32_t* buckets, int64_t nbuckets, Particles p, double4* src,
+                         cudaStream_t st);
 void launch_upward(Nodes nd, int64_t ninternal, cudaStream_t st);
 void launch_finalize(Nodes nd, int64_t nnodes, double gfac, int want_f32, cudaStream_t st);
-void launch_traverse_f64(const TravParams& P, const Mom* mom, int grid, cudaStream_t st);
+void launch_traverse_f64(const TravParams& P, const Mom* mom, int sms, cudaStream_t st);
 void launch_replay_f64(const TravParams& P, int grid, cudaStream_t st);
 void launch_kick_perturb(Particles p, int64_t n, double dt, int grid, cudaStream_t st);
 void launch_kick_half(Particles p, int64_t n, double dt, int grid, cudaStream_t st);
