@@ -18,13 +18,13 @@
 // region and goes on.  Only a full pool sets kErrPool (the host then repeats
 // the walk with larger pools).
 //
-// Phase B (eval_p2c2 / eval_p2c, eval_p2p): one warp per bucket streams its
+// Phase B (eval_p2c2, eval_p2p): one warp per bucket streams its
 // list in chunks of 64 entries and evaluates them with the packed FP32
 // instructions (two interactions per issue slot) on offsets relative to the
 // bucket's centre of mass.  Each staged node or source meets two targets per
 // packed instruction, so it is read from shared memory once for two (P2C)
-// or four (P2P) evaluations.  The P2C evaluation stores (or, for replica
-// walks after the first, adds) and eval_p2p adds.
+// or four (P2P) evaluations.  The P2C evaluation stores (or, for a later batch
+// of replicas, adds) and eval_p2p adds.
 #include "pt_internal.cuh"
 #include "pt_walk.cuh"
 #include "pt_f32.cuh"
@@ -52,14 +52,32 @@ __device__ unsigned long long g_prof[32];
 #endif
 
 constexpr int kWlWarps = 4;
-constexpr int kWlStack = 640;  // opened nodes pending (as the fused walk)
+constexpr int kWlStack = 672;  // opened nodes pending (21 levels x 28 + 32, and the roots of a batch of replicas)
 constexpr int kWlBuf = 64;
 
+template <bool kReps>
 struct WalkWarp {
   BucketGeom geom;
   int32_t stack[kWlStack];
+  uint8_t rep[kReps ? kWlStack : 4];  // the replica each pending node is walked for
   PROF_FIELDS
 };
+
+// Offsets of a batch of replicas (GravityVisitor's, in the replica loop's order
+// of examples/Gravity.C:35-41), computed by every CTA.
+struct RepOffsets {
+  double x[kMaxReps], y[kMaxReps], z[kMaxReps];
+};
+__device__ __forceinline__ void rep_offsets(const TravParams& P, RepOffsets& R) {
+  const int w = 2 * P.rep_n + 1;
+  for (int k = threadIdx.x; k < P.rep_count; k += blockDim.x) {
+    const int r = P.rep_first + k;
+    R.x[k] = __dmul_rn((double)(r / (w * w) - P.rep_n), P.period);
+    R.y[k] = __dmul_rn((double)(r / w % w - P.rep_n), P.period);
+    R.z[k] = __dmul_rn((double)(r % w - P.rep_n), P.period);
+  }
+  __syncthreads();
+}
 
 // Per-warp region of one pool: [cur, end).
 struct Region {
@@ -88,9 +106,10 @@ __device__ __forceinline__ bool ensure_region(Region& r, unsigned long long* cur
 // a new region of at least twice its new length.  False only if the pool is
 // full.  Warp-uniform; the list's entries were written before the __syncwarp
 // that ends each walk step.
+template <bool kReps>
 __device__ __forceinline__ bool make_room(int n, Region& r, unsigned long long& start, int32_t* __restrict__ pool,
-                                          unsigned long long* cursor, unsigned long long cap, unsigned region,
-                                          int lane) {
+                                          uint8_t* __restrict__ reps, unsigned long long* cursor,
+                                          unsigned long long cap, unsigned region, int lane) {
   if (r.cur + (unsigned long long)n <= r.end) return true;
   const unsigned long long len = r.cur - start;
   const unsigned long long want = max((unsigned long long)region, 2ull * (len + (unsigned long long)n));
@@ -101,7 +120,10 @@ __device__ __forceinline__ bool make_room(int n, Region& r, unsigned long long& 
     r.cur = r.end = cap;
     return false;
   }
-  for (unsigned long long k = lane; k < len; k += 32) pool[s + k] = pool[start + k];
+  for (unsigned long long k = lane; k < len; k += 32) {
+    pool[s + k] = pool[start + k];
+    if (kReps) reps[s + k] = reps[start + k];
+  }
   start = s;
   r.cur = s + len;
   r.end = s + want;
@@ -112,15 +134,21 @@ __device__ __forceinline__ bool make_room(int n, Region& r, unsigned long long& 
 #ifndef PT_WALK_MINB
 #define PT_WALK_MINB 7
 #endif
-// kOffset: the replica offset (P.ox, P.oy, P.oz) may be non-zero (periodic
-// walks); without it the walk skips three FP64 adds at the head of every
-// classification's dependent chain (c + 0.0 == c, so the tests are unchanged).
-template <bool kOffset>
+// kReps: a batch of replica offsets (periodic passes).  All replicas of a batch
+// are walked together -- their roots are tested in one step, and a step's four
+// opened nodes may belong to different replicas -- and an entry's replica goes to
+// a byte pool beside the lists, so that a bucket has one list for the batch.
+// (One walk and two evaluations per replica left the outer replicas' short lists
+// on a few lanes and read and wrote every particle's sums 54 times: 22.8 of the
+// 27.4 ms of a 128^3 lattice pass with 27 replicas.)
+template <bool kReps>
 __global__ void __launch_bounds__(kWlWarps * 32, PT_WALK_MINB) walk_lists(TravParams P, ListParams L,
                                                                          const Mom* __restrict__ mom) {
-  __shared__ WalkWarp warps[kWlWarps];
-  WalkWarp& w = warps[threadIdx.x >> 5];
+  __shared__ WalkWarp<kReps> warps[kWlWarps];
+  __shared__ RepOffsets offs[kReps ? 1 : 0 + 1];
+  WalkWarp<kReps>& w = warps[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
+  if (kReps) rep_offsets(P, offs[0]);
   unsigned long long c_pc = 0, c_open = 0;
   unsigned max_len = 0;
   Region rpc{0, 0}, rpp{0, 0};
@@ -165,11 +193,13 @@ __global__ void __launch_bounds__(kWlWarps * 32, PT_WALK_MINB) walk_lists(TravPa
     PROF_MARK(w, 0);
     while (true) {
       const int e = lane >> 3, c = lane & 7;
-      int node = -1;
+      int node = -1, rep = 0;
       if (pop < 0) {
-        if (lane == 0) node = 0;
+        if (lane < (kReps ? P.rep_count : 1)) node = 0;
+        rep = lane;
       } else if (e < nexp) {
         node = w.stack[pop + e] + c;
+        if (kReps) rep = w.rep[pop + e];
       }
       int cls = kClsNone;
       double gap2 = -1.0;
@@ -193,7 +223,7 @@ __global__ void __launch_bounds__(kWlWarps * 32, PT_WALK_MINB) walk_lists(TravPa
             r.type = tc & 7;
             r.count = tc >> 3;
           }
-          if (kOffset) cls = classify_node_gap(r, blo, bhi, g, P.ox, P.oy, P.oz, gap2);
+          if (kReps) cls = classify_node_gap(r, blo, bhi, g, offs[0].x[rep], offs[0].y[rep], offs[0].z[rep], gap2);
           else cls = classify_node_gap_nooff(r, blo, bhi, g, gap2);
         }
       }
@@ -213,18 +243,24 @@ __global__ void __launch_bounds__(kWlWarps * 32, PT_WALK_MINB) walk_lists(TravPa
         const int n = __popc(m);
         opens32 += n;  // internal children: accepted (P2C) here, opened below
         if (n && fits) {
-          fits = make_room(n, rpc, pc0, L.pc_pool, L.cursor + 0, L.cap_pc, L.region, lane);
-          if (fits && pc)
-            L.pc_pool[rpc.cur + __popc(m & lt)] =
-                node | (cls == kClsMono ? (int)0x80000000 : 0) | (near ? 0x40000000 : 0);
+          fits = make_room<kReps>(n, rpc, pc0, L.pc_pool, L.pc_rep, L.cursor + 0, L.cap_pc, L.region, lane);
+          if (fits && pc) {
+            const unsigned long long at = rpc.cur + __popc(m & lt);
+            L.pc_pool[at] = node | (cls == kClsMono ? (int)0x80000000 : 0) | (near ? 0x40000000 : 0);
+            if (kReps) L.pc_rep[at] = (uint8_t)rep;
+          }
           if (fits) rpc.cur += (unsigned long long)n;
         }
         const bool pp = (cls == kClsP2P);
         const unsigned mp = __ballot_sync(kFull, pp);
         const int npp = __popc(mp);
         if (npp && fits) {
-          fits = make_room(npp, rpp, pp0, L.pp_pool, L.cursor + 1, L.cap_pp, L.region, lane);
-          if (fits && pp) L.pp_pool[rpp.cur + __popc(mp & lt)] = node;
+          fits = make_room<kReps>(npp, rpp, pp0, L.pp_pool, L.pp_rep, L.cursor + 1, L.cap_pp, L.region, lane);
+          if (fits && pp) {
+            const unsigned long long at = rpp.cur + __popc(mp & lt);
+            L.pp_pool[at] = node;
+            if (kReps) L.pp_rep[at] = (uint8_t)rep;
+          }
           if (fits) rpp.cur += (unsigned long long)npp;
         }
       }
@@ -236,7 +272,11 @@ __global__ void __launch_bounds__(kWlWarps * 32, PT_WALK_MINB) walk_lists(TravPa
           ok = false;
           break;
         }
-        if (op) w.stack[sp + __popc(m & ((1u << lane) - 1u))] = r.first_child;
+        if (op) {
+          const int at = sp + __popc(m & ((1u << lane) - 1u));
+          w.stack[at] = r.first_child;
+          if (kReps) w.rep[at] = (uint8_t)rep;
+        }
         sp += __popc(m);
       }
       __syncwarp();
@@ -277,7 +317,7 @@ __global__ void __launch_bounds__(kWlWarps * 32, PT_WALK_MINB) walk_lists(TravPa
 
 // ---------------------------------------------------------------- phase B
 constexpr int kEvWarps = 4;
-// CTAs per SM of eval_p2c (72 registers, no spills; 6 and 8 measured 0.2 and
+// CTAs per SM of eval_p2c2 (72 registers, no spills; 6 and 8 measured 0.2 and
 // 0.3 ms slower at N = 2^24: more CTAs take shared memory from the L1 that
 // holds the node records)
 #ifndef PT_P2C_MINB
@@ -296,16 +336,6 @@ struct EvalWarp {
   int32_t ps0[kWlBuf];         // first particle of each leaf - its stream position
   float4 lof[kWlBuf];          // leaf offsets cm_leaf - cm_bucket (FP32)
   int32_t lsel[kWlBuf];        // leaves of the current kind in a block
-  PROF_FIELDS
-};
-
-// ... and of eval_p2c (kept apart: shared memory taken from one kernel's
-// CTAs is L1 lost to its node records)
-struct EvalWarpC {
-  BucketGeom geom;
-  float4 st[5][32];            // staged node pairs, five rows (offset, mass, traceless moments)
-  float4 ks[2][32];            // each lane's compensated sums and their compensations
-  int32_t spec[kWlBuf];        // the chunk's near and monopole entries (scalar pass)
   PROF_FIELDS
 };
 
@@ -428,37 +458,24 @@ __device__ __forceinline__ void ev_finish2(EvalWarp& w, const Kahan4& K, const E
   }
 }
 
-// Sum the G lane groups of each target and store or add the result.  P2C
-// (p2c): pot_full gets every node's potential, pot the quadrupole node()
-// terms only (the reference's potential: pmono, the monopole nodes' part, is
-// left out); P2P adds to pot_full only (GravityVisitor::leaf applies none).
-template <class W>
-__device__ __forceinline__ void ev_finish(W& w, const Kahan4& K, float pmono, const EvTarget& x,
-                                          const TravParams& P, int t0, int lane, bool p2c, bool store) {
+// Sum the G lane groups of each target and add the result (P2P of a single
+// target; GravityVisitor::leaf applies no potential, so pot_full only).
+__device__ __forceinline__ void ev_finish(EvalWarp& w, const Kahan4& K, const EvTarget& x, const TravParams& P,
+                                          int t0, int lane) {
   double* red = reinterpret_cast<double*>(&w.st[0][0]);
   __syncwarp();
 #pragma unroll
-  for (int k = 0; k < 4; k++) red[5 * lane + k] = (double)K.s[k] - (double)K.c[k];
-  red[5 * lane + 4] = (double)pmono;
+  for (int k = 0; k < 4; k++) red[4 * lane + k] = (double)K.s[k] - (double)K.c[k];
   __syncwarp();
   if (lane < x.nt) {
-    double v[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
     for (int gg = 0; gg < x.G; gg++)
-      for (int k = 0; k < 5; k++) v[k] += red[5 * (gg * x.nt + lane) + k];
+      for (int k = 0; k < 4; k++) v[k] += red[4 * (gg * x.nt + lane) + k];
     const int i = t0 + lane;
-    if (store) {
-      P.p.ax[i] = v[0];
-      P.p.ay[i] = v[1];
-      P.p.az[i] = v[2];
-      P.p.pot[i] = p2c ? v[3] - v[4] : 0.0;
-      P.p.potf[i] = v[3];
-    } else {
-      P.p.ax[i] += v[0];
-      P.p.ay[i] += v[1];
-      P.p.az[i] += v[2];
-      if (p2c) P.p.pot[i] += v[3] - v[4];
-      P.p.potf[i] += v[3];
-    }
+    P.p.ax[i] += v[0];
+    P.p.ay[i] += v[1];
+    P.p.az[i] += v[2];
+    P.p.potf[i] += v[3];
   }
   __syncwarp();
 }
@@ -491,11 +508,16 @@ __device__ __forceinline__ void ld_nc_f8(const void* p, float4& a, float4& b) {
       : "l"(p));
 }
 
-__device__ __forceinline__ float4 node_offset(const WalkRec* __restrict__ walk, int node, const TravParams& P,
+template <bool kReps>
+__device__ __forceinline__ float4 node_offset(const WalkRec* __restrict__ walk, int node, const RepOffsets* R, int rep,
                                               const BucketGeom& g) {
-  const double4 c = ld_nc_d4(walk + node);  // cm x, y, z, orsq | reach
-  return make_float4((float)((c.x + P.ox) - g.cm[0]), (float)((c.y + P.oy) - g.cm[1]),
-                     (float)((c.z + P.oz) - g.cm[2]), 0.f);
+  double4 c = ld_nc_d4(walk + node);  // cm x, y, z, orsq | reach
+  if (kReps) {
+    c.x += R->x[rep];
+    c.y += R->y[rep];
+    c.z += R->z[rep];
+  }
+  return make_float4((float)(c.x - g.cm[0]), (float)(c.y - g.cm[1]), (float)(c.z - g.cm[2]), 0.f);
 }
 
 // The FP32 node record (mass, soft, xx, xy), (xz, yy, yz, zz).
@@ -534,197 +556,20 @@ __device__ __noinline__ P2cTerm ev_p2c_scalar(float ox, float oy, float oz, floa
   return t;
 }
 
-// The staged node pairs k = grp, grp + G, ... of one chunk against this
-// lane's target (GravityVisitor::node, examples/GravityVisitor.h:184-224, in
-// packed FP32).  Near and monopole nodes are staged as zero-mass padding and
-// evaluated apart (ev_p2c_specials), so this loop has no branch.
-//
 // The moments are staged traceless, Qt = Q - (trace Q / 3) I.  With
 // a = 1/r, b = a^3, c = 3 b a^2, d = 5 c a^2 the reference's unsoftened terms
-// (qir = r.Q.r / 2, tr = trace Q / 2)
+// (qir = r.Q.r / 2, tr = trace Q / 2; GravityVisitor::node,
+// examples/GravityVisitor.h:184-224)
 //   pot = -M a - c qir + b tr,  acc = -(b M + d qir - c tr) r + c Q r
 // equal, since c r^2 = 3 b and d r^2 = 5 c,
 //   pot = -M a - c qt,          acc = -(b M + d qt) r + c Qt r
 // with qt = r.Qt.r / 2: the trace terms cancel exactly, which saves three of
-// 37 operations per evaluation and one staged row.
-__device__ __forceinline__ void ev_p2c_pairs(const EvalWarpC& w, const EvTarget& x, int npair, float2 ntx, float2 nty,
-                                             float2 ntz, float2& ax2, float2& ay2, float2& az2, float2& pp2,
-                                             float2& mm2) {
-  const float2 mthree = make_float2(-3.f, -3.f), m25 = make_float2(-2.5f, -2.5f), half = make_float2(0.5f, 0.5f);
-  const float4* sp = &w.st[0][x.grp];  // rows st[1..4] follow at +32 each
-  for (int k = x.grp; k < npair; k += x.G, sp += x.G) {
-    const float4 P0 = sp[0], P1 = sp[32];
-    const float2 rx = __fadd2_rn(make_float2(P0.x, P0.y), ntx);  // r' = o - t = -r
-    const float2 ry = __fadd2_rn(make_float2(P0.z, P0.w), nty);
-    const float2 rz = __fadd2_rn(make_float2(P1.x, P1.y), ntz);
-    float2 r2 = __fmul2_rn(rx, rx);
-    r2 = __ffma2_rn(ry, ry, r2);
-    r2 = __ffma2_rn(rz, rz, r2);
-    const float4 P2 = sp[64], P3 = sp[96], P4 = sp[128];
-    const float2 a = make_float2(rsqrtf(r2.x), rsqrtf(r2.y));
-    const float2 d2 = __fmul2_rn(a, a);
-    const float2 bb = __fmul2_rn(a, d2);                       // b = 1/r^3
-    const float2 nc = __fmul2_rn(__fmul2_rn(bb, d2), mthree);  // -c = -3/r^5
-    const float2 xx = make_float2(P2.x, P2.y), xy = make_float2(P2.z, P2.w);
-    const float2 xz = make_float2(P3.x, P3.y), yy = make_float2(P3.z, P3.w);
-    const float2 yz = make_float2(P4.x, P4.y), zz = make_float2(P4.z, P4.w);
-    const float2 qx = __ffma2_rn(xz, rz, __ffma2_rn(xy, ry, __fmul2_rn(xx, rx)));  // q' = Qt r' = -Qt r
-    const float2 qy = __ffma2_rn(yz, rz, __ffma2_rn(yy, ry, __fmul2_rn(xy, rx)));
-    const float2 qz = __ffma2_rn(zz, rz, __ffma2_rn(yz, ry, __fmul2_rn(xz, rx)));
-    const float2 cq = __fmul2_rn(nc, __ffma2_rn(qz, rz, __ffma2_rn(qy, ry, __fmul2_rn(qx, rx))));  // -2 c qt
-    const float2 M = make_float2(P1.z, P1.w);
-    // A = b M + d qt = b M - (5 / 2) a^2 (-2 c qt); acc += A r' - c q'; pot += -c qt - M a
-    const float2 A = __ffma2_rn(__fmul2_rn(d2, m25), cq, __fmul2_rn(bb, M));
-    ax2 = __ffma2_rn(nc, qx, __ffma2_rn(A, rx, ax2));
-    ay2 = __ffma2_rn(nc, qy, __ffma2_rn(A, ry, ay2));
-    az2 = __ffma2_rn(nc, qz, __ffma2_rn(A, rz, az2));
-    pp2 = __ffma2_rn(half, cq, pp2);
-    mm2 = __ffma2_rn(M, a, mm2);
-  }
-}
-
-// The chunk's near and monopole entries w.spec[0..ns), spread over the lane
-// groups, in scalar form; a monopole node's potential also goes to pmono
-// (left out of the reference's potential).
-__device__ __forceinline__ void ev_p2c_specials(const EvalWarpC& w, const TravParams& P, const EvTarget& x, int ns,
-                                                float2& ax2, float2& ay2, float2& az2, float2& pp2, float& pmono) {
-  const float qnan = __int_as_float(0x7fc00000);
-  for (int j = x.grp; j < ns; j += x.G) {
-    const int e = w.spec[j];
-    const int node = e & 0x3fffffff;
-    const float4 o = node_offset(P.walk, node, P, w.geom);
-    float4 r0, r1;  // (mass, soft, xx, xy), (xz, yy, yz, zz)
-    load_quadf(P.quadf, node, r0, r1);
-    const bool mono = e < 0;
-    const float4 q0 = mono ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(r0.z, r0.w, r1.x, r1.y);
-    const float2 q1 = mono ? make_float2(0.f, 0.f) : make_float2(r1.z, r1.w);
-    const P2cTerm t = ev_p2c_scalar(o.x, o.y, o.z, r0.x, mono ? qnan : r0.y, q0, q1, x.tx, x.ty, x.tz, x.ts);
-    ax2.x += t.ax;
-    ay2.x += t.ay;
-    az2.x += t.az;
-    pp2.x += t.pf;
-    if (mono) pmono += t.pf;
-  }
-}
-
-template <int kMinBlocks>
-__global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2c(TravParams P, ListParams L,
-                                                                     const Mom* __restrict__ mom) {
-  __shared__ EvalWarpC warps[kEvWarps];
-  EvalWarpC& w = warps[threadIdx.x >> 5];
-  const int lane = threadIdx.x & 31;
-  const float kPad = 1.0e10f;
-  int64_t b;
-  int tnode;
-  PROF_START(w);
-  while (next_bucket(P, lane, b, tnode)) {
-    if (tnode < 0 || tnode >= P.nnodes) continue;
-    const int64_t lb = b - P.b_begin;
-    const int64_t start = L.pc_start[lb];
-    const int count = L.pc_count[lb];
-    if (count == 0 && P.accumulate) continue;  // nothing to add (the first walk stores, even zeros)
-    __syncwarp();
-    if (lane == 0) load_bucket_geom(mom, tnode, w.geom);
-    __syncwarp();
-    const int tbase = P.walk[tnode].pstart, ntot = P.walk[tnode].pcount;
-    for (int tc = 0; tc < ntot; tc += 32) {
-      const int t0 = tbase + tc, nt = min(32, ntot - tc);
-      const EvTarget x = ev_target(P.p, w.geom, t0, nt, lane);
-      const float2 ntx = make_float2(-x.tx, -x.tx), nty = make_float2(-x.ty, -x.ty), ntz = make_float2(-x.tz, -x.tz);
-      // compensated sums in shared memory (added to once every four chunks)
-      w.ks[0][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-      w.ks[1][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-      // plain packed sums over four chunks, then one compensated add
-      float2 ax2 = make_float2(0.f, 0.f), ay2 = ax2, az2 = ax2, pp2 = ax2, mm2 = ax2;
-      float pmono = 0.f;  // the monopole nodes' potential (left out of pot)
-      // list entries of the coming chunk, loaded a chunk ahead so that only
-      // the node records wait at staging time
-      int en0 = (2 * lane < count) ? L.pc_pool[start + 2 * lane] : 0;
-      int en1 = (2 * lane + 1 < count) ? L.pc_pool[start + 2 * lane + 1] : 0;
-      PROF_MARK(w, 0);
-      for (int cs = 0; cs < count; cs += 64) {
-        const int ec[2] = {en0, en1};
-        if (cs + 64 < count) {
-          const int qn = cs + 64 + 2 * lane;
-          en0 = (qn < count) ? L.pc_pool[start + qn] : 0;
-          en1 = (qn + 1 < count) ? L.pc_pool[start + qn + 1] : 0;
-        }
-        // stage this lane's two nodes as a pair; near and monopole nodes
-        // (bits 30 / 31) become zero-mass padding and go to the scalar list
-        float4 o[2], r0[2], r1[2];
-        bool spec[2] = {false, false};
-#pragma unroll
-        for (int h = 0; h < 2; h++) {
-          const int q = cs + 2 * lane + h;
-          o[h] = make_float4(kPad, kPad, kPad, 0.f);
-          r0[h] = make_float4(0.f, 0.f, 0.f, 0.f);
-          r1[h] = r0[h];
-          if (q < count) {
-            const int e = ec[h];
-            spec[h] = (e & 0xc0000000) != 0;
-            if (!spec[h]) {
-              const int node = e & 0x3fffffff;
-              o[h] = node_offset(P.walk, node, P, w.geom);
-              load_quadf(P.quadf, node, r0[h], r1[h]);  // (mass, soft, xx, xy), (xz, yy, yz, zz)
-            }
-          }
-        }
-        const unsigned m0 = __ballot_sync(kFull, spec[0]), m1 = __ballot_sync(kFull, spec[1]);
-        const int ns = __popc(m0) + __popc(m1);
-        __syncwarp();
-        if (spec[0] || spec[1]) {  // chunk order: by lane, then h
-          const unsigned lt = (1u << lane) - 1u;
-          const int at = __popc(m0 & lt) + __popc(m1 & lt);
-          if (spec[0]) w.spec[at] = ec[0];
-          if (spec[1]) w.spec[at + (spec[0] ? 1 : 0)] = ec[1];
-        }
-#pragma unroll
-        for (int h = 0; h < 2; h++) {  // traceless moments: xx, yy, zz less a third of the trace
-          const float t3 = (r0[h].z + r1[h].y + r1[h].w) * (1.0f / 3.0f);
-          r0[h].z -= t3;
-          r1[h].y -= t3;
-          r1[h].w -= t3;
-        }
-        w.st[0][lane] = make_float4(o[0].x, o[1].x, o[0].y, o[1].y);
-        w.st[1][lane] = make_float4(o[0].z, o[1].z, r0[0].x, r0[1].x);
-        w.st[2][lane] = make_float4(r0[0].z, r0[1].z, r0[0].w, r0[1].w);
-        w.st[3][lane] = make_float4(r1[0].x, r1[1].x, r1[0].y, r1[1].y);
-        w.st[4][lane] = make_float4(r1[0].z, r1[1].z, r1[0].w, r1[1].w);
-        __syncwarp();
-        const int npair = (min(64, count - cs) + 1) >> 1;
-        PROF_MARK(w, 1);
-        if (x.grp < x.G) {
-          ev_p2c_pairs(w, x, npair, ntx, nty, ntz, ax2, ay2, az2, pp2, mm2);
-          PROF_MARK(w, 2);
-          if (ns) ev_p2c_specials(w, P, x, ns, ax2, ay2, az2, pp2, pmono);
-          PROF_MARK(w, 3);
-        }
-        if (((cs >> 6) & 3) == 3 || cs + 64 >= count) {
-          float4 ks = w.ks[0][lane], kc = w.ks[1][lane];
-          kahan_add(ks.x, kc.x, ax2.x + ax2.y);
-          kahan_add(ks.y, kc.y, ay2.x + ay2.y);
-          kahan_add(ks.z, kc.z, az2.x + az2.y);
-          kahan_add(ks.w, kc.w, (pp2.x + pp2.y) - (mm2.x + mm2.y));
-          w.ks[0][lane] = ks;
-          w.ks[1][lane] = kc;
-          ax2 = ay2 = az2 = pp2 = mm2 = make_float2(0.f, 0.f);
-        }
-      }
-      Kahan4 K;
-      {
-        const float4 ks = w.ks[0][lane], kc = w.ks[1][lane];
-        K.s[0] = ks.x; K.s[1] = ks.y; K.s[2] = ks.z; K.s[3] = ks.w;
-        K.c[0] = kc.x; K.c[1] = kc.y; K.c[2] = kc.z; K.c[3] = kc.w;
-      }
-      ev_finish(w, K, pmono, x, P, t0, lane, true, P.accumulate == 0);
-      PROF_MARK(w, 4);
-    }
-  }
-  PROF_MARK(w, 5);
-  PROF_FLUSH(w, 0);
-}
-
-// eval_p2c with two targets per lane: each staged node meets the lane's two
+// 37 operations per evaluation.  In the packed loop below, with r' = o - t = -r,
+// A = b M + d qt = b M - (5 / 2) a^2 (-2 c qt), acc += A r' - c Qt r', pot +=
+// -c qt - M a.  Near and monopole nodes are staged as zero-mass padding and
+// evaluated apart, so the loop has no branch.
+//
+// eval_p2c2, two targets per lane: each staged node meets the lane's two
 // targets in one packed instruction, so a node is read from shared memory
 // once for two evaluations.  The chunk's nodes are staged one per entry:
 // na = (offset x, y, z, mass), nq = traceless (xx, xy, xz, yy), nr =
@@ -736,14 +581,36 @@ struct EvalWarpC2 {
   float2 nr[64];
   float4 ks[4][32];  // compensated sums: target 1 (sum, compensation), target 2 (sum, compensation)
   int32_t spec[kWlBuf];
+  uint8_t srep[kWlBuf];
   PROF_FIELDS
 };
 
+// Compensated packed sum (Kahan): s + v with the rounding error kept in c.
+__device__ __forceinline__ void kahan_add2(float2& s, float2& c, float2 v) {
+  const float2 mone = make_float2(-1.f, -1.f);
+  const float2 y = __ffma2_rn(c, mone, v);
+  const float2 t = __fadd2_rn(s, y);
+  c = __ffma2_rn(y, mone, __ffma2_rn(s, mone, t));
+  s = t;
+}
+
+// The sums of a lane's two targets.  Over a batch of replicas (kComp) every term
+// is added with compensation: the replicas' attractions nearly cancel, and
+// plain sums over chunks that mix replicas left three times the rounding error
+// of sums replica by replica (128^3 lattice, pot_full 2.7e-4 against 9.5e-5 of
+// the FP64 values).  Otherwise plain sums over four chunks (pot as its two
+// halves: pp2 - mm2), then one compensated add.
+template <bool kComp>
+struct P2cSums {
+  float2 ax2, ay2, az2, pp2, mm2;
+  float2 cx2, cy2, cz2, cp2;  // compensations
+};
+
 // The chunk's nodes k = grp, grp + G, ... < nn against the lane's two
-// targets (halves of every packed value); the same terms as ev_p2c_pairs.
+// targets (halves of every packed value).
+template <bool kComp>
 __device__ __forceinline__ void ev_p2c_nodes2(const EvalWarpC2& w, const EvTarget2& x, int nn, float2 ntx,
-                                              float2 nty, float2 ntz, float2& ax2, float2& ay2, float2& az2,
-                                              float2& pp2, float2& mm2) {
+                                              float2 nty, float2 ntz, P2cSums<kComp>& S) {
   const float2 mthree = make_float2(-3.f, -3.f), m25 = make_float2(-2.5f, -2.5f), half = make_float2(0.5f, 0.5f);
   for (int k = x.grp; k < nn; k += x.G) {
     const float4 A = w.na[k];
@@ -767,18 +634,33 @@ __device__ __forceinline__ void ev_p2c_nodes2(const EvalWarpC2& w, const EvTarge
     const float2 cq = __fmul2_rn(nc, __ffma2_rn(qz, rz, __ffma2_rn(qy, ry, __fmul2_rn(qx, rx))));
     const float2 M = make_float2(A.w, A.w);
     const float2 AA = __ffma2_rn(__fmul2_rn(d2, m25), cq, __fmul2_rn(bb, M));
-    ax2 = __ffma2_rn(nc, qx, __ffma2_rn(AA, rx, ax2));
-    ay2 = __ffma2_rn(nc, qy, __ffma2_rn(AA, ry, ay2));
-    az2 = __ffma2_rn(nc, qz, __ffma2_rn(AA, rz, az2));
-    pp2 = __ffma2_rn(half, cq, pp2);
-    mm2 = __ffma2_rn(M, a, mm2);
+    if (kComp) {
+      kahan_add2(S.ax2, S.cx2, __ffma2_rn(nc, qx, __fmul2_rn(AA, rx)));
+      kahan_add2(S.ay2, S.cy2, __ffma2_rn(nc, qy, __fmul2_rn(AA, ry)));
+      kahan_add2(S.az2, S.cz2, __ffma2_rn(nc, qz, __fmul2_rn(AA, rz)));
+      kahan_add2(S.pp2, S.cp2, __ffma2_rn(make_float2(-M.x, -M.y), a, __fmul2_rn(half, cq)));
+    } else {
+      S.ax2 = __ffma2_rn(nc, qx, __ffma2_rn(AA, rx, S.ax2));
+      S.ay2 = __ffma2_rn(nc, qy, __ffma2_rn(AA, ry, S.ay2));
+      S.az2 = __ffma2_rn(nc, qz, __ffma2_rn(AA, rz, S.az2));
+      S.pp2 = __ffma2_rn(half, cq, S.pp2);
+      S.mm2 = __ffma2_rn(M, a, S.mm2);
+    }
   }
 }
 
-template <int kMinBlocks>
+template <bool kComp>
+__device__ __forceinline__ void add_term(float& s, float& c, float v) {
+  if (kComp) kahan_add(s, c, v);
+  else s += v;
+}
+
+template <int kMinBlocks, bool kReps>
 __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2c2(TravParams P, ListParams L,
                                                                       const Mom* __restrict__ mom) {
   __shared__ EvalWarpC2 warps[kEvWarps];
+  __shared__ RepOffsets offs[1];
+  if (kReps) rep_offsets(P, offs[0]);
   EvalWarpC2& w = warps[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const float kPad = 1.0e10f;
@@ -791,7 +673,7 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2c2(TravParam
     const int64_t lb = b - P.b_begin;
     const int64_t start = L.pc_start[lb];
     const int count = L.pc_count[lb];
-    if (count == 0 && P.accumulate) continue;  // nothing to add (the first walk stores, even zeros)
+    if (count == 0 && P.accumulate) continue;  // nothing to add (the first batch stores, even zeros)
     __syncwarp();
     if (lane == 0) load_bucket_geom(mom, tnode, w.geom);
     __syncwarp();
@@ -804,17 +686,27 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2c2(TravParam
                    ntz = make_float2(-x.tz.x, -x.tz.y);
 #pragma unroll
       for (int r = 0; r < 4; r++) w.ks[r][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-      float2 ax2 = make_float2(0.f, 0.f), ay2 = ax2, az2 = ax2, pp2 = ax2, mm2 = ax2;
+      P2cSums<kReps> S{};
       float2 pmono = make_float2(0.f, 0.f);  // the monopole nodes' potential (left out of pot)
       int en0 = (2 * lane < count) ? L.pc_pool[start + 2 * lane] : 0;
       int en1 = (2 * lane + 1 < count) ? L.pc_pool[start + 2 * lane + 1] : 0;
+      int rn0 = 0, rn1 = 0;
+      if (kReps) {
+        rn0 = (2 * lane < count) ? L.pc_rep[start + 2 * lane] : 0;
+        rn1 = (2 * lane + 1 < count) ? L.pc_rep[start + 2 * lane + 1] : 0;
+      }
       PROF_MARK(w, 0);
       for (int cs = 0; cs < count; cs += 64) {
         const int ec[2] = {en0, en1};
+        const int rc[2] = {rn0, rn1};
         if (cs + 64 < count) {
           const int qn = cs + 64 + 2 * lane;
           en0 = (qn < count) ? L.pc_pool[start + qn] : 0;
           en1 = (qn + 1 < count) ? L.pc_pool[start + qn + 1] : 0;
+          if (kReps) {
+            rn0 = (qn < count) ? L.pc_rep[start + qn] : 0;
+            rn1 = (qn + 1 < count) ? L.pc_rep[start + qn + 1] : 0;
+          }
         }
         float4 o[2], r0[2], r1[2];
         bool spec[2] = {false, false};
@@ -829,7 +721,7 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2c2(TravParam
             spec[h] = (e & 0xc0000000) != 0;
             if (!spec[h]) {
               const int node = e & 0x3fffffff;
-              o[h] = node_offset(P.walk, node, P, w.geom);
+              o[h] = node_offset<kReps>(P.walk, node, offs, rc[h], w.geom);
               load_quadf(P.quadf, node, r0[h], r1[h]);  // (mass, soft, xx, xy), (xz, yy, yz, zz)
             }
           }
@@ -840,8 +732,14 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2c2(TravParam
         if (spec[0] || spec[1]) {  // chunk order: by lane, then h
           const unsigned lt = (1u << lane) - 1u;
           const int at = __popc(m0 & lt) + __popc(m1 & lt);
-          if (spec[0]) w.spec[at] = ec[0];
-          if (spec[1]) w.spec[at + (spec[0] ? 1 : 0)] = ec[1];
+          if (spec[0]) {
+            w.spec[at] = ec[0];
+            if (kReps) w.srep[at] = (uint8_t)rc[0];
+          }
+          if (spec[1]) {
+            w.spec[at + (spec[0] ? 1 : 0)] = ec[1];
+            if (kReps) w.srep[at + (spec[0] ? 1 : 0)] = (uint8_t)rc[1];
+          }
         }
 #pragma unroll
         for (int h = 0; h < 2; h++) {  // traceless moments: xx, yy, zz less a third of the trace
@@ -854,12 +752,12 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2c2(TravParam
         const int nn = min(64, count - cs);
         PROF_MARK(w, 1);
         if (x.grp < x.G) {
-          ev_p2c_nodes2(w, x, nn, ntx, nty, ntz, ax2, ay2, az2, pp2, mm2);
+          ev_p2c_nodes2<kReps>(w, x, nn, ntx, nty, ntz, S);
           PROF_MARK(w, 2);
           for (int j = x.grp; j < ns; j += x.G) {  // near and monopole nodes, scalar
             const int e = w.spec[j];
             const int node = e & 0x3fffffff;
-            const float4 of = node_offset(P.walk, node, P, w.geom);
+            const float4 of = node_offset<kReps>(P.walk, node, offs, kReps ? w.srep[j] : 0, w.geom);
             float4 q0r, q1r;
             load_quadf(P.quadf, node, q0r, q1r);
             const bool mono = e < 0;
@@ -867,38 +765,44 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2c2(TravParam
             const float2 q1 = mono ? make_float2(0.f, 0.f) : make_float2(q1r.z, q1r.w);
             const float sf = mono ? qnan : q0r.y;
             const P2cTerm t = ev_p2c_scalar(of.x, of.y, of.z, q0r.x, sf, q0, q1, x.tx.x, x.ty.x, x.tz.x, x.ts.x);
-            ax2.x += t.ax;
-            ay2.x += t.ay;
-            az2.x += t.az;
-            pp2.x += t.pf;
+            add_term<kReps>(S.ax2.x, S.cx2.x, t.ax);
+            add_term<kReps>(S.ay2.x, S.cy2.x, t.ay);
+            add_term<kReps>(S.az2.x, S.cz2.x, t.az);
+            add_term<kReps>(S.pp2.x, S.cp2.x, t.pf);
             if (mono) pmono.x += t.pf;
             if (two) {
               const P2cTerm u = ev_p2c_scalar(of.x, of.y, of.z, q0r.x, sf, q0, q1, x.tx.y, x.ty.y, x.tz.y, x.ts.y);
-              ax2.y += u.ax;
-              ay2.y += u.ay;
-              az2.y += u.az;
-              pp2.y += u.pf;
+              add_term<kReps>(S.ax2.y, S.cx2.y, u.ax);
+              add_term<kReps>(S.ay2.y, S.cy2.y, u.ay);
+              add_term<kReps>(S.az2.y, S.cz2.y, u.az);
+              add_term<kReps>(S.pp2.y, S.cp2.y, u.pf);
               if (mono) pmono.y += u.pf;
             }
           }
           PROF_MARK(w, 3);
         }
-        if (((cs >> 6) & 3) == 3 || cs + 64 >= count) {
+        if (!kReps && (((cs >> 6) & 3) == 3 || cs + 64 >= count)) {
           float4 s1 = w.ks[0][lane], c1 = w.ks[1][lane], s2 = w.ks[2][lane], c2 = w.ks[3][lane];
-          kahan_add(s1.x, c1.x, ax2.x);
-          kahan_add(s1.y, c1.y, ay2.x);
-          kahan_add(s1.z, c1.z, az2.x);
-          kahan_add(s1.w, c1.w, pp2.x - mm2.x);
-          kahan_add(s2.x, c2.x, ax2.y);
-          kahan_add(s2.y, c2.y, ay2.y);
-          kahan_add(s2.z, c2.z, az2.y);
-          kahan_add(s2.w, c2.w, pp2.y - mm2.y);
+          kahan_add(s1.x, c1.x, S.ax2.x);
+          kahan_add(s1.y, c1.y, S.ay2.x);
+          kahan_add(s1.z, c1.z, S.az2.x);
+          kahan_add(s1.w, c1.w, S.pp2.x - S.mm2.x);
+          kahan_add(s2.x, c2.x, S.ax2.y);
+          kahan_add(s2.y, c2.y, S.ay2.y);
+          kahan_add(s2.z, c2.z, S.az2.y);
+          kahan_add(s2.w, c2.w, S.pp2.y - S.mm2.y);
           w.ks[0][lane] = s1;
           w.ks[1][lane] = c1;
           w.ks[2][lane] = s2;
           w.ks[3][lane] = c2;
-          ax2 = ay2 = az2 = pp2 = mm2 = make_float2(0.f, 0.f);
+          S = P2cSums<kReps>{};
         }
+      }
+      if (kReps) {  // the running sums and compensations, where the reduction reads them
+        w.ks[0][lane] = make_float4(S.ax2.x, S.ay2.x, S.az2.x, S.pp2.x);
+        w.ks[1][lane] = make_float4(S.cx2.x, S.cy2.x, S.cz2.x, S.cp2.x);
+        w.ks[2][lane] = make_float4(S.ax2.y, S.ay2.y, S.az2.y, S.pp2.y);
+        w.ks[3][lane] = make_float4(S.cx2.y, S.cy2.y, S.cz2.y, S.cp2.y);
       }
       // per target slot (group, target): ax, ay, az, pot_full, monopole part
       double* red = reinterpret_cast<double*>(&w.na[0]);  // na, nq, nr: 2560 bytes = 64 slots x 5
@@ -1170,10 +1074,11 @@ __device__ __forceinline__ void ev_p2p_leaves(EvalWarp& w, int base, int nleaves
 // (a separate marking pass over the list read every record twice: 0.6 ms at
 // N = 2^24).  Returns the source particles of the listed leaves, as the
 // reference counts P2P work (n_src * n_tgt per leaf(), src/Traverser.h:27).
-template <bool kTwo, class Tgt>
+template <bool kTwo, bool kReps, class Tgt>
 __device__ __forceinline__ unsigned long long ev_p2p_blocks(EvalWarp& w, const TravParams& P,
-                                                                  const ListParams& L, const Tgt& x, int64_t start,
-                                                                  int count, int lane, Kahan4& K) {
+                                                                  const ListParams& L, const RepOffsets* R,
+                                                                  const Tgt& x, int64_t start, int count, int lane,
+                                                                  Kahan4& K) {
   unsigned long long nsrc = 0;
   const unsigned lt = (1u << lane) - 1u;
   for (int blk = 0; blk < count; blk += 64) {
@@ -1195,12 +1100,17 @@ __device__ __forceinline__ unsigned long long ev_p2p_blocks(EvalWarp& w, const T
         ps[h] = __float_as_int(b.y);
         pc[h] = __float_as_int(b.z);
         const double smax = __hiloint2double(__float_as_int(a.y), __float_as_int(a.x));
-        const double cx = __dadd_rn(c.x, P.ox), cy = __dadd_rn(c.y, P.oy), cz = __dadd_rn(c.z, P.oz);
+        double cx = c.x, cy = c.y, cz = c.z;
+        if (kReps) {
+          const int rep = L.pp_rep[start + q];
+          cx += R->x[rep];
+          cy += R->y[rep];
+          cz += R->z[rep];
+        }
         const double gap2 = box_gap2_exact(w.geom.lo, w.geom.hi, cx, cy, cz);
         const double reach = c.w + smax + w.geom.soft_max;
         nr[h] = !(gap2 > reach * reach);
-        of[h] = make_float4((float)((c.x + P.ox) - w.geom.cm[0]), (float)((c.y + P.oy) - w.geom.cm[1]),
-                            (float)((c.z + P.oz) - w.geom.cm[2]), 0.f);
+        of[h] = make_float4((float)(cx - w.geom.cm[0]), (float)(cy - w.geom.cm[1]), (float)(cz - w.geom.cm[2]), 0.f);
       }
     }
     nsrc += __reduce_add_sync(kFull, (unsigned)(pc[0] + pc[1]));
@@ -1225,10 +1135,12 @@ __device__ __forceinline__ unsigned long long ev_p2p_blocks(EvalWarp& w, const T
   return nsrc;
 }
 
-template <int kMinBlocks>
+template <int kMinBlocks, bool kReps>
 __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2p(TravParams P, ListParams L,
                                                                      const Mom* __restrict__ mom) {
   __shared__ EvalWarp warps[kEvWarps];
+  __shared__ RepOffsets offs[1];
+  if (kReps) rep_offsets(P, offs[0]);
   EvalWarp& w = warps[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   unsigned long long c_pp = 0;
@@ -1240,7 +1152,7 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2p(TravParams
     const int64_t lb = b - P.b_begin;
     const int64_t start = L.pp_start[lb];
     const int count = L.pp_count[lb];
-    if (count == 0) continue;  // P2P only adds (the outer replica walks leave most lists empty)
+    if (count == 0) continue;  // P2P only adds
     __syncwarp();
     if (lane == 0) load_bucket_geom(mom, tnode, w.geom);
     __syncwarp();
@@ -1254,7 +1166,7 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2p(TravParams
         ev_two_zero(w, lane);
         Kahan4 K;
         K.zero();
-        nsrc = ev_p2p_blocks<true>(w, P, L, x, start, count, lane, K);
+        nsrc = ev_p2p_blocks<true, kReps>(w, P, L, offs, x, start, count, lane, K);
         ev_finish2(w, K, x, P, t0, lane);
         PROF_MARK(w, 4);
         continue;
@@ -1262,8 +1174,8 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2p(TravParams
       const EvTarget x = ev_target(P.p, w.geom, t0, nt, lane);
       Kahan4 K;
       K.zero();
-      nsrc = ev_p2p_blocks<false>(w, P, L, x, start, count, lane, K);
-      ev_finish(w, K, 0.f, x, P, t0, lane, false, false);
+      nsrc = ev_p2p_blocks<false, kReps>(w, P, L, offs, x, start, count, lane, K);
+      ev_finish(w, K, x, P, t0, lane);
       PROF_MARK(w, 4);
     }
     // P2P pairs as the reference counts them (n_src * n_tgt per leaf(),
@@ -1289,21 +1201,18 @@ int walk_lists_grid(int sms) { return sms * PT_WALK_MINB; }  // the CTAs residen
 
 void launch_walk_lists(const TravParams& P, const ListParams& L, const Mom* mom, int grid, cudaStream_t st) {
   note_launch();
-  if (P.ox == 0.0 && P.oy == 0.0 && P.oz == 0.0) walk_lists<false><<<grid, kWlWarps * 32, 0, st>>>(P, L, mom);
-  else walk_lists<true><<<grid, kWlWarps * 32, 0, st>>>(P, L, mom);
+  if (P.rep_count) walk_lists<true><<<grid, kWlWarps * 32, 0, st>>>(P, L, mom);
+  else walk_lists<false><<<grid, kWlWarps * 32, 0, st>>>(P, L, mom);
 }
 void launch_eval_lists(const TravParams& P, const TravParams& Q, const ListParams& L, const Mom* mom, int grid,
                        cudaStream_t st) {
+  const int threads = kEvWarps * 32;
   note_launch();
-  // the replica walks after the first (periodic passes) leave short P2C
-  // lists, where the one-target kernel's smaller per-bucket work measured
-  // faster (256^3 lattice pass 212 against 220 ms); the first walk and every
-  // non-periodic pass take the two-target kernel (Plummer N = 2^24: 3.5 ms
-  // faster)
-  if (P.accumulate) eval_p2c<PT_P2C_MINB><<<grid, kEvWarps * 32, 0, st>>>(P, L, mom);
-  else eval_p2c2<PT_P2C_MINB><<<grid, kEvWarps * 32, 0, st>>>(P, L, mom);
+  if (P.rep_count) eval_p2c2<PT_P2C_MINB, true><<<grid, threads, 0, st>>>(P, L, mom);
+  else eval_p2c2<PT_P2C_MINB, false><<<grid, threads, 0, st>>>(P, L, mom);
   note_launch();
-  eval_p2p<PT_P2P_MINB><<<grid, kEvWarps * 32, 0, st>>>(Q, L, mom);
+  if (P.rep_count) eval_p2p<PT_P2P_MINB, true><<<grid, threads, 0, st>>>(Q, L, mom);
+  else eval_p2p<PT_P2P_MINB, false><<<grid, threads, 0, st>>>(Q, L, mom);
 }
 
 }  // namespace pt

@@ -466,6 +466,14 @@ int ewald_correction_pass(pt_handle* h, int64_t b0, int64_t b1) {
   return PT_OK;
 }
 
+// The offset of replica r in the order of the loop of examples/Gravity.C:35-41.
+void replica_offset(const pt_handle* h, int r, TravParams& P) {
+  const int nr = h->cfg.n_replicas, w = 2 * nr + 1;
+  P.ox = (r / (w * w) - nr) * h->cfg.period;
+  P.oy = (r / w % w - nr) * h->cfg.period;
+  P.oz = (r % w - nr) * h->cfg.period;
+}
+
 // Two-phase mixed evaluation: walk_lists writes every bucket's interaction
 // list to the pools, then eval_p2c and eval_p2p evaluate them.  Pools are
 // sized from the previous pass with a quarter of headroom (a bucket whose list
@@ -494,9 +502,9 @@ int run_two_phase(pt_handle* h, TravParams& P) {
     const unsigned region = h->l_region;
     const unsigned long long slack = (unsigned long long)wgrid * 4 * region;
     const unsigned long long need_pc =
-        std::max<unsigned long long>(h->want_pc ? h->want_pc + slack : 0, 1024ull * nb + slack);
+        std::max<unsigned long long>(h->want_pc, 1024ull * nb + slack);
     const unsigned long long need_pp =
-        std::max<unsigned long long>(h->want_pp ? h->want_pp + slack : 0, 256ull * nb + slack);
+        std::max<unsigned long long>(h->want_pp, 256ull * nb + slack);
     if (need_pc > h->cap_pc || need_pp > h->cap_pp) {
       // a quarter of headroom, so that the pass-to-pass variation of the
       // reserved regions does not free and map the multi-GB pools again
@@ -505,25 +513,32 @@ int run_two_phase(pt_handle* h, TravParams& P) {
       dfree(h->pool_pp);
       h->cap_pc = h->cap_pp = 0;
       unsigned long long alloc_pc = need_pc + need_pc / 4, alloc_pp = need_pp + need_pp / 4;
-      if (cudaMalloc((void**)&h->pool_pc, alloc_pc * sizeof(int32_t)) != cudaSuccess ||
-          cudaMalloc((void**)&h->pool_pp, alloc_pp * sizeof(int32_t)) != cudaSuccess) {
+      // an entry, and in a periodic pass its replica (a byte, behind the entries)
+      const size_t per = sizeof(int32_t) + (h->cfg.periodic ? 1 : 0);
+      if (cudaMalloc((void**)&h->pool_pc, alloc_pc * per) != cudaSuccess ||
+          cudaMalloc((void**)&h->pool_pp, alloc_pp * per) != cudaSuccess) {
         cudaGetLastError();
         dfree(h->pool_pc);
         dfree(h->pool_pp);
         alloc_pc = need_pc;
         alloc_pp = need_pp;
       }
-      if ((!h->pool_pc && cudaMalloc((void**)&h->pool_pc, need_pc * sizeof(int32_t)) != cudaSuccess) ||
-          (!h->pool_pp && cudaMalloc((void**)&h->pool_pp, need_pp * sizeof(int32_t)) != cudaSuccess)) {
+      if ((!h->pool_pc && cudaMalloc((void**)&h->pool_pc, need_pc * per) != cudaSuccess) ||
+          (!h->pool_pp && cudaMalloc((void**)&h->pool_pp, need_pp * per) != cudaSuccess)) {
         // no room for the lists: this handle evaluates with the fused kernel from now on
         cudaGetLastError();
         dfree(h->pool_pc);
         dfree(h->pool_pp);
         h->two_phase = false;
         CK(cudaMemcpyAsync(h->d_counters, c0, sizeof(c0), cudaMemcpyHostToDevice, st));
-        CKR(zero_queue(h));
-        if (h->cfg.precision == PT_FP64_LISTS) launch_traverse_f64(P, h->nd.mom, h->sms, st);
-        else launch_traverse_mixed(P, h->nd.mom, h->sms * 16, st);
+        for (int k = 0; k < std::max(1, P.rep_count); k++) {  // the batch's replicas one by one
+          TravParams A = P;
+          if (P.rep_count) replica_offset(h, P.rep_first + k, A);
+          A.accumulate = P.accumulate || k > 0;
+          CKR(zero_queue(h));
+          if (h->cfg.precision == PT_FP64_LISTS) launch_traverse_f64(A, h->nd.mom, h->sms, st);
+          else launch_traverse_mixed(A, h->nd.mom, h->sms * 16, st);
+        }
         CK(cudaGetLastError());
         return PT_OK;
       }
@@ -532,6 +547,10 @@ int run_two_phase(pt_handle* h, TravParams& P) {
     }
     L.pc_pool = h->pool_pc;
     L.pp_pool = h->pool_pp;
+    if (h->cfg.periodic) {
+      L.pc_rep = reinterpret_cast<uint8_t*>(h->pool_pc + h->cap_pc);
+      L.pp_rep = reinterpret_cast<uint8_t*>(h->pool_pp + h->cap_pp);
+    }
     L.cursor = h->d_lcur;
     L.cap_pc = h->cap_pc;
     L.cap_pp = h->cap_pp;
@@ -556,9 +575,12 @@ int run_two_phase(pt_handle* h, TravParams& P) {
     // the cursors count reserved regions (also refused ones): at most the pool size is used
     const unsigned long long used_pc = std::min(cur[0], h->cap_pc), used_pp = std::min(cur[1], h->cap_pp);
     if (!(status & kErrPool)) {
-      // next pass: room for this pass's lists and a quarter more
-      h->want_pc = std::max<unsigned long long>(h->want_pc, used_pc + used_pc / 4);
-      h->want_pp = std::max<unsigned long long>(h->want_pp, used_pp + used_pp / 4);
+      // next pass: room for this pass's regions and a sixteenth more (a pool is
+      // allocated a quarter larger than asked for, so it serves the next passes
+      // as it is: asking for a quarter more here made every handle's second pass
+      // allocate again, 129 instead of 90 ms at N = 2^24)
+      h->want_pc = std::max<unsigned long long>(h->want_pc, used_pc + used_pc / 16);
+      h->want_pp = std::max<unsigned long long>(h->want_pp, used_pp + used_pp / 16);
       break;
     }
     if (attempt >= 6) return fail(h, PT_E_NOMEM, "interaction lists outgrow their pools");
@@ -711,19 +733,22 @@ int traverse(pt_handle* h, int64_t b0, int64_t b1) {
   // GravityVisitor offsets (X, Y, Z) * L in that loop order; every walk after
   // the first continues each particle's sums
   const int nr = h->cfg.periodic ? h->cfg.n_replicas : 0;
-  const double L = h->cfg.period;
-  bool first = true;
-  for (int X = -nr; X <= nr; X++)
-    for (int Y = -nr; Y <= nr; Y++)
-      for (int Z = -nr; Z <= nr; Z++) {
-        P.ox = X * L;
-        P.oy = Y * L;
-        P.oz = Z * L;
-        P.accumulate = first ? 0 : 1;
-        first = false;
-        CKR(zero_queue(h));
-        CKR(run_traversal(h, P, grid));
-      }
+  const int reps = (2 * nr + 1) * (2 * nr + 1) * (2 * nr + 1);
+  // the two-phase forms take the replicas in batches, the mixed one up to
+  // kMaxReps at a time; the others one by one
+  int per = 1;
+  P.rep_n = nr;
+  P.period = h->cfg.period;
+  for (int r = 0; r < reps; r += per) {
+    const bool lists_form = (h->cfg.precision == PT_MIXED || h->cfg.precision == PT_FP64_LISTS) && h->two_phase;
+    per = h->cfg.precision == PT_MIXED && lists_form ? std::min(kMaxReps, reps - r) : 1;
+    if (h->cfg.periodic) replica_offset(h, r, P);
+    P.rep_first = r;
+    P.rep_count = reps > 1 && lists_form ? per : 0;
+    P.accumulate = r > 0;
+    CKR(zero_queue(h));
+    CKR(run_traversal(h, P, grid));
+  }
   if (h->cfg.periodic) CKR(ewald_correction_pass(h, b0, b1));
   CK(cudaEventRecord(h->ev[6], st));
   if (two_phase_record && h->tp_lists_valid) CKR(lists_from_pools(h));

@@ -18,6 +18,7 @@ constexpr int kTypeLeaf = 1;           // Node<Data>::Type numbering, src/Node.h
 constexpr int kTypeEmpty = 2;
 constexpr int kTypeInternal = 6;
 constexpr int kMinParticleNode = 6;    // examples/GravityVisitor.h:35
+constexpr int kMaxReps = 32;           // replicas the list kernels take in one batch (their roots: one lane each)
 
 // Device status word bits (written by kernels, read by the host after a pass).
 enum : unsigned {
@@ -134,6 +135,10 @@ struct TravParams {
   const int32_t* buckets; // bucket b -> node index (DFS order)
   int64_t b_begin, b_end;
   double ox, oy, oz;      // GravityVisitor offset (periodic replicas; 0 otherwise)
+  // list kernels: a batch of replicas, number rep_first .. rep_first + rep_count
+  // - 1 of the (2 rep_n + 1)^3 in the replica loop's order (rep_count = 0: none)
+  int rep_n, rep_first, rep_count;
+  double period;
   int64_t nnodes;
   int mode;               // 0 evaluate, 1 count lists only, 2 evaluate + record lists
   int accumulate;         // add to the stored accelerations (replica walks after the first)
@@ -157,6 +162,7 @@ struct TravParams {
 struct ListParams {
   int32_t* pc_pool;
   int32_t* pp_pool;
+  uint8_t *pc_rep, *pp_rep;    // the entries' replicas in the batch (periodic passes; else null)
   unsigned long long* cursor;  // [0] P2C pool, [1] P2P pool
   unsigned long long cap_pc, cap_pp;
   unsigned region, thresh;     // region size; least space left before a bucket starts
