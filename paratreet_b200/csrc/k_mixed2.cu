@@ -427,9 +427,38 @@ __device__ __forceinline__ void ev_two_zero(EvalWarp& w, int lane) {
   w.st[4][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// ev_finish for two-target lanes (P2P: adds to ax, ay, az and pot_full).
-__device__ __forceinline__ void ev_finish2(EvalWarp& w, const Kahan4& K, const EvTarget2& x, const TravParams& P,
-                                           int t0, int lane) {
+// Target t0 + lane's P2P sums v: added to ax, ay, az and pot_full (GravityVisitor::
+// leaf applies no potential).  A team's warps bring their sums together first
+// and warp 0 adds them, in the warps' order.
+template <int kTeam>
+__device__ __forceinline__ void ev_add(double (*team)[32][4], double v[4], int nt, const TravParams& P, int t0,
+                                       int lane) {
+  if (kTeam > 1) {
+    const int q = threadIdx.x >> 5;
+#pragma unroll
+    for (int k = 0; k < 4; k++) team[q][lane][k] = v[k];
+    __syncthreads();
+    if (q == 0) {
+#pragma unroll
+      for (int o = 1; o < kTeam; o++)
+        for (int k = 0; k < 4; k++) v[k] += team[o][lane][k];
+    }
+    __syncthreads();
+    if (q != 0) return;
+  }
+  if (lane < nt) {
+    const int i = t0 + lane;
+    P.p.ax[i] += v[0];
+    P.p.ay[i] += v[1];
+    P.p.az[i] += v[2];
+    P.p.potf[i] += v[3];
+  }
+}
+
+// Sum the G lane groups of each target, two targets per lane.
+template <int kTeam>
+__device__ __forceinline__ void ev_finish2(EvalWarp& w, double (*team)[32][4], const Kahan4& K, const EvTarget2& x,
+                                           const TravParams& P, int t0, int lane) {
   const float4 s2 = w.st[3][lane], c2 = w.st[4][lane];
   double* red = reinterpret_cast<double*>(&w.st[0][0]);
   __syncwarp();
@@ -446,38 +475,28 @@ __device__ __forceinline__ void ev_finish2(EvalWarp& w, const Kahan4& K, const E
     }
   }
   __syncwarp();
-  if (lane < x.nt) {
-    double v[4] = {0.0, 0.0, 0.0, 0.0};
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  if (lane < x.nt)
     for (int gg = 0; gg < x.G; gg++)
       for (int k = 0; k < 4; k++) v[k] += red[4 * (gg * x.nt + lane) + k];
-    const int i = t0 + lane;
-    P.p.ax[i] += v[0];
-    P.p.ay[i] += v[1];
-    P.p.az[i] += v[2];
-    P.p.potf[i] += v[3];
-  }
+  ev_add<kTeam>(team, v, x.nt, P, t0, lane);
 }
 
-// Sum the G lane groups of each target and add the result (P2P of a single
-// target; GravityVisitor::leaf applies no potential, so pot_full only).
-__device__ __forceinline__ void ev_finish(EvalWarp& w, const Kahan4& K, const EvTarget& x, const TravParams& P,
-                                          int t0, int lane) {
+// The same for a single target.
+template <int kTeam>
+__device__ __forceinline__ void ev_finish(EvalWarp& w, double (*team)[32][4], const Kahan4& K, const EvTarget& x,
+                                          const TravParams& P, int t0, int lane) {
   double* red = reinterpret_cast<double*>(&w.st[0][0]);
   __syncwarp();
 #pragma unroll
   for (int k = 0; k < 4; k++) red[4 * lane + k] = (double)K.s[k] - (double)K.c[k];
   __syncwarp();
-  if (lane < x.nt) {
-    double v[4] = {0.0, 0.0, 0.0, 0.0};
+  double v[4] = {0.0, 0.0, 0.0, 0.0};
+  if (lane < x.nt)
     for (int gg = 0; gg < x.G; gg++)
       for (int k = 0; k < 4; k++) v[k] += red[4 * (gg * x.nt + lane) + k];
-    const int i = t0 + lane;
-    P.p.ax[i] += v[0];
-    P.p.ay[i] += v[1];
-    P.p.az[i] += v[2];
-    P.p.potf[i] += v[3];
-  }
   __syncwarp();
+  ev_add<kTeam>(team, v, x.nt, P, t0, lane);
 }
 
 __device__ __forceinline__ bool next_bucket(const TravParams& P, int lane, int64_t& b, int& tnode) {
@@ -1135,24 +1154,43 @@ __device__ __forceinline__ unsigned long long ev_p2p_blocks(EvalWarp& w, const T
   return nsrc;
 }
 
-template <int kMinBlocks, bool kReps>
+// kTeam = 4: a CTA's warps share a bucket, each a quarter of its list (with few
+// buckets a pass takes as long as the longest list).
+template <int kMinBlocks, bool kReps, int kTeam>
 __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2p(TravParams P, ListParams L,
                                                                      const Mom* __restrict__ mom) {
   __shared__ EvalWarp warps[kEvWarps];
   __shared__ RepOffsets offs[1];
+  __shared__ double team[kTeam > 1 ? kTeam : 1][32][4];
+  __shared__ unsigned team_b;
   if (kReps) rep_offsets(P, offs[0]);
   EvalWarp& w = warps[threadIdx.x >> 5];
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
   unsigned long long c_pp = 0;
-  int64_t b;
-  int tnode;
   PROF_START(w);
-  while (next_bucket(P, lane, b, tnode)) {
+  while (true) {
+    unsigned bi;
+    if (kTeam > 1) {
+      if (threadIdx.x == 0) team_b = atomicAdd(P.work, 1u);
+      __syncthreads();
+      bi = team_b;
+      __syncthreads();
+    } else {
+      bi = grab_bucket(P.work, P.smq, P.batch, lane);
+    }
+    const int64_t b = P.b_begin + (int64_t)bi;
+    if (b >= P.b_end) break;
+    const int tnode = P.buckets[b];
     if (tnode < 0 || tnode >= P.nnodes) continue;
     const int64_t lb = b - P.b_begin;
-    const int64_t start = L.pp_start[lb];
-    const int count = L.pp_count[lb];
+    int64_t start = L.pp_start[lb];
+    int count = L.pp_count[lb];
     if (count == 0) continue;  // P2P only adds
+    if (kTeam > 1) {
+      const int per = (count + kTeam - 1) / kTeam, c0 = min(count, q * per);
+      start += c0;
+      count = min(count - c0, per);
+    }
     __syncwarp();
     if (lane == 0) load_bucket_geom(mom, tnode, w.geom);
     __syncwarp();
@@ -1161,27 +1199,27 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2p(TravParams
     PROF_MARK(w, 0);
     for (int tc = 0; tc < ntot; tc += 32) {
       const int t0 = tbase + tc, nt = min(32, ntot - tc);
+      Kahan4 K;
+      K.zero();
       if (ev_two_targets(nt)) {
         const EvTarget2 x = ev_target2(P.p, w.geom, t0, nt, lane);
         ev_two_zero(w, lane);
-        Kahan4 K;
-        K.zero();
         nsrc = ev_p2p_blocks<true, kReps>(w, P, L, offs, x, start, count, lane, K);
-        ev_finish2(w, K, x, P, t0, lane);
-        PROF_MARK(w, 4);
-        continue;
+        ev_finish2<kTeam>(w, team, K, x, P, t0, lane);
+      } else {
+        const EvTarget x = ev_target(P.p, w.geom, t0, nt, lane);
+        nsrc = ev_p2p_blocks<false, kReps>(w, P, L, offs, x, start, count, lane, K);
+        ev_finish<kTeam>(w, team, K, x, P, t0, lane);
       }
-      const EvTarget x = ev_target(P.p, w.geom, t0, nt, lane);
-      Kahan4 K;
-      K.zero();
-      nsrc = ev_p2p_blocks<false, kReps>(w, P, L, offs, x, start, count, lane, K);
-      ev_finish(w, K, x, P, t0, lane);
       PROF_MARK(w, 4);
     }
     // P2P pairs as the reference counts them (n_src * n_tgt per leaf(),
     // src/Traverser.h:27); the walk wrote the bucket's P2C work before
     c_pp += nsrc * (unsigned long long)ntot;
-    if (P.bucket_work && lane == 0) P.bucket_work[b] += nsrc * (unsigned long long)ntot;
+    if (P.bucket_work && lane == 0) {
+      if (kTeam > 1) atomicAdd(P.bucket_work + b, nsrc * (unsigned long long)ntot);
+      else P.bucket_work[b] += nsrc * (unsigned long long)ntot;
+    }
   }
   PROF_MARK(w, 5);
   PROF_FLUSH(w, 8);
@@ -1204,15 +1242,26 @@ void launch_walk_lists(const TravParams& P, const ListParams& L, const Mom* mom,
   if (P.rep_count) walk_lists<true><<<grid, kWlWarps * 32, 0, st>>>(P, L, mom);
   else walk_lists<false><<<grid, kWlWarps * 32, 0, st>>>(P, L, mom);
 }
-void launch_eval_lists(const TravParams& P, const TravParams& Q, const ListParams& L, const Mom* mom, int grid,
+void launch_eval_lists(const TravParams& P, const TravParams& Q, const ListParams& L, const Mom* mom, int sms,
                        cudaStream_t st) {
+  const int grid = 16 * sms;
   const int threads = kEvWarps * 32;
   note_launch();
   if (P.rep_count) eval_p2c2<PT_P2C_MINB, true><<<grid, threads, 0, st>>>(P, L, mom);
   else eval_p2c2<PT_P2C_MINB, false><<<grid, threads, 0, st>>>(P, L, mom);
   note_launch();
-  if (P.rep_count) eval_p2p<PT_P2P_MINB, true><<<grid, threads, 0, st>>>(Q, L, mom);
-  else eval_p2p<PT_P2P_MINB, false><<<grid, threads, 0, st>>>(Q, L, mom);
+  // Up to 96 buckets per SM (28 warps are resident), a CTA per bucket: the
+  // traversal of 4,000 particles 0.18 -> 0.13 ms, of 10,000 0.23-0.34 -> 0.18-
+  // 0.19, of 40,000 in buckets of 32 0.73 -> 0.47 and of 80,000 1.00 -> 0.80
+  // (Plummer); beyond it no difference.
+  const bool team = P.b_end - P.b_begin <= (int64_t)96 * sms;
+  if (P.rep_count) {
+    if (team) eval_p2p<PT_P2P_MINB, true, kEvWarps><<<grid, threads, 0, st>>>(Q, L, mom);
+    else eval_p2p<PT_P2P_MINB, true, 1><<<grid, threads, 0, st>>>(Q, L, mom);
+  } else {
+    if (team) eval_p2p<PT_P2P_MINB, false, kEvWarps><<<grid, threads, 0, st>>>(Q, L, mom);
+    else eval_p2p<PT_P2P_MINB, false, 1><<<grid, threads, 0, st>>>(Q, L, mom);
+  }
 }
 
 }  // namespace pt

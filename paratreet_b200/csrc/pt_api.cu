@@ -597,7 +597,7 @@ int run_two_phase(pt_handle* h, TravParams& P) {
   TravParams F = P;  // the P2P evaluation's
   use_queue(h, F, 2);
   if (h->cfg.precision == PT_FP64_LISTS) launch_eval_lists_f64(E, L, h->nd.mom, h->sms * 16, st, F.work);
-  else launch_eval_lists(E, F, L, h->nd.mom, h->sms * 16, st);
+  else launch_eval_lists(E, F, L, h->nd.mom, h->sms, st);
   CK(cudaGetLastError());
   h->tp_lists_valid = (P.b_begin == 0 && P.b_end == h->nbuckets && !h->cfg.periodic);
   return PT_OK;
