@@ -426,6 +426,9 @@ int ewald_correction_pass(pt_handle* h, int64_t b0, int64_t b1) {
         const int h2 = hx * hx + hy * hy + hz * hz;
         if (h2 == 0) continue;
         if (h2 > hcut * hcut) continue;
+        // h and -h have the same coefficient and add the same: the first of the
+        // two in this order stands for both
+        if (hx > 0 || (hx == 0 && (hy > 0 || (hy == 0 && hz > 0)))) continue;
         const double g0 = std::exp(-k4 * h2) / (M_PI * h2 * L);
         const double g1 = 2 * M_PI / L * g0;
         const double g2 = -2 * M_PI / L * g1;
@@ -436,7 +439,7 @@ int ewald_correction_pass(pt_handle* h, int64_t b0, int64_t b1) {
         double mfacc = 0.0;
         mfacc -= g2 * Qmir;
         mfacc -= g0 * root.mass;
-        tab.push_back(make_double4(2 * M_PI / L * hx, 2 * M_PI / L * hy, 2 * M_PI / L * hz, mfacc));
+        tab.push_back(make_double4(2 * M_PI / L * hx, 2 * M_PI / L * hy, 2 * M_PI / L * hz, 2.0 * mfacc));
       }
   if ((int)tab.size() > h->htab_cap) {
     CKR(dalloc(h, &h->d_htab, tab.size()));
