@@ -43,6 +43,10 @@ constexpr int kKnnStack = 640;   // pending frames: 4 popped per step, <= 32 pus
 constexpr int kKnnLeaves = 128;  // leaves buffered between flushes
 constexpr int kKnnChunk = 128;   // candidates staged per pass over the targets
 constexpr int kKnnNone = 0x7fffffff;
+// Passing candidates of a batch of 32 that are inserted one by one (about 20
+// instructions each); more are sorted and merged.  10^6 particles: 7.3, 6.9, 6.8,
+// 6.8 and 7.6 ms per density pass at 12, 16, 20, 24 and 32.
+constexpr int kKnnFew = 20;
 
 struct KnnWarp {
   double cx[kKnnChunk], cy[kKnnChunk], cz[kKnnChunk];  // staged candidates
@@ -111,17 +115,15 @@ __device__ __forceinline__ void knn_merge(double& ld, int& li, double bd, int bi
   for (int j = 16; j > 0; j >>= 1) knn_stage(ld, li, j, true, lane);
 }
 
-// Insert one candidate (cd, ci), known to beat the list's last entry.
+// Insert one candidate (cd, ci); one behind the whole list (no lane past it)
+// changes nothing, so an earlier insertion that raised the bar needs no test.
 __device__ __forceinline__ void knn_insert(double& ld, int& li, double cd, int ci, int lane) {
   const int pos = __popc(__ballot_sync(kFull, knn_before(ld, li, cd, ci)));  // entries that stay ahead
   const double ud = __shfl_up_sync(kFull, ld, 1);
   const int ui = __shfl_up_sync(kFull, li, 1);
-  if (lane == pos) {
-    ld = cd;
-    li = ci;
-  } else if (lane > pos) {
-    ld = ud;
-    li = ui;
+  if (lane >= pos) {
+    ld = lane == pos ? cd : ud;
+    li = lane == pos ? ci : ui;
   }
 }
 
@@ -154,28 +156,23 @@ __device__ __forceinline__ void knn_chunk(KnnWarp& w, int nt, int cnt, double* _
         li = Li[t * 32 + lane];
         loaded = true;
       }
-      if (__popc(m) <= 12) {
+      if (__popc(m) <= kKnnFew) {
         unsigned r = m;
         while (r) {
           const int src = __ffs(r) - 1;
           r &= r - 1u;
           const double cd = __shfl_sync(kFull, d2, src);
           const int cj = __shfl_sync(kFull, j, src);
-          // an earlier insertion of this batch may have raised the bar past it
-          if (knn_before(cd, cj, kd, ki)) {
-            knn_insert(ld, li, cd, cj, lane);
-            kd = __shfl_sync(kFull, ld, 31);
-            ki = __shfl_sync(kFull, li, 31);
-          }
+          knn_insert(ld, li, cd, cj, lane);
         }
       } else {
         double cd = pass ? d2 : CUDART_INF;
         int cj = pass ? j : kKnnNone;
         knn_sort32(cd, cj, lane);
         knn_merge(ld, li, cd, cj, lane);
-        kd = __shfl_sync(kFull, ld, 31);
-        ki = __shfl_sync(kFull, li, 31);
       }
+      kd = __shfl_sync(kFull, ld, 31);
+      ki = __shfl_sync(kFull, li, 31);
     }
     if (loaded) {
       Ld[t * 32 + lane] = ld;
@@ -331,8 +328,9 @@ __global__ void __launch_bounds__(kKnnWarps * 32, 7) sph_density_kernel(Particle
               const double* hi = mom[node].hi;
               const double nlo[3] = {lo[0], lo[1], lo[2]}, nhi[3] = {hi[0], hi[1], hi[2]};
               keep = box_box_gap2(nlo, nhi, blo, bhi) <= rmax * (1.0 + 1e-13);
-              // then the per-target test itself (DensityVisitor::open)
-              if (keep) {
+              // then, for a leaf, the per-target test itself (DensityVisitor::
+              // open; on Internal nodes it cost more than the visits it saved)
+              if (keep && !internal) {
                 keep = false;
                 for (int t = 0; t < nt && !keep; t++)
                   keep = box_d2(nlo, nhi, w.tx[t], w.ty[t], w.tz[t]) <= w.kd[t];
