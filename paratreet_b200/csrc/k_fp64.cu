@@ -45,25 +45,15 @@ __device__ __forceinline__ LaneMom lane_mom_clear() { return {0.0, 0.0, 0.0, DBL
 __device__ __forceinline__ int quad_i(int r) { return r < 3 ? 0 : r < 5 ? 1 : 2; }
 __device__ __forceinline__ int quad_j(int r) { return r < 3 ? r : r == 3 ? 1 : 2; }
 
-// q += (m2, lin2, quad2), a particle (quad2 = 0, leaf = true) or a child's
-// moments: MultipoleMoments::operator+=(Particle), examples/MultipoleMoments.h:
-// 274-353, and CentroidData::operator+= with MultipoleMoments::
-// operator+=(MultipoleMoments).  The group's lanes call it together.
-template <bool kLeaf>
-__device__ __forceinline__ void lane_mom_add(LaneMom& q, double m2, double lin2, double quad2, int r, unsigned gm) {
+// q += particle (m2, lin2): MultipoleMoments::operator+=(Particle),
+// examples/MultipoleMoments.h:274-353.  The group's lanes call it together.
+__device__ __forceinline__ void lane_mom_add(LaneMom& q, double m2, double lin2, int r, unsigned gm) {
   const double m1 = q.mass;
   q.mass += m2;
   if (q.mass == 0.0) {
     q.lin = 0.5 * (q.lin + lin2);
     return;
   }
-  if (!kLeaf && m1 == 0.0) {
-    q.mass = m2;
-    q.lin = lin2;
-    q.quad = quad2;
-    return;
-  }
-  if (!kLeaf && m2 == 0.0) return;
   const double old = q.lin;
   q.lin = (m1 * q.lin + m2 * lin2) / q.mass;
   const double d = old - q.lin, e = lin2 - q.lin;
@@ -71,8 +61,7 @@ __device__ __forceinline__ void lane_mom_add(LaneMom& q, double m2, double lin2,
   const double di = __shfl_sync(gm, d, i, 8), dj = __shfl_sync(gm, d, j, 8);
   const double ei = __shfl_sync(gm, e, i, 8), ej = __shfl_sync(gm, e, j, 8);
   q.quad += m1 * di * dj;
-  if (kLeaf) q.quad += m2 * ei * ej;
-  else q.quad += quad2 + m2 * ei * ej;
+  q.quad += m2 * ei * ej;
 }
 
 // The group's moments to the node's record.
@@ -116,7 +105,7 @@ __global__ void __launch_bounds__(256) leaf_moments(Nodes nd, const int32_t* __r
     if (src) {  // the FP64 evaluation's source records (x, y, z, m)
       if (r < 4) reinterpret_cast<double*>(src + j)[r] = r < 3 ? lin : pm;
     }
-    lane_mom_add<true>(q, pm, lin, 0.0, r, gm);
+    lane_mom_add(q, pm, lin, r, gm);
     if (lin < q.lo) q.lo = lin;
     if (lin > q.hi) q.hi = lin;
     smax = fmax(smax, lin);  // lane 3: the softening
@@ -143,7 +132,8 @@ __global__ void __launch_bounds__(256) leaf_moments(Nodes nd, const int32_t* __r
 // The nodes without Internal children start; the group that brings a parent its
 // last finished Internal child goes on with the parent (a counter per node, no
 // waiting).  The children's moments are read in one round (lane c child c) and
-// wait in shared memory while the group adds them in the order the reference's
+// wait in shared memory while the group adds them (CentroidData::operator+= with
+// MultipoleMoments::operator+=(MultipoleMoments)) in the order the reference's
 // FIFO delivers them.  One launch per level, one thread per node and a load
 // chain per child took 98 us at N = 4096 and 207 us at 2^20 (10-20 us per
 // level); this form with every lane doing all of a combine 48 us at 4096; this 38.
@@ -179,14 +169,47 @@ __global__ void __launch_bounds__(kClimbThreads) upward_climb(Nodes nd, int64_t 
     for (int o = 4; o; o >>= 1) cnt += __shfl_xor_sync(gm, cnt, o);
     __syncwarp(gm);
     LaneMom q = lane_mom_clear();
-    const int lin = 1 + min(r, 3), quad = 6 + min(r, 5), d = min(r, 2);
+    const int lin = 1 + min(r, 3), quad = 6 + min(r, 5), dim = min(r, 2);
     int src = 0;
+    // first the serial chain of masses and centres (a division per child), then
+    // the second moments, whose shuffles do not wait for one another
+    double m1[8], m2[8], od[8], nw[8], qd[8];
+    unsigned copy = 0, add = 0;
+#pragma unroll
     for (int a = 0; a < 8; a++) {
       src = __ffs(__ballot_sync(gm, rank == a) & gm) - 1 - (lane & 24);
       const double* c = K[src];
-      if (c[12 + d] < q.lo) q.lo = c[12 + d];
-      if (c[15 + d] > q.hi) q.hi = c[15 + d];
-      lane_mom_add<false>(q, c[0], c[lin], c[quad], r, gm);
+      if (c[12 + dim] < q.lo) q.lo = c[12 + dim];
+      if (c[15 + dim] > q.hi) q.hi = c[15 + dim];
+      const double l2 = c[lin];
+      m1[a] = q.mass;
+      m2[a] = c[0];
+      qd[a] = c[quad];
+      od[a] = q.lin;
+      q.mass += m2[a];
+      if (q.mass == 0.0) {
+        q.lin = 0.5 * (q.lin + l2);
+      } else if (m1[a] == 0.0) {
+        q.mass = m2[a];
+        q.lin = l2;
+        copy |= 1u << a;
+      } else if (m2[a] != 0.0) {
+        q.lin = (m1[a] * q.lin + m2[a] * l2) / q.mass;
+        add |= 1u << a;
+      }
+      od[a] -= q.lin;
+      nw[a] = l2 - q.lin;
+    }
+    const int qi = quad_i(r), qj = quad_j(r);
+#pragma unroll
+    for (int a = 0; a < 8; a++) {
+      const double di = __shfl_sync(gm, od[a], qi, 8), dj = __shfl_sync(gm, od[a], qj, 8);
+      const double ei = __shfl_sync(gm, nw[a], qi, 8), ej = __shfl_sync(gm, nw[a], qj, 8);
+      if ((copy >> a) & 1u) q.quad = qd[a];
+      if ((add >> a) & 1u) {
+        q.quad += m1[a] * di * dj;
+        q.quad += qd[a] + m2[a] * ei * ej;
+      }
     }
     double e;
     {

@@ -23,6 +23,14 @@
 
 using namespace pt;
 
+// What a pass writes for the host, and the counters' copy from before a list walk
+// (restored if the walk is repeated with larger pools).
+struct Words {
+  unsigned long long counters[3], lcur[3], saved[3];
+  unsigned status, ticket;
+  uint32_t total[kMaxDepth + 1];
+};
+
 struct pt_handle {
   pt_config cfg{};
   std::string err;
@@ -45,6 +53,10 @@ struct pt_handle {
   double* bbox_partial = nullptr;
   int bbox_blocks = 0;
   double* d_uni = nullptr;  // 12 doubles
+  // small device words in one block (Words), so that one copy brings the host all
+  // it reads back, into pinned memory
+  Words* d_words = nullptr;
+  Words* pin = nullptr;
   unsigned* d_status = nullptr;
   unsigned* d_ticket = nullptr;  // CTAs that finished the bounding box (0 between passes)
   unsigned long long* d_counters = nullptr;  // 3
@@ -262,10 +274,17 @@ int grow_nodes(pt_handle* h, int64_t need) {
   return PT_OK;
 }
 
-int read_status(pt_handle* h) {
-  unsigned st = 0;
-  CK(cudaMemcpyAsync(&st, h->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
+// The small words, as they stand after the work issued so far (synchronises).
+int read_words(pt_handle* h) {
+  CK(cudaMemcpyAsync(h->pin, h->d_words, sizeof(Words), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
+  return PT_OK;
+}
+
+// read_words and the status among them.
+int read_status(pt_handle* h) {
+  CKR(read_words(h));
+  const unsigned st = h->pin->status;
   if (st) {
     CK(cudaMemsetAsync(h->d_status, 0, sizeof(unsigned), h->stream));
     std::string m = "device status:";
@@ -328,9 +347,8 @@ int build_tree(pt_handle* h) {
   cudaStream_t st = h->stream;
   const int64_t n = h->n;
   launch_tree_count(h->p.key, n, h->cfg.bucket, h->tree_counts, h->d_total, st);
-  uint32_t tot[kMaxDepth + 1];  // Internal nodes of each level, leaves
-  CK(cudaMemcpyAsync(tot, h->d_total, sizeof(tot), cudaMemcpyDeviceToHost, st));
   CKR(read_status(h));  // synchronises; a failed sort ends the pass here
+  const uint32_t* tot = h->pin->total;  // Internal nodes of each level, leaves
   int64_t ni = 0;
   int depth = 0;
   for (int l = 0; l < kMaxDepth; l++) {
@@ -495,11 +513,11 @@ int run_two_phase(pt_handle* h, TravParams& P) {
     CKR(dalloc(h, &h->l_pp_count, cap));
     h->l_nb_cap = cap;
   }
-  if (!h->d_lcur) CKR(dalloc(h, &h->d_lcur, 3));
   const int wgrid = (int)std::max<int64_t>(1, std::min<int64_t>(walk_lists_grid(h->sms), (nb + 3) / 4));
-  unsigned long long c0[3];
-  CK(cudaMemcpyAsync(c0, h->d_counters, sizeof(c0), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+  CK(cudaMemcpyAsync(h->d_words->saved, h->d_counters, sizeof(h->d_words->saved), cudaMemcpyDeviceToDevice, st));
+  auto restore_counters = [&]() {
+    return cudaMemcpyAsync(h->d_counters, h->d_words->saved, sizeof(h->d_words->saved), cudaMemcpyDeviceToDevice, st);
+  };
   ListParams L{};
   for (int attempt = 0;; attempt++) {
     const unsigned region = h->l_region;
@@ -533,7 +551,7 @@ int run_two_phase(pt_handle* h, TravParams& P) {
         dfree(h->pool_pc);
         dfree(h->pool_pp);
         h->two_phase = false;
-        CK(cudaMemcpyAsync(h->d_counters, c0, sizeof(c0), cudaMemcpyHostToDevice, st));
+        CK(restore_counters());
         for (int k = 0; k < std::max(1, P.rep_count); k++) {  // the batch's replicas one by one
           TravParams A = P;
           if (P.rep_count) replica_offset(h, P.rep_first + k, A);
@@ -570,11 +588,9 @@ int run_two_phase(pt_handle* h, TravParams& P) {
     use_queue(h, A, 0);
     launch_walk_lists(A, L, h->nd.mom, wgrid, st);
     CK(cudaGetLastError());
-    unsigned status = 0;
-    unsigned long long cur[3];
-    CK(cudaMemcpyAsync(&status, h->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-    CK(cudaMemcpyAsync(cur, h->d_lcur, sizeof(cur), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    CKR(read_words(h));
+    unsigned status = h->pin->status;
+    const unsigned long long* cur = h->pin->lcur;
     // the cursors count reserved regions (also refused ones): at most the pool size is used
     const unsigned long long used_pc = std::min(cur[0], h->cap_pc), used_pp = std::min(cur[1], h->cap_pp);
     if (!(status & kErrPool)) {
@@ -591,7 +607,7 @@ int run_two_phase(pt_handle* h, TravParams& P) {
     // stop reserving once their pool is full)
     status &= ~kErrPool;
     CK(cudaMemcpyAsync(h->d_status, &status, sizeof(unsigned), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(h->d_counters, c0, sizeof(c0), cudaMemcpyHostToDevice, st));
+    CK(restore_counters());
     h->want_pc = std::max(2 * h->cap_pc, cur[0] + cur[0] / 2);
     h->want_pp = std::max(2 * h->cap_pp, cur[1] + cur[1] / 2);
   }
@@ -775,9 +791,7 @@ int forces(pt_handle* h, int64_t b0, int64_t b1) {
   CKR(upward(h));
   CKR(traverse(h, b0, b1));
   CKR(read_status(h));
-  unsigned long long c[3];
-  CK(cudaMemcpyAsync(c, h->d_counters, sizeof(c), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
+  const unsigned long long* c = h->pin->counters;
   pt_counters& k = h->last;
   k.n_pp = c[0];
   k.n_pc = c[1];
@@ -816,11 +830,19 @@ int timestep(pt_handle* h, double* dt) {
   return PT_OK;
 }
 
-int unpermute_f64(pt_handle* h, const double* dsrc, double* host_out) {
-  if (!host_out) return PT_OK;
-  launch_scatter_f64(dsrc, h->tmp[0], h->p.order, h->n, grid_for(h, h->n), h->stream);
-  CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(host_out, h->tmp[0], h->n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+// Sorted arrays to the caller's, in the caller's order (null outputs are left
+// out): each array is scattered to a buffer of its own, so that only the end is
+// waited for.
+int unpermute_all(pt_handle* h, const double* const* dsrc, double* const* host_out, int count) {
+  const int g = grid_for(h, h->n);
+  for (int k = 0; k < count; k++) {
+    if (!host_out[k]) continue;
+    double* const t = h->tmp[k];
+    launch_scatter_f64(dsrc[k], t, h->p.order, h->n, g, h->stream);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(host_out[k], t, h->n * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+  }
+  CK(cudaStreamSynchronize(h->stream));
   return PT_OK;
 }
 
@@ -897,14 +919,17 @@ int pt_create(const pt_config* cfg, pt_handle** out) {
   h->bbox_blocks = h->sms * 4;
   if (dalloc(h, &h->bbox_partial, 6 * (size_t)h->bbox_blocks) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_uni, 12) != PT_OK) return bail(PT_E_NOMEM);
-  if (dalloc(h, &h->d_status, 2) != PT_OK) return bail(PT_E_NOMEM);
-  h->d_ticket = h->d_status + 1;
-  if (dalloc(h, &h->d_counters, 3) != PT_OK) return bail(PT_E_NOMEM);
+  if (dalloc(h, &h->d_words, 1) != PT_OK) return bail(PT_E_NOMEM);
+  if (cudaMallocHost((void**)&h->pin, sizeof(Words)) != cudaSuccess) return bail(PT_E_NOMEM);
+  h->d_status = &h->d_words->status;
+  h->d_ticket = &h->d_words->ticket;
+  h->d_counters = h->d_words->counters;
+  h->d_lcur = h->d_words->lcur;
+  h->d_total = h->d_words->total;
   if (dalloc(h, &h->d_work, 1) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_queue, 3 * kQueueWords) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_vmax2, 1) != PT_OK) return bail(PT_E_NOMEM);
-  if (dalloc(h, &h->d_total, tree_columns()) != PT_OK) return bail(PT_E_NOMEM);
-  if (cudaMemset(h->d_status, 0, 2 * sizeof(unsigned)) != cudaSuccess) return bail(PT_E_CUDA);
+  if (cudaMemset(h->d_words, 0, sizeof(Words)) != cudaSuccess) return bail(PT_E_CUDA);
   *out = h;
   return PT_OK;
 }
@@ -913,8 +938,8 @@ int pt_destroy(pt_handle* h) {
   if (!h) return PT_OK;
   cudaSetDevice(h->cfg.device);
   if (h->stream) cudaStreamSynchronize(h->stream);
-  dfree(h->slab); dfree(h->d_total); dfree(h->bbox_partial); dfree(h->d_uni);
-  dfree(h->d_status); dfree(h->d_counters); dfree(h->d_work); dfree(h->d_vmax2); dfree(h->src); dfree(h->srcf); dfree(h->softf);
+  dfree(h->slab); dfree(h->bbox_partial); dfree(h->d_uni);
+  dfree(h->d_words); dfree(h->d_work); dfree(h->d_vmax2); dfree(h->src); dfree(h->srcf); dfree(h->softf);
   Nodes& o = h->nd;
   dfree(o.key); dfree(o.type); dfree(o.depth); dfree(o.pstart); dfree(o.pcount); dfree(o.parent);
   dfree(o.first_child); dfree(o.count); dfree(o.mom); dfree(o.walk); dfree(o.walks); dfree(o.quad); dfree(o.quadf);
@@ -923,9 +948,10 @@ int pt_destroy(pt_handle* h) {
   dfree(h->list_kind); dfree(h->dsum); dfree(h->adj); dfree(h->nadj); dfree(h->d_htab); dfree(h->ewd); dfree(h->sph); dfree(h->sph_nbr); dfree(h->sph_nd2);
   dfree(h->sph_list_d); dfree(h->sph_list_i); dfree(h->sph_state);
   dfree(h->pool_pc); dfree(h->pool_pp); dfree(h->l_pc_start); dfree(h->l_pp_start); dfree(h->l_pc_count);
-  dfree(h->l_pp_count); dfree(h->d_lcur); dfree(h->d_queue);
+  dfree(h->l_pp_count); dfree(h->d_queue);
   for (auto& e : h->ev)
     if (e) cudaEventDestroy(e);
+  if (h->pin) cudaFreeHost(h->pin);
   if (h->own_stream) cudaStreamDestroy(h->own_stream);
   delete h;
   return PT_OK;
@@ -1003,11 +1029,7 @@ int pt_get_accel(pt_handle* h, double* ax, double* ay, double* az, double* pot, 
   cudaSetDevice(h->cfg.device);
   const double* src[5] = {h->p.ax, h->p.ay, h->p.az, h->p.pot, h->p.potf};
   double* dst[5] = {ax, ay, az, pot, pot_full};
-  for (int i = 0; i < 5; i++) {
-    CKR(unpermute_f64(h, src[i], dst[i]));
-    if (dst[i]) CK(cudaStreamSynchronize(h->stream));
-  }
-  return PT_OK;
+  return unpermute_all(h, src, dst, 5);
 }
 
 int pt_device_accel(pt_handle* h, double** ax, double** ay, double** az, double** pot, double** pot_full,
@@ -1072,10 +1094,9 @@ int pt_sph_density(pt_handle* h, double* density, double* ball_sq, int32_t* nbr,
   if (n == 0) return PT_OK;
   const bool want_nbr = nbr != nullptr;
   CKR(sph_density_device(h, want_nbr));
-  CKR(unpermute_f64(h, h->sph, density));
-  CK(cudaStreamSynchronize(st));
-  CKR(unpermute_f64(h, h->sph + n, ball_sq));
-  CK(cudaStreamSynchronize(st));
+  const double* src[2] = {h->sph, h->sph + n};
+  double* dst[2] = {density, ball_sq};
+  CKR(unpermute_all(h, src, dst, 2));
   if (want_nbr) {
     // neighbours of sorted particle i -> caller order, each list sorted by (d2, caller index)
     std::vector<int32_t> hn((size_t)n * k), order(n);
@@ -1122,11 +1143,7 @@ int pt_sph_pressure(pt_handle* h, const double* u, double* density, double* ax, 
   CKR(read_status(h));
   double* dst[5] = {density, ax, ay, az, pdv};
   const double* src[5] = {h->sph, out, out + n, out + 2 * n, out + 3 * n};
-  for (int i = 0; i < 5; i++) {
-    CKR(unpermute_f64(h, src[i], dst[i]));
-    CK(cudaStreamSynchronize(st));
-  }
-  return PT_OK;
+  return unpermute_all(h, src, dst, 5);
 }
 
 // nsteps iterations of the SPH example: density pass, pressure pass with the
@@ -1244,11 +1261,7 @@ int pt_get_state(pt_handle* h, double* x, double* y, double* z, double* vx, doub
   cudaSetDevice(h->cfg.device);
   const double* src[6] = {h->p.x, h->p.y, h->p.z, h->p.vx, h->p.vy, h->p.vz};
   double* dst[6] = {x, y, z, vx, vy, vz};
-  for (int i = 0; i < 6; i++) {
-    CKR(unpermute_f64(h, src[i], dst[i]));
-    if (dst[i]) CK(cudaStreamSynchronize(h->stream));
-  }
-  return PT_OK;
+  return unpermute_all(h, src, dst, 6);
 }
 
 int pt_last_dt(const pt_handle* h, double* dt) {
