@@ -33,7 +33,7 @@ namespace pt {
 
 // Moments of one node held by eight lanes (r = lane & 7): lane r < 3 has centre
 // coordinate r and the box along it, lane 3 the softening, lane r < 6 the second
-// moment (i, j) of kQi / kQj; the mass is on every lane.  A combine then takes one
+// moment (quad_i, quad_j); the mass is on every lane.  A combine then takes one
 // IEEE division per lane instead of four in a row on one lane, and the
 // additions of the reference's moments stay in its order.
 struct LaneMom {
@@ -44,25 +44,6 @@ __device__ __forceinline__ LaneMom lane_mom_clear() { return {0.0, 0.0, 0.0, DBL
 // second moments in the order of Mom: xx xy xz yy yz zz
 __device__ __forceinline__ int quad_i(int r) { return r < 3 ? 0 : r < 5 ? 1 : 2; }
 __device__ __forceinline__ int quad_j(int r) { return r < 3 ? r : r == 3 ? 1 : 2; }
-
-// q += particle (m2, lin2): MultipoleMoments::operator+=(Particle),
-// examples/MultipoleMoments.h:274-353.  The group's lanes call it together.
-__device__ __forceinline__ void lane_mom_add(LaneMom& q, double m2, double lin2, int r, unsigned gm) {
-  const double m1 = q.mass;
-  q.mass += m2;
-  if (q.mass == 0.0) {
-    q.lin = 0.5 * (q.lin + lin2);
-    return;
-  }
-  const double old = q.lin;
-  q.lin = (m1 * q.lin + m2 * lin2) / q.mass;
-  const double d = old - q.lin, e = lin2 - q.lin;
-  const int i = quad_i(r), j = quad_j(r);
-  const double di = __shfl_sync(gm, d, i, 8), dj = __shfl_sync(gm, d, j, 8);
-  const double ei = __shfl_sync(gm, e, i, 8), ej = __shfl_sync(gm, e, j, 8);
-  q.quad += m1 * di * dj;
-  q.quad += m2 * ei * ej;
-}
 
 // The group's moments to the node's record.
 __device__ __forceinline__ void lane_mom_store(Mom* __restrict__ out, const LaneMom& q, double radius, double reach,
@@ -81,50 +62,77 @@ __device__ __forceinline__ void lane_mom_store(Mom* __restrict__ out, const Lane
 }
 static_assert(sizeof(Mom) == 20 * sizeof(double), "lane_mom_store writes Mom's twenty doubles");
 
-// CentroidData(particles, n, depth) of every bucket, eight lanes per leaf.  (One
-// thread per node, four divisions in a row per particle, took 15-29 us at up to
-// 10^5 particles; this 9 us at 4096 and 10,000.)
+// CentroidData(particles, n, depth) of every bucket, four lanes per leaf: lane
+// r < 3 centre coordinate r and the box along it, lane 3 the softening, each with
+// one or two of the second moments; MultipoleMoments::operator+=(Particle),
+// examples/MultipoleMoments.h:274-353, particle by particle.  (One thread per
+// node, four divisions in a row per particle: 16-29 us at up to 10^5 particles,
+// 495 us at 2^24; eight lanes with one second moment each: 9 and 934 us, twice
+// the warps for the same chain.)
 __global__ void __launch_bounds__(256) leaf_moments(Nodes nd, const int32_t* __restrict__ buckets, int64_t nbuckets,
                                                     Particles p, double4* __restrict__ src) {
-  const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3;
+  const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 2;
   if (g >= nbuckets) return;
-  const int lane = threadIdx.x & 31, r = lane & 7;
-  const unsigned gm = 0xffu << (lane & 24);
+  const int lane = threadIdx.x & 31, r = lane & 3;
+  const unsigned gm = 0xfu << (lane & 28);
   const int node = buckets[g];
   const int s0 = nd.pstart[node], sn = nd.pcount[node];
   const double* const field = r == 0 ? p.x : r == 1 ? p.y : r == 2 ? p.z : p.soft;
-  LaneMom q = lane_mom_clear();
-  double smax = 0.0;
+  double mass = 0.0, lin = 0.0, lo = DBL_MAX, hi = -DBL_MAX, smax = 0.0;
+  double qa = 0.0, qb = 0.0;  // xx xy xz yy by lane, and yz zz on lanes 0 and 1
   double v = field[s0], m = p.m[s0];
   for (int j = s0; j < s0 + sn; j++) {
-    const double lin = v, pm = m;
+    const double l2 = v, m2 = m, m1 = mass;
     if (j + 1 < s0 + sn) {
       v = field[j + 1];
       m = p.m[j + 1];
     }
-    if (src) {  // the FP64 evaluation's source records (x, y, z, m)
-      if (r < 4) reinterpret_cast<double*>(src + j)[r] = r < 3 ? lin : pm;
+    // the FP64 evaluation's source records (x, y, z, m)
+    if (src) reinterpret_cast<double*>(src + j)[r] = r < 3 ? l2 : m2;
+    if (l2 < lo) lo = l2;
+    if (l2 > hi) hi = l2;
+    smax = fmax(smax, l2);  // lane 3: the softening
+    mass += m2;
+    if (mass == 0.0) {
+      lin = 0.5 * (lin + l2);
+      continue;
     }
-    lane_mom_add(q, pm, lin, r, gm);
-    if (lin < q.lo) q.lo = lin;
-    if (lin > q.hi) q.hi = lin;
-    smax = fmax(smax, lin);  // lane 3: the softening
+    const double old = lin;
+    lin = (m1 * lin + m2 * l2) / mass;
+    const double d = old - lin, e = l2 - lin;
+    const double d0 = __shfl_sync(gm, d, 0, 4), d1 = __shfl_sync(gm, d, 1, 4), d2 = __shfl_sync(gm, d, 2, 4);
+    const double e0 = __shfl_sync(gm, e, 0, 4), e1 = __shfl_sync(gm, e, 1, 4), e2 = __shfl_sync(gm, e, 2, 4);
+    const bool yy = r == 3;
+    qa += m1 * (yy ? d1 : d0) * (yy ? d1 : d);
+    qa += m2 * (yy ? e1 : e0) * (yy ? e1 : e);
+    qb += m1 * (r == 0 ? d1 : d2) * d2;
+    qb += m2 * (r == 0 ? e1 : e2) * e2;
   }
-  const double w = q.hi - q.lo;
-  const double wx = __shfl_sync(gm, w, 0, 8), wy = __shfl_sync(gm, w, 1, 8), wz = __shfl_sync(gm, w, 2, 8);
-  const double radius = sn > 1 ? 0.5 * sqrt(wx * wx + wy * wy + wz * wz) : 1.0;
+  const double w = hi - lo;
+  const double wx = __shfl_sync(gm, w, 0, 4), wy = __shfl_sync(gm, w, 1, 4), wz = __shfl_sync(gm, w, 2, 4);
   // not part of the reference's data: reach and max softening of the leaf,
   // used only to select the mixed form's unsoftened fast path
-  const double cx = __shfl_sync(gm, q.lin, 0, 8), cy = __shfl_sync(gm, q.lin, 1, 8), cz = __shfl_sync(gm, q.lin, 2, 8);
+  const double cx = __shfl_sync(gm, lin, 0, 4), cy = __shfl_sync(gm, lin, 1, 4), cz = __shfl_sync(gm, lin, 2, 4);
   double r2max = 0.0;
-  for (int j = s0 + r; j < s0 + sn; j += 8) {
+  for (int j = s0 + r; j < s0 + sn; j += 4) {
     const double dx = p.x[j] - cx, dy = p.y[j] - cy, dz = p.z[j] - cz;
     r2max = fmax(r2max, dx * dx + dy * dy + dz * dz);
   }
-#pragma unroll
-  for (int o = 4; o; o >>= 1) r2max = fmax(r2max, __shfl_xor_sync(gm, r2max, o));
-  smax = __shfl_sync(gm, smax, 3, 8);
-  lane_mom_store(nd.mom + node, q, radius, sqrt(r2max), smax, r);
+  r2max = fmax(r2max, __shfl_xor_sync(gm, r2max, 2));
+  r2max = fmax(r2max, __shfl_xor_sync(gm, r2max, 1));
+  double* const o = reinterpret_cast<double*>(nd.mom + node);  // mass cm soft radius | xx .. zz | lo hi | reach soft_max
+  o[1 + r] = lin;
+  o[6 + r] = qa;
+  if (r < 2) o[10 + r] = qb;
+  if (r < 3) {
+    o[12 + r] = lo;
+    o[15 + r] = hi;
+  } else {
+    o[19] = smax;
+  }
+  if (r == 0) o[0] = mass;
+  if (r == 1) o[5] = sn > 1 ? 0.5 * sqrt(wx * wx + wy * wy + wz * wz) : 1.0;
+  if (r == 2) o[18] = sqrt(r2max);
   if (r == 0) nd.count[node] = sn;
 }
 
@@ -844,7 +852,7 @@ static inline unsigned blocks_for(int64_t n, int t = 256) { return (unsigned)((n
 
 void launch_leaf_moments(Nodes nd, const int32_t* buckets, int64_t nbuckets, Particles p, double4* src,
                          cudaStream_t st) {
-  if (nbuckets > 0) { note_launch(); leaf_moments<<<blocks_for(8 * nbuckets), 256, 0, st>>>(nd, buckets, nbuckets, p, src); }
+  if (nbuckets > 0) { note_launch(); leaf_moments<<<blocks_for(4 * nbuckets), 256, 0, st>>>(nd, buckets, nbuckets, p, src); }
 }
 void launch_upward(Nodes nd, int64_t ninternal, cudaStream_t st) {
   if (ninternal > 0) { note_launch(); upward_climb<<<blocks_for(8 * ninternal, kClimbThreads), kClimbThreads, 0, st>>>(nd, ninternal); }

@@ -431,17 +431,17 @@ __device__ __forceinline__ void ev_two_zero(EvalWarp& w, int lane) {
 // leaf applies no potential).  A team's warps bring their sums together first
 // and warp 0 adds them, in the warps' order.
 template <int kTeam>
-__device__ __forceinline__ void ev_add(double (*team)[32][4], double v[4], int nt, const TravParams& P, int t0,
+__device__ __forceinline__ void ev_add(double* team, double v[4], int nt, const TravParams& P, int t0,
                                        int lane) {
   if (kTeam > 1) {
     const int q = threadIdx.x >> 5;
 #pragma unroll
-    for (int k = 0; k < 4; k++) team[q][lane][k] = v[k];
+    for (int k = 0; k < 4; k++) team[(q * 32 + lane) * 4 + k] = v[k];
     __syncthreads();
     if (q == 0) {
 #pragma unroll
       for (int o = 1; o < kTeam; o++)
-        for (int k = 0; k < 4; k++) v[k] += team[o][lane][k];
+        for (int k = 0; k < 4; k++) v[k] += team[(o * 32 + lane) * 4 + k];
     }
     __syncthreads();
     if (q != 0) return;
@@ -457,7 +457,7 @@ __device__ __forceinline__ void ev_add(double (*team)[32][4], double v[4], int n
 
 // Sum the G lane groups of each target, two targets per lane.
 template <int kTeam>
-__device__ __forceinline__ void ev_finish2(EvalWarp& w, double (*team)[32][4], const Kahan4& K, const EvTarget2& x,
+__device__ __forceinline__ void ev_finish2(EvalWarp& w, double* team, const Kahan4& K, const EvTarget2& x,
                                            const TravParams& P, int t0, int lane) {
   const float4 s2 = w.st[3][lane], c2 = w.st[4][lane];
   double* red = reinterpret_cast<double*>(&w.st[0][0]);
@@ -484,7 +484,7 @@ __device__ __forceinline__ void ev_finish2(EvalWarp& w, double (*team)[32][4], c
 
 // The same for a single target.
 template <int kTeam>
-__device__ __forceinline__ void ev_finish(EvalWarp& w, double (*team)[32][4], const Kahan4& K, const EvTarget& x,
+__device__ __forceinline__ void ev_finish(EvalWarp& w, double* team, const Kahan4& K, const EvTarget& x,
                                           const TravParams& P, int t0, int lane) {
   double* red = reinterpret_cast<double*>(&w.st[0][0]);
   __syncwarp();
@@ -1161,7 +1161,7 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2p(TravParams
                                                                      const Mom* __restrict__ mom) {
   __shared__ EvalWarp warps[kEvWarps];
   __shared__ RepOffsets offs[1];
-  __shared__ double team[kTeam > 1 ? kTeam : 1][32][4];
+  __shared__ double team[kTeam > 1 ? kTeam * 128 : 1];  // a team's sums, [warp][target][4]
   __shared__ unsigned team_b;
   if (kReps) rep_offsets(P, offs[0]);
   EvalWarp& w = warps[threadIdx.x >> 5];
