@@ -76,7 +76,7 @@ __device__ __forceinline__ void spline_b_db(double r2, double ir, double twoh, d
 // Work layout of adjoint_lists: one warp per bucket, the bucket's n_t targets
 // two per lane in groups of h = ceil(n_t / 2) lanes, replicated over
 // G = floor(32 / h) lane groups (as the evaluation kernels do).  A chunk of up
-// to 32 list nodes, or of 32 source particles of the listed leaves, is staged
+// to 64 list nodes, or of 64 source particles of the listed leaves, is staged
 // in shared memory with one adjoint accumulator row per staged slot; group g
 // takes the slots g, g + G, ...  Inside a group, at step s lane t handles its
 // group's slot number (s + t) mod L (L = max(h, the group's slots)), so no two
@@ -85,10 +85,14 @@ __device__ __forceinline__ void spline_b_db(double r2, double ir, double twoh, d
 // target-side terms stay in registers; the source-side ones are added to the
 // slot's row and flushed with one atomic add per slot and value after the
 // chunk.  Atomic adds make the last bits of the results order-dependent.
+// Slots per chunk: a chunk of n takes max(h, n / G) steps, so with buckets of 5
+// targets (h = 3, G = 10) 32 slots keep 75% of the lanes busy and 64 keep 86%.
+constexpr int kAdjSlots = 64;
+
 struct AdjWarp {
-  double st[12][32];   // staged slot data: P2C cm x/y/z, M, xx, xy, xz, yy, yz, zz, kind, soft; P2P x/y/z, m, soft
-  double acc[10][32];  // per slot adjoint rows: node (cm x/y/z, M, 6 moments) or source (x/y/z, m)
-  int32_t sidx[32];    // the slot's node or particle index
+  double st[12][kAdjSlots];   // staged slot data: P2C cm x/y/z, M, xx, xy, xz, yy, yz, zz, kind, soft; P2P x/y/z, m, soft
+  double acc[10][kAdjSlots];  // per slot adjoint rows: node (cm x/y/z, M, 6 moments) or source (x/y/z, m)
+  int32_t sidx[kAdjSlots];    // the slot's node or particle index
   int32_t lnode[32];   // P2P: the window's leaves
   int32_t lincl[32];   // P2P: inclusive prefix of their particle counts
   int32_t lpst[32];    // P2P: their first particles
@@ -235,11 +239,11 @@ __device__ __forceinline__ AdjTgt adj_load_target(const AdjParams& A, int i) {
   return t;
 }
 
-// CTAs per SM of adjoint_lists: 5 (96 registers, a little spilled) measured
-// faster than the 4 that 124 registers allow (13.0 -> 11.7 ms); 6 and 7 spill
-// far more (14.4 and 15.8 ms)
+// CTAs per SM of adjoint_lists: 4 (126 registers, 47 KB of shared memory each).
+// Hernquist N = 262,144, theta 0.6: 10.3 ms; with chunks of 32 slots 5 CTAs (96
+// registers, some spilled) took 11.1 and 4 took 10.8 ms.
 #ifndef PT_ADJ_MINB
-#define PT_ADJ_MINB 5
+#define PT_ADJ_MINB 4
 #endif
 __global__ void __launch_bounds__(kAdjWarps * 32, PT_ADJ_MINB) adjoint_lists(AdjParams A) {
   __shared__ AdjWarp warps[kAdjWarps];
@@ -276,50 +280,63 @@ __global__ void __launch_bounds__(kAdjWarps * 32, PT_ADJ_MINB) adjoint_lists(Adj
       if (x.two) x.b = adj_load_target(A, t0 + x.t2);
       double g[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // target-side sums of the lane's targets
       ADJ_MARK(0);
-      // P2C: the list's nodes, 32 at a time
-      for (int64_t win = e0; win < e1; win += 32) {
-        const int64_t e = win + lane;
-        int node = -1, kind = 0;
-        if (e < e1) {
-          kind = A.list_kind[e];
-          node = A.list_node[e];
-          if (node < 0 || node >= A.nnodes) {
-            atomicOr(A.status, kErrCapacity);
-            kind = 0;
-          } else if (kind != 0 && A.walk[node].count == 0) {
-            kind = 0;  // node() of an empty node adds nothing
+      // P2C: the list's nodes, kAdjSlots at a time
+      for (int64_t win = e0; win < e1; win += kAdjSlots) {
+        int node[2];
+        bool sel[2];
+        int kind[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+          const int64_t e = win + lane + 32 * u;
+          node[u] = -1;
+          kind[u] = 0;
+          if (e < e1) {
+            kind[u] = A.list_kind[e];
+            node[u] = A.list_node[e];
+            if (node[u] < 0 || node[u] >= A.nnodes) {
+              atomicOr(A.status, kErrCapacity);
+              kind[u] = 0;
+            } else if (kind[u] != 0 && A.walk[node[u]].count == 0) {
+              kind[u] = 0;  // node() of an empty node adds nothing
+            }
           }
+          sel[u] = kind[u] != 0;
         }
-        const bool sel = e < e1 && kind != 0;
-        const unsigned m = __ballot_sync(kAdjFull, sel);
-        const int n = __popc(m);
+        const unsigned m0 = __ballot_sync(kAdjFull, sel[0]), m1 = __ballot_sync(kAdjFull, sel[1]);
+        const int n = __popc(m0) + __popc(m1);
         if (n == 0) continue;
         __syncwarp();
-        if (sel) {
-          const int k = __popc(m & ((1u << lane) - 1u));
-          const WalkRec& r = A.walk[node];
-          const QuadRec q = A.quad[node];
-          w.sidx[k] = node;
-          w.st[0][k] = r.cm[0]; w.st[1][k] = r.cm[1]; w.st[2][k] = r.cm[2];
-          w.st[3][k] = q.mass;
-          w.st[4][k] = q.xx; w.st[5][k] = q.xy; w.st[6][k] = q.xz;
-          w.st[7][k] = q.yy; w.st[8][k] = q.yz; w.st[9][k] = q.zz;
-          w.st[10][k] = (double)kind;
-          w.st[11][k] = q.soft;
-        }
 #pragma unroll
-        for (int q = 0; q < 10; q++) w.acc[q][lane] = 0.0;
+        for (int u = 0; u < 2; u++) {
+          if (sel[u]) {
+            const unsigned lt = (1u << lane) - 1u;
+            const int k = u ? __popc(m0) + __popc(m1 & lt) : __popc(m0 & lt);
+            const WalkRec& r = A.walk[node[u]];
+            const QuadRec q = A.quad[node[u]];
+            w.sidx[k] = node[u];
+            w.st[0][k] = r.cm[0]; w.st[1][k] = r.cm[1]; w.st[2][k] = r.cm[2];
+            w.st[3][k] = q.mass;
+            w.st[4][k] = q.xx; w.st[5][k] = q.xy; w.st[6][k] = q.xz;
+            w.st[7][k] = q.yy; w.st[8][k] = q.yz; w.st[9][k] = q.zz;
+            w.st[10][k] = (double)kind[u];
+            w.st[11][k] = q.soft;
+          }
+        }
+        for (int k = lane; k < n; k += 32) {
+#pragma unroll
+          for (int q = 0; q < 10; q++) w.acc[q][k] = 0.0;
+        }
         __syncwarp();
         adj_rotate<true>(w, n, x, g, A.status);
-        if (lane < n) {
-          double* na = A.nadj + 10 * (int64_t)w.sidx[lane];
+        for (int k = lane; k < n; k += 32) {
+          double* na = A.nadj + 10 * (int64_t)w.sidx[k];
 #pragma unroll
-          for (int q = 0; q < 10; q++) atomicAdd(na + q, w.acc[q][lane]);
+          for (int q = 0; q < 10; q++) atomicAdd(na + q, w.acc[q][k]);
         }
         __syncwarp();
       }
       ADJ_MARK(1);
-      // P2P: the listed leaves' particles, 32 at a time
+      // P2P: the listed leaves' particles, kAdjSlots at a time
       for (int64_t win = e0; win < e1; win += 32) {
         const int64_t e = win + lane;
         int node = -1;
@@ -350,10 +367,10 @@ __global__ void __launch_bounds__(kAdjWarps * 32, PT_ADJ_MINB) adjoint_lists(Adj
           w.lpst[k] = pst;
         }
         __syncwarp();
-        for (int cs = 0; cs < total; cs += 32) {
-          const int q = cs + lane;
-          const int n = min(32, total - cs);
-          if (q < total) {
+        for (int cs = 0; cs < total; cs += kAdjSlots) {
+          const int n = min(kAdjSlots, total - cs);
+          for (int k = lane; k < n; k += 32) {
+            const int q = cs + k;
             int lo = 0, hi = nl - 1;  // the first leaf with inclusive prefix > q
             while (lo < hi) {
               const int mid = (lo + hi) >> 1;
@@ -362,20 +379,20 @@ __global__ void __launch_bounds__(kAdjWarps * 32, PT_ADJ_MINB) adjoint_lists(Adj
             }
             const int first = (lo == 0) ? 0 : w.lincl[lo - 1];
             const int j = w.lpst[lo] + (q - first);
-            w.sidx[lane] = j;
-            w.st[0][lane] = A.p.x[j]; w.st[1][lane] = A.p.y[j]; w.st[2][lane] = A.p.z[j];
-            w.st[3][lane] = A.p.m[j]; w.st[4][lane] = A.p.soft[j];
-          }
+            w.sidx[k] = j;
+            w.st[0][k] = A.p.x[j]; w.st[1][k] = A.p.y[j]; w.st[2][k] = A.p.z[j];
+            w.st[3][k] = A.p.m[j]; w.st[4][k] = A.p.soft[j];
 #pragma unroll
-          for (int r = 0; r < 4; r++) w.acc[r][lane] = 0.0;
+            for (int r = 0; r < 4; r++) w.acc[r][k] = 0.0;
+          }
           __syncwarp();
           adj_rotate<false>(w, n, x, g, A.status);
-          if (lane < n) {
-            const int j = w.sidx[lane];
-            atomicAdd(&A.gx[j], w.acc[0][lane]);
-            atomicAdd(&A.gy[j], w.acc[1][lane]);
-            atomicAdd(&A.gz[j], w.acc[2][lane]);
-            atomicAdd(&A.gm[j], w.acc[3][lane]);
+          for (int k = lane; k < n; k += 32) {
+            const int j = w.sidx[k];
+            atomicAdd(&A.gx[j], w.acc[0][k]);
+            atomicAdd(&A.gy[j], w.acc[1][k]);
+            atomicAdd(&A.gz[j], w.acc[2][k]);
+            atomicAdd(&A.gm[j], w.acc[3][k]);
           }
           __syncwarp();
         }
