@@ -172,6 +172,96 @@ __global__ void __launch_bounds__(256) pools_to_csr(const int32_t* __restrict__ 
   }
 }
 
+// Exclusive prefix of pc_count + pp_count over the buckets, in three launches:
+// sums of tiles of 1024 buckets, their prefix by one CTA, the buckets' offsets.
+constexpr int kListThreads = 256, kListTile = 1024;
+
+__device__ __forceinline__ int64_t warp_scan_i64(int64_t v, int lane) {
+  for (int o = 1; o < 32; o <<= 1) {
+    const int64_t y = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += y;
+  }
+  return v;
+}
+
+// Exclusive prefix of v over the CTA's threads; *all = the sum.
+__device__ __forceinline__ int64_t block_scan_i64(int64_t v, int64_t* ws, int64_t* all) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t inc = warp_scan_i64(v, lane);
+  if (lane == 31) ws[w] = inc;
+  __syncthreads();
+  int64_t before = 0, sum = 0;
+  for (int q = 0; q < kListThreads / 32; q++) {
+    if (q < w) before += ws[q];
+    sum += ws[q];
+  }
+  __syncthreads();
+  *all = sum;
+  return before + inc - v;
+}
+
+__global__ void __launch_bounds__(kListThreads) list_tile_sums(const int32_t* __restrict__ pc,
+                                                              const int32_t* __restrict__ pp, int64_t nb,
+                                                              int64_t* __restrict__ tiles) {
+  __shared__ int64_t ws[kListThreads / 32];
+  int64_t v = 0, all;
+  for (int k = threadIdx.x; k < kListTile; k += kListThreads) {
+    const int64_t b = (int64_t)blockIdx.x * kListTile + k;
+    if (b < nb) v += (int64_t)pc[b] + pp[b];
+  }
+  block_scan_i64(v, ws, &all);
+  if (threadIdx.x == 0) tiles[blockIdx.x] = all;
+}
+
+__global__ void __launch_bounds__(kListThreads) list_tile_scan(int64_t* __restrict__ tiles, int64_t n,
+                                                              unsigned long long* __restrict__ total) {
+  __shared__ int64_t ws[kListThreads / 32];
+  int64_t carry = 0;
+  for (int64_t base = 0; base < n; base += kListThreads) {
+    const int64_t i = base + threadIdx.x;
+    const int64_t v = i < n ? tiles[i] : 0;
+    int64_t all;
+    const int64_t before = block_scan_i64(v, ws, &all);
+    if (i < n) tiles[i] = carry + before;
+    carry += all;
+  }
+  if (threadIdx.x == 0) *total = (unsigned long long)carry;
+}
+
+__global__ void __launch_bounds__(kListThreads) list_offsets(const int32_t* __restrict__ pc,
+                                                            const int32_t* __restrict__ pp, int64_t nb,
+                                                            const int64_t* __restrict__ tiles,
+                                                            int64_t* __restrict__ off) {
+  __shared__ int64_t ws[kListThreads / 32];
+  constexpr int kPer = kListTile / kListThreads;
+  const int64_t b0 = (int64_t)blockIdx.x * kListTile + threadIdx.x * kPer;
+  int64_t v[kPer], sum = 0, all;
+#pragma unroll
+  for (int k = 0; k < kPer; k++) {
+    v[k] = b0 + k < nb ? (int64_t)pc[b0 + k] + pp[b0 + k] : 0;
+    sum += v[k];
+  }
+  int64_t at = tiles[blockIdx.x] + block_scan_i64(sum, ws, &all);
+#pragma unroll
+  for (int k = 0; k < kPer; k++) {
+    if (b0 + k <= nb) off[b0 + k] = at;  // off[nb]: the total
+    at += v[k];
+  }
+}
+
+int64_t list_tiles(int64_t nb) { return nb / kListTile + 1; }  // nb + 1 offsets
+
+void launch_list_offsets(const int32_t* pc_count, const int32_t* pp_count, int64_t nb, int64_t* tiles, int64_t* off,
+                         unsigned long long* total, cudaStream_t st) {
+  const int64_t n = list_tiles(nb);
+  note_launch();
+  list_tile_sums<<<(unsigned)n, kListThreads, 0, st>>>(pc_count, pp_count, nb, tiles);
+  note_launch();
+  list_tile_scan<<<1, kListThreads, 0, st>>>(tiles, n, total);
+  note_launch();
+  list_offsets<<<(unsigned)n, kListThreads, 0, st>>>(pc_count, pp_count, nb, tiles, off);
+}
+
 void launch_pools_to_csr(const int32_t* pc_pool, const int32_t* pp_pool, const int64_t* pc_start,
                          const int32_t* pc_count, const int64_t* pp_start, const int32_t* pp_count, int64_t nb,
                          const int64_t* off, int32_t* node, int8_t* kind, cudaStream_t st) {

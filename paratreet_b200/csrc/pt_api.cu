@@ -26,7 +26,7 @@ using namespace pt;
 // What a pass writes for the host, and the counters' copy from before a list walk
 // (restored if the walk is repeated with larger pools).
 struct Words {
-  unsigned long long counters[3], lcur[3], saved[3];
+  unsigned long long counters[3], lcur[3], saved[3], list_total;
   unsigned status, ticket;
   uint32_t total[kMaxDepth + 1];
 };
@@ -125,6 +125,8 @@ struct pt_handle {
   double* adj = nullptr;  // adjoint scratch: cotangent (3N) and gradients (4N), sorted + caller order,
                           // then pt_adjoint's caller-order input and output (7N)
   int64_t adj_cap = 0;
+  double* chain = nullptr;  // pt_chain_grad's states and checkpoints
+  int64_t chain_cap = 0;
   double* nadj = nullptr;  // 10 adjoint values per node
   int64_t nadj_cap = 0;
 };
@@ -640,24 +642,24 @@ int lists_from_pools(pt_handle* h) {
   cudaStream_t st = h->stream;
   const int64_t nb = h->nbuckets;
   if (nb + 1 > h->list_off_cap) {
-    CKR(dalloc(h, &h->list_count, nb + 1));
-    CKR(dalloc(h, &h->list_off, nb + 1));
-    h->list_off_cap = nb + 1;
+    const int64_t cap = nb + nb / 8 + 64;
+    h->list_off_cap = 0;
+    CKR(dalloc(h, &h->list_count, cap));
+    CKR(dalloc(h, &h->list_off, cap));
+    h->list_off_cap = cap;
   }
-  std::vector<int32_t> cpc(nb), cpp(nb);
-  std::vector<int64_t> off(nb + 1);
-  CK(cudaMemcpyAsync(cpc.data(), h->l_pc_count, nb * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(cpp.data(), h->l_pp_count, nb * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  off[0] = 0;
-  for (int64_t i = 0; i < nb; i++) off[i + 1] = off[i] + cpc[i] + cpp[i];
-  h->list_total = off[nb];
+  // list_count is the scan's scratch here (the FP64 form's counting walk uses it)
+  launch_list_offsets(h->l_pc_count, h->l_pp_count, nb, h->list_count, h->list_off, &h->d_words->list_total, st);
+  CK(cudaGetLastError());
+  CKR(read_words(h));
+  h->list_total = (int64_t)h->pin->list_total;
   if (h->list_total > h->list_cap) {
-    CKR(dalloc(h, &h->list_node, h->list_total));
-    CKR(dalloc(h, &h->list_kind, h->list_total));
-    h->list_cap = h->list_total;
+    const int64_t cap = h->list_total + h->list_total / 8;
+    h->list_cap = 0;
+    CKR(dalloc(h, &h->list_node, cap));
+    CKR(dalloc(h, &h->list_kind, cap));
+    h->list_cap = cap;
   }
-  CK(cudaMemcpyAsync(h->list_off, off.data(), (nb + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
   launch_pools_to_csr(h->pool_pc, h->pool_pp, h->l_pc_start, h->l_pc_count, h->l_pp_start, h->l_pp_count, nb,
                       h->list_off, h->list_node, h->list_kind, st);
   CK(cudaGetLastError());
@@ -945,7 +947,7 @@ int pt_destroy(pt_handle* h) {
   dfree(o.first_child); dfree(o.count); dfree(o.mom); dfree(o.walk); dfree(o.walks); dfree(o.quad); dfree(o.quadf);
   dfree(o.fifo); dfree(o.inode); dfree(o.npend); dfree(o.arrived);
   dfree(h->buckets); dfree(h->bucket_work); dfree(h->list_count); dfree(h->list_off); dfree(h->list_node);
-  dfree(h->list_kind); dfree(h->dsum); dfree(h->adj); dfree(h->nadj); dfree(h->d_htab); dfree(h->ewd); dfree(h->sph); dfree(h->sph_nbr); dfree(h->sph_nd2);
+  dfree(h->list_kind); dfree(h->dsum); dfree(h->adj); dfree(h->nadj); dfree(h->chain); dfree(h->d_htab); dfree(h->ewd); dfree(h->sph); dfree(h->sph_nbr); dfree(h->sph_nd2);
   dfree(h->sph_list_d); dfree(h->sph_list_i); dfree(h->sph_state);
   dfree(h->pool_pc); dfree(h->pool_pp); dfree(h->l_pc_start); dfree(h->l_pp_start); dfree(h->l_pc_count);
   dfree(h->l_pp_count); dfree(h->d_queue);
@@ -1600,7 +1602,7 @@ int adjoint_device(pt_handle* h, const double* cx, const double* cy, const doubl
   A.nadj = h->nadj;
   A.work = h->d_work;
   A.status = h->d_status;
-  launch_adjoint(A, h->sms * 8, st);
+  launch_adjoint(A, h->sms, st);
   CK(cudaGetLastError());
   double* outs[4] = {gx, gy, gz, gm};
   for (int k = 0; k < 4; k++) {
@@ -1730,9 +1732,12 @@ extern "C" int pt_chain_grad(pt_handle* h, int nsteps, double dt, int ckpt_every
                 off_A = 14 * n, off_Y = 17 * n, off_xb = 20 * n, off_vb = 23 * n, off_mb = 26 * n, off_pd = 27 * n,
                 off_ck = 30 * n, off_seg = off_ck + (int64_t)nck * 6 * n;
   const int64_t total = off_seg + (int64_t)(C + 1) * 3 * n;
-  DevBuf buf;
-  CK(cudaMalloc((void**)&buf.p, total * sizeof(double)));
-  double* B = buf.p;
+  if (total > h->chain_cap) {
+    h->chain_cap = 0;
+    CKR(dalloc(h, &h->chain, total));
+    h->chain_cap = total;
+  }
+  double* B = h->chain;
   double *X0 = B + off_X0, *V0 = B + off_V0, *M0 = B + off_M0, *S0 = B + off_S0, *X = B + off_X, *V = B + off_V,
          *A = B + off_A, *Y = B + off_Y, *xb = B + off_xb, *vb = B + off_vb, *mb = B + off_mb, *pd = B + off_pd,
          *ck = B + off_ck, *seg = B + off_seg;

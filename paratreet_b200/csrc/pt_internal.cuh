@@ -191,6 +191,7 @@ struct AdjParams {
   const int32_t* parent;
   const int32_t* buckets;
   int64_t nbuckets, nnodes;
+  int slices;  // pieces each bucket's list is cut into (set by the launcher)
   const int64_t* list_off;
   const int32_t* list_node;
   const int8_t* list_kind;

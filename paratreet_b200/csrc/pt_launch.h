@@ -95,9 +95,14 @@ void launch_sph_density(Particles p, int64_t n, const Mom* mom, const WalkRec* w
                         cudaStream_t st);
 
 // k_adjoint.cu
-void launch_adjoint(const AdjParams& A, int grid, cudaStream_t st);
+void launch_adjoint(const AdjParams& A, int sms, cudaStream_t st);
 
 // k_util.cu
+// CSR offsets of the two-phase lists: off[b] = entries of the buckets before b
+// (nb + 1 of them) and *total; tiles: list_tiles(nb) + 1 scratch words
+int64_t list_tiles(int64_t nb);
+void launch_list_offsets(const int32_t* pc_count, const int32_t* pp_count, int64_t nb, int64_t* tiles, int64_t* off,
+                         unsigned long long* total, cudaStream_t st);
 void launch_pools_to_csr(const int32_t* pc_pool, const int32_t* pp_pool, const int64_t* pc_start,
                          const int32_t* pc_count, const int64_t* pp_start, const int32_t* pp_count, int64_t nb,
                          const int64_t* off, int32_t* node, int8_t* kind, cudaStream_t st);
