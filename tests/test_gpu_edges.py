@@ -44,7 +44,7 @@ def assert_tree_and_forces(p, bucket, theta, traversal="transposed"):
         return s.counters()["n_buckets"]
 
 
-@pytest.mark.parametrize("n", [1023, 1024, 1025, 2049, 12287, 12288, 12289])
+@pytest.mark.parametrize("n", [1023, 1024, 1025, 2049, 16383, 16384, 16385])
 def test_tiles_and_sorts_bit_exact(n):
     assert_tree_and_forces(ics.mixture(n, seed=n, clump_a=0.02), 8, 0.9)
 
