@@ -328,9 +328,8 @@ __global__ void __launch_bounds__(kKnnWarps * 32, 7) sph_density_kernel(Particle
               const double* hi = mom[node].hi;
               const double nlo[3] = {lo[0], lo[1], lo[2]}, nhi[3] = {hi[0], hi[1], hi[2]};
               keep = box_box_gap2(nlo, nhi, blo, bhi) <= rmax * (1.0 + 1e-13);
-              // then, for a leaf, the per-target test itself (DensityVisitor::
-              // open; on Internal nodes it cost more than the visits it saved)
-              if (keep && !internal) {
+              // then the per-target test itself (DensityVisitor::open)
+              if (keep) {
                 keep = false;
                 for (int t = 0; t < nt && !keep; t++)
                   keep = box_d2(nlo, nhi, w.tx[t], w.ty[t], w.tz[t]) <= w.kd[t];
