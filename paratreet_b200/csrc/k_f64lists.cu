@@ -3,7 +3,7 @@
 //
 // The comparator of the mixed form: the same walk_lists lists (so the same
 // leaf() and node() interactions as the reference's traversal), evaluated
-// with the same work layout as eval_p2c / eval_p2p (one warp per bucket, the
+// with the same work layout as eval_p2c2 / eval_p2p (one warp per bucket, the
 // bucket's targets replicated over G = floor(32 / n_t) lane groups, 32-entry
 // chunks staged in shared memory), but in FP64 with the reference's
 // expressions on absolute positions: GravityVisitor::leaf and ::node

@@ -498,7 +498,7 @@ void replica_offset(const pt_handle* h, int r, TravParams& P) {
 }
 
 // Two-phase mixed evaluation: walk_lists writes every bucket's interaction
-// list to the pools, then eval_p2c and eval_p2p evaluate them.  Pools are
+// list to the pools, then eval_p2c2 and eval_p2p evaluate them.  Pools are
 // sized from the previous pass with a quarter of headroom (a bucket whose list
 // outgrows its warp's region moves it to a new region inside the walk); only
 // a pass whose lists fill a pool is repeated (counters restored) with pools

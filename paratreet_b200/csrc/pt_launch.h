@@ -72,7 +72,7 @@ void launch_ewald_recip(const double* x, const double* y, const double* z, const
 // k_mixed2.cu
 int walk_lists_grid(int sms);
 void launch_walk_lists(const TravParams& P, const ListParams& L, const Mom* mom, int grid, cudaStream_t st);
-// eval_p2c (store or add per P.accumulate) then eval_p2p (add); P and Q differ in
+// eval_p2c2 (store or add per P.accumulate) then eval_p2p (add); P and Q differ in
 // their bucket queues (zeroed by the caller)
 void launch_eval_lists(const TravParams& P, const TravParams& Q, const ListParams& L, const Mom* mom, int sms,
                        cudaStream_t st);
