@@ -69,6 +69,7 @@ struct pt_handle {
   int64_t cap_srcf = 0;
 
   Nodes nd{};
+  unsigned char* node_slab = nullptr;  // the node arrays, one allocation
   int64_t node_cap = 0, nnodes = 0, ninternal = 0;
   int depth = 0;  // deepest level of the tree
   int32_t* buckets = nullptr;
@@ -249,29 +250,45 @@ int ensure_particles(pt_handle* h, int64_t n) {
   return PT_OK;
 }
 
-// Room for `need` nodes; the arrays hold nothing that outlives a build.
+// Room for `need` nodes; the arrays hold nothing that outlives a build.  One
+// allocation for all of them: a new handle's first pass made 17 here.
 int grow_nodes(pt_handle* h, int64_t need) {
   if (need <= h->node_cap) return PT_OK;
   const int64_t nc = std::max<int64_t>(need + need / 4, 1024);
-  Nodes& o = h->nd;
+  Nodes o{};
+  size_t bytes = 0;
+  unsigned char* base = nullptr;  // null: count the bytes
+  auto take = [&](auto** ptr, size_t count) {
+    if (base) *ptr = reinterpret_cast<std::remove_reference_t<decltype(*ptr)>>(base + bytes);
+    bytes += (count * sizeof(**ptr) + 255) / 256 * 256;
+  };
+  auto take_all = [&]() {
+    bytes = 0;
+    take(&o.mom, nc);
+    take(&o.walk, nc);
+    take(&o.walks, walk_sib_size(nc));
+    take(&o.quad, nc);
+    take(&o.quadf, nc);
+    take(&o.inode, nc / 8 + 1);
+    take(&o.key, nc);
+    take(&o.fifo, nc);
+    take(&o.type, nc);
+    take(&o.depth, nc);
+    take(&o.pstart, nc);
+    take(&o.pcount, nc);
+    take(&o.parent, nc);
+    take(&o.first_child, nc);
+    take(&o.count, nc);
+    take(&o.npend, nc);
+    take(&o.arrived, nc);
+  };
+  take_all();
   h->node_cap = 0;
-  CKR(dalloc(h, &o.key, nc));
-  CKR(dalloc(h, &o.type, nc));
-  CKR(dalloc(h, &o.depth, nc));
-  CKR(dalloc(h, &o.pstart, nc));
-  CKR(dalloc(h, &o.pcount, nc));
-  CKR(dalloc(h, &o.parent, nc));
-  CKR(dalloc(h, &o.first_child, nc));
-  CKR(dalloc(h, &o.count, nc));
-  CKR(dalloc(h, &o.mom, nc));
-  CKR(dalloc(h, &o.walk, nc));
-  CKR(dalloc(h, &o.walks, walk_sib_size(nc)));
-  CKR(dalloc(h, &o.quad, nc));
-  CKR(dalloc(h, &o.quadf, nc));
-  CKR(dalloc(h, &o.fifo, nc));
-  CKR(dalloc(h, &o.inode, nc / 8 + 1));
-  CKR(dalloc(h, &o.npend, nc));
-  CKR(dalloc(h, &o.arrived, nc));
+  h->nd = Nodes{};
+  CKR(dalloc(h, &h->node_slab, bytes));
+  base = h->node_slab;
+  take_all();
+  h->nd = o;
   h->node_cap = nc;
   return PT_OK;
 }
@@ -358,12 +375,11 @@ int build_tree(pt_handle* h) {
     if (tot[l]) depth = l + 1;
   }
   const int64_t nl = tot[kMaxDepth];
-  h->nnodes = 0;
+  h->nnodes = h->nbuckets = 0;
   CKR(grow_nodes(h, 1 + 8 * ni));
   h->nnodes = 1 + 8 * ni;
   h->ninternal = ni;
   h->depth = depth;
-  h->nbuckets = 0;
   if (nl > h->cap_buckets) {
     // an eighth of headroom: the bucket count drifts from pass to pass as the
     // particles move, and a cudaFree on every new maximum would stall the device
@@ -509,10 +525,11 @@ int run_two_phase(pt_handle* h, TravParams& P) {
   if (nb <= 0) return PT_OK;
   if (nb > h->l_nb_cap) {
     const int64_t cap = nb + nb / 8 + 64;  // headroom, as for the bucket arrays
-    CKR(dalloc(h, &h->l_pc_start, cap));
-    CKR(dalloc(h, &h->l_pp_start, cap));
-    CKR(dalloc(h, &h->l_pc_count, cap));
-    CKR(dalloc(h, &h->l_pp_count, cap));
+    h->l_nb_cap = 0;
+    CKR(dalloc(h, &h->l_pc_start, 3 * cap));  // two arrays of starts, two of 32-bit counts
+    h->l_pp_start = h->l_pc_start + cap;
+    h->l_pc_count = reinterpret_cast<int32_t*>(h->l_pp_start + cap);
+    h->l_pp_count = h->l_pc_count + cap;
     h->l_nb_cap = cap;
   }
   const int wgrid = (int)std::max<int64_t>(1, std::min<int64_t>(walk_lists_grid(h->sms), (nb + 3) / 4));
@@ -942,15 +959,12 @@ int pt_destroy(pt_handle* h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   dfree(h->slab); dfree(h->bbox_partial); dfree(h->d_uni);
   dfree(h->d_words); dfree(h->d_work); dfree(h->d_vmax2); dfree(h->src); dfree(h->srcf); dfree(h->softf);
-  Nodes& o = h->nd;
-  dfree(o.key); dfree(o.type); dfree(o.depth); dfree(o.pstart); dfree(o.pcount); dfree(o.parent);
-  dfree(o.first_child); dfree(o.count); dfree(o.mom); dfree(o.walk); dfree(o.walks); dfree(o.quad); dfree(o.quadf);
-  dfree(o.fifo); dfree(o.inode); dfree(o.npend); dfree(o.arrived);
+  dfree(h->node_slab);
   dfree(h->buckets); dfree(h->bucket_work); dfree(h->list_count); dfree(h->list_off); dfree(h->list_node);
   dfree(h->list_kind); dfree(h->dsum); dfree(h->adj); dfree(h->nadj); dfree(h->chain); dfree(h->d_htab); dfree(h->ewd); dfree(h->sph); dfree(h->sph_nbr); dfree(h->sph_nd2);
   dfree(h->sph_list_d); dfree(h->sph_list_i); dfree(h->sph_state);
-  dfree(h->pool_pc); dfree(h->pool_pp); dfree(h->l_pc_start); dfree(h->l_pp_start); dfree(h->l_pc_count);
-  dfree(h->l_pp_count); dfree(h->d_queue);
+  dfree(h->pool_pc); dfree(h->pool_pp); dfree(h->l_pc_start);
+  dfree(h->d_queue);
   for (auto& e : h->ev)
     if (e) cudaEventDestroy(e);
   if (h->pin) cudaFreeHost(h->pin);
