@@ -22,10 +22,13 @@
 // The look-back only waits on tiles that claimed their index earlier and
 // publish their counts before waiting on anything, so it always ends; the spin
 // is still bounded (spin_limit polls of an unpublished tile, 2^21 by default)
-// and reports kErrSort instead of hanging.  A look-back cut short only
-// under-counts a digit's exclusive prefix, so every destination stays inside
-// [0, n), but the output is then not a permutation: the caller checks the
-// status word before it uses the sorted indices.
+// and reports kErrSort instead of hanging.  A look-back cut short under-counts a
+// digit's exclusive prefix: its own pass still writes inside [0, n), but leaves
+// slots of the output as they were, and a later pass may then hold more keys of
+// a digit than the histogram of the original keys says, whose destinations run
+// past n.  Those are left out (the write is bounded).  The output is not a
+// permutation: the caller checks the status word before it uses the sorted
+// indices.
 #include <algorithm>
 
 #include "pt_internal.cuh"
@@ -207,8 +210,12 @@ __global__ void __launch_bounds__(kSortThreads, 2) radix_onesweep(const uint64_t
     const uint64_t key = S.key[i];
     const uint32_t dd = (uint32_t)((key >> shift) & 0xff);
     const uint32_t dst = S.gbase[dd] + ((uint32_t)i - S.dstart[dd]);
-    kout[dst] = key;
-    vout[dst] = S.val[i];
+    if (dst < n) {
+      kout[dst] = key;
+      vout[dst] = S.val[i];
+    } else {  // only behind a pass whose look-back gave up
+      atomicOr(status, kErrSort);
+    }
   }
 }
 

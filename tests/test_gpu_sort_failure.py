@@ -5,9 +5,9 @@ look-back over earlier tiles that polls an unpublished tile a bounded number
 of times.  With the bound set to 0 a look-back gives up at the first tile it
 finds unpublished, which on a multi-tile sort happens in practice on every
 pass.  The force pass must then return PT_E_DEVICE naming the sort, stop
-before it permutes the particles (a look-back cut short writes in bounds but
-not a permutation), and leave the handle usable: with the default bound the
-next pass equals a fresh handle's bit for bit.  No wait in this test is left
+before it permutes the particles (look-backs cut short leave no permutation), and
+leave the handle usable: with the default bound the next pass equals a fresh
+handle's bit for bit.  No wait in this test is left
 to run out on its own; the bound only cuts waits short."""
 import numpy as np
 import pytest
@@ -44,3 +44,33 @@ def test_sort_lookback_limit_reports_and_recovers():
         got = s.accelerations()
     for k in ("ax", "ay", "az", "pot", "pot_full"):
         assert np.array_equal(got[k], want[k]), k
+
+
+# both tile sizes; with a limit above 0 only some look-backs give up, which is
+# what can send a later digit pass past the end (tests/test_sort_lookback_model.py)
+@pytest.mark.parametrize("n", [300_001, (1 << 21) + 5])
+@pytest.mark.parametrize("polls", [0, 1, 4])
+def test_failed_sort_leaves_the_particles(n, polls):
+    from paratreet_b200._lib import PtError
+    from paratreet_b200.gravity import GravitySimulation
+
+    p = ics.plummer(n, seed=6, soft=1e-3)
+    failed = 0
+    with GravitySimulation(max_particles_per_leaf=32, theta=1.0, precision="mixed") as s:
+        s.set_particles(p)
+        s.start_down()  # the particles are in key order, and the alternate buffers full
+        want = s.keys()
+        s.set_sort_spin_limit(polls)
+        for _ in range(6):
+            try:
+                s.start_down()
+            except PtError as e:
+                assert "radix sort look-back timed out" in str(e)
+                failed += 1
+            st = s.state()
+            for k in ("x", "y", "z", "vx", "vy", "vz"):
+                assert np.array_equal(st[k], p[k]), k
+        assert failed or polls > 0
+        s.set_sort_spin_limit()
+        s.start_down()
+        assert np.array_equal(s.keys(), want)
