@@ -152,6 +152,12 @@ int pt_set_sort_spin_limit(pt_handle* h, int64_t polls);
  * knob; entries < 64 is PT_E_ARG. */
 int pt_set_list_region(pt_handle* h, int64_t entries);
 
+/* Failure-path control of the handle's device memory, for tests: an allocation
+ * of more than `bytes` is refused as cudaMalloc refuses one that does not fit.
+ * A call that cannot do without it returns PT_E_NOMEM; the handle stays usable.
+ * 0 (the default): no limit.  bytes < 0 is PT_E_ARG. */
+int pt_set_alloc_limit(pt_handle* h, int64_t bytes);
+
 /* Particles -------------------------------------------------------------- */
 /* Replaces Reader::load + the universe reduction (src/Reader.C:11-107,
  * src/Driver.h:96-107): copies FP64 host SoA to the device.  soft is the

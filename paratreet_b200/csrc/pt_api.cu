@@ -38,6 +38,7 @@ struct pt_handle {
   cudaStream_t stream = nullptr;
   cudaStream_t own_stream = nullptr;
 
+  int64_t alloc_limit = 0;  // largest device allocation (pt_set_alloc_limit; 0: no limit)
   int64_t n = 0, cap_n = 0;
   Particles p{};
   unsigned char* slab = nullptr;  // every per-particle array below, one allocation
@@ -185,6 +186,13 @@ int fail(pt_handle* h, int code, const std::string& msg) {
     if (r_ != PT_OK) return r_; \
   } while (0)
 
+// cudaMalloc within the handle's limit.
+template <typename T>
+cudaError_t device_malloc(const pt_handle* h, T** ptr, size_t bytes) {
+  if (h->alloc_limit > 0 && bytes > (size_t)h->alloc_limit) return cudaErrorMemoryAllocation;
+  return cudaMalloc((void**)ptr, bytes);
+}
+
 template <typename T>
 int dalloc(pt_handle* h, T** ptr, size_t count) {
   if (*ptr) {
@@ -192,7 +200,7 @@ int dalloc(pt_handle* h, T** ptr, size_t count) {
     *ptr = nullptr;
   }
   if (count == 0) count = 1;
-  CK(cudaMalloc((void**)ptr, count * sizeof(T)));
+  CK(device_malloc(h, ptr, count * sizeof(T)));
   return PT_OK;
 }
 
@@ -367,6 +375,9 @@ int build_tree(pt_handle* h) {
   const int64_t n = h->n;
   launch_tree_count(h->p.key, n, h->cfg.bucket, h->tree_counts, h->d_total, st);
   CKR(read_status(h));  // synchronises; a failed sort ends the pass here
+  // the particles are in a new order from here on: results of an earlier pass no
+  // longer line up with it
+  h->have_forces = h->forces_current = h->lists_valid = h->tp_lists_valid = false;
   const uint32_t* tot = h->pin->total;  // Internal nodes of each level, leaves
   int64_t ni = 0;
   int depth = 0;
@@ -555,16 +566,16 @@ int run_two_phase(pt_handle* h, TravParams& P) {
       unsigned long long alloc_pc = need_pc + need_pc / 4, alloc_pp = need_pp + need_pp / 4;
       // an entry, and in a periodic pass its replica (a byte, behind the entries)
       const size_t per = sizeof(int32_t) + (h->cfg.periodic ? 1 : 0);
-      if (cudaMalloc((void**)&h->pool_pc, alloc_pc * per) != cudaSuccess ||
-          cudaMalloc((void**)&h->pool_pp, alloc_pp * per) != cudaSuccess) {
+      if (device_malloc(h, &h->pool_pc, alloc_pc * per) != cudaSuccess ||
+          device_malloc(h, &h->pool_pp, alloc_pp * per) != cudaSuccess) {
         cudaGetLastError();
         dfree(h->pool_pc);
         dfree(h->pool_pp);
         alloc_pc = need_pc;
         alloc_pp = need_pp;
       }
-      if ((!h->pool_pc && cudaMalloc((void**)&h->pool_pc, need_pc * per) != cudaSuccess) ||
-          (!h->pool_pp && cudaMalloc((void**)&h->pool_pp, need_pp * per) != cudaSuccess)) {
+      if ((!h->pool_pc && device_malloc(h, &h->pool_pc, need_pc * per) != cudaSuccess) ||
+          (!h->pool_pp && device_malloc(h, &h->pool_pp, need_pp * per) != cudaSuccess)) {
         // no room for the lists: this handle evaluates with the fused kernel from now on
         cudaGetLastError();
         dfree(h->pool_pc);
@@ -808,8 +819,12 @@ int forces(pt_handle* h, int64_t b0, int64_t b1) {
   CKR(keys_and_sort(h));
   CKR(build_tree(h));
   CKR(upward(h));
-  CKR(traverse(h, b0, b1));
-  CKR(read_status(h));
+  int rc = traverse(h, b0, b1);
+  if (rc == PT_OK) rc = read_status(h);
+  if (rc != PT_OK) {
+    h->lists_valid = h->tp_lists_valid = false;
+    return rc;
+  }
   const unsigned long long* c = h->pin->counters;
   pt_counters& k = h->last;
   k.n_pp = c[0];
@@ -1005,6 +1020,12 @@ int pt_set_list_region(pt_handle* h, int64_t entries) {
   return PT_OK;
 }
 
+int pt_set_alloc_limit(pt_handle* h, int64_t bytes) {
+  if (!h || bytes < 0) return PT_E_ARG;
+  h->alloc_limit = bytes;
+  return PT_OK;
+}
+
 int pt_set_particles(pt_handle* h, int64_t n, const double* x, const double* y, const double* z, const double* vx,
                      const double* vy, const double* vz, const double* m, const double* soft) {
   if (!h) return PT_E_ARG;
@@ -1071,10 +1092,6 @@ static int sph_density_device(pt_handle* h, bool want_nbr) {
   CKR(keys_and_sort(h));
   CKR(build_tree(h));
   CKR(upward(h, false));
-  // the particle arrays were re-sorted: results of an earlier force pass no longer line up
-  h->have_forces = false;
-  h->forces_current = false;
-  h->lists_valid = false;
   if (7 * n > h->sph_cap) {
     CKR(dalloc(h, &h->sph, 7 * n));
     h->sph_cap = 7 * n;
@@ -1404,7 +1421,7 @@ int pt_get_list_digests(pt_handle* h, int which, uint64_t* digest, int64_t* coun
   cudaSetDevice(h->cfg.device);
   cudaStream_t st = h->stream;
   DevBuf buf;
-  CK(cudaMalloc((void**)&buf.p, 2 * nb * sizeof(double)));
+  CK(device_malloc(h, &buf.p, 2 * nb * sizeof(double)));
   unsigned long long* d_dig = reinterpret_cast<unsigned long long*>(buf.p);
   int64_t* d_cnt = reinterpret_cast<int64_t*>(buf.p + nb);
   if (which == 0)

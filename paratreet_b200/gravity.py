@@ -157,6 +157,11 @@ class GravitySimulation:
         tests: smaller regions move the buckets' lists more often)."""
         self._check(self._lib.pt_set_list_region(self._h, int(entries)))
 
+    def set_alloc_limit(self, nbytes: int = 0):
+        """Failure-path control of the device memory (tests): allocations of more
+        than nbytes are refused (0: no limit)."""
+        self._check(self._lib.pt_set_alloc_limit(self._h, int(nbytes)))
+
     # -- particles ----------------------------------------------------------
     def set_particles(self, p: dict):
         arrs = [np.ascontiguousarray(p[k], dtype=np.float64) for k in _FIELDS]
