@@ -175,9 +175,11 @@ int fail(pt_handle* h, int code, const std::string& msg) {
 #define CK(call)                                                                               \
   do {                                                                                         \
     cudaError_t e_ = (call);                                                                   \
-    if (e_ != cudaSuccess)                                                                     \
+    if (e_ != cudaSuccess) {                                                                   \
+      cudaGetLastError(); /* or the next launch's check reports this error again */            \
       return fail(h, (e_ == cudaErrorMemoryAllocation) ? PT_E_NOMEM : PT_E_CUDA,               \
                   std::string(#call) + ": " + cudaGetErrorString(e_));                         \
+    }                                                                                          \
   } while (0)
 
 #define CKR(expr)              \
@@ -189,7 +191,9 @@ int fail(pt_handle* h, int code, const std::string& msg) {
 // cudaMalloc within the handle's limit.
 template <typename T>
 cudaError_t device_malloc(const pt_handle* h, T** ptr, size_t bytes) {
-  if (h->alloc_limit > 0 && bytes > (size_t)h->alloc_limit) return cudaErrorMemoryAllocation;
+  // a refused allocation asks for more than any device has, so that the runtime's
+  // error state is that of a failed call
+  if (h->alloc_limit > 0 && bytes > (size_t)h->alloc_limit) bytes = (size_t)1 << 62;
   return cudaMalloc((void**)ptr, bytes);
 }
 
