@@ -112,7 +112,7 @@ struct pt_handle {
   int64_t sph_state_cap = 0;
 
   double4* d_htab = nullptr;  // Ewald reciprocal table (h vector, hCfac)
-  int htab_cap = 0;
+  int64_t htab_cap = 0;
   double* ewd = nullptr;  // Ewald direct-sum scratch
   int64_t ewd_cap = 0;
 
@@ -206,6 +206,20 @@ int dalloc(pt_handle* h, T** ptr, size_t count) {
   if (count == 0) count = 1;
   CK(device_malloc(h, ptr, count * sizeof(T)));
   return PT_OK;
+}
+
+// Room for `need` elements in each of the arrays that share the capacity `cap`,
+// with `want` of them where they are allocated anew.  The old arrays go first, so
+// the capacity is 0 until all of the new ones are there: after a refused
+// allocation the next call allocates again instead of using a null array.
+template <typename... T>
+int reserve(pt_handle* h, int64_t& cap, int64_t need, int64_t want, T**... arrays) {
+  if (need <= cap) return PT_OK;
+  cap = 0;
+  int rc = PT_OK;
+  (void)(((rc = dalloc(h, arrays, (size_t)want)) == PT_OK) && ...);
+  if (rc == PT_OK) cap = want;
+  return rc;
 }
 
 int zero_queue(pt_handle* h) {
@@ -392,17 +406,12 @@ int build_tree(pt_handle* h) {
   const int64_t nl = tot[kMaxDepth];
   h->nnodes = h->nbuckets = 0;
   CKR(grow_nodes(h, 1 + 8 * ni));
+  // an eighth of headroom: the bucket count drifts from pass to pass as the
+  // particles move, and a cudaFree on every new maximum would stall the device
+  CKR(reserve(h, h->cap_buckets, nl, nl + nl / 8 + 64, &h->buckets, &h->bucket_work));
   h->nnodes = 1 + 8 * ni;
   h->ninternal = ni;
   h->depth = depth;
-  if (nl > h->cap_buckets) {
-    // an eighth of headroom: the bucket count drifts from pass to pass as the
-    // particles move, and a cudaFree on every new maximum would stall the device
-    const int64_t cap = (int64_t)nl + nl / 8 + 64;
-    CKR(dalloc(h, &h->buckets, cap));
-    CKR(dalloc(h, &h->bucket_work, cap));
-    h->cap_buckets = cap;
-  }
   h->nbuckets = nl;
   launch_tree_emit(h->nd, h->p.key, n, h->cfg.bucket, h->tree_counts, h->d_total, ni, h->node_cap, nl, h->buckets,
                    h->d_status, st);
@@ -411,13 +420,7 @@ int build_tree(pt_handle* h) {
   return PT_OK;
 }
 
-int ensure_src(pt_handle* h) {
-  if (h->cap_src >= h->cap_n) return PT_OK;
-  h->cap_src = 0;
-  CKR(dalloc(h, &h->src, h->cap_n));
-  h->cap_src = h->cap_n;
-  return PT_OK;
-}
+int ensure_src(pt_handle* h) { return reserve(h, h->cap_src, h->cap_n, h->cap_n, &h->src); }
 
 // K6: moments, upward pass, traversal records.
 int upward(pt_handle* h, bool walk = true) {
@@ -432,11 +435,7 @@ int upward(pt_handle* h, bool walk = true) {
   const int mixed = h->cfg.precision == PT_MIXED;
   launch_finalize(h->nd, h->nnodes, gfac, mixed, st);
   if (mixed) {
-    if (h->cap_srcf < h->cap_n) {
-      CKR(dalloc(h, &h->srcf, h->cap_n));
-      CKR(dalloc(h, &h->softf, h->cap_n));
-      h->cap_srcf = h->cap_n;
-    }
+    CKR(reserve(h, h->cap_srcf, h->cap_n, h->cap_n, &h->srcf, &h->softf));
     launch_prep_sources(h->buckets, h->nbuckets, h->nd.walk, h->p, h->srcf, h->softf, st);
   }
   CK(cudaGetLastError());
@@ -492,10 +491,7 @@ int ewald_correction_pass(pt_handle* h, int64_t b0, int64_t b1) {
         mfacc -= g0 * root.mass;
         tab.push_back(make_double4(2 * M_PI / L * hx, 2 * M_PI / L * hy, 2 * M_PI / L * hz, 2.0 * mfacc));
       }
-  if ((int)tab.size() > h->htab_cap) {
-    CKR(dalloc(h, &h->d_htab, tab.size()));
-    h->htab_cap = (int)tab.size();
-  }
+  CKR(reserve(h, h->htab_cap, (int64_t)tab.size(), (int64_t)tab.size(), &h->d_htab));
   if (!tab.empty())
     CK(cudaMemcpyAsync(h->d_htab, tab.data(), tab.size() * sizeof(double4), cudaMemcpyHostToDevice, st));
   EwaldRoot R{};
@@ -673,25 +669,13 @@ int run_traversal(pt_handle* h, TravParams& P, int grid) {
 int lists_from_pools(pt_handle* h) {
   cudaStream_t st = h->stream;
   const int64_t nb = h->nbuckets;
-  if (nb + 1 > h->list_off_cap) {
-    const int64_t cap = nb + nb / 8 + 64;
-    h->list_off_cap = 0;
-    CKR(dalloc(h, &h->list_count, cap));
-    CKR(dalloc(h, &h->list_off, cap));
-    h->list_off_cap = cap;
-  }
+  CKR(reserve(h, h->list_off_cap, nb + 1, nb + nb / 8 + 64, &h->list_count, &h->list_off));
   // list_count is the scan's scratch here (the FP64 form's counting walk uses it)
   launch_list_offsets(h->l_pc_count, h->l_pp_count, nb, h->list_count, h->list_off, &h->d_words->list_total, st);
   CK(cudaGetLastError());
   CKR(read_words(h));
   h->list_total = (int64_t)h->pin->list_total;
-  if (h->list_total > h->list_cap) {
-    const int64_t cap = h->list_total + h->list_total / 8;
-    h->list_cap = 0;
-    CKR(dalloc(h, &h->list_node, cap));
-    CKR(dalloc(h, &h->list_kind, cap));
-    h->list_cap = cap;
-  }
+  CKR(reserve(h, h->list_cap, h->list_total, h->list_total + h->list_total / 8, &h->list_node, &h->list_kind));
   launch_pools_to_csr(h->pool_pc, h->pool_pp, h->l_pc_start, h->l_pc_count, h->l_pp_start, h->l_pp_count, nb,
                       h->list_off, h->list_node, h->list_kind, st);
   CK(cudaGetLastError());
@@ -742,11 +726,7 @@ int traverse(pt_handle* h, int64_t b0, int64_t b1) {
                                 b0 == 0 && b1 == h->nbuckets &&
                                 (h->cfg.precision == PT_MIXED || h->cfg.precision == PT_FP64_LISTS);
   if (h->cfg.record_lists && nb > 0 && !two_phase_record) {
-    if (nb + 1 > h->list_off_cap) {
-      CKR(dalloc(h, &h->list_count, nb + 1));
-      CKR(dalloc(h, &h->list_off, nb + 1));
-      h->list_off_cap = nb + 1;
-    }
+    CKR(reserve(h, h->list_off_cap, nb + 1, nb + 1, &h->list_count, &h->list_off));
     h->list_nb = nb + 1;
     P.mode = 1;
     P.list_count = h->list_count;
@@ -758,11 +738,7 @@ int traverse(pt_handle* h, int64_t b0, int64_t b1) {
     off[0] = 0;
     for (int64_t i = 0; i < nb; i++) off[i + 1] = off[i] + cnt[i];
     h->list_total = off[nb];
-    if (h->list_total > h->list_cap) {
-      CKR(dalloc(h, &h->list_node, h->list_total));
-      CKR(dalloc(h, &h->list_kind, h->list_total));
-      h->list_cap = h->list_total;
-    }
+    CKR(reserve(h, h->list_cap, h->list_total, h->list_total, &h->list_node, &h->list_kind));
     CK(cudaMemcpyAsync(h->list_off, off.data(), (nb + 1) * sizeof(int64_t), cudaMemcpyHostToDevice, st));
     CK(cudaMemsetAsync(h->d_counters, 0, 3 * sizeof(unsigned long long), st));
     P.mode = 2;
@@ -1096,23 +1072,12 @@ static int sph_density_device(pt_handle* h, bool want_nbr) {
   CKR(keys_and_sort(h));
   CKR(build_tree(h));
   CKR(upward(h, false));
-  if (7 * n > h->sph_cap) {
-    CKR(dalloc(h, &h->sph, 7 * n));
-    h->sph_cap = 7 * n;
-  }
-  if (want_nbr && n * k > h->sph_nbr_cap) {
-    CKR(dalloc(h, &h->sph_nbr, n * k));
-    CKR(dalloc(h, &h->sph_nd2, n * k));
-    h->sph_nbr_cap = n * k;
-  }
+  CKR(reserve(h, h->sph_cap, 7 * n, 7 * n, &h->sph));
+  if (want_nbr) CKR(reserve(h, h->sph_nbr_cap, n * k, n * k, &h->sph_nbr, &h->sph_nd2));
   // per-warp candidate lists of the neighbour search: 32 targets x 32 entries
   const int kgrid = h->sms * 7;
   const int64_t slots = sph_knn_slots(kgrid);
-  if (slots * 1024 > h->sph_list_cap) {
-    CKR(dalloc(h, &h->sph_list_d, slots * 1024));
-    CKR(dalloc(h, &h->sph_list_i, slots * 1024));
-    h->sph_list_cap = slots * 1024;
-  }
+  CKR(reserve(h, h->sph_list_cap, slots * 1024, slots * 1024, &h->sph_list_d, &h->sph_list_i));
   CK(cudaMemsetAsync(h->d_work, 0, sizeof(unsigned), st));
   launch_sph_density(h->p, n, h->nd.mom, h->nd.walk, h->buckets, h->nbuckets, h->nnodes, h->sph, h->sph + n,
                      want_nbr ? h->sph_nbr : nullptr, want_nbr ? h->sph_nd2 : nullptr, h->sph_list_d,
@@ -1196,10 +1161,7 @@ int pt_sph_step(pt_handle* h, int nsteps, double* u, double* u_pred, double* vpx
   cudaStream_t st = h->stream;
   const int64_t n = h->n;
   if (n == 0 || nsteps == 0) return PT_OK;
-  if (8 * n > h->sph_state_cap) {
-    CKR(dalloc(h, &h->sph_state, 8 * n));
-    h->sph_state_cap = 8 * n;
-  }
+  CKR(reserve(h, h->sph_state_cap, 8 * n, 8 * n, &h->sph_state));
   double* cs = h->sph_state;  // caller order: u, u_pred, vpx, vpy, vpz
   double* vps = cs + 5 * n;   // sorted v_pred
   double* in[5] = {u, u_pred, vpx, vpy, vpz};
@@ -1460,10 +1422,7 @@ int pt_direct_sum(pt_handle* h, int64_t nt, const int32_t* targets, double* ax, 
   int nsplit = std::max(1, std::min(256, (4 * h->sms + tb - 1) / tb));
   if (n < 4096) nsplit = 1;
   const int64_t need = 5 * n + 4 * nt * nsplit + nt;
-  if (need > h->dsum_cap) {
-    CKR(dalloc(h, &h->dsum, need));
-    h->dsum_cap = need;
-  }
+  CKR(reserve(h, h->dsum_cap, need, need, &h->dsum));
   // caller-order copies of x, y, z, m, soft
   const double* src[5] = {h->p.x, h->p.y, h->p.z, h->p.m, h->p.soft};
   for (int k = 0; k < 5; k++) launch_scatter_f64(src[k], h->dsum + k * n, h->p.order, n, grid_for(h, n), st);
@@ -1527,10 +1486,7 @@ int pt_ewald_direct_sum(pt_handle* h, int64_t nt, const int32_t* targets, double
   const int64_t off_kv = (off_S + 2 * (nk + 1) + 3) / 4 * 4;
   const int64_t off_tgt = off_kv + 4 * (nk + 1);
   const int64_t need = off_tgt + nt / 2 + 1;
-  if (need > h->ewd_cap) {
-    CKR(dalloc(h, &h->ewd, need));
-    h->ewd_cap = need;
-  }
+  CKR(reserve(h, h->ewd_cap, need, need, &h->ewd));
   double* c = h->ewd;
   const double* src[5] = {h->p.x, h->p.y, h->p.z, h->p.m, h->p.soft};
   for (int k = 0; k < 5; k++) launch_scatter_f64(src[k], c + k * n, h->p.order, n, grid_for(h, n), st);
@@ -1569,16 +1525,9 @@ namespace {
 
 int ensure_adjoint(pt_handle* h) {
   const int64_t need = 21 * std::max<int64_t>(h->n, 1);
-  if (need > h->adj_cap) {
-    CKR(dalloc(h, &h->adj, need));
-    h->adj_cap = need;
-  }
+  CKR(reserve(h, h->adj_cap, need, need, &h->adj));
   const int64_t nneed = 10 * std::max<int64_t>(h->nnodes, 1);
-  if (nneed > h->nadj_cap) {
-    CKR(dalloc(h, &h->nadj, nneed));
-    h->nadj_cap = nneed;
-  }
-  return PT_OK;
+  return reserve(h, h->nadj_cap, nneed, nneed, &h->nadj);
 }
 
 bool lists_cover_all(const pt_handle* h) {
@@ -1767,11 +1716,7 @@ extern "C" int pt_chain_grad(pt_handle* h, int nsteps, double dt, int ckpt_every
                 off_A = 14 * n, off_Y = 17 * n, off_xb = 20 * n, off_vb = 23 * n, off_mb = 26 * n, off_pd = 27 * n,
                 off_ck = 30 * n, off_seg = off_ck + (int64_t)nck * 6 * n;
   const int64_t total = off_seg + (int64_t)(C + 1) * 3 * n;
-  if (total > h->chain_cap) {
-    h->chain_cap = 0;
-    CKR(dalloc(h, &h->chain, total));
-    h->chain_cap = total;
-  }
+  CKR(reserve(h, h->chain_cap, total, total, &h->chain));
   double* B = h->chain;
   double *X0 = B + off_X0, *V0 = B + off_V0, *M0 = B + off_M0, *S0 = B + off_S0, *X = B + off_X, *V = B + off_V,
          *A = B + off_A, *Y = B + off_Y, *xb = B + off_xb, *vb = B + off_vb, *mb = B + off_mb, *pd = B + off_pd,

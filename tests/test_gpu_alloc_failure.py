@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from paratreet_b200 import ics
+from paratreet_b200._lib import PtError
 
 pytestmark = pytest.mark.gpu
 
@@ -18,7 +19,6 @@ def sim(**kw):
 
 
 def refused(call, code):
-    from paratreet_b200._lib import PtError
     with pytest.raises(PtError) as e:
         call()
     assert e.value.code == code, e.value
@@ -94,3 +94,76 @@ def test_sph_pass_drops_earlier_lists():
         refused(s.accelerations, STATE)
         s.start_down()
         s.list_digests("two_phase")
+
+
+# limits between the sizes of a pass's arrays: the refused one is another each
+# time (n = 20,000: 0.5 MB of bucket counters at most, 2 MB of node arrays, 4 MB
+# of particles, the list pools far larger)
+@pytest.mark.parametrize("precision", ["fp64", "mixed", "fp64_lists"])
+@pytest.mark.parametrize("record", [False, True])
+def test_refused_growth_is_tried_again(precision, record):
+    """A handle that served a small system meets a larger one under a limit, then
+    the larger one without it, and the small one again."""
+    small, large = ics.plummer(600, seed=2, soft=1e-2), ics.plummer(20000, seed=3, soft=1e-2)
+    kw = dict(precision=precision, record_lists=record, max_particles_per_leaf=4, theta=0.9)
+    want = {}
+    for name, p in (("small", small), ("large", large)):
+        with sim(**kw) as f:
+            f.set_particles(p)
+            f.start_down()
+            want[name] = f.accelerations()
+    failed = set()
+    tol = 1e-4 if precision == "mixed" else 1e-12
+    for limit in [1 << k for k in range(8, 24)]:
+        with sim(**kw) as s:
+            s.set_particles(small)
+            s.start_down()
+            s.set_particles(large)
+            s.set_alloc_limit(limit)
+            for _ in range(2):
+                try:
+                    s.start_down()
+                except PtError as e:
+                    assert e.code == NOMEM
+                    failed.add(limit)
+                    refused(s.accelerations, STATE)
+            s.set_alloc_limit(0)
+            for name, p in (("small", small), ("large", large)):
+                s.set_particles(p)
+                s.start_down()
+                a = s.accelerations()
+                for k in OUT[:3]:  # the forms that replace refused list pools sum in another order
+                    assert np.abs(a[k] - want[name][k]).max() <= tol * np.abs(want[name][k]).max(), (limit, k)
+    assert len(failed) >= 4
+
+
+def test_refused_sph_and_adjoint_arrays_are_tried_again():
+    small, large = ics.plummer(600, seed=2, soft=1e-2), ics.plummer(6000, seed=3, soft=1e-2)
+    for limit in [1 << k for k in range(12, 22)]:
+        with sim(precision="fp64", record_lists=True) as s, sim(precision="fp64", record_lists=True) as f:
+            for h in (s, f):
+                h.set_particles(small)
+                h.sph_density(neighbors=True)
+                h.start_down()
+                h.adjoint(small["x"], small["y"], small["z"])
+                h.set_particles(large)
+            s.set_alloc_limit(limit)
+            for call in (s.sph_density, lambda: s.sph_density(neighbors=True), s.start_down,
+                         lambda: s.adjoint(large["x"], large["y"], large["z"])):
+                try:
+                    call()
+                except PtError as e:
+                    assert e.code in (NOMEM, STATE)
+            s.set_alloc_limit(0)
+            out = []
+            for h in (s, f):
+                d = h.sph_density(neighbors=True)
+                h.start_down()
+                out.append((d, h.accelerations(), h.adjoint(large["x"], large["y"], large["z"])))
+            for a, b in zip(out[0][0], out[1][0]):
+                assert np.array_equal(a, b)
+            for k in OUT:
+                assert np.array_equal(out[0][1][k], out[1][1][k])
+            for k in ("gx", "gy", "gz", "gm"):  # atomic adds: the last bits vary
+                b = out[1][2][k]
+                assert np.abs(out[0][2][k] - b).max() <= 1e-9 * np.abs(b).max()
