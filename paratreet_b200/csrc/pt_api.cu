@@ -209,16 +209,19 @@ int dalloc(pt_handle* h, T** ptr, size_t count) {
 }
 
 // Room for `need` elements in each of the arrays that share the capacity `cap`,
-// with `want` of them where they are allocated anew.  The old arrays go first, so
-// the capacity is 0 until all of the new ones are there: after a refused
+// with `want` of them where they are allocated anew and that fits.  The old arrays
+// go first, so the capacity is 0 until all of the new ones are there: after a refused
 // allocation the next call allocates again instead of using a null array.
 template <typename... T>
 int reserve(pt_handle* h, int64_t& cap, int64_t need, int64_t want, T**... arrays) {
   if (need <= cap) return PT_OK;
   cap = 0;
   int rc = PT_OK;
-  (void)(((rc = dalloc(h, arrays, (size_t)want)) == PT_OK) && ...);
-  if (rc == PT_OK) cap = want;
+  for (const int64_t count : {std::max(need, want), need}) {
+    (void)(((rc = dalloc(h, arrays, (size_t)count)) == PT_OK) && ...);
+    if (rc == PT_OK) cap = count;
+    if (rc != PT_E_NOMEM || count == need) break;
+  }
   return rc;
 }
 

@@ -167,3 +167,27 @@ def test_refused_sph_and_adjoint_arrays_are_tried_again():
             for k in ("gx", "gy", "gz", "gm"):  # atomic adds: the last bits vary
                 b = out[1][2][k]
                 assert np.abs(out[0][2][k] - b).max() <= 1e-9 * np.abs(b).max()
+
+
+def test_headroom_gives_way():
+    """Recorded lists that fit without the eighth of headroom: n entries of four
+    bytes are the largest allocation of this pass behind the first handle's."""
+    p = ics.plummer(30000, seed=5, soft=1e-2)
+    kw = dict(precision="fp64_lists", record_lists=True, max_particles_per_leaf=4, theta=0.5)
+    with sim(**kw) as f:
+        f.set_particles(p)
+        f.start_down()
+        total = int(f.lists().offsets[-1])
+        want = f.accelerations()
+    q = ics.plummer(30000, seed=5, soft=1e-2)
+    with sim(**dict(kw, theta=0.9)) as s:  # shorter lists: every other array has its size
+        s.set_particles(q)
+        s.start_down()
+        assert s.lists().offsets[-1] * 9 // 8 < total
+        s.set_theta(0.5)
+        s.set_alloc_limit(4 * total + 256)
+        s.start_down()
+        assert int(s.lists().offsets[-1]) == total
+        a = s.accelerations()
+    for k in OUT:
+        assert np.array_equal(a[k], want[k]), k
