@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(kE64Warps * 32) eval_p2c_f64(TravParams P, Lis
     const int count = L.pc_count[lb];
     if (count == 0 && P.accumulate) continue;  // nothing to add (the first walk stores, even zeros)
     const int tbase = P.walk[tnode].pstart, ntot = P.walk[tnode].pcount;
+    add_p2c_work(P, b, count, ntot, lane);
     for (int tc = 0; tc < ntot; tc += 32) {
       const int t0 = tbase + tc, nt = min(32, ntot - tc);
       const E64Target x = e64_target(P.p, t0, nt, lane);

@@ -299,11 +299,6 @@ __global__ void __launch_bounds__(kWlWarps * 32, PT_WALK_MINB) walk_lists(TravPa
     max_len = max(max_len, max(npc, npp));
     c_pc += (unsigned long long)npc * (unsigned long long)ntot;
     c_open += opens32;
-    if (P.bucket_work && lane == 0) {  // eval_p2p adds the P2P pairs
-      unsigned long long wk = (unsigned long long)npc * (unsigned long long)ntot;
-      if (P.accumulate) wk += P.bucket_work[b];
-      P.bucket_work[b] = wk;
-    }
     PROF_MARK(w, 4);
   }
   PROF_MARK(w, 5);
@@ -697,6 +692,7 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2c2(TravParam
     if (lane == 0) load_bucket_geom(mom, tnode, w.geom);
     __syncwarp();
     const int tbase = P.walk[tnode].pstart, ntot = P.walk[tnode].pcount;
+    add_p2c_work(P, b, count, ntot, lane);
     for (int tc = 0; tc < ntot; tc += 32) {
       const int t0 = tbase + tc, nt = min(32, ntot - tc);
       const EvTarget2 x = ev_target2(P.p, w.geom, t0, nt, lane);
@@ -1214,7 +1210,7 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2p(TravParams
       PROF_MARK(w, 4);
     }
     // P2P pairs as the reference counts them (n_src * n_tgt per leaf(),
-    // src/Traverser.h:27); the walk wrote the bucket's P2C work before
+    // src/Traverser.h:27); eval_p2c2 wrote the bucket's P2C work before
     c_pp += nsrc * (unsigned long long)ntot;
     if (P.bucket_work && lane == 0) {
       if (kTeam > 1) atomicAdd(P.bucket_work + b, nsrc * (unsigned long long)ntot);

@@ -378,6 +378,17 @@ __device__ __forceinline__ unsigned grab_bucket(unsigned* work, unsigned long lo
   return __shfl_sync(kFull, bi, 0);
 }
 
+// A bucket's P2C evaluations (list entries times targets) in bucket_work, before
+// its P2P pairs are added.  Written by the P2C evaluation, which runs once per
+// batch of replicas; the walk that writes the lists may be repeated.
+__device__ __forceinline__ void add_p2c_work(const TravParams& P, int64_t b, int count, int ntot, int lane) {
+  if (P.bucket_work && lane == 0) {
+    unsigned long long wk = (unsigned long long)count * (unsigned long long)ntot;
+    if (P.accumulate) wk += P.bucket_work[b];
+    P.bucket_work[b] = wk;
+  }
+}
+
 // Sink that only counts the interaction list of a bucket.
 struct ListCounter {
   int64_t n;

@@ -130,3 +130,28 @@ def test_mixed_replica_batches_over_bucket_ranges():
             parts.append(s.accelerations())
     for k in OUT:
         assert np.allclose(parts[0][k] + parts[1][k], full[k], rtol=0, atol=1e-6), k
+
+
+# a later replica's (batch's) lists outgrow the pools: the walk of that batch is
+# repeated, which costs a launch in the first pass and none in the second
+@pytest.mark.parametrize("prec,nrep,theta", [("fp64_lists", 1, 0.25), ("mixed", 2, 0.35)])
+def test_repeated_walk_counts_its_work_once(prec, nrep, theta):
+    p = ics.lattice(12, seed=3, rms_cells=0.3, soft_cells=0.2)
+    kw = dict(max_particles_per_leaf=1, theta=theta, periodic=True, n_replicas=nrep)
+    with sim(precision="fp64", **kw) as s:
+        s.set_particles(p)
+        s.start_down()
+        want, c0 = s.bucket_work(), s.counters()
+    with sim(precision=prec, **kw) as s:
+        s.set_list_region(64)
+        s.set_particles(p)
+        s.start_down()
+        first, c1 = s.bucket_work(), s.counters()
+        s.start_down()
+        second, c2 = s.bucket_work(), s.counters()
+    print(prec, "launches", c1["launches"], c2["launches"], "entries per bucket", c0["n_pc"] / c0["n_buckets"], c0["n_pp"] / c0["n_buckets"])
+    assert c1["launches"] > c2["launches"]
+    for c in (c1, c2):
+        assert [c[k] for k in ("n_pp", "n_pc", "n_open")] == [c0[k] for k in ("n_pp", "n_pc", "n_open")]
+    assert np.array_equal(second, want)
+    assert np.array_equal(first, want)
