@@ -106,7 +106,7 @@ __device__ __forceinline__ bool ensure_region(Region& r, unsigned long long* cur
 // a new region of at least twice its new length.  False only if the pool is
 // full.  Warp-uniform; the list's entries were written before the __syncwarp
 // that ends each walk step.
-template <bool kReps>
+template <bool kBytes>
 __device__ __forceinline__ bool make_room(int n, Region& r, unsigned long long& start, int32_t* __restrict__ pool,
                                           uint8_t* __restrict__ reps, unsigned long long* cursor,
                                           unsigned long long cap, unsigned region, int lane) {
@@ -122,7 +122,7 @@ __device__ __forceinline__ bool make_room(int n, Region& r, unsigned long long& 
   }
   for (unsigned long long k = lane; k < len; k += 32) {
     pool[s + k] = pool[start + k];
-    if (kReps) reps[s + k] = reps[start + k];
+    if (kBytes) reps[s + k] = reps[start + k];
   }
   start = s;
   r.cur = s + len;
@@ -134,18 +134,20 @@ __device__ __forceinline__ bool make_room(int n, Region& r, unsigned long long& 
 #ifndef PT_WALK_MINB
 #define PT_WALK_MINB 7
 #endif
-// kReps: a batch of replica offsets (periodic passes).  All replicas of a batch
+// kReps: a batch of replica offsets (periodic passes); kBytes: of more than one.  All replicas of a batch
 // are walked together -- their roots are tested in one step, and a step's four
 // opened nodes may belong to different replicas -- and an entry's replica goes to
-// a byte pool beside the lists, so that a bucket has one list for the batch.
+// a byte pool beside the lists (a batch of one has none: a test of the pointer in
+// the loops instead cost 0.9% of the 128^3 lattice pass), so that a bucket has one
+// list for the batch.
 // (One walk and two evaluations per replica left the outer replicas' short lists
 // on a few lanes and read and wrote every particle's sums 54 times: 22.8 of the
 // 27.4 ms of a 128^3 lattice pass with 27 replicas.)
-template <bool kReps>
+template <bool kReps, bool kBytes>
 __global__ void __launch_bounds__(kWlWarps * 32, PT_WALK_MINB) walk_lists(TravParams P, ListParams L,
                                                                          const Mom* __restrict__ mom) {
   __shared__ WalkWarp<kReps> warps[kWlWarps];
-  __shared__ RepOffsets offs[kReps ? 1 : 0 + 1];
+  __shared__ RepOffsets offs[1];
   WalkWarp<kReps>& w = warps[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   if (kReps) rep_offsets(P, offs[0]);
@@ -243,11 +245,11 @@ __global__ void __launch_bounds__(kWlWarps * 32, PT_WALK_MINB) walk_lists(TravPa
         const int n = __popc(m);
         opens32 += n;  // internal children: accepted (P2C) here, opened below
         if (n && fits) {
-          fits = make_room<kReps>(n, rpc, pc0, L.pc_pool, L.pc_rep, L.cursor + 0, L.cap_pc, L.region, lane);
+          fits = make_room<kBytes>(n, rpc, pc0, L.pc_pool, L.pc_rep, L.cursor + 0, L.cap_pc, L.region, lane);
           if (fits && pc) {
             const unsigned long long at = rpc.cur + __popc(m & lt);
             L.pc_pool[at] = node | (cls == kClsMono ? (int)0x80000000 : 0) | (near ? 0x40000000 : 0);
-            if (kReps) L.pc_rep[at] = (uint8_t)rep;
+            if (kBytes) L.pc_rep[at] = (uint8_t)rep;
           }
           if (fits) rpc.cur += (unsigned long long)n;
         }
@@ -255,11 +257,11 @@ __global__ void __launch_bounds__(kWlWarps * 32, PT_WALK_MINB) walk_lists(TravPa
         const unsigned mp = __ballot_sync(kFull, pp);
         const int npp = __popc(mp);
         if (npp && fits) {
-          fits = make_room<kReps>(npp, rpp, pp0, L.pp_pool, L.pp_rep, L.cursor + 1, L.cap_pp, L.region, lane);
+          fits = make_room<kBytes>(npp, rpp, pp0, L.pp_pool, L.pp_rep, L.cursor + 1, L.cap_pp, L.region, lane);
           if (fits && pp) {
             const unsigned long long at = rpp.cur + __popc(mp & lt);
             L.pp_pool[at] = node;
-            if (kReps) L.pp_rep[at] = (uint8_t)rep;
+            if (kBytes) L.pp_rep[at] = (uint8_t)rep;
           }
           if (fits) rpp.cur += (unsigned long long)npp;
         }
@@ -669,7 +671,7 @@ __device__ __forceinline__ void add_term(float& s, float& c, float v) {
   else s += v;
 }
 
-template <int kMinBlocks, bool kReps>
+template <int kMinBlocks, bool kReps, bool kBytes>
 __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2c2(TravParams P, ListParams L,
                                                                       const Mom* __restrict__ mom) {
   __shared__ EvalWarpC2 warps[kEvWarps];
@@ -706,7 +708,7 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2c2(TravParam
       int en0 = (2 * lane < count) ? L.pc_pool[start + 2 * lane] : 0;
       int en1 = (2 * lane + 1 < count) ? L.pc_pool[start + 2 * lane + 1] : 0;
       int rn0 = 0, rn1 = 0;
-      if (kReps) {
+      if (kBytes) {
         rn0 = (2 * lane < count) ? L.pc_rep[start + 2 * lane] : 0;
         rn1 = (2 * lane + 1 < count) ? L.pc_rep[start + 2 * lane + 1] : 0;
       }
@@ -718,7 +720,7 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2c2(TravParam
           const int qn = cs + 64 + 2 * lane;
           en0 = (qn < count) ? L.pc_pool[start + qn] : 0;
           en1 = (qn + 1 < count) ? L.pc_pool[start + qn + 1] : 0;
-          if (kReps) {
+          if (kBytes) {
             rn0 = (qn < count) ? L.pc_rep[start + qn] : 0;
             rn1 = (qn + 1 < count) ? L.pc_rep[start + qn + 1] : 0;
           }
@@ -1089,7 +1091,7 @@ __device__ __forceinline__ void ev_p2p_leaves(EvalWarp& w, int base, int nleaves
 // (a separate marking pass over the list read every record twice: 0.6 ms at
 // N = 2^24).  Returns the source particles of the listed leaves, as the
 // reference counts P2P work (n_src * n_tgt per leaf(), src/Traverser.h:27).
-template <bool kTwo, bool kReps, class Tgt>
+template <bool kTwo, bool kReps, bool kBytes, class Tgt>
 __device__ __forceinline__ unsigned long long ev_p2p_blocks(EvalWarp& w, const TravParams& P,
                                                                   const ListParams& L, const RepOffsets* R,
                                                                   const Tgt& x, int64_t start, int count, int lane,
@@ -1117,7 +1119,7 @@ __device__ __forceinline__ unsigned long long ev_p2p_blocks(EvalWarp& w, const T
         const double smax = __hiloint2double(__float_as_int(a.y), __float_as_int(a.x));
         double cx = c.x, cy = c.y, cz = c.z;
         if (kReps) {
-          const int rep = L.pp_rep[start + q];
+          const int rep = kBytes ? L.pp_rep[start + q] : 0;
           cx += R->x[rep];
           cy += R->y[rep];
           cz += R->z[rep];
@@ -1152,7 +1154,7 @@ __device__ __forceinline__ unsigned long long ev_p2p_blocks(EvalWarp& w, const T
 
 // kTeam = 4: a CTA's warps share a bucket, each a quarter of its list (with few
 // buckets a pass takes as long as the longest list).
-template <int kMinBlocks, bool kReps, int kTeam>
+template <int kMinBlocks, bool kReps, bool kBytes, int kTeam>
 __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2p(TravParams P, ListParams L,
                                                                      const Mom* __restrict__ mom) {
   __shared__ EvalWarp warps[kEvWarps];
@@ -1200,11 +1202,11 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2p(TravParams
       if (ev_two_targets(nt)) {
         const EvTarget2 x = ev_target2(P.p, w.geom, t0, nt, lane);
         ev_two_zero(w, lane);
-        nsrc = ev_p2p_blocks<true, kReps>(w, P, L, offs, x, start, count, lane, K);
+        nsrc = ev_p2p_blocks<true, kReps, kBytes>(w, P, L, offs, x, start, count, lane, K);
         ev_finish2<kTeam>(w, team, K, x, P, t0, lane);
       } else {
         const EvTarget x = ev_target(P.p, w.geom, t0, nt, lane);
-        nsrc = ev_p2p_blocks<false, kReps>(w, P, L, offs, x, start, count, lane, K);
+        nsrc = ev_p2p_blocks<false, kReps, kBytes>(w, P, L, offs, x, start, count, lane, K);
         ev_finish<kTeam>(w, team, K, x, P, t0, lane);
       }
       PROF_MARK(w, 4);
@@ -1235,29 +1237,34 @@ int walk_lists_grid(int sms) { return sms * PT_WALK_MINB; }  // the CTAs residen
 
 void launch_walk_lists(const TravParams& P, const ListParams& L, const Mom* mom, int grid, cudaStream_t st) {
   note_launch();
-  if (P.rep_count) walk_lists<true><<<grid, kWlWarps * 32, 0, st>>>(P, L, mom);
-  else walk_lists<false><<<grid, kWlWarps * 32, 0, st>>>(P, L, mom);
+  const int threads = kWlWarps * 32;
+  if (P.rep_count > 1) walk_lists<true, true><<<grid, threads, 0, st>>>(P, L, mom);
+  else if (P.rep_count) walk_lists<true, false><<<grid, threads, 0, st>>>(P, L, mom);
+  else walk_lists<false, false><<<grid, threads, 0, st>>>(P, L, mom);
 }
-void launch_eval_lists(const TravParams& P, const TravParams& Q, const ListParams& L, const Mom* mom, int sms,
-                       cudaStream_t st) {
+
+template <bool kReps, bool kBytes>
+static void launch_eval(const TravParams& P, const TravParams& Q, const ListParams& L, const Mom* mom, int sms,
+                        cudaStream_t st) {
   const int grid = 16 * sms;
   const int threads = kEvWarps * 32;
   note_launch();
-  if (P.rep_count) eval_p2c2<PT_P2C_MINB, true><<<grid, threads, 0, st>>>(P, L, mom);
-  else eval_p2c2<PT_P2C_MINB, false><<<grid, threads, 0, st>>>(P, L, mom);
+  eval_p2c2<PT_P2C_MINB, kReps, kBytes><<<grid, threads, 0, st>>>(P, L, mom);
   note_launch();
   // Up to 96 buckets per SM (28 warps are resident), a CTA per bucket: the
   // traversal of 4,000 particles 0.18 -> 0.13 ms, of 10,000 0.23-0.34 -> 0.18-
   // 0.19, of 40,000 in buckets of 32 0.73 -> 0.47 and of 80,000 1.00 -> 0.80
   // (Plummer); beyond it no difference.
-  const bool team = P.b_end - P.b_begin <= (int64_t)96 * sms;
-  if (P.rep_count) {
-    if (team) eval_p2p<PT_P2P_MINB, true, kEvWarps><<<grid, threads, 0, st>>>(Q, L, mom);
-    else eval_p2p<PT_P2P_MINB, true, 1><<<grid, threads, 0, st>>>(Q, L, mom);
-  } else {
-    if (team) eval_p2p<PT_P2P_MINB, false, kEvWarps><<<grid, threads, 0, st>>>(Q, L, mom);
-    else eval_p2p<PT_P2P_MINB, false, 1><<<grid, threads, 0, st>>>(Q, L, mom);
-  }
+  if (P.b_end - P.b_begin <= (int64_t)96 * sms)
+    eval_p2p<PT_P2P_MINB, kReps, kBytes, kEvWarps><<<grid, threads, 0, st>>>(Q, L, mom);
+  else
+    eval_p2p<PT_P2P_MINB, kReps, kBytes, 1><<<grid, threads, 0, st>>>(Q, L, mom);
+}
+void launch_eval_lists(const TravParams& P, const TravParams& Q, const ListParams& L, const Mom* mom, int sms,
+                       cudaStream_t st) {
+  if (P.rep_count > 1) launch_eval<true, true>(P, Q, L, mom, sms, st);
+  else if (P.rep_count) launch_eval<true, false>(P, Q, L, mom, sms, st);
+  else launch_eval<false, false>(P, Q, L, mom, sms, st);
 }
 
 }  // namespace pt

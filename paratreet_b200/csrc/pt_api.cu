@@ -93,6 +93,8 @@ struct pt_handle {
   bool two_phase = true;  // PT_MIXED_FUSED=1 selects the fused walk + evaluate kernel
   int32_t *pool_pc = nullptr, *pool_pp = nullptr;
   unsigned long long cap_pc = 0, cap_pp = 0;    // allocated entries of each pool
+  bool pool_reps = false;       // ... with a byte per entry behind them
+  int rep_batch = kMaxReps;     // replicas a mixed periodic pass takes in one batch
   unsigned long long want_pc = 0, want_pp = 0;  // entries the next pass should have
   int64_t *l_pc_start = nullptr, *l_pp_start = nullptr;
   int32_t *l_pc_count = nullptr, *l_pp_count = nullptr;
@@ -533,6 +535,7 @@ void replica_offset(const pt_handle* h, int r, TravParams& P) {
 // outgrows its warp's region moves it to a new region inside the walk); only
 // a pass whose lists fill a pool is repeated (counters restored) with pools
 // twice as large, which happens at most on the first passes of a handle.
+constexpr int kFewerReplicas = 1;  // run_two_phase: no room for a batch's lists, h->rep_batch is smaller now
 int run_two_phase(pt_handle* h, TravParams& P) {
   cudaStream_t st = h->stream;
   const int64_t nb = P.b_end - P.b_begin;
@@ -559,7 +562,9 @@ int run_two_phase(pt_handle* h, TravParams& P) {
         std::max<unsigned long long>(h->want_pc, 1024ull * nb + slack);
     const unsigned long long need_pp =
         std::max<unsigned long long>(h->want_pp, 256ull * nb + slack);
-    if (need_pc > h->cap_pc || need_pp > h->cap_pp) {
+    // an entry, and where a batch has several replicas its replica (a byte)
+    const bool reps = P.rep_count > 1;
+    if (need_pc > h->cap_pc || need_pp > h->cap_pp || (reps && !h->pool_reps)) {
       // a quarter of headroom, so that the pass-to-pass variation of the
       // reserved regions does not free and map the multi-GB pools again
       // (which costs more than a whole pass); without room for it, the bare need
@@ -567,8 +572,7 @@ int run_two_phase(pt_handle* h, TravParams& P) {
       dfree(h->pool_pp);
       h->cap_pc = h->cap_pp = 0;
       unsigned long long alloc_pc = need_pc + need_pc / 4, alloc_pp = need_pp + need_pp / 4;
-      // an entry, and in a periodic pass its replica (a byte, behind the entries)
-      const size_t per = sizeof(int32_t) + (h->cfg.periodic ? 1 : 0);
+      const size_t per = sizeof(int32_t) + (reps ? 1 : 0);
       if (device_malloc(h, &h->pool_pc, alloc_pc * per) != cudaSuccess ||
           device_malloc(h, &h->pool_pp, alloc_pp * per) != cudaSuccess) {
         cudaGetLastError();
@@ -579,29 +583,30 @@ int run_two_phase(pt_handle* h, TravParams& P) {
       }
       if ((!h->pool_pc && device_malloc(h, &h->pool_pc, need_pc * per) != cudaSuccess) ||
           (!h->pool_pp && device_malloc(h, &h->pool_pp, need_pp * per) != cudaSuccess)) {
-        // no room for the lists: this handle evaluates with the fused kernel from now on
         cudaGetLastError();
         dfree(h->pool_pc);
         dfree(h->pool_pp);
-        h->two_phase = false;
         CK(restore_counters());
-        for (int k = 0; k < std::max(1, P.rep_count); k++) {  // the batch's replicas one by one
-          TravParams A = P;
-          if (P.rep_count) replica_offset(h, P.rep_first + k, A);
-          A.accumulate = P.accumulate || k > 0;
-          CKR(zero_queue(h));
-          if (h->cfg.precision == PT_FP64_LISTS) launch_traverse_f64(A, h->nd.mom, h->sms, st);
-          else launch_traverse_mixed(A, h->nd.mom, h->sms * 16, st);
+        if (reps) {  // no room for the lists of so many replicas
+          h->rep_batch = P.rep_count / 2;
+          h->want_pc = h->want_pp = 0;
+          return kFewerReplicas;
         }
+        // no room for the lists: this handle evaluates with the fused kernel from now on
+        h->two_phase = false;
+        CKR(zero_queue(h));
+        if (h->cfg.precision == PT_FP64_LISTS) launch_traverse_f64(P, h->nd.mom, h->sms, st);
+        else launch_traverse_mixed(P, h->nd.mom, h->sms * 16, st);
         CK(cudaGetLastError());
         return PT_OK;
       }
       h->cap_pc = alloc_pc;
       h->cap_pp = alloc_pp;
+      h->pool_reps = reps;
     }
     L.pc_pool = h->pool_pc;
     L.pp_pool = h->pool_pp;
-    if (h->cfg.periodic) {
+    if (reps) {
       L.pc_rep = reinterpret_cast<uint8_t*>(h->pool_pc + h->cap_pc);
       L.pp_rep = reinterpret_cast<uint8_t*>(h->pool_pp + h->cap_pp);
     }
@@ -766,20 +771,22 @@ int traverse(pt_handle* h, int64_t b0, int64_t b1) {
   // the first continues each particle's sums
   const int nr = h->cfg.periodic ? h->cfg.n_replicas : 0;
   const int reps = (2 * nr + 1) * (2 * nr + 1) * (2 * nr + 1);
-  // the two-phase forms take the replicas in batches, the mixed one up to
-  // kMaxReps at a time; the others one by one
+  // the mixed two-phase form takes the replicas in batches of up to kMaxReps, of
+  // fewer where the lists of so many do not fit; the others one by one
   int per = 1;
   P.rep_n = nr;
   P.period = h->cfg.period;
   for (int r = 0; r < reps; r += per) {
     const bool lists_form = (h->cfg.precision == PT_MIXED || h->cfg.precision == PT_FP64_LISTS) && h->two_phase;
-    per = h->cfg.precision == PT_MIXED && lists_form ? std::min(kMaxReps, reps - r) : 1;
+    per = h->cfg.precision == PT_MIXED && lists_form ? std::min(h->rep_batch, reps - r) : 1;
     if (h->cfg.periodic) replica_offset(h, r, P);
     P.rep_first = r;
     P.rep_count = reps > 1 && lists_form ? per : 0;
     P.accumulate = r > 0;
     CKR(zero_queue(h));
-    CKR(run_traversal(h, P, grid));
+    const int rc = run_traversal(h, P, grid);
+    if (rc == kFewerReplicas) per = 0;  // the same replicas again
+    else CKR(rc);
   }
   if (h->cfg.periodic) CKR(ewald_correction_pass(h, b0, b1));
   CK(cudaEventRecord(h->ev[6], st));
@@ -868,6 +875,7 @@ int set_particles_impl(pt_handle* h, int64_t n, const double* const src[8], cuda
   for (int i = 0; i < 8 && n > 0; i++)
     if (!src[i]) return fail(h, PT_E_ARG, "null particle array");
   CKR(ensure_particles(h, n));
+  if (n != h->n) h->rep_batch = kMaxReps;
   h->n = n;
   double* dst[8] = {h->p.x, h->p.y, h->p.z, h->p.vx, h->p.vy, h->p.vz, h->p.m, h->p.soft};
   for (int i = 0; i < 8 && n > 0; i++)

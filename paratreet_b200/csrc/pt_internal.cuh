@@ -162,7 +162,7 @@ struct TravParams {
 struct ListParams {
   int32_t* pc_pool;
   int32_t* pp_pool;
-  uint8_t *pc_rep, *pp_rep;    // the entries' replicas in the batch (periodic passes; else null)
+  uint8_t *pc_rep, *pp_rep;    // the entries' replicas in a batch of several (else null)
   unsigned long long* cursor;  // [0] P2C pool, [1] P2P pool
   unsigned long long cap_pc, cap_pp;
   unsigned region, thresh;     // region size; least space left before a bucket starts

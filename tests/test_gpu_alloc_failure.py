@@ -191,3 +191,38 @@ def test_headroom_gives_way():
         a = s.accelerations()
     for k in OUT:
         assert np.array_equal(a[k], want[k]), k
+
+
+# bytes per entry of the first pools: 13 leaves batches of one replica (no replica
+# bytes), 20 of half the 27
+@pytest.mark.parametrize("nrep,room", [(1, 13), (1, 20), (2, 13)])
+def test_replica_lists_that_do_not_fit_take_smaller_batches(nrep, room):
+    """The lists of a full batch of replicas outgrow the limit, those of a few fit:
+    the pass takes fewer replicas at a time instead of the fused form, which
+    leaves no potential (pot) of the quadrupole terms."""
+    p = ics.lattice(24, seed=6, rms_cells=0.3, soft_cells=0.3)
+    kw = dict(precision="mixed", max_particles_per_leaf=4, theta=0.4, periodic=True, n_replicas=nrep)
+    out, counts, launches = [], [], []
+    # as test_mixed_replica_batches_match_fp64 (tests/test_gpu_edges.py)
+    scale = {"a": 1, "p": (2 * nrep + 1) ** 2}
+    for limit in (0, 1):
+        with sim(**kw) as s:
+            s.set_list_region(64)
+            s.set_particles(p)
+            if limit:
+                s.set_alloc_limit(room * (1024 * nb + 148 * 7 * 4 * 64))
+            s.start_down()
+            nb = s.counters()["n_buckets"]
+            out.append(s.accelerations())
+            c = s.counters()
+            counts.append((c["n_pp"], c["n_pc"], c["n_open"], int(s.bucket_work().sum())))
+            s.start_down()
+            again = s.accelerations()
+            launches.append((c["launches"], s.counters()["launches"]))
+            for k in OUT:
+                assert np.abs(again[k] - out[-1][k]).max() < 1e-5 * scale[k[0]], k
+    print("launches", launches)
+    assert counts[0] == counts[1]
+    assert launches[1][1] > launches[0][1]
+    for k in OUT:
+        assert np.abs(out[0][k] - out[1][k]).max() < 1e-5 * scale[k[0]], k
