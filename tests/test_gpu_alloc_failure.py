@@ -226,3 +226,21 @@ def test_replica_lists_that_do_not_fit_take_smaller_batches(nrep, room):
     assert launches[1][1] > launches[0][1]
     for k in OUT:
         assert np.abs(out[0][k] - out[1][k]).max() < 1e-5 * scale[k[0]], k
+
+
+def test_fused_form_in_the_middle_of_a_pass_leaves_no_potential():
+    """Where even one replica's lists do not fit, the replicas before it must not
+    leave their part of pot: the fused form has none (pot_full has it)."""
+    p = ics.lattice(24, seed=6, rms_cells=0.3, soft_cells=0.3)
+    with sim(precision="mixed", max_particles_per_leaf=4, theta=0.4, periodic=True, n_replicas=1) as s:
+        s.set_list_region(64)
+        s.set_particles(p)
+        s.set_alloc_limit(8 * (1024 * 8583 + 148 * 7 * 4 * 64))  # 8583 buckets
+        s.start_down()
+        assert s.counters()["n_buckets"] == 8583
+        first, n1 = s.accelerations(), s.counters()["launches"]
+        s.start_down()  # fused from the first replica on
+        second, n2 = s.accelerations(), s.counters()["launches"]
+    assert n1 != n2
+    for k in OUT:
+        assert np.abs(first[k] - second[k]).max() < 1e-5 * (1 if k[0] == "a" else 9), k
