@@ -124,6 +124,7 @@ struct pt_handle {
   double last_dt = 0.0;
   bool have_forces = false;     // a force pass ran since the particles were set
   bool forces_current = false;  // ... and the positions have not moved since
+  bool keys_valid = false;      // the keys are sorted and line up with the particles
   bool trav_range_partial = false;
 
   double* adj = nullptr;  // adjoint scratch: cotangent (3N) and gradients (4N), sorted + caller order,
@@ -357,6 +358,7 @@ int keys_and_sort(pt_handle* h) {
   cudaStream_t st = h->stream;
   const int64_t n = h->n;
   const int g = grid_for(h, n);
+  h->keys_valid = false;
   launch_bbox(h->p.x, h->p.y, h->p.z, n, h->bbox_partial, h->bbox_blocks, h->d_ticket, h->d_uni, h->d_status, st);
   launch_keys(h->p.x, h->p.y, h->p.z, n, h->d_uni, h->p.key, h->idx, g, st);
   CK(cudaGetLastError());
@@ -401,6 +403,7 @@ int build_tree(pt_handle* h) {
   // the particles are in a new order from here on: results of an earlier pass no
   // longer line up with it
   h->have_forces = h->forces_current = h->lists_valid = h->tp_lists_valid = false;
+  h->keys_valid = true;
   const uint32_t* tot = h->pin->total;  // Internal nodes of each level, leaves
   int64_t ni = 0;
   int depth = 0;
@@ -1284,6 +1287,7 @@ int pt_get_keys(pt_handle* h, uint64_t* keys) {
   if (!h || !keys) return PT_E_ARG;
   if (!h->have_forces) return fail(h, PT_E_STATE, "no force pass yet");
   if (h->n == 0) return PT_OK;
+  if (!h->keys_valid) return fail(h, PT_E_STATE, "the keys were lost in a failed pass");
   cudaSetDevice(h->cfg.device);
   launch_scatter_u64(h->p.key, h->key_alt, h->p.order, h->n, grid_for(h, h->n), h->stream);
   CK(cudaGetLastError());

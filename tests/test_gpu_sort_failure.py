@@ -74,3 +74,34 @@ def test_failed_sort_leaves_the_particles(n, polls):
         s.set_sort_spin_limit()
         s.start_down()
         assert np.array_equal(s.keys(), want)
+
+
+def test_failed_sort_keeps_results_but_no_keys():
+    """The accelerations of the pass before a failed sort still line up with the
+    particles; its keys were overwritten."""
+    from paratreet_b200._lib import PtError
+    from paratreet_b200.gravity import GravitySimulation
+
+    n = (1 << 21) + 5
+    p = ics.plummer(n, seed=6, soft=1e-3)
+    with GravitySimulation(max_particles_per_leaf=32, theta=1.0, precision="mixed") as s:
+        s.set_particles(p)
+        s.start_down()
+        want, keys = s.accelerations(), s.keys()
+        s.set_sort_spin_limit(0)
+        for _ in range(6):
+            try:
+                s.start_down()
+            except PtError:
+                break
+        else:
+            pytest.fail("no look-back gave up in 6 passes with a spin limit of 0")
+        got = s.accelerations()
+        for k in want:
+            assert np.array_equal(got[k], want[k]), k
+        with pytest.raises(PtError) as e:
+            s.keys()
+        assert e.value.code == -4
+        s.set_sort_spin_limit()
+        s.start_down()
+        assert np.array_equal(s.keys(), keys)
