@@ -424,13 +424,33 @@ __device__ __forceinline__ void ev_two_zero(EvalWarp& w, int lane) {
   w.st[4][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-// Target t0 + lane's P2P sums v: added to ax, ay, az and pot_full (GravityVisitor::
-// leaf applies no potential).  A team's warps bring their sums together first
-// and warp 0 adds them, in the warps' order.
+// One target's P2P sums, added to ax, ay, az and pot_full (GravityVisitor::leaf
+// applies no potential).
+__device__ __forceinline__ void ev_add(const TravParams& P, int i, const double v[4]) {
+  P.p.ax[i] += v[0];
+  P.p.ay[i] += v[1];
+  P.p.az[i] += v[2];
+  P.p.potf[i] += v[3];
+}
+
+// The sums of G lane groups per target in red (4 per group and target), added to
+// the targets t0 ...; a team's warps bring their sums together first and warp 0
+// adds them, in the warps' order.
 template <int kTeam>
-__device__ __forceinline__ void ev_add(double* team, double v[4], int nt, const TravParams& P, int t0,
-                                       int lane) {
-  if (kTeam > 1) {
+__device__ __forceinline__ void ev_reduce(const double* red, double* team, int G, int nt, const TravParams& P, int t0,
+                                          int lane) {
+  if constexpr (kTeam == 1) {
+    if (lane < nt) {
+      double v[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int gg = 0; gg < G; gg++)
+        for (int k = 0; k < 4; k++) v[k] += red[4 * (gg * nt + lane) + k];
+      ev_add(P, t0 + lane, v);
+    }
+  } else {
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    if (lane < nt)
+      for (int gg = 0; gg < G; gg++)
+        for (int k = 0; k < 4; k++) v[k] += red[4 * (gg * nt + lane) + k];
     const int q = threadIdx.x >> 5;
 #pragma unroll
     for (int k = 0; k < 4; k++) team[(q * 32 + lane) * 4 + k] = v[k];
@@ -441,14 +461,7 @@ __device__ __forceinline__ void ev_add(double* team, double v[4], int nt, const 
         for (int k = 0; k < 4; k++) v[k] += team[(o * 32 + lane) * 4 + k];
     }
     __syncthreads();
-    if (q != 0) return;
-  }
-  if (lane < nt) {
-    const int i = t0 + lane;
-    P.p.ax[i] += v[0];
-    P.p.ay[i] += v[1];
-    P.p.az[i] += v[2];
-    P.p.potf[i] += v[3];
+    if (q == 0 && lane < nt) ev_add(P, t0 + lane, v);
   }
 }
 
@@ -472,11 +485,7 @@ __device__ __forceinline__ void ev_finish2(EvalWarp& w, double* team, const Kaha
     }
   }
   __syncwarp();
-  double v[4] = {0.0, 0.0, 0.0, 0.0};
-  if (lane < x.nt)
-    for (int gg = 0; gg < x.G; gg++)
-      for (int k = 0; k < 4; k++) v[k] += red[4 * (gg * x.nt + lane) + k];
-  ev_add<kTeam>(team, v, x.nt, P, t0, lane);
+  ev_reduce<kTeam>(red, team, x.G, x.nt, P, t0, lane);
 }
 
 // The same for a single target.
@@ -488,12 +497,8 @@ __device__ __forceinline__ void ev_finish(EvalWarp& w, double* team, const Kahan
 #pragma unroll
   for (int k = 0; k < 4; k++) red[4 * lane + k] = (double)K.s[k] - (double)K.c[k];
   __syncwarp();
-  double v[4] = {0.0, 0.0, 0.0, 0.0};
-  if (lane < x.nt)
-    for (int gg = 0; gg < x.G; gg++)
-      for (int k = 0; k < 4; k++) v[k] += red[4 * (gg * x.nt + lane) + k];
+  ev_reduce<kTeam>(red, team, x.G, x.nt, P, t0, lane);
   __syncwarp();
-  ev_add<kTeam>(team, v, x.nt, P, t0, lane);
 }
 
 __device__ __forceinline__ bool next_bucket(const TravParams& P, int lane, int64_t& b, int& tnode) {
@@ -1152,8 +1157,48 @@ __device__ __forceinline__ unsigned long long ev_p2p_blocks(EvalWarp& w, const T
   return nsrc;
 }
 
+// One bucket's P2P: its targets against the entries [start, start + count) of its
+// list (a team's warp: its share).  Returns the pairs.
+template <bool kReps, bool kBytes, int kTeam>
+__device__ __forceinline__ unsigned long long ev_p2p_bucket(EvalWarp& w, double* team, const TravParams& P,
+                                                            const ListParams& L, const RepOffsets* R,
+                                                            const Mom* __restrict__ mom, int tnode, int64_t start,
+                                                            int count, int lane) {
+  __syncwarp();
+  if (lane == 0) load_bucket_geom(mom, tnode, w.geom);
+  __syncwarp();
+  const int tbase = P.walk[tnode].pstart, ntot = P.walk[tnode].pcount;
+  unsigned long long nsrc = 0;
+  PROF_MARK(w, 0);
+  for (int tc = 0; tc < ntot; tc += 32) {
+    const int t0 = tbase + tc, nt = min(32, ntot - tc);
+    if (ev_two_targets(nt)) {
+      const EvTarget2 x = ev_target2(P.p, w.geom, t0, nt, lane);
+      ev_two_zero(w, lane);
+      Kahan4 K;
+      K.zero();
+      nsrc = ev_p2p_blocks<true, kReps, kBytes>(w, P, L, R, x, start, count, lane, K);
+      ev_finish2<kTeam>(w, team, K, x, P, t0, lane);
+      PROF_MARK(w, 4);
+      continue;
+    }
+    const EvTarget x = ev_target(P.p, w.geom, t0, nt, lane);
+    Kahan4 K;
+    K.zero();
+    nsrc = ev_p2p_blocks<false, kReps, kBytes>(w, P, L, R, x, start, count, lane, K);
+    ev_finish<kTeam>(w, team, K, x, P, t0, lane);
+    PROF_MARK(w, 4);
+  }
+  // P2P pairs as the reference counts them (n_src * n_tgt per leaf(),
+  // src/Traverser.h:27)
+  return nsrc * (unsigned long long)ntot;
+}
+
 // kTeam = 4: a CTA's warps share a bucket, each a quarter of its list (with few
-// buckets a pass takes as long as the longest list).
+// buckets a pass takes as long as the longest list).  eval_p2c2 wrote the bucket's
+// P2C work to bucket_work before.  The one-warp form has a bucket loop and a
+// reduction of its own (ev_reduce): sharing the team's cost it 1.3% at N = 2^24
+// (35.0 against 34.55 ms) and 1.7% at 1.5e6 (10.4 against 10.24 ms).
 template <int kMinBlocks, bool kReps, bool kBytes, int kTeam>
 __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2p(TravParams P, ListParams L,
                                                                      const Mom* __restrict__ mom) {
@@ -1163,60 +1208,40 @@ __global__ void __launch_bounds__(kEvWarps * 32, kMinBlocks) eval_p2p(TravParams
   __shared__ unsigned team_b;
   if (kReps) rep_offsets(P, offs[0]);
   EvalWarp& w = warps[threadIdx.x >> 5];
-  const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   unsigned long long c_pp = 0;
   PROF_START(w);
-  while (true) {
-    unsigned bi;
-    if (kTeam > 1) {
+  if constexpr (kTeam == 1) {
+    int64_t b;
+    int tnode;
+    while (next_bucket(P, lane, b, tnode)) {
+      if (tnode < 0 || tnode >= P.nnodes) continue;
+      const int64_t start = L.pp_start[b - P.b_begin];
+      const int count = L.pp_count[b - P.b_begin];
+      if (count == 0) continue;  // P2P only adds
+      const unsigned long long pairs =
+          ev_p2p_bucket<kReps, kBytes, 1>(w, team, P, L, offs, mom, tnode, start, count, lane);
+      c_pp += pairs;
+      if (P.bucket_work && lane == 0) P.bucket_work[b] += pairs;
+    }
+  } else {
+    const int q = threadIdx.x >> 5;
+    while (true) {
       if (threadIdx.x == 0) team_b = atomicAdd(P.work, 1u);
       __syncthreads();
-      bi = team_b;
+      const int64_t b = P.b_begin + (int64_t)team_b;
       __syncthreads();
-    } else {
-      bi = grab_bucket(P.work, P.smq, P.batch, lane);
-    }
-    const int64_t b = P.b_begin + (int64_t)bi;
-    if (b >= P.b_end) break;
-    const int tnode = P.buckets[b];
-    if (tnode < 0 || tnode >= P.nnodes) continue;
-    const int64_t lb = b - P.b_begin;
-    int64_t start = L.pp_start[lb];
-    int count = L.pp_count[lb];
-    if (count == 0) continue;  // P2P only adds
-    if (kTeam > 1) {
+      if (b >= P.b_end) break;
+      const int tnode = P.buckets[b];
+      if (tnode < 0 || tnode >= P.nnodes) continue;
+      const int64_t start = L.pp_start[b - P.b_begin];
+      const int count = L.pp_count[b - P.b_begin];
+      if (count == 0) continue;
       const int per = (count + kTeam - 1) / kTeam, c0 = min(count, q * per);
-      start += c0;
-      count = min(count - c0, per);
-    }
-    __syncwarp();
-    if (lane == 0) load_bucket_geom(mom, tnode, w.geom);
-    __syncwarp();
-    const int tbase = P.walk[tnode].pstart, ntot = P.walk[tnode].pcount;
-    unsigned long long nsrc = 0;
-    PROF_MARK(w, 0);
-    for (int tc = 0; tc < ntot; tc += 32) {
-      const int t0 = tbase + tc, nt = min(32, ntot - tc);
-      Kahan4 K;
-      K.zero();
-      if (ev_two_targets(nt)) {
-        const EvTarget2 x = ev_target2(P.p, w.geom, t0, nt, lane);
-        ev_two_zero(w, lane);
-        nsrc = ev_p2p_blocks<true, kReps, kBytes>(w, P, L, offs, x, start, count, lane, K);
-        ev_finish2<kTeam>(w, team, K, x, P, t0, lane);
-      } else {
-        const EvTarget x = ev_target(P.p, w.geom, t0, nt, lane);
-        nsrc = ev_p2p_blocks<false, kReps, kBytes>(w, P, L, offs, x, start, count, lane, K);
-        ev_finish<kTeam>(w, team, K, x, P, t0, lane);
-      }
-      PROF_MARK(w, 4);
-    }
-    // P2P pairs as the reference counts them (n_src * n_tgt per leaf(),
-    // src/Traverser.h:27); eval_p2c2 wrote the bucket's P2C work before
-    c_pp += nsrc * (unsigned long long)ntot;
-    if (P.bucket_work && lane == 0) {
-      if (kTeam > 1) atomicAdd(P.bucket_work + b, nsrc * (unsigned long long)ntot);
-      else P.bucket_work[b] += nsrc * (unsigned long long)ntot;
+      const unsigned long long pairs = ev_p2p_bucket<kReps, kBytes, kTeam>(w, team, P, L, offs, mom, tnode, start + c0,
+                                                                           min(count - c0, per), lane);
+      c_pp += pairs;
+      if (P.bucket_work && lane == 0) atomicAdd(P.bucket_work + b, pairs);
     }
   }
   PROF_MARK(w, 5);
