@@ -44,7 +44,9 @@ constexpr int64_t kSortSmallMax = 1 << 19;
 constexpr unsigned long long kFlagAggregate = 1ull << 32;
 constexpr unsigned long long kFlagInclusive = 2ull << 32;
 constexpr int kTagShift = 34;
-constexpr unsigned kTags = 1u << 30;  // pass tags 1 .. kTags - 1; 0 = memory as it was cleared
+// pass tags 1 .. kTags - 1; 0 = memory as it was cleared.  A clear every 127 sorts
+// costs nothing to speak of, and an ordinary run starts the tags over.
+constexpr unsigned kTags = 1u << 10;
 
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
   unsigned long long v;

@@ -155,3 +155,75 @@ def test_repeated_walk_counts_its_work_once(prec, nrep, theta):
         assert [c[k] for k in ("n_pp", "n_pc", "n_open")] == [c0[k] for k in ("n_pp", "n_pc", "n_open")]
     assert np.array_equal(second, want)
     assert np.array_equal(first, want)
+
+
+def test_one_handle_across_sizes():
+    """One handle keeps its sort scratch (look-back words of both tile sizes,
+    told apart by their tags), node arrays and list descriptors from size to size:
+    every pass is a fresh handle's bit for bit."""
+    sizes = [(1 << 19) + 1, 20000, 5000, (1 << 19) - 1, 300, 1 << 20, 16384, 16385, (1 << 19) + 1]
+    kw = dict(max_particles_per_leaf=32, theta=1.2)
+    for prec in ("fp64", "mixed"):
+        with sim(precision=prec, **kw) as s:
+            for n in sizes:
+                p = ics.mixture(n, seed=n)
+                s.set_particles(p)
+                s.start_down()
+                got, keys = s.accelerations(), s.keys()
+                with sim(precision=prec, **kw) as f:
+                    f.set_particles(p)
+                    f.start_down()
+                    want = f.accelerations()
+                    assert np.array_equal(keys, f.keys()), (prec, n)
+                for k in OUT:
+                    assert np.array_equal(got[k], want[k]), (prec, n, k)
+
+
+@pytest.mark.parametrize("n", [20000, (1 << 19) + 1])
+def test_sort_tags_start_over(n):
+    """The look-back words are cleared after 127 sorts, and the tags begin again."""
+    p, q = ics.plummer(n, seed=21), ics.mixture(n, seed=22)
+    with sim(max_particles_per_leaf=32, theta=1.5, precision="mixed") as s:
+        want = []
+        for r in (p, q):
+            s.set_particles(r)
+            s.start_down()
+            want.append((s.keys(), s.accelerations()))
+        for k in range(270):
+            i = k % 2
+            s.set_particles((p, q)[i])
+            s.start_down()
+            if 120 <= k < 132 or 246 <= k < 260 or k > 266:
+                assert np.array_equal(s.keys(), want[i][0]), k
+                a = s.accelerations()
+                for c in OUT:
+                    assert np.array_equal(a[c], want[i][1][c]), (k, c)
+
+
+# a bucket's list is cut into min(8, 75,776 / buckets) slices on 148 SMs: eight, a
+# few, two, and one
+@pytest.mark.parametrize("n", [9000, 40000, 55000, 120000])
+def test_adjoint_slices_match_finite_differences(n):
+    """The derivative along one direction of all positions and masses, against
+    central differences of the frozen lists.  h = 1e-6 of the positions' scale:
+    truncation (h / softening)^2 = 2.5e-9, rounding below 1e-16 sqrt(n) / h = 4e-8
+    of the objective."""
+    p = ics.plummer(n, seed=12, soft=0.02)
+    rng = np.random.default_rng(3)
+    cot, d = rng.normal(size=(3, n)), rng.normal(size=(4, n))
+    h = 1e-6
+    with sim(max_particles_per_leaf=4, record_lists=True) as s:
+        s.set_particles(p)
+        s.start_down()
+        nb = s.counters()["n_buckets"]
+        g = s.adjoint(*cot)
+
+        def objective(sign):
+            a = s.forces_frozen(*[p[k] + sign * h * d[i] for i, k in enumerate("xyz")], p["m"] * (1 + sign * h * d[3]))
+            return sum(float(np.dot(cot[i], a[k])) for i, k in enumerate(("ax", "ay", "az")))
+
+        fd = (objective(1) - objective(-1)) / (2 * h)
+    parts = [float(np.dot(g["g" + k], d[i])) for i, k in enumerate("xyz")] + [float(np.dot(g["gm"], p["m"] * d[3]))]
+    scale = max(abs(v) for v in parts)
+    print(n, "buckets", nb, "slices", max(1, min(8, 75776 // nb)), "fd", fd, "adjoint", sum(parts))
+    assert abs(fd - sum(parts)) < 1e-5 * scale
