@@ -95,8 +95,7 @@ struct AdjWarp {
   double st[12][kAdjSlots];   // staged slot data: P2C cm x/y/z, M, xx, xy, xz, yy, yz, zz, kind, soft; P2P x/y/z, m, soft
   double acc[10][kAdjSlots];  // per slot adjoint rows: node (cm x/y/z, M, 6 moments) or source (x/y/z, m)
   int32_t sidx[kAdjSlots];    // the slot's node or particle index
-  int32_t lnode[32];   // P2P: the window's leaves
-  int32_t lincl[32];   // P2P: inclusive prefix of their particle counts
+  int32_t lincl[32];   // P2P: inclusive prefix of the window's leaves' particle counts
   int32_t lpst[32];    // P2P: their first particles
 };
 
@@ -370,7 +369,6 @@ __global__ void __launch_bounds__(kAdjWarps * 32, PT_ADJ_MINB) adjoint_lists(Adj
         __syncwarp();
         if (sel) {
           const int k = __popc(m & ((1u << lane) - 1u));
-          w.lnode[k] = node;
           w.lincl[k] = inc;
           w.lpst[k] = pst;
         }

@@ -66,9 +66,10 @@ static_assert(sizeof(Mom) == 20 * sizeof(double), "lane_mom_store writes Mom's t
 // r < 3 centre coordinate r and the box along it, lane 3 the softening, each with
 // one or two of the second moments; MultipoleMoments::operator+=(Particle),
 // examples/MultipoleMoments.h:274-353, particle by particle.  (One thread per
-// node, four divisions in a row per particle: 16-29 us at up to 10^5 particles,
-// 495 us at 2^24; eight lanes with one second moment each: 9 and 934 us, twice
-// the warps for the same chain.)
+// node, four divisions in a row per particle: 14 us at 10^4 and 15 at 10^5
+// particles in buckets of 16, 51 us at 2^20, 504 us at 2^24 in buckets of 32; this
+// 8, 10, 59 and 673 us: four times the warps for the same chain, which pays where
+// the nodes are few.  Eight lanes with one second moment each: 934 us at 2^24.)
 __global__ void __launch_bounds__(256) leaf_moments(Nodes nd, const int32_t* __restrict__ buckets, int64_t nbuckets,
                                                     Particles p, double4* __restrict__ src) {
   const int64_t g = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 2;

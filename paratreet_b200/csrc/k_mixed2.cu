@@ -509,9 +509,6 @@ __device__ __forceinline__ bool next_bucket(const TravParams& P, int lane, int64
   return true;
 }
 
-// FP32 offset of a node's centre of mass (plus the replica offset) from the
-// bucket's, computed in FP64 as the walk computes it.
-
 // 256-bit loads (sm_100): half a 64-byte walk record, or a whole 32-byte
 // FP32 node record, with one instruction (the read-only path: these kernels
 // never write the node arrays)
@@ -529,6 +526,8 @@ __device__ __forceinline__ void ld_nc_f8(const void* p, float4& a, float4& b) {
       : "l"(p));
 }
 
+// FP32 offset of a node's centre of mass (plus the replica offset) from the
+// bucket's, computed in FP64 as the walk computes it.
 template <bool kReps>
 __device__ __forceinline__ float4 node_offset(const WalkRec* __restrict__ walk, int node, const RepOffsets* R, int rep,
                                               const BucketGeom& g) {

@@ -9,14 +9,14 @@
 //   histogram  one pass over the keys builds all eight 256-bin digit
 //              histograms (shared-memory atomics, then global atomics), and
 //              one small kernel turns each into exclusive digit offsets;
-//   pass       per digit, each CTA claims the next 4096-key tile from an atomic
-//              counter (so every earlier tile is already running), ranks its
+//   pass       per digit, each CTA claims the next tile (4096 keys; 1024 up to 2^19
+//              keys) from an atomic counter (so every earlier tile is already running), ranks its
 //              keys stably with __match_any_sync (lane order = key order in a
 //              round, rounds and warps in order), publishes its per-digit
 //              counts, and resolves the counts of all earlier tiles by
 //              decoupled look-back on 64-bit status words (tag | flag | count;
 //              a word of another tag is one an earlier pass left, so the words
-//              are never cleared between passes).  The
+//              are cleared only when the tags start over).  The
 //              ranked tile is staged in shared memory and written out with
 //              consecutive threads on consecutive destinations.
 // The look-back only waits on tiles that claimed their index earlier and
@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(kSortThreads, 2) radix_onesweep(const uint64_t
 // ---------------------------------------------------------------- small sort
 // Up to kRankMax keys: every key's place is the number of keys before it, counted
 // against all of them (n^2 comparisons cost less than eight dependent digit
-// passes of about 11 us: 91 us at N = 4096 and 10,000).  A CTA places 64 keys, two
+// passes, figures below).  A CTA places 64 keys, two
 // per lane, its warps taking every 16th group of 16 keys.
 constexpr int kRankThreads = 512;
 constexpr int kRankWarps = kRankThreads / 32;

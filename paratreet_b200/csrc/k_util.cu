@@ -15,18 +15,6 @@ __global__ void __launch_bounds__(256) iota_kernel(int32_t* __restrict__ out, in
     out[i] = (int32_t)i;
 }
 
-__global__ void __launch_bounds__(256) inverse_kernel(const int32_t* __restrict__ order, int32_t* __restrict__ inv,
-                                                      int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    inv[order[i]] = (int32_t)i;
-}
-
-__global__ void __launch_bounds__(256) map_kernel(const int32_t* __restrict__ inv, const int32_t* __restrict__ in,
-                                                  int32_t* __restrict__ out, int64_t n) {
-  int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  if (i < n) out[i] = inv[in[i]];
-}
-
 // y += alpha * x for three arrays (the chain's kick and drift, caller order).
 __global__ void __launch_bounds__(256) axpy3_kernel(int64_t n, double alpha, const double* __restrict__ x0,
                                                     const double* __restrict__ x1, const double* __restrict__ x2,
@@ -74,12 +62,6 @@ void launch_scatter_u64(const uint64_t* in, uint64_t* out, const int32_t* order,
 void launch_iota_i32(int32_t* out, int64_t n, int grid, cudaStream_t st) {
   if (n > 0) { note_launch(); iota_kernel<<<grid, 256, 0, st>>>(out, n); }
 }
-void launch_inverse_perm(const int32_t* order, int32_t* inv, int64_t n, int grid, cudaStream_t st) {
-  if (n > 0) { note_launch(); inverse_kernel<<<grid, 256, 0, st>>>(order, inv, n); }
-}
-void launch_map_index(const int32_t* inv, const int32_t* in, int32_t* out, int64_t n, cudaStream_t st) {
-  if (n > 0) { note_launch(); map_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(inv, in, out, n); }
-}
 
 // ------------------------------------------------- interaction-list digests
 // Order-independent digest of one bucket's interaction list: the sum (mod
@@ -118,8 +100,8 @@ __global__ void __launch_bounds__(256) digest_recorded(const int64_t* __restrict
   }
 }
 
-// Two-phase lists: per bucket a P2C run (bit 31 monopole, bit 30 near) and a
-// P2P run (bit 31 near) in the pools, one warp per bucket.
+// Two-phase lists: per bucket a P2C run (bit 31 monopole, bit 30 near) and a P2P
+// run in the pools, one warp per bucket.
 __global__ void __launch_bounds__(256) digest_two_phase(const int32_t* __restrict__ pc_pool,
                                                         const int32_t* __restrict__ pp_pool,
                                                         const int64_t* __restrict__ pc_start,

@@ -344,8 +344,6 @@ int read_status(pt_handle* h) {
     std::string m = "device status:";
     if (st & kErrNonFinite) m += " non-finite particle position;";
     if (st & kErrStack) m += " traversal stack overflow;";
-    if (st & kErrBucketTooBig) m += " bucket larger than 32;";
-    if (st & kErrListOverflow) m += " interaction list overflow;";
     if (st & kErrCapacity) m += " capacity exceeded;";
     if (st & kErrAdjointSoftened) m += " adjoint met a softened quadrupole term (not differentiated);";
     if (st & kErrSort) m += " radix sort look-back timed out;";
@@ -965,7 +963,10 @@ int pt_create(const pt_config* cfg, pt_handle** out) {
   if (dalloc(h, &h->d_work, 1) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_queue, 3 * kQueueWords) != PT_OK) return bail(PT_E_NOMEM);
   if (dalloc(h, &h->d_vmax2, 1) != PT_OK) return bail(PT_E_NOMEM);
-  if (cudaMemset(h->d_words, 0, sizeof(Words)) != cudaSuccess) return bail(PT_E_CUDA);
+  // (on the handle's stream: it does not wait for the default stream's work)
+  if (cudaMemsetAsync(h->d_words, 0, sizeof(Words), h->own_stream) != cudaSuccess ||
+      cudaStreamSynchronize(h->own_stream) != cudaSuccess)
+    return bail(PT_E_CUDA);
   *out = h;
   return PT_OK;
 }

@@ -24,8 +24,6 @@ constexpr int kMaxReps = 32;           // replicas the list kernels take in one 
 enum : unsigned {
   kErrNonFinite = 1u << 0,
   kErrStack = 1u << 1,
-  kErrBucketTooBig = 1u << 2,
-  kErrListOverflow = 1u << 3,
   kErrCapacity = 1u << 4,
   kErrAdjointSoftened = 1u << 5,
   kErrSort = 1u << 6,                 // radix sort look-back gave up waiting
@@ -156,7 +154,7 @@ struct TravParams {
 };
 
 // Interaction lists of the two-phase mixed traversal (k_mixed2.cu): two pools
-// of node indices (bit 31 = monopole for P2C, near for P2P), per-warp regions
+// of node indices (P2C: bit 31 = monopole, bit 30 = near), per-warp regions
 // reserved from the cursors, and per bucket (index b - b_begin) the start and
 // length of its contiguous list in each pool.
 struct ListParams {

@@ -115,8 +115,6 @@ void launch_scatter_f64(const double* in, double* out, const int32_t* order, int
 void launch_scatter_u64(const uint64_t* in, uint64_t* out, const int32_t* order, int64_t n, int grid,
                         cudaStream_t st);
 void launch_iota_i32(int32_t* out, int64_t n, int grid, cudaStream_t st);
-void launch_inverse_perm(const int32_t* order, int32_t* inv, int64_t n, int grid, cudaStream_t st);
-void launch_map_index(const int32_t* inv, const int32_t* in, int32_t* out, int64_t n, cudaStream_t st);
 void launch_axpy1(int64_t n, double alpha, const double* x, double* y, int grid, cudaStream_t st);
 void launch_axpy3(int64_t n, double alpha, const double* x0, const double* x1, const double* x2, double* y0,
                   double* y1, double* y2, int grid, cudaStream_t st);

@@ -9,13 +9,15 @@
 // handed to GravityVisitor::node (P2C), an EmptyLeaf is skipped.  Per target
 // particle the interactions are applied in exactly that order.
 //
-// B200 mapping: one warp owns one bucket (lanes = target particles).  When a
-// node is opened, lanes 0..7 classify its 8 contiguous children in parallel
-// (64-byte WalkRec each, one coalesced 512-byte read) into P2P / P2C
-// (quadrupole) / P2C (softened monopole, GravityVisitor::openSoftening) /
-// open; four ballots give the per-child masks (a frame's bits: P2P 0-7, P2C
-// quadrupole 8-15, P2C monopole 16-23, open 24-31).  The terminal children
-// before the first opened child are handed to the evaluator in child order, the
+// B200 mapping: one warp owns one bucket (lanes = target particles).  A step of the
+// pre-order walk takes up to four opened nodes of a frame (the breadth-first one a
+// single node, from the 64-byte records): lanes 8e .. 8e + 7 classify the children of
+// the e-th in parallel (contiguous; their classification fields come from the
+// sibling blocks, walk_sib_index) into P2P / P2C (quadrupole) / P2C (softened
+// monopole, GravityVisitor::openSoftening) / open; four ballots give the per-child
+// masks (a frame's bits: P2P 0-7, P2C quadrupole 8-15, P2C monopole 16-23, open
+// 24-31).  The terminal children before the first opened child are handed to the
+// evaluator in child order, the
 // rest waits on a per-warp shared-memory stack (walk_preorder).  Every decision
 // is warp-uniform.  The tests use
 // __dadd_rn/__dmul_rn so that they evaluate identically (no FMA contraction)
@@ -38,7 +40,8 @@ enum : int { kClsNone = 0, kClsP2P = 1, kClsQuad = 2, kClsOpen = 3, kClsMono = 4
 // d = lo - c if positive, else c - hi if positive, else nothing; summed x, y,
 // z).  Written with selects: an axis without a gap adds 0 * 0, which leaves
 // the (non-negative) sum unchanged, so the value is the branchy form's bit for
-// bit.
+// bit.  Space::intersect(box, centre, rsq) is gap <= rsq (GravityVisitor::open,
+// :180, and ::openSoftening, :127).
 __device__ __forceinline__ double box_gap2_exact(const double lo[3], const double hi[3], double cx, double cy,
                                                  double cz) {
   const double c[3] = {cx, cy, cz};
@@ -50,13 +53,6 @@ __device__ __forceinline__ double box_gap2_exact(const double lo[3], const doubl
     dsq = __dadd_rn(dsq, __dmul_rn(d, d));
   }
   return dsq;
-}
-
-// Space::intersect(box, centre, rsq): intersect iff the gap is <= rsq.  Used
-// by GravityVisitor::open (:180) and ::openSoftening (:127).
-__device__ __forceinline__ bool box_sphere_exact(const double lo[3], const double hi[3], double cx,
-                                                 double cy, double cz, double rsq) {
-  return box_gap2_exact(lo, hi, cx, cy, cz) <= rsq;
 }
 
 // Squared distance from a point to a box (0 inside); conservative helper.
@@ -81,12 +77,6 @@ __device__ __forceinline__ bool open_softening_gap(double scx, double scy, doubl
   double rs = __dadd_rn(r1, r2);
   if (d2 <= __dmul_rn(rs, rs)) return true;
   return gap2 <= __dmul_rn(r1, r1);
-}
-
-__device__ __forceinline__ bool open_softening_exact(double scx, double scy, double scz, double ssoft,
-                                                     double tcx, double tcy, double tcz, double tsoft,
-                                                     const double lo[3], const double hi[3]) {
-  return open_softening_gap(scx, scy, scz, ssoft, tcx, tcy, tcz, tsoft, box_gap2_exact(lo, hi, scx, scy, scz));
 }
 
 // Whether a P2P leaf may hold a pair that GravityVisitor::leaf softens (or
