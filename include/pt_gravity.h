@@ -140,7 +140,7 @@ int pt_set_precision(pt_handle* h, int precision);
  * times (default 2^21, which is never reached in practice) and then gives up.
  * The force pass then stops before it permutes the particles and returns
  * PT_E_DEVICE ("radix sort look-back timed out"); the handle keeps its last
- * consistent state and the next call sorts afresh.  0 gives up at the first
+ * consistent state (all but the keys, pt_get_keys) and the next call sorts afresh.  0 gives up at the first
  * poll of an unpublished tile.  polls < 0 is PT_E_ARG. */
 int pt_set_sort_spin_limit(pt_handle* h, int64_t polls);
 
