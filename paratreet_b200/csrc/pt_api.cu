@@ -558,6 +558,11 @@ int run_two_phase(pt_handle* h, TravParams& P) {
   auto restore_counters = [&]() {
     return cudaMemcpyAsync(h->d_counters, h->d_words->saved, sizeof(h->d_words->saved), cudaMemcpyDeviceToDevice, st);
   };
+  auto fewer_replicas = [&]() {  // the lists of so many do not fit
+    h->rep_batch = P.rep_count / 2;
+    h->want_pc = h->want_pp = 0;
+    return kFewerReplicas;
+  };
   ListParams L{};
   for (int attempt = 0;; attempt++) {
     const unsigned region = h->l_region;
@@ -591,11 +596,7 @@ int run_two_phase(pt_handle* h, TravParams& P) {
         dfree(h->pool_pc);
         dfree(h->pool_pp);
         CK(restore_counters());
-        if (reps) {  // no room for the lists of so many replicas
-          h->rep_batch = P.rep_count / 2;
-          h->want_pc = h->want_pp = 0;
-          return kFewerReplicas;
-        }
+        if (reps) return fewer_replicas();
         // no room for the lists: this handle evaluates with the fused kernel from now on
         h->two_phase = false;
         CKR(zero_queue(h));
@@ -650,6 +651,7 @@ int run_two_phase(pt_handle* h, TravParams& P) {
     status &= ~kErrPool;
     CK(cudaMemcpyAsync(h->d_status, &status, sizeof(unsigned), cudaMemcpyHostToDevice, st));
     CK(restore_counters());
+    if (attempt >= 6) return reps ? fewer_replicas() : fail(h, PT_E_NOMEM, "interaction lists outgrow their pools");
     h->want_pc = std::max(2 * h->cap_pc, cur[0] + cur[0] / 2);
     h->want_pp = std::max(2 * h->cap_pp, cur[1] + cur[1] / 2);
   }

@@ -228,6 +228,27 @@ def test_replica_lists_that_do_not_fit_take_smaller_batches(nrep, room):
         assert np.abs(out[0][k] - out[1][k]).max() < 1e-5 * scale[k[0]], k
 
 
+def test_ordered_walk_in_the_middle_of_a_pass():
+    """PT_FP64_LISTS under the same limit: the replicas whose lists do not fit are
+    walked in order, the sums before them stay, and no work is counted twice."""
+    p = ics.lattice(24, seed=6, rms_cells=0.3, soft_cells=0.3)
+    kw = dict(max_particles_per_leaf=4, theta=0.4, periodic=True, n_replicas=1)
+    out = []
+    for prec in ("fp64", "fp64_lists"):
+        with sim(precision=prec, **kw) as s:
+            s.set_list_region(64)
+            s.set_particles(p)
+            s.set_alloc_limit(8 * (1024 * 8583 + 148 * 7 * 4 * 64))  # 8583 buckets
+            s.start_down()
+            out.append((s.accelerations(), s.bucket_work(), s.counters()))
+    (a, wa, ca), (b, wb, cb) = out
+    assert ca["n_buckets"] == 8583 and cb["launches"] != ca["launches"]
+    assert np.array_equal(wa, wb)
+    assert all(ca[k] == cb[k] for k in ("n_pp", "n_pc", "n_open"))
+    for k in OUT:  # sums of 27 replicas of size 1 each in another order
+        assert np.abs(a[k] - b[k]).max() <= 1e-11 * (1 if k[0] == "a" else 27), k
+
+
 def test_fused_form_in_the_middle_of_a_pass_leaves_no_potential():
     """Where even one replica's lists do not fit, the replicas before it must not
     leave their part of pot: the fused form has none (pot_full has it)."""
