@@ -956,7 +956,7 @@ int pt_create(const pt_config* cfg, pt_handle** out) {
   h->pin = static_cast<Words*>(std::aligned_alloc(kPage, kPage));
   if (!h->pin) return bail(PT_E_NOMEM);
   h->pinned = cudaHostRegister(h->pin, kPage, cudaHostRegisterDefault) == cudaSuccess;
-  if (!h->pinned) return bail(PT_E_CUDA);
+  if (!h->pinned) cudaGetLastError();  // the copies work from pageable memory too
   h->d_status = &h->d_words->status;
   h->d_ticket = &h->d_words->ticket;
   h->d_counters = h->d_words->counters;
